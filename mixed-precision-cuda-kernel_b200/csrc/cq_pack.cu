@@ -103,41 +103,294 @@ __global__ void pack_codes_kernel(const void* __restrict__ w, int is_f32, const 
   }
 }
 
-// ------------------------------------------------------------------ dense unpack
-// llama/qlinear.py:120-162: dense[n, k] = cherry ? cherry_weight : fp16((q + 0.5) * s).
-// A 32x32 (k, n) tile per block: codes are read with n contiguous, the dense matrix is
-// written with k contiguous.
-__global__ void unpack_dense_kernel(const uint8_t* __restrict__ q, const __half* __restrict__ scales,
-                                    const __half* __restrict__ cw, const int16_t* __restrict__ idx,
-                                    int bits, int K, int N, int C, int G, __half* __restrict__ dense) {
-  __shared__ __half tile[32][33];
-  const int k0 = blockIdx.x * 32, n0 = blockIdx.y * 32;
-  const int tx = threadIdx.x, ty = threadIdx.y;  // 32 x 8
-  for (int kk = ty; kk < 32; kk += 8) {
-    const int k = k0 + kk, n = n0 + tx;
-    __half v = __float2half(0.f);
-    if (k < K && n < N) {
-      // rank of k among the sorted cherry columns
-      int low = 0, high = C;
-      while (low < high) {
-        const int mid = (low + high) >> 1;
-        if ((int)idx[mid] < k) low = mid + 1; else high = mid;
+// One pass over the weights for the group sizes in use (64, multiples of 128, one group per row): a block owns
+// PK_ROWS output rows of one group (two 64-wide ones), reads them once in chunks of 128 compact columns, reduces
+// the maxima and writes scales and codes.  The general pair of kernels above reads the matrix twice, lanes a row
+// apart, and divides per weight.  The loads are 2 bytes a lane, 64 contiguous bytes a warp, because the removed
+// cherry columns leave the compact columns at any alignment; the tile turns them so that a thread quantises 32
+// columns of one row and the byte stores have 32 consecutive rows a warp.  Groups of more than one chunk are read
+// a second time for the codes (mostly from L2).  4096 x 11008 4-bit: 58 us (114 MB, bound by the issue rate: about 25
+// instructions per weight), 415 us for sort, cherries, scales and codes in four kernels.
+constexpr int PK_ROWS = 64, PK_COLS = 128, PK_THREADS = 256;
+
+template <typename T> struct PackTile;
+template <> struct PackTile<__half> {
+  static constexpr int STRIDE = PK_COLS + 8;        // 272 B: the 16-byte reads of 8 rows hit 8 different bank groups
+  static __device__ __forceinline__ float f(__half v) { return __half2float(v); }
+};
+template <> struct PackTile<float> {
+  static constexpr int STRIDE = PK_COLS + 4;
+  static __device__ __forceinline__ float f(float v) { return v; }
+};
+
+// fp16(w / s) for fp16 w and s (held as floats), r = RN(1 / s).  One residual step after w * r (Markstein's division
+// with fused multiply-add) leaves a relative error of at most 2^-24 (1 + 2^-20); a quotient of two 11-bit significands
+// is never closer than 2^-23 to a midpoint of two fp16 numbers without being one exactly representable, so the fp16
+// rounding is that of the exact quotient.  For an infinite s the caller passes 0 in the residual's place: the result is
+// then w * 0, as w / infinity is.  An exact division per weight took half of the kernel's instructions.
+__device__ __forceinline__ float div_fp16(float w, float s_residual, float r) {
+  const float q = __fmul_rn(w, r);
+  return __fmaf_rn(__fmaf_rn(-q, s_residual, w), r, q);
+}
+
+template <typename T, int BITS>
+__global__ void __launch_bounds__(PK_THREADS, sizeof(T) == 2 ? 5 : 3) pack_fused_kernel(
+    const T* __restrict__ w, const int16_t* __restrict__ idx, int K, int N, int C, int G, int span, int n_tiles,
+    int n_spans, __half* __restrict__ scales, uint8_t* __restrict__ q, __half* __restrict__ cw) {
+  constexpr int ST = PackTile<T>::STRIDE, VEC = 16 / sizeof(T);
+  __shared__ __align__(16) T tile[PK_ROWS * ST];
+  __shared__ float red[4][PK_ROWS];
+  __shared__ int source[PK_COLS];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int n0 = (int)(blockIdx.x % n_tiles) * PK_ROWS, sp = (int)(blockIdx.x / n_tiles);
+  const int rows = min(PK_ROWS, N - n0);
+  if (sp >= n_spans) {
+    // the last block of a row tile copies its cherry columns: cherry_weight[c, n] = fp16(W[n, idx[c]])
+    for (int id = tid; id < C * PK_ROWS; id += PK_THREADS) {
+      const int r = id % PK_ROWS, c = id / PK_ROWS;
+      if (r < rows) cw[(size_t)c * N + n0 + r] = __float2half_rn(PackTile<T>::f(w[(size_t)(n0 + r) * K + idx[c]]));
+    }
+    return;
+  }
+  const int Kc = K - C;
+  const int k_begin = sp * span, k_end = min(Kc, k_begin + span);
+  const int n_chunks = (k_end - k_begin + PK_COLS - 1) / PK_COLS;
+  const int row = tid & (PK_ROWS - 1), part = tid / PK_ROWS;      // this thread's 32 columns of the tile
+  const bool two = G == 64;                                       // two groups in the block's 128 columns
+
+  auto load_chunk = [&](int k0) {
+    // lane l of every warp loads compact columns k0 + 32 j + l; rows go round over the warps
+    __syncthreads();
+    if (tid < PK_COLS) {
+      const int kc = k0 + tid;
+      source[tid] = kc < k_end ? kc + cherry_shift(idx, C, kc) : -1;
+    }
+    __syncthreads();
+    int col[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) col[j] = source[32 * j + lane];
+    const T* src = w + (size_t)(n0 + min(warp, rows - 1)) * K;
+    const size_t step = (size_t)(PK_THREADS / 32) * K;
+#pragma unroll 4
+    for (int r = warp; r < PK_ROWS; r += PK_THREADS / 32) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) tile[r * ST + 32 * j + lane] = col[j] >= 0 ? src[col[j]] : (T)0.f;
+      if (r + PK_THREADS / 32 < rows) src += step;               // (rows past the matrix repeat one of its rows)
+    }
+    __syncthreads();
+  };
+  uint4 raw[32 / VEC];
+  auto read_part = [&]() {
+#pragma unroll
+    for (int i = 0; i < 32 / VEC; ++i) raw[i] = reinterpret_cast<const uint4*>(tile + row * ST + 32 * part)[i];
+  };
+  // two consecutive values
+  auto pair = [&](int i) {
+    const uint32_t* u = reinterpret_cast<const uint32_t*>(raw);
+    if constexpr (sizeof(T) == 2)
+      return __half22float2(*reinterpret_cast<const __half2*>(&u[i >> 1]));
+    else
+      return make_float2(__uint_as_float(u[i]), __uint_as_float(u[i + 1]));
+  };
+
+  float mx = 0.f;
+  for (int c = 0; c < n_chunks; ++c) {
+    load_chunk(k_begin + c * PK_COLS);
+    read_part();
+#pragma unroll
+    for (int i = 0; i < 32; i += 2) {
+      const float2 f = pair(i);
+      mx = fmaxf(mx, fmaxf(fabsf(f.x), fabsf(f.y)));
+    }
+  }
+  red[part][row] = mx;
+  __syncthreads();
+  if (two)
+    mx = fmaxf(red[part & 2][row], red[(part & 2) + 1][row]);
+  else
+    mx = fmaxf(fmaxf(red[0][row], red[1][row]), fmaxf(red[2][row], red[3][row]));
+  const float div = (float)(1 << (BITS - 1));
+  __half sh;
+  if constexpr (sizeof(T) == 4) {
+    sh = __float2half_rn(__fdiv_rn(__fadd_rn(mx, 1e-6f), div));
+  } else {
+    const __half a = __float2half_rn(__fadd_rn(mx, 1e-6f));       // fp16 add, rounded once
+    sh = __float2half_rn(__fdiv_rn(__half2float(a), div));        // fp16 divide, rounded once
+  }
+  const int grp = k_begin / G + (two ? (part >> 1) : 0);
+  if (row < rows && (part == 0 || (two && part == 2)) && grp < (Kc + G - 1) / G) scales[(size_t)grp * N + n0 + row] = sh;
+
+  const float s = __half2float(sh), rs = __frcp_rn(s), s_residual = s < 65536.f ? s : 0.f;
+  const float qmax = (float)((double)(1 << (BITS - 1)) - 1e-2);
+  for (int c = 0; c < n_chunks; ++c) {
+    const int k0 = k_begin + c * PK_COLS;
+    if (n_chunks > 1) {
+      load_chunk(k0);
+      read_part();
+    }
+#pragma unroll
+    for (int o = 0; o < 4; ++o) {
+      uint32_t word = 0;
+#pragma unroll
+      for (int i = 0; i < 8; i += 2) {
+        float2 r = pair(8 * o + i);
+        if constexpr (sizeof(T) == 2)                             // fp16 / fp16 is rounded to fp16
+          r = __half22float2(__floats2half2_rn(div_fp16(r.x, s_residual, rs), div_fp16(r.y, s_residual, rs)));
+        else
+          r = make_float2(__fdiv_rn(r.x, s), __fdiv_rn(r.y, s));
+        r.x = fminf(fmaxf(r.x, -qmax), qmax);
+        r.y = fminf(fmaxf(r.y, -qmax), qmax);
+        // adding 1.5 * 2^23 (+ the code offset) rounds to the nearest integer, ties to even, like rint
+        const float magic = 12582912.f + (float)(1 << (BITS - 1));
+        word |= (__float_as_uint(__fadd_rn(__fsub_rn(r.x, 0.5f), magic)) & ((1u << BITS) - 1)) << (BITS * i);
+        word |= (__float_as_uint(__fadd_rn(__fsub_rn(r.y, 0.5f), magic)) & ((1u << BITS) - 1)) << (BITS * (i + 1));
       }
-      if (low < C && (int)idx[low] == k) {
-        v = cw[(size_t)low * N + n];
-      } else {
-        const int kc = k - low;
-        const int u = (int)cq_ref_code(q, bits, kc, n, N);
-        const __half a = __float2half_rn((float)(u - (1 << (bits - 1))) + 0.5f);
-        v = __float2half_rn(__fmul_rn(__half2float(a), __half2float(scales[(size_t)(kc / G) * N + n])));
+      const int oct = (k0 >> 3) + 4 * part + o;
+      if (row < rows && 8 * oct < k_end) {
+        uint8_t* dst = q + (size_t)oct * BITS * N + n0 + row;
+#pragma unroll
+        for (int b = 0; b < BITS; ++b) dst[(size_t)b * N] = (uint8_t)(word >> (8 * b));
       }
     }
-    tile[kk][tx] = v;
+  }
+}
+
+// ------------------------------------------------------------------ dense unpack
+// llama/qlinear.py:120-162: dense[n, k] = cherry ? cherry_weight : fp16((q + 0.5) * s).
+// A block writes 64 rows x 128 columns: a thread makes one octet of 8 original columns of four consecutive rows.
+// Without a cherry column or a group boundary inside, the octet's codes are 8 consecutive compact columns: the bytes
+// of two compact octets (one 32-bit load per byte row covers the four rows), shifted by the position inside the first.
+// Pairs of codes become the low mantissa bits of 1024 + u, minus (1024 + off), times the scale: each step but the
+// last exact, so the product is rounded once as in the reference.  The tile in shared memory (16-byte slots, slot
+// number XOR row quad against bank conflicts) turns the octets into rows of 256 contiguous bytes.  11008 x 4096 3-bit:
+// 52 us (108 MB), 296 us with a binary search, a byte-wise code fetch and two divisions per element.
+constexpr int UP_ROWS = 64, UP_COLS = 128;
+
+__device__ __forceinline__ uint32_t load_quad(const uint8_t* p, bool aligned) {
+  if (aligned) return __ldg(reinterpret_cast<const uint32_t*>(p));
+  return (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
+}
+
+// codes 2 i, 2 i + 1 of a word as fp16 (u - off)
+template <int BITS> __device__ __forceinline__ __half2 code_pair(uint32_t word, int i) {
+  const uint32_t x = word >> (2 * BITS * i);
+  constexpr uint32_t M = (1u << BITS) - 1;
+  const uint32_t v = (x & M) | ((x << (16 - BITS)) & (M << 16)) | 0x64006400u;
+  constexpr uint32_t CENTER = BITS == 4 ? 0x64076407u : 0x64036403u;       // 1024 + floor(off)
+  const uint32_t half = 0x38003800u;
+  const __half2 d = __hsub2(*reinterpret_cast<const __half2*>(&v), *reinterpret_cast<const __half2*>(&CENTER));
+  return __hsub2(d, *reinterpret_cast<const __half2*>(&half));
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
+    const uint8_t* __restrict__ q, const __half* __restrict__ scales, const __half* __restrict__ cw,
+    const int16_t* __restrict__ idx, int K, int N, int C, int G, int g_shift, __half* __restrict__ dense, int aligned) {
+  __shared__ __align__(16) uint4 tile[UP_ROWS * (UP_COLS / 8)];
+  __shared__ int before[UP_COLS / 8 + 1];           // cherry columns before each octet
+  const int tid = threadIdx.x, nq = tid & 15, oct = tid >> 4;
+  const int k0 = blockIdx.x * UP_COLS, n0 = blockIdx.y * UP_ROWS;
+  const int k = k0 + 8 * oct, n = n0 + 4 * nq;
+  const int Kc = K - C, n_oct = Kc / 8;
+  if (tid <= UP_COLS / 8) {
+    const int kk = k0 + 8 * tid;
+    int low = 0, high = C;
+    while (low < high) {
+      const int mid = (low + high) >> 1;
+      if ((int)idx[mid] < kk) low = mid + 1; else high = mid;
+    }
+    before[tid] = low;
   }
   __syncthreads();
-  for (int nn = ty; nn < 32; nn += 8) {
-    const int n = n0 + nn, k = k0 + tx;
-    if (k < K && n < N) dense[(size_t)n * K + k] = tile[tx][nn];
+  if (k < K && n < N) {
+    const int low = before[oct], kc = k - low, o = kc >> 3, r = kc & 7;
+    const bool cherry = before[oct + 1] != low;
+    // the bytes of compact octets o and o + 1, four rows in each word
+    uint32_t b[2][BITS];
+    const uint8_t* src = q + (size_t)o * BITS * N + n;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < BITS; ++i)
+        b[h][i] = (o + h < n_oct && (h == 0 || r)) ? load_quad(src + (size_t)(h * BITS + i) * N, aligned & 1) : 0u;
+    auto group_of = [&](int c) { return g_shift >= 0 ? c >> g_shift : c / G; };
+    const int g = group_of(kc), split = (g + 1) * G - kc;       // codes 0 .. split - 1 belong to group g
+    unsigned long long s0 = 0, s1 = 0;                          // the four rows' scales of groups g and g + 1
+    const bool whole = split >= 8;
+    if (!cherry) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        s0 |= (unsigned long long)__half_as_ushort(scales[(size_t)g * N + n + j]) << (16 * j);
+        if (!whole) s1 |= (unsigned long long)__half_as_ushort(scales[(size_t)(g + 1) * N + n + j]) << (16 * j);
+      }
+    }
+    // (groups narrower than 8 columns can put more than two into an octet: the general path below)
+    const bool general = cherry || (!whole && G < 8);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t w[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const uint32_t sel = (uint32_t)j | ((uint32_t)(4 + j) << 4);
+        const uint32_t lo = __byte_perm(b[h][0], b[h][1], sel);
+        const uint32_t hi = BITS == 4 ? __byte_perm(b[h][2], b[h][BITS - 1], sel) : ((b[h][2] >> (8 * j)) & 0xFFu);
+        w[h] = __byte_perm(lo, hi, 0x5410);
+      }
+      // the eight codes from column kc on
+      uint32_t word;
+      if (BITS == 4)
+        word = __funnelshift_r(w[0], w[1], 4 * r);
+      else
+        word = ((w[0] & 0xFFFFFFu) >> (3 * r)) | (r ? w[1] << (24 - 3 * r) : 0u);
+      if (!general) {
+        const uint32_t sa = (uint32_t)(s0 >> (16 * j)) & 0xFFFFu, sb = (uint32_t)(s1 >> (16 * j)) & 0xFFFFu;
+        uint32_t p[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t sc = whole ? (sa | (sa << 16)) : ((2 * i < split ? sa : sb) | ((2 * i + 1 < split ? sa : sb) << 16));
+          const __half2 v = __hmul2(code_pair<BITS>(word, i), *reinterpret_cast<const __half2*>(&sc));
+          p[i] = *reinterpret_cast<const uint32_t*>(&v);
+        }
+        tile[(4 * nq + j) * 16 + (oct ^ nq)] = make_uint4(p[0], p[1], p[2], p[3]);
+      }
+    }
+    if (general) {
+      // column by column
+#pragma unroll 1
+      for (int j = 0; j < 4; ++j) {
+        __half* dst = reinterpret_cast<__half*>(&tile[(4 * nq + j) * 16 + (oct ^ nq)]);
+        int m = low;
+#pragma unroll 1
+        for (int e = 0; e < 8; ++e) {
+          while (m < C && (int)idx[m] < k + e) ++m;
+          if (m < C && (int)idx[m] == k + e) {
+            dst[e] = cw[(size_t)m * N + n + j];
+          } else {
+            const int c = k + e - m;
+            const uint32_t u = cq_ref_code(q, BITS, c, n + j, N);
+            const float a = (float)((int)u - (1 << (BITS - 1))) + 0.5f;
+            dst[e] = __float2half_rn(__fmul_rn(a, __half2float(scales[(size_t)group_of(c) * N + n + j])));
+          }
+        }
+      }
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int id = tid + 256 * i, rr = id >> 4, oo = id & 15;
+    const int nn = n0 + rr, kk = k0 + 8 * oo;
+    if (nn < N && kk < K) {
+      const uint4 v = tile[rr * 16 + (oo ^ (rr >> 2))];
+      __half* dst = dense + (size_t)nn * K + kk;
+      if (aligned & 2) {
+        *reinterpret_cast<uint4*>(dst) = v;
+      } else {
+        const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dst[e] = __ushort_as_half((unsigned short)(u[e >> 1] >> (16 * (e & 1))));
+      }
+    }
   }
 }
 
@@ -183,12 +436,28 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
   if (rc) return rc;
   cudaStream_t st = (cudaStream_t)stream;
   const int T = 256;
-  if (C > 0) {
-    pack_sort_kernel<<<nblocks(C, T), T, 0, st>>>(cherry_unsorted, C, cherry_indices);
+  if (C > 0) pack_sort_kernel<<<nblocks(C, T), T, 0, st>>>(cherry_unsorted, C, cherry_indices);
+  const int ng = (K - C + G - 1) / G;
+  if (G == 64 || G % PK_COLS == 0 || ng == 1) {
+    const int span = G == 64 ? PK_COLS : (ng == 1 ? (K - C) : G);         // compact columns a block owns
+    const int n_tiles = (N + PK_ROWS - 1) / PK_ROWS, n_spans = (K - C + span - 1) / span;
+    const long long blocks = (long long)n_tiles * (n_spans + (C > 0));
+    if (blocks <= 0x7fffffffll) {
+      auto launch = [&](auto kernel, auto* wp) {
+        kernel<<<(unsigned)blocks, PK_THREADS, 0, st>>>(wp, cherry_indices, K, N, C, G, span, n_tiles, n_spans,
+                                                       (__half*)scales, qweight, (__half*)cherry_weight);
+      };
+      if (weight_is_f32)
+        bits == 4 ? launch(pack_fused_kernel<float, 4>, (const float*)weight) : launch(pack_fused_kernel<float, 3>, (const float*)weight);
+      else
+        bits == 4 ? launch(pack_fused_kernel<__half, 4>, (const __half*)weight) : launch(pack_fused_kernel<__half, 3>, (const __half*)weight);
+      CQ_CUDA_TRY(cudaGetLastError());
+      return CQ_OK;
+    }
+  }
+  if (C > 0)
     pack_cherry_kernel<<<nblocks((long long)C * N, T), T, 0, st>>>(weight, weight_is_f32, cherry_indices, K, N, C,
                                                                   (__half*)cherry_weight);
-  }
-  const int ng = (K - C + G - 1) / G;
   pack_scales_kernel<<<nblocks((long long)ng * N * 32, T), T, 0, st>>>(weight, weight_is_f32, cherry_indices, bits,
                                                                       K, N, C, G, (__half*)scales);
   pack_codes_kernel<<<nblocks((long long)((K - C) / 8) * N, T), T, 0, st>>>(
@@ -204,10 +473,14 @@ extern "C" int cq_unpack_dense(const uint8_t* qweight, const void* scales, const
   if (C > 0 && (!cherry_weight || !cherry_indices)) return CQ_ERR_BAD_ARG;
   const int rc = check_dims(bits, K, N, C, &G);
   if (rc) return rc;
-  dim3 grid((K + 31) / 32, (N + 31) / 32), block(32, 8);
-  unpack_dense_kernel<<<grid, block, 0, (cudaStream_t)stream>>>(qweight, (const __half*)scales,
-                                                                (const __half*)cherry_weight, cherry_indices, bits,
-                                                                K, N, C, G, (__half*)dense);
+  dim3 grid((K + UP_COLS - 1) / UP_COLS, (N + UP_ROWS - 1) / UP_ROWS);
+  const int aligned = (((uintptr_t)qweight & 3) == 0 ? 1 : 0) | (((uintptr_t)dense & 15) == 0 ? 2 : 0);
+  int g_shift = -1;
+  if ((G & (G - 1)) == 0)
+    for (g_shift = 0; (1 << g_shift) < G;) ++g_shift;
+  auto kernel = bits == 4 ? unpack_dense_kernel<4> : unpack_dense_kernel<3>;
+  kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(qweight, (const __half*)scales, (const __half*)cherry_weight,
+                                                 cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
   CQ_CUDA_TRY(cudaGetLastError());
   return CQ_OK;
 }

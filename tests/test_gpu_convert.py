@@ -1,0 +1,64 @@
+"""The one-pass conversion kernels against the numpy oracle and the torch expressions they replace, byte for byte, at the
+edges of their tiles: rows that are not a multiple of 64, columns that are not a multiple of 128, groups of one chunk, of
+several and of a whole row, octets with cherry columns and group boundaries inside."""
+import numpy as np
+import pytest
+
+from oracle import cherryq_oracle as O
+from test_gpu_parity import dev, gpu_pack, gpu_unpack, ptr
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def cabi():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    from cherryq_b200 import _cabi
+    _cabi.lib()
+    return _cabi
+
+
+def layer(K, N, C, dtype, seed):
+    rng = np.random.default_rng(seed)
+    w = (rng.normal(size=(N, K)) * 0.02).astype(dtype)
+    idx = rng.permutation(K)[:C]
+    if C:
+        idx[:min(C, 8)] = np.arange(min(C, 8)) + 8                 # a whole octet of cherries
+        idx = np.unique(idx)
+        idx = np.concatenate([idx, np.setdiff1d(np.arange(K), idx)[:C - len(idx)]])
+        w[:, idx] = (rng.normal(size=(N, C)) * 0.2).astype(dtype)
+        idx = rng.permutation(idx)
+    w[0] = 0                                                       # the smallest scale
+    w[1] = np.asarray(0.5 * np.sign(w[1].astype(np.float32) + 1e-9), dtype)     # quotients on the code boundaries
+    w[2, ::3] = np.asarray(6e-8, dtype)                            # subnormal in fp16
+    w[3] *= np.asarray(1000, dtype)
+    return w, idx
+
+
+@pytest.mark.parametrize("dtype", [np.float16, np.float32])
+@pytest.mark.parametrize("K,N,bits,G,C", [
+    (8, 8, 4, 128, 0), (136, 72, 3, 64, 8), (1024, 64, 4, 128, 8), (1032, 136, 3, 128, 16), (1040, 56, 4, 256, 24),
+    (2048, 200, 3, 2048, 8), (512, 64, 4, 96, 16), (4096, 128, 3, 64, 128), (640, 8, 4, 640, 200)])
+def test_pack_and_unpack(cabi, K, N, bits, G, C, dtype):
+    w, idx = layer(K, N, C, dtype, K + N)
+    ref = O.pack(w, idx, bits, G)
+    got = gpu_pack(cabi, w, idx, bits, G)
+    for key in ("qweight", "scales", "cherry_weight", "cherry_indices"):
+        assert np.array_equal(got[key].view(np.uint8), ref[key].view(np.uint8)), key
+    dense = O.unpack(ref["qweight"], ref["scales"], ref["cherry_weight"], ref["cherry_indices"], bits, G, K)
+    assert np.array_equal(gpu_unpack(cabi, ref, bits, K, G).view(np.uint16), dense.view(np.uint16))
+
+
+def test_unpack_into_unaligned_buffers(cabi):
+    K, N, bits, G, C = 264, 72, 3, 128, 8
+    w, idx = layer(K, N, C, np.float16, 5)
+    ref = O.pack(w, idx, bits, G)
+    t = [dev(ref[k]) for k in ("scales", "cherry_weight", "cherry_indices")]
+    q = torch.zeros(ref["qweight"].size + 1, dtype=torch.uint8, device="cuda")
+    q[1:] = dev(ref["qweight"]).flatten()
+    out = torch.zeros(N * K + 1, dtype=torch.float16, device="cuda")
+    cabi.check(cabi.lib().cq_unpack_dense(q.data_ptr() + 1, *[ptr(a) for a in t], bits, K, N, C, G, out.data_ptr() + 2, None), "unpack")
+    dense = O.unpack(ref["qweight"], ref["scales"], ref["cherry_weight"], ref["cherry_indices"], bits, G, K)
+    assert np.array_equal(out[1:].cpu().numpy().view(np.uint16), dense.view(np.uint16).ravel())
