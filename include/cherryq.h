@@ -365,6 +365,13 @@ int cq_pack(const void* weight, int weight_is_f32, const int32_t* cherry_unsorte
             uint8_t* qweight, void* scales_f16, void* cherry_weight_f16,
             int16_t* cherry_indices, void* tmp, cq_stream_t stream);
 
+/* Fake-quantised weight of the training-side layer (llama/cherry_linear.py:69-99): weight (N, K) row-major, dtype 0 =
+ * fp16, 1 = fp32, 2 = bf16, 16-byte aligned like `out`; quantised: K bytes, 0 for a cherry column; bits 2..4; G >= 8
+ * quantised columns share a scale.  ste != 0: out = (real - weight) + weight, each rounded to the type, the value of the
+ * straight-through expression.  table: device scratch of K / 8 words. */
+int cq_fake_quant(const void* weight, int dtype, const uint8_t* quantised, int bits, int K, int N, int G, int ste,
+                  void* out, uint32_t* table, cq_stream_t stream);
+
 /* dense: (N, K) fp16 = what QuantLinear.unpack() returns. */
 int cq_unpack_dense(const uint8_t* qweight, const void* scales_f16,
                     const void* cherry_weight_f16, const int16_t* cherry_indices,

@@ -12,7 +12,28 @@ import math
 import torch
 import torch.nn as nn
 
+from . import load_quant_cuda
 from .quantizer import FullSymQuantizer
+
+
+class _StraightThrough(torch.autograd.Function):
+    """(real - w).detach() + w as one kernel: the value of the expression, the gradient of `+ w`."""
+
+    @staticmethod
+    def forward(ctx, weight, quantised, bits, group_size):
+        return load_quant_cuda().fake_quant(weight, quantised, bits, group_size, True)
+
+    @staticmethod
+    def backward(ctx, grad):
+        return grad, None, None, None
+
+
+def _plain_eager():
+    """No tracer, compiler, functorch transform, forward-mode level or dispatch / function mode sees the operations."""
+    return (not torch.compiler.is_compiling() and not torch.jit.is_tracing()
+            and torch._C._functorch.peek_interpreter_stack() is None
+            and torch.autograd.forward_ad._current_level < 0
+            and torch._C._len_torch_dispatch_stack() == 0 and torch._C._len_torch_function_stack() == 0)
 
 
 class QuantLinear(nn.Linear):
@@ -51,10 +72,23 @@ class QuantLinear(nn.Linear):
                                                          self.weight_layerwise))
         return torch.cat(out, dim=-1)
 
+    def _one_pass(self, weight):
+        """Whether the kernel takes this weight; everything else goes through the torch expressions below, which also
+        raise what they raise (one group per row or layer-wide scales are not defined for them)."""
+        return (weight.is_cuda and type(weight) in (torch.Tensor, nn.Parameter) and weight.layout == torch.strided
+                and weight.dtype in (torch.float16, torch.bfloat16, torch.float32) and weight.dim() == 2
+                and weight.is_contiguous() and weight.numel() > 0 and weight.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
+                and not self.weight_layerwise and self.group_size >= 8 and weight.shape[1] < (1 << 24)
+                and weight.shape[1] // self.group_size < 12000 and self.quantizer is FullSymQuantizer and _plain_eager())
+
     def _adjust_weight(self, weight, ste=True):
         assert not self.training or self.cherry_indices_registered, "`cherry_indices` is not registered yet."
         cherry = self.cherry_indices.long()
         quant_idx = torch.ones(weight.shape[1], dtype=torch.bool, device=weight.device).scatter(-1, cherry, 0)
+        if self._one_pass(weight):
+            if ste:
+                return _StraightThrough.apply(weight, quant_idx, self.w_bits, self.group_size)
+            return load_quant_cuda().fake_quant(weight.detach(), quant_idx, self.w_bits, self.group_size, False)
         quant_idx = quant_idx.nonzero().squeeze(1)
         qw = weight.detach().index_select(-1, quant_idx)
         s = self._expand_scaling_factors(self._get_scaling_factors(qw), qw)

@@ -196,6 +196,23 @@ std::vector<torch::Tensor> pack(torch::Tensor weight, torch::Tensor cherry_unsor
   return {qweight, scales, cw, idx};
 }
 
+// Fake-quantised training weight (llama/cherry_linear.py:69-99); `quantised` marks the columns that are not cherries.
+torch::Tensor fake_quant(torch::Tensor weight, torch::Tensor quantised, int bits, int group_size, bool ste) {
+  const at::cuda::OptionalCUDAGuard device_guard(device_of(weight));
+  TORCH_CHECK(weight.is_cuda() && weight.dim() == 2 && weight.is_contiguous(), "weight must be a contiguous 2-D CUDA tensor");
+  const auto t = weight.scalar_type();
+  TORCH_CHECK(t == torch::kFloat16 || t == torch::kFloat32 || t == torch::kBFloat16, "weight must be float16, float32 or bfloat16");
+  check_tensor(quantised, "quantised", torch::kBool, weight);
+  TORCH_CHECK(quantised.numel() == weight.size(1), "quantised must have one entry per column");
+  auto out = torch::empty_like(weight);
+  auto table = torch::empty({weight.size(1) / 8}, weight.options().dtype(torch::kInt32));
+  check_status(cq_fake_quant(weight.data_ptr(), t == torch::kFloat16 ? 0 : (t == torch::kFloat32 ? 1 : 2),
+                             (const uint8_t*)quantised.data_ptr(), bits, (int)weight.size(1), (int)weight.size(0), group_size,
+                             ste ? 1 : 0, out.data_ptr(), (uint32_t*)table.data_ptr(), current_stream()),
+               "fake_quant");
+  return out;
+}
+
 // GPU QuantLinear.unpack (llama/qlinear.py:120-162): dense (N, K) fp16.
 torch::Tensor unpack_dense(torch::Tensor qweight, torch::Tensor scales, torch::Tensor cherry_weight,
                            torch::Tensor cherry_indices, int bits, int in_features, int group_size) {
@@ -595,6 +612,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("Dequantize3Normal", &Dequantize3Normal, "Dequantize3Normal");
   m.def("Dequantize4Normal", &Dequantize4Normal, "Dequantize4Normal");
   m.def("pack", &pack, "GPU QuantLinear.pack");
+  m.def("fake_quant", &fake_quant, "fake-quantised training weight");
   m.def("unpack_dense", &unpack_dense, "GPU QuantLinear.unpack");
   m.def("cache_clear", []() {
     check_status(cq_cache_clear(), "cache_clear");

@@ -62,3 +62,26 @@ def test_unpack_into_unaligned_buffers(cabi):
     cabi.check(cabi.lib().cq_unpack_dense(q.data_ptr() + 1, *[ptr(a) for a in t], bits, K, N, C, G, out.data_ptr() + 2, None), "unpack")
     dense = O.unpack(ref["qweight"], ref["scales"], ref["cherry_weight"], ref["cherry_indices"], bits, G, K)
     assert np.array_equal(out[1:].cpu().numpy().view(np.uint16), dense.view(np.uint16).ravel())
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("K,N,bits,G,C", [(128, 3, 4, 128, 8), (264, 5, 3, 64, 16), (1032, 9, 4, 100, 40), (4096, 6, 2, 128, 16),
+                                         (2312, 7, 4, 4096, 8)])
+def test_fake_quantised_weight(pkg, K, N, bits, G, C, dtype):
+    """The kernel's weight and gradient equal the torch expressions', infinite and NaN weights included."""
+    from cherryq_b200 import cherry_linear as CL
+    w, idx = layer(K, max(N, 4), C, np.float32, K + bits)
+    w[3, 5], w[2, 70] = np.inf, np.nan
+    lin = CL.QuantLinear(K, w.shape[0], w_bits=bits, group_size=G, cherryq=True, cherry_fraction=C / K).cuda().to(dtype).train()
+    lin.weight.data.copy_(dev(w))
+    lin.register_cherry_indices(dev(idx.astype(np.int32)))
+    assert lin._one_pass(lin.weight)
+    got = lin._adjust_weight(lin.weight), lin._adjust_weight(lin.weight, ste=False)
+    lin._one_pass = lambda weight: False
+    ref = lin._adjust_weight(lin.weight), lin._adjust_weight(lin.weight, ste=False)
+    for a, b in zip(got, ref):
+        assert a.dtype == b.dtype and torch.equal(a.isnan(), b.isnan())
+        assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0))
+    g = torch.randn_like(lin.weight)
+    got[0].backward(g)
+    assert torch.equal(lin.weight.grad, g)
