@@ -6,60 +6,74 @@
 // dequantised matrix to memory.  This is the only part of the path that is a dense
 // contraction, so it runs on the 5th-generation tensor cores:
 //
-//   * A operand = weights, 128 rows per CTA tile, dequantised to fp16 by the row's own thread
-//     (one thread = one weight row = one TENSOR MEMORY lane) and stored straight into tensor
-//     memory with tcgen05.st: exponent-trick unpack (AND-OR into the bits of 1024.0), one exact
-//     subtraction and one multiplication by the group scale per fp16 pair, which reproduces
+//   * A operand = weights, 256 rows per tile, 128 in each CTA of a pair, dequantised to fp16 by the
+//     row's own thread (one thread = one weight row = one TENSOR MEMORY lane) and stored straight
+//     into tensor memory with tcgen05.st: exponent-trick unpack (AND-OR into the bits of 1024.0), one
+//     exact subtraction and one multiplication by the group scale per fp16 pair, which reproduces
 //     unpack()'s fp16 values bit for bit;
-//   * B operand = NT tokens of activations per CTA tile (NT = 256, or 128 for calls of at most 128
-//     rows), prepared once per call by a small pre-pass kernel (gather into compact column
-//     order, canonical K-major UMMA layout) so that the main kernel moves them with plain bulk
-//     async copies;
-//   * D = 128 rows x NT tokens fp32 in tensor memory, accumulated over the whole K by
-//     tcgen05.mma.cta_group::1.kind::f16 (A from TMEM, M = 128, N = NT, K = 16 per instruction);
-//     with NT = 128 there are two accumulator buffers, so that the fp16 store of one tile overlaps
-//     the MMAs of the next.
+//   * B operand = NT tokens of activations per tile (NT = 32 .. 256 in steps of 32), half of them in each CTA,
+//     prepared once per call by a small pre-pass kernel (gather into compact column order, canonical
+//     K-major UMMA layout) so that the main kernel moves them with plain bulk async copies;
+//   * D = 256 rows x NT tokens fp32 in tensor memory (128 rows per CTA), accumulated over K by
+//     tcgen05.mma.cta_group::2.kind::f16 (A from TMEM, M = 256, N = NT, K = 16 per instruction).
 //
-// Warp roles (704 threads, one CTA per SM, persistent over (token block, row tile) units):
-//   warps 0-15  four decode groups (items go round-robin), thread r of a group = row r; a group
-//               needs about twice the time the tensor core spends on an item, hence four of them
-//   warp 16     MMA issuer (one lane); owns the tensor-memory allocation
-//   warp 17     producer (one lane): bulk copies of weight items and activation tiles
-//   warps 18-21 epilogue: tcgen05.ld of a finished tile, fp16 store to y
+// Why pairs: a lone CTA with 128 x 256 tiles has to bring 64 KB of activations and 8 KB of weights into shared memory
+// per 128 columns, about 70 bytes a cycle at the tensor core's rate, more than an SM gets from L2; in a pair each CTA
+// brings half of the activations.
+//
+// Work: (token block, pair of row tiles) units x items (cherry items, then granules of 128 columns).  Clusters take
+// whole units round-robin; the units that do not fill a last wave - all of them in a call of few tokens - are cut
+// into equal runs of items, one run per cluster.  A unit that more than one cluster worked on is summed from fp32
+// partial tiles, in item order, by the cluster that arrives last (no cluster waits for another; sums do not depend on
+// timing).
+//
+// Warp roles (736 threads, one CTA per SM, persistent over its work list):
+//   warps 0-15  four decode groups (items go round-robin), thread r of a group = row r
+//   warp 16     MMA issuer (one lane, leader CTA); owns the tensor-memory allocation
+//   warps 17-18 producers (one lane each): bulk copies of weight items / activation tiles; each issue costs its thread
+//               a few hundred cycles, so they are two and keep their addresses and phases without a division
+//   warps 19-22 epilogue: tcgen05.ld of a finished tile into shared memory (which frees the accumulator), then
+//               16-byte stores to y
 // Every wait is bounded and reports into the status word instead of hanging.
-#include <cstdlib>
+//
+// Bound and state: 4096 -> 11008 4-bit, 2048 rows: 144 us = 1.28 PFLOP/s (739 us through QuantLinear and 195 us by itself
+// with lone CTAs of 128 x 256 tiles); 8192 -> 28672 3-bit, 2048 rows: 657 us = 1.46 PFLOP/s, tensor-bound.  16 rows: 18 and
+// 52 us (31 and 76): an item then takes about 740 cycles, the eight MMAs' reads of A from tensor memory and their issue,
+// against 365 that its weights need to arrive from HBM.
+#include <cmath>
 
 #include "cq_tile.cuh"
 
 namespace {
 
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
-// NT = tokens per tile = UMMA N: 256 (one accumulator buffer; the MMA runs at its full rate) or 128
-// (two accumulator buffers; less padding for few tokens).
 constexpr int NGRP = 4;                 // decode groups of four warps
 constexpr int NA = 4;                   // A slots in tensor memory (64 columns each), one per decode group
 constexpr int A_COLS = 64;
 constexpr int D_BASE = NA * A_COLS;
 constexpr int TMEM_COLS = 512;
-constexpr int SW = 4;                   // weight ring stages
-constexpr int NTHREADS = (NGRP * 4 + 6) * 32;
-// one K = 16 step of the B operand: [token group of 8][k half][8 tokens][16 B] = NT * 32 bytes;
-// a granule is 8 steps, a cherry item one
-__host__ __device__ constexpr int b_kstep_bytes(int nt) { return nt * 32; }
-__host__ __device__ constexpr int b_gran_bytes(int nt) { return nt * 256; }
+constexpr int SW_MAX = 12, SB_MAX = 12; // most weight / activation ring stages
+constexpr int NTHREADS = (NGRP * 4 + 7) * 32;
+constexpr int STAGE_THREADS = 128;     // a block of the pre-pass fits beside a CTA of the main kernel
+constexpr int N_BARS = 2 * SW_MAX + 2 * SB_MAX + 2 * NA + 4;
+// A CTA's half of the B operand of one K = 16 step: [token group of 8][k half][8 tokens][16 B] = NT / 2 * 32 bytes;
+// a granule is 8 steps, a cherry item one.
+__host__ __device__ constexpr int b_kstep_bytes(int nt) { return nt * 16; }
+__host__ __device__ constexpr int b_gran_bytes(int nt) { return nt * 128; }
 
 struct PrefillParams {
   const uint8_t* stream;     // tile-layout weight stream
-  const uint8_t* xb;         // staged activations: [token block][cherry items][granules]
+  const uint8_t* xb;         // staged activations: [token block][half][cherry items][granules]
   __half* y;
   uint32_t* status;
-  int M, N, n_gran, n_tile, n_cher, gran_bytes, tile_bytes, ldy, accumulate;
-  uint32_t n_units;          // token blocks x row tiles
-  unsigned long long xb_blk_bytes;
-  int wstage_bytes, sb, off_wring, off_bring, off_bar;   // sb = activation ring stages
-  int split;                 // parts the items of a unit are divided into (split-K), 1 = none
-  float* partial;            // [unit][part][row tile][128 rows][NT] fp32 partial tiles (split > 1)
-  uint32_t* arrived;         // [unit] parts finished so far (split > 1)
+  int M, N, n_gran, n_tile, n_cher, gran_bytes, tile_bytes, ldy, accumulate, vec_y;
+  int nt;                    // tokens per block
+  uint32_t n_units;          // token blocks x pairs of row tiles
+  uint32_t sk_units, sk_clusters;   // the first sk_units units are cut into runs of items for sk_clusters clusters
+  unsigned long long xb_half_bytes;
+  int wstage_bytes, sw, sb, off_wring, off_bring, off_stage, off_bar;   // sw, sb = ring stages
+  float* partial;            // [cluster][first / last run][CTA of the pair][token][128 rows] fp32
+  uint32_t* arrived;         // [cut unit][CTA of the pair] runs finished so far
 };
 
 // ------------------------------------------------------------------ PTX helpers
@@ -86,16 +100,16 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
 // which wait failed in the status word and lets the caller run on to the common exit.
 __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
                                             uint32_t* status, uint32_t code) {
-  // bounded in polls and in time (about one second of the device's nanosecond timer)
+  // bounded in polls and in time (about one second of the device's nanosecond timer, read once some polls have failed)
   const uint32_t limit = *abort_flag ? 1u : WAIT_LIMIT;
-  unsigned long long t0;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t0));
+  unsigned long long t0 = 0;
   for (uint32_t it = 0; it < limit; ++it) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 63u) == 63u) {
+    if ((it & 255u) == 255u) {
       unsigned long long t1;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
-      if (t1 - t0 > 1000000000ull) break;
+      if (t0 == 0) t0 = t1;
+      else if (t1 - t0 > 1000000000ull) break;
     }
   }
   *abort_flag = 1;
@@ -121,18 +135,40 @@ __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
   return d;
 }
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
+// the same shared-memory offset in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
 }
-// D[tmem_d] (+)= A[tmem_a] * B[desc_b]: fp16 inputs, fp32 accumulate, shape from the instruction descriptor
+// What an arrival in the other CTA announces is read there by the tensor core only (tensor memory, ordered by the
+// tcgen05 fences, and tiles written by the async proxy), so it needs no cluster-wide fence: release.cluster here and
+// acquire.cluster in the waits made an item of 128 columns take 1500 cycles whatever its number of tokens.
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_bar) : "memory");
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// arrives on the barrier at this offset in both CTAs when every MMA issued so far has finished
+__device__ __forceinline__ void tc_commit_pair(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+               ::"r"(bar), "h"((unsigned short)3) : "memory");
+}
+// D[tmem_d] (+)= A[tmem_a] * B[desc_b] over the pair: fp16 inputs, fp32 accumulate, shape from the instruction descriptor
 __device__ __forceinline__ void umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t acc) {
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, {%5, %5, %5, %5}, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc), "r"(0u) : "memory");
+      "tcgen05.mma.cta_group::2.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(acc) : "memory");
 }
 __device__ __forceinline__ void tmem_st16(uint32_t addr, const uint32_t* v) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
@@ -205,199 +241,323 @@ __device__ __forceinline__ void dequant3(uint32_t w0, uint32_t w1, uint32_t w2, 
 }
 
 // ------------------------------------------------------------------ activation pre-pass
-// xb[token block][item][...] in the layout the MMA reads from shared memory: per K = 16 step
-// [token group of 8][k half][token in group][8 fp16]; cherry items (16 cherry columns) first, then
-// the granules (128 compact columns = 8 steps).  Tokens past M are not written.
-__global__ void prefill_stage_x_kernel(const __half* __restrict__ x, int ldx, int M, const uint32_t* __restrict__ osh,
-                                       const uint16_t* __restrict__ cidx, int C, int Kc, int n_gran, int n_cher,
-                                       uint8_t* __restrict__ xb, unsigned long long blk_bytes, int n_mblk, int NT) {
-  const int per_tok = 2 * n_cher + 16 * n_gran;            // octets per token
-  // Only real tokens are staged: the padding columns of the last token block feed accumulator
-  // columns that are never read back (each output column depends on its own token only).
-  const long long total = (long long)M * per_tok;
-  (void)n_mblk;
-  const int B_KSTEP_BYTES = b_kstep_bytes(NT), B_GRAN_BYTES = b_gran_bytes(NT), B_CHER_BYTES = B_KSTEP_BYTES;
-  for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < total;
-       id += (long long)gridDim.x * blockDim.x) {
-    const int m = (int)(id / per_tok), oi = (int)(id % per_tok);
-    const int mb = m / NT, ml = m % NT;
-    unsigned short h[8];
+// xb[token block][half of the block][item][...] in the layout the MMA reads from shared memory: per K = 16 step
+// [token group of 8][k half][token in group][8 fp16]; cherry items (16 cherry columns) first, then the granules
+// (128 compact columns = 8 steps).  A warp stages four octets of eight tokens (128 contiguous bytes per octet) and goes
+// on to the next GROUPS - 1 token groups with the same columns, all their loads in flight together.  An octet without a
+// cherry column inside is two aligned 16-byte loads and a shift by its position in them.
+// Tokens past M are not written: the padding feeds accumulator columns that are never read back (each output
+// column depends on its own token only).  Also clears the arrival counters of the main kernel.
+// the eight halves that start `off` halves into the two vectors
+__device__ __forceinline__ uint4 shift_halves(uint4 lo, uint4 hi, int off) {
+  uint32_t w[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-    for (int e = 0; e < 8; ++e) h[e] = 0;
-    uint8_t* dst;
-    const unsigned short* xr = reinterpret_cast<const unsigned short*>(x) + (size_t)m * ldx;
-    if (oi < 2 * n_cher) {
-      const int j = oi >> 1, hh = oi & 1;
-      if (m < M) {
+  for (int i = 0; i < 6; ++i) w[i] = (off & 4) ? w[i + 2] : w[i];
+#pragma unroll
+  for (int i = 0; i < 5; ++i) w[i] = (off & 2) ? w[i + 1] : w[i];
+  const uint32_t s = 16 * (off & 1);
+  return make_uint4(__funnelshift_r(w[0], w[1], s), __funnelshift_r(w[1], w[2], s), __funnelshift_r(w[2], w[3], s),
+                    __funnelshift_r(w[3], w[4], s));
+}
+template <int GROUPS>
+__global__ void __launch_bounds__(STAGE_THREADS, 10) prefill_stage_x_kernel(
+    const __half* __restrict__ x, int ldx, int M, const uint32_t* __restrict__ osh, const uint16_t* __restrict__ cidx,
+    int C, int Kc, int n_gran, int n_cher, uint8_t* __restrict__ xb, unsigned long long half_bytes, int NT,
+    uint32_t* __restrict__ arrived, int n_arrived, int aligned16) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int n_oct = 2 * n_cher + 16 * n_gran;              // octets per token
+  const int lane = threadIdx.x & 31, HT = NT >> 1;
+  const int oi = (blockIdx.x * (STAGE_THREADS / 32) + (threadIdx.x >> 5)) * 4 + (lane >> 3);
+  const unsigned short* xs = reinterpret_cast<const unsigned short*>(x);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  // where the octet's columns are
+  const bool cherry = oi < 2 * n_cher;
+  const int o = oi - 2 * n_cher, k0 = 8 * o;
+  int lo0 = 0, lo7 = 0;
+  bool empty = oi >= n_oct;
+  size_t dst0;
+  if (cherry) {
+    dst0 = (size_t)(oi >> 1) * b_kstep_bytes(NT) + (oi & 1) * 128;
+  } else {
+    dst0 = (size_t)n_cher * b_kstep_bytes(NT) + (size_t)(o >> 4) * b_gran_bytes(NT) + ((o & 15) >> 1) * b_kstep_bytes(NT) + (o & 1) * 128;
+    const uint32_t sh = empty ? 0xFFFFFFFFu : osh[o];
+    empty = sh == 0xFFFFFFFFu;
+    lo0 = (int)(sh & 0xFFFFu);
+    lo7 = (int)(sh >> 16);
+  }
+  const bool plain = !cherry && !empty && lo0 == lo7 && aligned16;
+  const int c0 = k0 + lo0, off = c0 & 7;
+  if (blockIdx.x == 0 && blockIdx.y == 0)
+    for (int i = threadIdx.x; i < n_arrived; i += STAGE_THREADS) arrived[i] = 0u;
+  if (oi >= n_oct) return;
+  for (int tg0 = blockIdx.y * GROUPS; tg0 < (M + 7) >> 3; tg0 += gridDim.y * GROUPS) {
+    uint4 v[GROUPS], v2[GROUPS];
+#pragma unroll
+    for (int u = 0; u < GROUPS; ++u) {
+      const int m = (tg0 + u) * 8 + (lane & 7);
+      v[u] = v2[u] = make_uint4(0, 0, 0, 0);
+      if (plain && m < M) {
+        // (K is a multiple of 8 and all eight columns exist: the second vector, where needed, lies inside the row)
+        const uint4* src = reinterpret_cast<const uint4*>(xs + (size_t)m * ldx + (c0 - off));
+        v[u] = __ldg(src);
+        if (off) v2[u] = __ldg(src + 1);
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < GROUPS; ++u) {
+      const int m = (tg0 + u) * 8 + (lane & 7);
+      if (m >= M) break;
+      if (plain) {
+        v[u] = shift_halves(v[u], v2[u], off);
+      } else if (!empty) {
+        const unsigned short* xr = xs + (size_t)m * ldx;
+        unsigned short h[8];
+        int sft = lo0;
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const int c = 16 * j + 8 * hh + e;
-          if (c < C) h[e] = __ldg(xr + cidx[c]);
-        }
-      }
-      dst = xb + (size_t)mb * blk_bytes + (size_t)j * B_CHER_BYTES + (ml >> 3) * 256 + hh * 128 + (ml & 7) * 16;
-    } else {
-      const int o = oi - 2 * n_cher, g = o >> 4, oo = o & 15;
-      const int k0 = 8 * o;
-      const uint32_t sh = osh[o];
-      if (m < M && sh != 0xFFFFFFFFu) {
-        const int lo0 = (int)(sh & 0xFFFFu), lo7 = (int)(sh >> 16);
-        if (lo0 == lo7 && ((k0 + lo0) & 1) == 0 && (((uintptr_t)xr) & 3) == 0) {
-          // eight consecutive columns at a 4-byte aligned address (K' is a multiple of 8: all exist)
-          const uint32_t* s32 = reinterpret_cast<const uint32_t*>(xr + k0 + lo0);
-#pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t w = __ldg(s32 + i);
-            h[2 * i] = (unsigned short)(w & 0xFFFFu);
-            h[2 * i + 1] = (unsigned short)(w >> 16);
-          }
-        } else {
-          int sft = lo0;
-#pragma unroll
-          for (int e = 0; e < 8; ++e) {
+          h[e] = 0;
+          if (cherry) {
+            const int c = 8 * oi + e;
+            if (c < C) h[e] = __ldg(xr + cidx[c]);
+          } else {
             // cherry columns inside the octet: the shift grows from lo0 to lo7 along it
             while (sft < lo7 && (int)cidx[sft] - sft <= k0 + e) ++sft;
             if (k0 + e < Kc) h[e] = __ldg(xr + k0 + e + sft);
           }
         }
+        v[u] = make_uint4((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16),
+                          (uint32_t)h[4] | ((uint32_t)h[5] << 16), (uint32_t)h[6] | ((uint32_t)h[7] << 16));
       }
-      dst = xb + (size_t)mb * blk_bytes + (size_t)n_cher * B_CHER_BYTES + (size_t)g * B_GRAN_BYTES +
-            (oo >> 1) * B_KSTEP_BYTES + (ml >> 3) * 256 + (oo & 1) * 128 + (ml & 7) * 16;
+      const int mb = m / NT, ml = m - mb * NT, hf = ml >= HT, mt = ml - hf * HT;
+      *reinterpret_cast<uint4*>(xb + (size_t)(2 * mb + hf) * half_bytes + dst0 + (mt >> 3) * 256 + (mt & 7) * 16) = v[u];
     }
-    uint4 v;
-    v.x = (uint32_t)h[0] | ((uint32_t)h[1] << 16);
-    v.y = (uint32_t)h[2] | ((uint32_t)h[3] << 16);
-    v.z = (uint32_t)h[4] | ((uint32_t)h[5] << 16);
-    v.w = (uint32_t)h[6] | ((uint32_t)h[7] << 16);
-    *reinterpret_cast<uint4*>(dst) = v;
   }
 }
 
+// ------------------------------------------------------------------ work list of a cluster
+struct Work {
+  uint32_t unit, j0, j1;     // items [j0, j1) of this unit
+  int run;                   // -1: a whole unit; 0 / 1: the first / last run of this cluster, a part of its unit
+};
+// first item of cluster c's run over the cut units
+__device__ __forceinline__ uint32_t run_begin(const PrefillParams& p, uint32_t c, uint32_t total) {
+  return c * total / p.sk_clusters;        // (74 clusters x 73 units x a few thousand items at most: fits 32 bits)
+}
+struct WorkList {
+  uint32_t b, e, b0, u, ipt, n_units, clusters;
+  __device__ __forceinline__ WorkList(const PrefillParams& p, uint32_t cluster, uint32_t n_clusters, uint32_t ipt_)
+      : b(0), e(0), b0(0), u(p.sk_units + cluster), ipt(ipt_), n_units(p.n_units), clusters(n_clusters) {
+    if (cluster < p.sk_clusters) {
+      const uint32_t total = p.sk_units * ipt;
+      b0 = b = run_begin(p, cluster, total);
+      e = run_begin(p, cluster + 1, total);
+    }
+  }
+  __device__ __forceinline__ bool next(Work& w) {
+    if (b < e) {
+      w.unit = b / ipt;
+      w.j0 = b - w.unit * ipt;
+      w.j1 = min(ipt, w.j0 + (e - b));
+      w.run = (w.j0 == 0 && w.j1 == ipt) ? -1 : (b == b0 ? 0 : 1);
+      b += w.j1 - w.j0;
+      return true;
+    }
+    if (u >= n_units) return false;
+    w.unit = u;
+    w.j0 = 0;
+    w.j1 = ipt;
+    w.run = -1;
+    u += clusters;
+    return true;
+  }
+};
+
+// position in a ring of stages: slot, parity of its current round, rounds completed
+struct Ring {
+  uint32_t slot = 0, phase = 0, round = 0;
+  __device__ __forceinline__ void advance(uint32_t stages) {
+    if (++slot == stages) {
+      slot = 0;
+      phase ^= 1;
+      ++round;
+    }
+  }
+  // the last use of every slot used so far
+  template <typename F> __device__ __forceinline__ void each_last(uint32_t stages, F f) const {
+    for (uint32_t s = 0; s < stages; ++s) {
+      if (s < slot) f(s, phase);
+      else if (round) f(s, phase ^ 1);
+    }
+  }
+};
+
 // ------------------------------------------------------------------ main kernel
-// RT = row tiles of 128 rows per unit: with two, one staged activation tile feeds two weight tiles,
-// which halves the activation bytes an SM has to pull from L2 per flop.
-template <int BITS, int SETS, int NT, int RT>
+template <int BITS, int SETS>
 __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillParams p) {
-  constexpr int W_MMA = NGRP * 4, W_PROD = NGRP * 4 + 1;
-  constexpr int ND = (NT * RT == 128) ? 2 : 1;            // accumulator buffers (RT * NT columns each)
-  constexpr int SBMAX = 4;
-  constexpr int B_KSTEP_BYTES = b_kstep_bytes(NT), B_GRAN_BYTES = b_gran_bytes(NT), B_CHER_BYTES = B_KSTEP_BYTES;
-  // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = NT, M = 128
-  constexpr uint32_t IDESC = (1u << 4) | ((uint32_t)(NT >> 3) << 17) | (8u << 24);
+  constexpr int W_MMA = NGRP * 4, W_PROD_W = NGRP * 4 + 1, W_PROD_B = NGRP * 4 + 2;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int s_abort;
   __shared__ uint32_t s_tmem;
   __shared__ int s_last;
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const uint32_t grid = gridDim.x, cta = blockIdx.x;
+  uint32_t rank;
+  asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  const uint32_t cluster = blockIdx.x >> 1, n_clusters = gridDim.x >> 1;
+  const uint32_t NT = (uint32_t)p.nt;
+  const uint32_t ND = NT <= 128 ? 2 : 1;                   // accumulator buffers of NT columns
   const uint32_t NCH = (uint32_t)p.n_cher, IPT = NCH + (uint32_t)p.n_gran;
-  const uint32_t NTILE = (uint32_t)p.n_tile;
-  const uint32_t NPAIR = (NTILE + RT - 1) / RT;          // units per token block
-  const uint32_t SB = (uint32_t)p.sb;
-  const uint32_t SPLIT = (uint32_t)p.split;
-  const uint32_t n_work = p.n_units * SPLIT;               // work items: (unit, part), part fastest
+  const uint32_t NTILE = (uint32_t)p.n_tile, NPAIR = (NTILE + 1) / 2;
+  const uint32_t SW = (uint32_t)p.sw, SB = (uint32_t)p.sb;
+  const uint32_t B_KSTEP_BYTES = b_kstep_bytes(NT), B_GRAN_BYTES = b_gran_bytes(NT), B_CHER_BYTES = B_KSTEP_BYTES;
 
   const uint32_t bar0 = smem_u32(smem + p.off_bar);
   auto B_WFULL = [&](uint32_t s) { return bar0 + 8 * s; };
-  auto B_WEMPTY = [&](uint32_t s) { return bar0 + 8 * (SW + s); };
-  auto B_BFULL = [&](uint32_t s) { return bar0 + 8 * (2 * SW + s); };
-  auto B_BEMPTY = [&](uint32_t s) { return bar0 + 8 * (2 * SW + SBMAX + s); };
-  auto B_AFULL = [&](uint32_t a) { return bar0 + 8 * (2 * SW + 2 * SBMAX + a); };
-  auto B_AEMPTY = [&](uint32_t a) { return bar0 + 8 * (2 * SW + 2 * SBMAX + NA + a); };
-  auto B_DFULL = [&](uint32_t d) { return bar0 + 8 * (2 * SW + 2 * SBMAX + 2 * NA + d); };
-  auto B_DEMPTY = [&](uint32_t d) { return bar0 + 8 * (2 * SW + 2 * SBMAX + 2 * NA + 2 + d); };
+  auto B_WEMPTY = [&](uint32_t s) { return bar0 + 8 * (SW_MAX + s); };
+  auto B_BFULL = [&](uint32_t s) { return bar0 + 8 * (2 * SW_MAX + s); };
+  // leader's: item ready in both CTAs (A in tensor memory, activations in shared memory)
+  auto B_READY = [&](uint32_t a) { return bar0 + 8 * (2 * SW_MAX + 2 * SB_MAX + a); };
+  auto B_AEMPTY = [&](uint32_t a) { return bar0 + 8 * (2 * SW_MAX + 2 * SB_MAX + NA + a); };
+  // with as many activation stages as A slots one commit releases both
+  auto B_BEMPTY = [&](uint32_t s) { return SB == NA ? B_AEMPTY(s) : bar0 + 8 * (2 * SW_MAX + SB_MAX + s); };
+  auto B_DFULL = [&](uint32_t d) { return bar0 + 8 * (2 * SW_MAX + 2 * SB_MAX + 2 * NA + d); };
+  auto B_DEMPTY = [&](uint32_t d) { return bar0 + 8 * (2 * SW_MAX + 2 * SB_MAX + 2 * NA + 2 + d); };
 
   if (tid == 0) {
     s_abort = 0;
     for (uint32_t s = 0; s < SW; ++s) { mbar_init(B_WFULL(s), 1); mbar_init(B_WEMPTY(s), 4); }
-    for (uint32_t s = 0; s < SB; ++s) { mbar_init(B_BFULL(s), 1); mbar_init(B_BEMPTY(s), 1); }
-    for (uint32_t a = 0; a < NA; ++a) { mbar_init(B_AFULL(a), 4); mbar_init(B_AEMPTY(a), 1); }
-    for (uint32_t d = 0; d < ND; ++d) { mbar_init(B_DFULL(d), 1); mbar_init(B_DEMPTY(d), 4); }
+    for (uint32_t s = 0; s < SB; ++s) {
+      mbar_init(B_BFULL(s), 1);
+      if (SB != NA) mbar_init(B_BEMPTY(s), 1);
+    }
+    for (uint32_t a = 0; a < NA; ++a) { mbar_init(B_READY(a), 8); mbar_init(B_AEMPTY(a), 1); }
+    for (uint32_t d = 0; d < 2; ++d) { mbar_init(B_DFULL(d), 1); mbar_init(B_DEMPTY(d), 8); }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if (warp == W_MMA) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(TMEM_COLS) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&s_tmem)), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   tc_fence_before();
   __syncthreads();
+  cluster_sync();                                          // the peer's barriers exist before anything arrives on them
   tc_fence_after();
   const uint32_t tmem = s_tmem;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
-  if (warp == W_PROD) {
-    // ================================================================ producer
+  if (warp == W_PROD_W) {
+    // ================================================================ weight producer
+    // (starts at once: the first ring of weights streams while the pre-pass still stages the activations)
+    if (lane == 0) {
+      const uint32_t wring = smem_u32(smem + p.off_wring);
+      Ring ring;
+      WorkList wl(p, cluster, n_clusters, IPT);
+      Work w;
+      while (wl.next(w)) {
+        // (an odd number of row tiles: the last pair's second CTA repeats the last tile, its results are dropped)
+        const uint32_t tile = min(2 * (w.unit % NPAIR) + rank, NTILE - 1);
+        const uint32_t c0 = min(w.j0, NCH);
+        const uint8_t* src = p.stream + (size_t)tile * p.tile_bytes + (size_t)c0 * CQT_CHER_BYTES + (size_t)(w.j0 - c0) * p.gran_bytes;
+        for (uint32_t j = w.j0; j < w.j1; ++j) {
+          const uint32_t bytes = j < NCH ? (uint32_t)CQT_CHER_BYTES : (uint32_t)p.gran_bytes;
+          if (ring.round) mbar_wait(B_WEMPTY(ring.slot), ring.phase ^ 1, &s_abort, p.status, 1u);
+          if (*(volatile int*)&s_abort) break;
+          mbar_expect_tx(B_WFULL(ring.slot), bytes);
+          bulk_g2s(wring + ring.slot * (uint32_t)p.wstage_bytes, src, bytes, B_WFULL(ring.slot));
+          src += bytes;
+          ring.advance(SW);
+        }
+      }
+      // No copy is in flight when this thread leaves, also after a wait that ran out (bounded like every wait).
+      int own = 0;
+      ring.each_last(SW, [&](uint32_t slot, uint32_t phase) { mbar_wait(B_WFULL(slot), phase, &own, p.status, 512u); });
+    }
+  } else if (warp == W_PROD_B) {
+    // ================================================================ activation producer
     if (lane == 0) {
       // the staged activations are written by the kernel launched just before this one
       asm volatile("griddepcontrol.wait;" ::: "memory");
-      const uint32_t wring = smem_u32(smem + p.off_wring), bring = smem_u32(smem + p.off_bring);
-      uint32_t n = 0, nb = 0;      // weight items and activation tiles issued so far
-      for (uint32_t wk = cta; wk < n_work; wk += grid) {
-        const uint32_t u = wk / SPLIT, part = wk - u * SPLIT;
-        const uint32_t j0 = part * IPT / SPLIT, j1 = (part + 1) * IPT / SPLIT;
-        const uint32_t mb = u / NPAIR, t0 = (u - mb * NPAIR) * RT;
-        const uint32_t ntr = min((uint32_t)RT, NTILE - t0);
-        // offsets of item j0 inside a row tile's block and inside the token block's staged activations
-        const uint32_t c0 = min(j0, NCH), g0 = j0 - c0;
-        size_t woff = (size_t)c0 * CQT_CHER_BYTES + (size_t)g0 * p.gran_bytes;
-        const uint8_t* bsrc = p.xb + (size_t)mb * p.xb_blk_bytes + (size_t)c0 * B_CHER_BYTES + (size_t)g0 * B_GRAN_BYTES;
-        for (uint32_t j = j0; j < j1; ++j, ++nb) {
-          const bool cherry = j < NCH;
-          const uint32_t sb = nb % SB;
-          const uint32_t wbytes = cherry ? (uint32_t)CQT_CHER_BYTES : (uint32_t)p.gran_bytes;
-          const uint32_t bbytes = cherry ? (uint32_t)B_CHER_BYTES : (uint32_t)B_GRAN_BYTES;
-          for (uint32_t rt = 0; rt < ntr; ++rt, ++n) {
-            const uint32_t sw = n % SW;
-            if (n >= SW) mbar_wait(B_WEMPTY(sw), ((n / SW) - 1) & 1, &s_abort, p.status, 1u);
-            mbar_expect_tx(B_WFULL(sw), wbytes);
-            bulk_g2s(wring + sw * (uint32_t)p.wstage_bytes, p.stream + (size_t)(t0 + rt) * p.tile_bytes + woff, wbytes,
-                     B_WFULL(sw));
+      const uint32_t bring = smem_u32(smem + p.off_bring);
+      Ring ring;
+      WorkList wl(p, cluster, n_clusters, IPT);
+      Work w;
+      while (wl.next(w)) {
+        const uint32_t mb = w.unit / NPAIR;
+        const bool real = (int)(mb * NT + rank * (NT >> 1)) < p.M;       // this half of the block holds tokens
+        const uint32_t c0 = min(w.j0, NCH);
+        const uint8_t* src = p.xb + (size_t)(2 * mb + rank) * p.xb_half_bytes + (size_t)c0 * B_CHER_BYTES +
+                             (size_t)(w.j0 - c0) * B_GRAN_BYTES;
+        for (uint32_t j = w.j0; j < w.j1; ++j) {
+          const uint32_t bytes = j < NCH ? B_CHER_BYTES : B_GRAN_BYTES;
+          if (ring.round) mbar_wait(B_BEMPTY(ring.slot), ring.phase ^ 1, &s_abort, p.status, 2u);
+          if (*(volatile int*)&s_abort) break;
+          if (real) {
+            mbar_expect_tx(B_BFULL(ring.slot), bytes);
+            bulk_g2s(bring + ring.slot * B_GRAN_BYTES, src, bytes, B_BFULL(ring.slot));
+          } else {
+            mbar_arrive(B_BFULL(ring.slot));
           }
-          if (nb >= SB) mbar_wait(B_BEMPTY(sb), ((nb / SB) - 1) & 1, &s_abort, p.status, 2u);
-          mbar_expect_tx(B_BFULL(sb), bbytes);
-          bulk_g2s(bring + sb * (uint32_t)B_GRAN_BYTES, bsrc, bbytes, B_BFULL(sb));
-          woff += wbytes;
-          bsrc += bbytes;
+          src += bytes;
+          ring.advance(SB);
         }
       }
+      // No copy and no arrival of a tcgen05.commit is in flight when this thread leaves: a late one would land in the
+      // barriers of the next kernel's CTA (the decode groups wait for theirs below).
+      int own = 0;
+      ring.each_last(SB, [&](uint32_t slot, uint32_t phase) {
+        mbar_wait(B_BFULL(slot), phase, &own, p.status, 512u);
+        mbar_wait(B_BEMPTY(slot), phase, &own, p.status, 512u);
+      });
     }
   } else if (warp == W_MMA) {
-    // ================================================================ MMA issuer
-    if (lane == 0) {
+    if (rank == 0) {
+      // ================================================================ MMA issuer (leader CTA)
+      // The whole warp walks the list and one elected lane issues: addresses and descriptors then stay in uniform
+      // registers, where the MMA takes them (all of tensor memory is allocated, so its base is column 0).
+      // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = NT, M = 256
+      const uint32_t IDESC = (1u << 4) | ((NT >> 3) << 17) | (16u << 24);
       const uint32_t bring = smem_u32(smem + p.off_bring);
-      uint32_t n = 0, nb = 0, lu = 0;
-      for (uint32_t wk = cta; wk < n_work; wk += grid, ++lu) {
-        const uint32_t u = wk / SPLIT, part = wk - u * SPLIT;
-        const uint32_t j0 = part * IPT / SPLIT, j1 = (part + 1) * IPT / SPLIT;
-        const uint32_t mb = u / NPAIR, t0 = (u - mb * NPAIR) * RT;
-        const uint32_t ntr = min((uint32_t)RT, NTILE - t0);
-        const uint32_t dbuf = lu % ND;
-        if (lu >= ND) mbar_wait(B_DEMPTY(dbuf), ((lu / ND) - 1) & 1, &s_abort, p.status, 4u);
-        for (uint32_t j = j0; j < j1; ++j, ++nb) {
-          const uint32_t sb = nb % SB;
-          mbar_wait(B_BFULL(sb), (nb / SB) & 1, &s_abort, p.status, 16u);
-          const uint32_t bbase = bring + sb * (uint32_t)B_GRAN_BYTES;
-          for (uint32_t rt = 0; rt < ntr; ++rt, ++n) {
-            const uint32_t a = n % NA;
-            const uint32_t td = tmem + D_BASE + (dbuf * RT + rt) * NT;
-            mbar_wait(B_AFULL(a), (n / NA) & 1, &s_abort, p.status, 8u);
-            tc_fence_after();
-            const uint32_t ta = tmem + a * A_COLS;
-            if (j < NCH) {
-              umma_ts(td, ta, smem_desc(bbase, 8, 16), IDESC, j != j0);
-            } else {
-#pragma unroll
-              for (uint32_t ks = 0; ks < 8; ++ks)
-                umma_ts(td, ta + ks * 8, smem_desc(bbase + ks * B_KSTEP_BYTES, 8, 16), IDESC, (j != j0 || ks != 0));
-            }
-            tc_commit(B_AEMPTY(a));
-          }
-          tc_commit(B_BEMPTY(sb));
-        }
-        tc_commit(B_DFULL(dbuf));
+      if (tmem != 0) {
+        s_abort = 1;
+        if (p.status && lane == 0) atomicOr(p.status, 1024u);
       }
+      __syncwarp();
+      uint32_t lu = 0;
+      Ring rb, ra;
+      WorkList wl(p, cluster, n_clusters, IPT);
+      Work w;
+      for (; wl.next(w); ++lu) {
+        const uint32_t dbuf = lu % ND;
+        const uint32_t td = D_BASE + dbuf * NT;
+        if (lu >= ND) mbar_wait(B_DEMPTY(dbuf), ((lu / ND) - 1) & 1, &s_abort, p.status, 4u);
+        tc_fence_after();
+        for (uint32_t j = w.j0; j < w.j1; ++j) {
+          // one wait an item: everything that stands between two items idles the tensor core
+          const bool ok = mbar_wait(B_READY(ra.slot), ra.phase, &s_abort, p.status, 8u);
+          if (!__all_sync(0xffffffffu, ok)) break;           // nothing is issued on operands that never came
+          tc_fence_after();
+          const uint64_t bdesc = smem_desc(bring + rb.slot * B_GRAN_BYTES, 8, 16);
+          const uint32_t ta = ra.slot * A_COLS;
+          if (elect_one()) {
+            if (j < NCH) {
+              umma_ts(td, ta, bdesc, IDESC, j != w.j0);
+            } else {
+              umma_ts(td, ta, bdesc, IDESC, j != w.j0);
+#pragma unroll
+              for (uint32_t ks = 1; ks < 8; ++ks) umma_ts(td, ta + ks * 8, bdesc + ks * (B_KSTEP_BYTES >> 4), IDESC, 1u);
+            }
+            tc_commit_pair(B_AEMPTY(ra.slot));
+            if (SB != NA) tc_commit_pair(B_BEMPTY(rb.slot));
+          }
+          __syncwarp();
+          ra.advance(NA);
+          rb.advance(SB);
+        }
+        if (elect_one()) tc_commit_pair(B_DFULL(dbuf));
+        __syncwarp();
+      }
+      if (*(volatile int*)&s_abort) __nanosleep(100000);     // (after a wait that ran out: let issued MMAs finish)
     }
   } else if (warp < W_MMA) {
     // ================================================================ decode groups
@@ -405,17 +565,20 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     const int row = (warp & 3) * 32 + lane;                 // row of the tile = tensor-memory lane
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const uint8_t* wring = smem + p.off_wring;
-    uint32_t n = 0;
-    for (uint32_t wk = cta; wk < n_work; wk += grid) {
-      const uint32_t u = wk / SPLIT, part = wk - u * SPLIT;
-      const uint32_t j0 = part * IPT / SPLIT, j1 = (part + 1) * IPT / SPLIT;
-      const uint32_t mbu = u / NPAIR, t0 = (u - mbu * NPAIR) * RT;
-      const uint32_t ntr = min((uint32_t)RT, NTILE - t0);
-      for (uint32_t jj = 0; jj < (j1 - j0) * ntr; ++jj, ++n) {
-        const uint32_t j = j0 + jj / ntr;          // items of the work item: (item j, row tile 0), (j, 1), ...
+    static_assert(NA == NGRP, "a decode group owns one A slot");
+    uint32_t n = 0, turn = 0;                               // items so far; items of this group so far
+    const uint32_t a = grp;
+    Ring ring, rb;
+    const uint32_t ready = rank == 0 ? B_READY(a) : cluster_addr(B_READY(a), 0);
+    WorkList wl(p, cluster, n_clusters, IPT);
+    Work w;
+    while (wl.next(w)) {
+      for (uint32_t j = w.j0; j < w.j1; ++j, ++n) {
+        const uint32_t sw = ring.slot, wphase = ring.phase, sb = rb.slot, bphase = rb.phase;
+        ring.advance(SW);
+        rb.advance(SB);
         if ((int)(n % NGRP) != grp) continue;
-        const uint32_t sw = n % SW, a = n % NA;
-        mbar_wait(B_WFULL(sw), (n / SW) & 1, &s_abort, p.status, 32u);
+        mbar_wait(B_WFULL(sw), wphase, &s_abort, p.status, 32u);
         const uint8_t* item = wring + (size_t)sw * p.wstage_bytes;
         const bool cherry = j < NCH;
         uint4 raw[BITS];
@@ -432,7 +595,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(B_WEMPTY(sw));
-        if (n >= NA) mbar_wait(B_AEMPTY(a), ((n / NA) - 1) & 1, &s_abort, p.status, 64u);
+        if (turn) mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_abort, p.status, 64u);
+        ++turn;
         tc_fence_after();
         const uint32_t ta = tmem + lane_addr + a * A_COLS;
         if (cherry) {
@@ -465,101 +629,160 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(B_AFULL(a));
+        if (lane == 0) {
+          // The group's first warp also answers for the activation tile.  (No wait by parity comes a round early: the
+          // MMAs of item n - 4 are done, so the slot's last tile, of an item n - SB <= n - 4, has landed.)
+          if ((warp & 3) == 0) mbar_wait(B_BFULL(sb), bphase, &s_abort, p.status, 16u);
+          if (rank == 0) mbar_arrive(ready);
+          else mbar_arrive_cluster(ready);
+        }
       }
     }
+    if (turn) mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_abort, p.status, 64u);
   } else {
     // ================================================================ epilogue (last four warps)
     const int quad = warp & 3;                              // the tensor-memory lanes this warp may read
     const int row = quad * 32 + lane;
     const uint32_t lane_addr = (uint32_t)(quad * 32) << 16;
+    const int etid = tid - (NGRP * 4 + 3) * 32;             // 0..127 among the epilogue threads
+    const int ewarp = etid >> 5;
+    __half* stage = reinterpret_cast<__half*>(smem + p.off_stage);      // [token][128 rows]
+    auto epi_sync = [&]() { asm volatile("bar.sync 2, 128;" ::: "memory"); };
     asm volatile("griddepcontrol.wait;" ::: "memory");
-    const int etid = tid - (NGRP * 4 + 2) * 32;             // 0..127 among the epilogue threads
     uint32_t lu = 0;
-    for (uint32_t wk = cta; wk < n_work; wk += grid, ++lu) {
-      const uint32_t u = wk / SPLIT, part = wk - u * SPLIT;
-      const uint32_t mb = u / NPAIR, t0 = (u - mb * NPAIR) * RT;
-      const uint32_t ntr = min((uint32_t)RT, NTILE - t0);
+    WorkList wl(p, cluster, n_clusters, IPT);
+    Work w;
+    for (; wl.next(w); ++lu) {
+      const uint32_t mb = w.unit / NPAIR, tile = 2 * (w.unit % NPAIR) + rank;
       const uint32_t dbuf = lu % ND;
-      mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_abort, p.status, 128u);
-      tc_fence_after();
-      const int tok0 = (int)mb * NT;
-      // 16-token chunks of this block that hold real tokens (the rest of the tile is padding)
-      const int n_chunks = min(NT / 16, (p.M - tok0 + 15) / 16);
-      auto store_row = [&](const float (&v)[16], int n_row, int c) {
-        if (n_row < p.N) {
+      const uint32_t d_lu = tmem + lane_addr + D_BASE + dbuf * NT;
+      const int tok0 = (int)(mb * NT), ntok = min((int)NT, p.M - tok0);
+      const int n0 = (int)tile * 128, nrows = min(128, p.N - n0);       // <= 0: the repeated tile of an odd pair
+      if (w.run < 0) {
+        if (p.accumulate && nrows > 0) {
+          // the old outputs into the staging area while the MMAs run
+          for (int i = etid; i < ntok * 16; i += 128) {
+            const int t = i >> 4, r8 = (i & 15) * 8;
+            if (r8 < nrows) {
+              const __half* yp = p.y + (size_t)(tok0 + t) * p.ldy + n0 + r8;
+              if (p.vec_y) {
+                *reinterpret_cast<uint4*>(stage + t * 128 + r8) = *reinterpret_cast<const uint4*>(yp);
+              } else {
 #pragma unroll
-          for (int e = 0; e < 16; ++e) {
-            const int tok = tok0 + c * 16 + e;
-            if (tok < p.M) {
-              __half* yp = p.y + (size_t)tok * p.ldy + n_row;
-              float val = v[e];
-              if (p.accumulate) val += __half2float(*yp);
-              *yp = __float2half(val);
+                for (int e = 0; e < 8; ++e) stage[t * 128 + r8 + e] = yp[e];
+              }
+            }
+          }
+          epi_sync();
+        }
+        mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_abort, p.status, 128u);
+        tc_fence_after();
+        // (NT is a multiple of 32: a 32-column step may read padding, never past the accumulator)
+#pragma unroll 1
+        for (int c = 0; c < ntok; c += 32) {
+          float v[2][16];
+          tmem_ld16(d_lu + c, v[0]);
+          tmem_ld16(d_lu + c + 16, v[1]);
+          tmem_wait_ld();
+          __half* sp = stage + c * 128 + row;
+          if (p.accumulate) {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sp[e * 128] = __float2half(v[e >> 4][e & 15] + __half2float(sp[e * 128]));
+          } else {
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sp[e * 128] = __float2half(v[e >> 4][e & 15]);
+          }
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_cluster(cluster_addr(B_DEMPTY(dbuf), 0));
+        epi_sync();
+        for (int i = etid; i < ntok * 16; i += 128) {
+          const int t = i >> 4, r8 = (i & 15) * 8;
+          if (r8 < nrows) {
+            __half* yp = p.y + (size_t)(tok0 + t) * p.ldy + n0 + r8;
+            if (p.vec_y) {
+              *reinterpret_cast<uint4*>(yp) = *reinterpret_cast<const uint4*>(stage + t * 128 + r8);
+            } else {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) yp[e] = stage[t * 128 + r8 + e];
             }
           }
         }
-      };
-      if (SPLIT == 1) {
-        for (uint32_t rt = 0; rt < ntr; ++rt) {
-          const int n_row = (int)(t0 + rt) * 128 + row;
-#pragma unroll 1
-          for (int c = 0; c < n_chunks; ++c) {
-            float v[16];
-            tmem_ld16(tmem + lane_addr + D_BASE + (dbuf * RT + rt) * NT + c * 16, v);
-            tmem_wait_ld();
-            store_row(v, n_row, c);
-          }
-        }
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(B_DEMPTY(dbuf));
+        epi_sync();
       } else {
-        // split-K: park this part's fp32 tile; the part that arrives last adds the parts in a fixed
-        // order (deterministic sums) and stores the outputs
-        float* mine = p.partial + ((size_t)(u * SPLIT + part) * RT) * 128 * NT;
-        for (uint32_t rt = 0; rt < ntr; ++rt) {
+        // a part of a unit: park the fp32 tile; the cluster that arrives last adds the parts in item order and
+        // stores the outputs
+        const size_t part_floats = (size_t)NT * 128;
+        float* mine = p.partial + ((size_t)(cluster * 2 + w.run) * 2 + rank) * part_floats;
+        mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_abort, p.status, 128u);
+        tc_fence_after();
 #pragma unroll 1
-          for (int c = 0; c < n_chunks; ++c) {
-            float v[16];
-            tmem_ld16(tmem + lane_addr + D_BASE + (dbuf * RT + rt) * NT + c * 16, v);
-            tmem_wait_ld();
-            float4* dst = reinterpret_cast<float4*>(mine + ((size_t)rt * 128 + row) * NT + c * 16);
+        for (int c = 0; c < ntok; c += 32) {
+          float v[2][16];
+          tmem_ld16(d_lu + c, v[0]);
+          tmem_ld16(d_lu + c + 16, v[1]);
+          tmem_wait_ld();
 #pragma unroll
-            for (int e = 0; e < 4; ++e) dst[e] = make_float4(v[4 * e], v[4 * e + 1], v[4 * e + 2], v[4 * e + 3]);
-          }
+          for (int e = 0; e < 32; ++e) mine[(c + e) * 128 + row] = v[e >> 4][e & 15];
         }
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(B_DEMPTY(dbuf));
+        if (lane == 0) mbar_arrive_cluster(cluster_addr(B_DEMPTY(dbuf), 0));
+        // clusters whose runs touch this unit
+        const uint32_t total = p.sk_units * IPT, i0 = w.unit * IPT;
+        const uint32_t c_first = ((i0 + 1) * p.sk_clusters - 1) / total, c_last = ((i0 + IPT) * p.sk_clusters - 1) / total;
         __threadfence();
-        asm volatile("bar.sync 2, 128;" ::: "memory");
-        if (etid == 0) s_last = (atomicAdd(p.arrived + u, 1u) == SPLIT - 1) ? 1 : 0;
-        asm volatile("bar.sync 2, 128;" ::: "memory");
-        if (s_last) {
+        epi_sync();
+        if (etid == 0) s_last = (atomicAdd(p.arrived + 2 * w.unit + rank, 1u) == c_last - c_first) ? 1 : 0;
+        epi_sync();
+        if (s_last && nrows > 0) {
           __threadfence();
-          const float* base = p.partial + ((size_t)(u * SPLIT) * RT) * 128 * NT;
-          for (uint32_t rt = 0; rt < ntr; ++rt) {
-            const int n_row = (int)(t0 + rt) * 128 + row;
-#pragma unroll 1
-            for (int c = 0; c < n_chunks; ++c) {
-              float v[16];
+          // a warp takes every fourth token, a lane four rows of it, four tokens' loads in flight; only the first
+          // cluster's run can have begun in an earlier unit (its part is then that cluster's last)
+          const uint32_t run0 = run_begin(p, c_first, total) >= i0 ? 0u : 1u;
+          const float4* parts = reinterpret_cast<const float4*>(p.partial + (size_t)(c_first * 4 + rank) * part_floats) + lane;
+          const size_t part_step = part_floats;               // one cluster's four parts, in float4
+          for (int t0 = ewarp; t0 < ntok; t0 += 16) {
+            float4 sum[4];
 #pragma unroll
-              for (int e = 0; e < 16; ++e) v[e] = 0.f;
-              for (uint32_t q = 0; q < SPLIT; ++q) {
-                const float4* src = reinterpret_cast<const float4*>(base + (((size_t)q * RT + rt) * 128 + row) * NT + c * 16);
+            for (int u = 0; u < 4; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (uint32_t c = 0; c <= c_last - c_first; ++c) {
+              const float4* src = parts + c * part_step + (c == 0 ? run0 * (part_floats / 2) : 0);
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
-                  const float4 f = __ldcg(src + e);
-                  v[4 * e] += f.x; v[4 * e + 1] += f.y; v[4 * e + 2] += f.z; v[4 * e + 3] += f.w;
+              for (int u = 0; u < 4; ++u) {
+                const int t = min(t0 + 4 * u, ntok - 1);
+                const float4 f = __ldcg(src + (size_t)t * 32);
+                sum[u].x += f.x; sum[u].y += f.y; sum[u].z += f.z; sum[u].w += f.w;
+              }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+              const int t = t0 + 4 * u;
+              const float4 s = sum[u];
+              if (t >= ntok) break;
+              if (4 * lane < nrows) {
+                __half* yp = p.y + (size_t)(tok0 + t) * p.ldy + n0 + 4 * lane;
+                float r[4] = {s.x, s.y, s.z, s.w};
+                if (p.accumulate) {
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) r[e] += __half2float(yp[e]);
+                }
+                if (p.vec_y) {
+                  const __half2 a = __floats2half2_rn(r[0], r[1]), b = __floats2half2_rn(r[2], r[3]);
+                  uint2 o;
+                  o.x = *reinterpret_cast<const uint32_t*>(&a);
+                  o.y = *reinterpret_cast<const uint32_t*>(&b);
+                  *reinterpret_cast<uint2*>(yp) = o;
+                } else {
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) yp[e] = __float2half(r[e]);
                 }
               }
-              store_row(v, n_row, c);
             }
           }
-          if (etid == 0) p.arrived[u] = 0u;          // ready for the next call
         }
-        asm volatile("bar.sync 2, 128;" ::: "memory");
+        epi_sync();
       }
     }
   }
@@ -567,9 +790,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
   // ------------------------------------------------------------------ teardown
   tc_fence_before();
   __syncthreads();
+  cluster_sync();              // no CTA leaves while the other may still signal its barriers or read its shared memory
   tc_fence_after();
   if (warp == W_MMA) {
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
   }
 }
 
@@ -581,7 +805,7 @@ PDeviceInfo pdevice_info(int dev) {
     cudaDeviceProp prop;
     if (cudaGetDeviceProperties(&prop, dev) != cudaSuccess) return PDeviceInfo();
     cache[dev].sms = prop.multiProcessorCount;
-    cache[dev].max_smem = (int)prop.sharedMemPerBlockOptin - 1024;
+    cache[dev].max_smem = (int)prop.sharedMemPerBlockOptin - 256;     // (the kernel's static variables)
     cache[dev].ok = true;
   }
   return cache[dev];
@@ -590,63 +814,63 @@ PDeviceInfo pdevice_info(int dev) {
 int palign_up(int v, int a) { return (v + a - 1) / a * a; }
 
 typedef void (*PKernelFn)(const PrefillParams);
-template <int NT, int RT>
 PKernelFn ppick(int bits, int sets) {
-  if (bits == 4) return sets == 1 ? cq_prefill_kernel<4, 1, NT, RT> : cq_prefill_kernel<4, 2, NT, RT>;
-  return sets == 1 ? cq_prefill_kernel<3, 1, NT, RT> : cq_prefill_kernel<3, 2, NT, RT>;
-}
-
-// Tile shape for a call of M rows: 0 = 128 rows x 128 tokens (two accumulator buffers), 1 = 128 x 256,
-// 2 = 256 x 128.
-int tile_shape(int M, int n_tile) {
-  (void)n_tile;
-  // measured on 4096 -> 11008, 2048 tokens: 128 x 256 tiles 938 TFLOP/s, 128 x 128 673, 256 x 128 613: the
-  // tensor-memory MMA only reaches its rate at N = 256
-  return M > 128 ? 1 : 0;
-}
-
-unsigned long long xb_block_bytes(const cq_tlayer* L, int nt) {
-  return (unsigned long long)L->n_cher * b_kstep_bytes(nt) + (unsigned long long)L->n_gran * b_gran_bytes(nt);
-}
-
-// Split-K for calls whose units do not fill the SMs (few tokens): into how many parts the items of
-// a unit are divided so that the parts fill the SMs about evenly.
-constexpr int MAX_SPLIT = 4;
-int pick_split(int n_units, int items, int sms) {
-  int best = 1;
-  if (n_units < sms) {
-    double best_t = 1.0;                                   // makespan, in whole units
-    for (int sp = 2; sp <= MAX_SPLIT; ++sp) {
-      const int waves = (n_units * sp + sms - 1) / sms;
-      const double t = (double)waves / sp + 0.04 * sp;     // + a small cost per part for the reduction
-      if (t < best_t - 1e-9) { best_t = t; best = sp; }
-    }
-  }
-  if (best > items) best = items;
-  return best < 1 ? 1 : best;
+  if (bits == 4) return sets == 1 ? cq_prefill_kernel<4, 1> : cq_prefill_kernel<4, 2>;
+  return sets == 1 ? cq_prefill_kernel<3, 1> : cq_prefill_kernel<3, 2>;
 }
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
+// the pair MMA takes N = 32 .. 256 in steps of 32; blocks of equal size, so that 300 rows are two of 160
+int token_blocks(int M) { return (M + 255) / 256; }
+int block_tokens(int M) {
+  const int nb = token_blocks(M);
+  return ((M + nb - 1) / nb + 31) & ~31;
+}
+unsigned long long xb_half_bytes(const cq_tlayer* L, int nt) {
+  return (unsigned long long)L->n_cher * b_kstep_bytes(nt) + (unsigned long long)L->n_gran * b_gran_bytes(nt);
+}
+size_t part_bytes(int nt) { return (size_t)nt * 128 * sizeof(float); }
 
-// Workspace: staged activations | fp32 partial tiles of split-K | arrival counters (one per unit).
+// Weight stages used of those that fit: a multiple of the decode groups.  Items go round the groups, so a slot then always
+// belongs to one group, which has finished the slot's last round before it waits for the next: a wait by parity that
+// comes a round early (another group's item of the slot not yet landed) would pass at once.
+constexpr int weight_stages(int fit) { return (fit > SW_MAX ? SW_MAX : fit) / NGRP * NGRP; }
+static_assert(SW_MAX % NGRP == 0 && weight_stages(5) == 4 && weight_stages(11) == 8 && weight_stages(30) == 12, "ring / group binding");
+
+// Workspace: staged activations | fp32 partial tiles (two per CTA) | arrival counters.  Covers every smaller call too.
 size_t xb_bytes_for(const cq_tlayer* L, int M) {
-  // (both tile widths stage the same bytes per token; round up to the wider one)
-  const size_t n_mblk = ((size_t)M + 255) / 256;
-  return align256(n_mblk * (size_t)xb_block_bytes(L, 256));
+  const size_t per_token = (size_t)L->n_cher * 32 + (size_t)L->n_gran * 256;
+  return align256(((size_t)M + 32 * (size_t)token_blocks(M)) * per_token);
 }
-// Split-K only happens while the units do not fill the SMs: at most 255 units of MAX_SPLIT parts.
-size_t partial_bytes_for(const cq_tlayer* L, int M) {
-  const int nt = M > 128 ? 256 : 128;
-  const size_t units = (((size_t)M + nt - 1) / nt) * (size_t)L->n_tile;
-  return units < 256 ? align256(units * MAX_SPLIT * 128 * nt * sizeof(float)) : 0;
+size_t partial_bytes_for(int M, int clusters) {
+  const int nt = M >= 256 ? 256 : (M + 31) & ~31;
+  return (size_t)clusters * 4 * part_bytes(nt);
 }
-constexpr size_t COUNTER_BYTES = 256 * sizeof(uint32_t);
+
+// Over how many clusters the `rem` units that do not fill a wave are cut, 0 = they stay whole.  In SM cycles: an item
+// takes the tensor core 4 NT, or about 365 until its weights have come from HBM; a part costs the last arriver a read
+// of its fp32 tile, about 7 NT, and a fixed 300.
+int pick_runs(uint32_t rem, uint32_t items, int nt, int clusters) {
+  const double t_item = 4.0 * nt > 365.0 ? 4.0 * nt : 365.0, t_part = 300.0 + 7.0 * nt;
+  double best = (double)items * t_item;
+  int runs = 0;
+  for (int g = (int)rem + 1; g <= clusters; ++g) {
+    const double t = std::ceil((double)rem * items / g) * t_item + ((double)g / rem + 1.0) * t_part;
+    if (t < best) { best = t; runs = g; }
+  }
+  return runs;
+}
 
 }  // namespace
 
 extern "C" size_t cq_tlayer_gemm_workspace_bytes(const cq_tlayer* L, int M) {
   if (!L || M < 1) return 0;
-  return xb_bytes_for(L, M) + partial_bytes_for(L, M) + COUNTER_BYTES;
+  int dev = 0;
+  PDeviceInfo di;
+  if (cudaGetDevice(&dev) == cudaSuccess) di = pdevice_info(dev);
+  else (void)cudaGetLastError();
+  const int clusters = (di.ok ? di.sms : 148) / 2;
+  return xb_bytes_for(L, M) + partial_bytes_for(M, clusters) + align256((size_t)clusters * 2 * sizeof(uint32_t));
 }
 
 extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* y, int ldy, int M, int accumulate,
@@ -660,20 +884,9 @@ extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* 
   if (!di.ok) return CQ_ERR_NO_DEVICE;
   cudaStream_t st = (cudaStream_t)stream;
   const uint8_t* blob = (const uint8_t*)L->blob;
-  const int shape = tile_shape(M, L->n_tile);
-  const int NT = shape == 1 ? 256 : 128, RT = shape == 2 ? 2 : 1;
-  const int n_mblk = (M + NT - 1) / NT;
-  const unsigned long long blk = xb_block_bytes(L, NT);
-
-  {
-    const long long total = (long long)M * (2 * L->n_cher + 16 * L->n_gran);
-    long long blocks = (total + 255) / 256;
-    if (blocks > 148 * 32) blocks = 148 * 32;
-    prefill_stage_x_kernel<<<(int)blocks, 256, 0, st>>>(
-        (const __half*)x, ldx, M, (const uint32_t*)(blob + L->off_osh), (const uint16_t*)(blob + L->off_cidx), L->C,
-        L->Kc, L->n_gran, L->n_cher, (uint8_t*)workspace, blk, n_mblk, NT);
-    CQ_CUDA_TRY(cudaGetLastError());
-  }
+  const int NT = block_tokens(M), n_mblk = (M + NT - 1) / NT;
+  const int clusters = di.sms / 2, n_pair = (L->n_tile + 1) / 2;
+  const uint32_t items = (uint32_t)(L->n_cher + L->n_gran);
 
   PrefillParams p;
   p.stream = blob + L->off_stream;
@@ -682,41 +895,66 @@ extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* 
   p.status = status_word;
   p.M = M; p.N = L->N; p.n_gran = L->n_gran; p.n_tile = L->n_tile; p.n_cher = L->n_cher;
   p.gran_bytes = L->gran_bytes; p.tile_bytes = L->tile_bytes; p.ldy = ldy; p.accumulate = accumulate;
-  p.n_units = (uint32_t)n_mblk * (uint32_t)((L->n_tile + RT - 1) / RT);
-  // Split-K pays for decode-sized batches only: the reduction costs about 4 us per 16-token chunk
-  // (measured: 128 tokens through 4096 -> 11008 take 61 us in three parts against 37 us unsplit, 16
-  // tokens through 4096 -> 4096 21 us in four parts against 35 us).
-  p.split = (M <= 32 && p.n_units < 256 && partial_bytes_for(L, M) > 0 && RT == 1)
-                ? pick_split((int)p.n_units, L->n_cher + L->n_gran, di.sms) : 1;
+  p.vec_y = ((uintptr_t)y & 15) == 0 && ldy % 8 == 0;
+  p.nt = NT;
+  p.n_units = (uint32_t)n_mblk * (uint32_t)n_pair;
+  const uint32_t rem = p.n_units % (uint32_t)clusters;
+  p.sk_clusters = rem ? (uint32_t)pick_runs(rem, items, NT, clusters) : 0;
+  p.sk_units = p.sk_clusters ? rem : 0;
   p.partial = (float*)((uint8_t*)workspace + xb_bytes_for(L, M));
-  p.arrived = (uint32_t*)((uint8_t*)workspace + xb_bytes_for(L, M) + partial_bytes_for(L, M));
-  if (p.split > 1) CQ_CUDA_TRY(cudaMemsetAsync(p.arrived, 0, COUNTER_BYTES, st));
-  p.xb_blk_bytes = blk;
-  p.wstage_bytes = palign_up(L->gran_bytes > CQT_CHER_BYTES ? L->gran_bytes : CQT_CHER_BYTES, 128);
-  int off = 0;
-  p.off_bar = off;   off = palign_up(off + (2 * SW + 2 * 4 + 2 * NA + 4) * 8, 128);
-  p.off_wring = off; off = palign_up(off + SW * p.wstage_bytes, 128);
-  p.off_bring = off;
-  p.sb = (di.max_smem - off) / b_gran_bytes(NT);
-  if (p.sb > 4) p.sb = 4;
-  if (p.sb < 2) return CQ_ERR_TOO_LARGE;
-  const int smem = off + p.sb * b_gran_bytes(NT);
-  int grid = di.sms;
-  if ((uint32_t)grid > p.n_units * (uint32_t)p.split) grid = (int)(p.n_units * (uint32_t)p.split);
+  p.arrived = (uint32_t*)((uint8_t*)workspace + xb_bytes_for(L, M) + partial_bytes_for(M, clusters));
+  p.xb_half_bytes = xb_half_bytes(L, NT);
+  const uint32_t used = p.n_units >= (uint32_t)clusters ? (uint32_t)clusters : (p.sk_clusters ? p.sk_clusters : p.n_units);
 
-  PKernelFn fn = shape == 1 ? ppick<256, 1>(L->bits, L->sets)
-                            : (shape == 2 ? ppick<128, 2>(L->bits, L->sets) : ppick<128, 1>(L->bits, L->sets));
-  CQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(NTHREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 2;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.stream = st;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  {
+    const int quads = (2 * L->n_cher + 16 * L->n_gran + 3) / 4, groups = (M + 7) / 8;
+    // four token groups a thread once that still fills the SMs (2048 rows of 5120: 10 us against 18), one below it
+    // (64 rows of 4096: four would add 4 us of latency to a 24 us call)
+    const int gx = (quads + STAGE_THREADS / 32 - 1) / (STAGE_THREADS / 32);
+    const bool four = (long long)gx * ((groups + 3) / 4) >= 10ll * di.sms;
+    const int gy = four ? (groups + 3) / 4 : groups;
+    cfg.gridDim = dim3(gx, gy < 65535 ? gy : 65535);
+    cfg.blockDim = dim3(STAGE_THREADS);
+    cfg.numAttrs = 1;
+    const int aligned16 = ((uintptr_t)x & 15) == 0 && ldx % 8 == 0;
+    CQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, four ? prefill_stage_x_kernel<4> : prefill_stage_x_kernel<1>, (const __half*)x, ldx, M,
+                                   (const uint32_t*)(blob + L->off_osh), (const uint16_t*)(blob + L->off_cidx), (int)L->C,
+                                   (int)L->Kc, (int)L->n_gran, (int)L->n_cher, (uint8_t*)workspace, p.xb_half_bytes, NT,
+                                   p.arrived, (int)(2 * p.sk_units), aligned16));
+  }
+
+  // shared memory: barriers, output staging tile, activation ring, and weights in what is left
+  p.wstage_bytes = palign_up(L->gran_bytes > CQT_CHER_BYTES ? L->gran_bytes : CQT_CHER_BYTES, 128);
+  int off = 0;
+  p.off_bar = off;   off = palign_up(off + N_BARS * 8, 128);
+  p.off_stage = off; off += NT * 128 * 2;
+  p.sb = (di.max_smem - off - NGRP * p.wstage_bytes) / b_gran_bytes(NT);
+  if (p.sb > NA) {
+    const int even = (di.max_smem - off) / (p.wstage_bytes + b_gran_bytes(NT));       // about as many stages of both
+    p.sb = even < NA ? NA : (even > SB_MAX ? SB_MAX : even);
+  }
+  p.off_bring = off; off += p.sb * b_gran_bytes(NT);
+  p.off_wring = off;
+  p.sw = weight_stages((di.max_smem - off) / p.wstage_bytes);
+  if (p.sb < NA || p.sw < NGRP) return CQ_ERR_TOO_LARGE;
+  const int smem = off + p.sw * p.wstage_bytes;
+
+  PKernelFn fn = ppick(L->bits, L->sets);
+  CQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  cfg.gridDim = dim3(2 * used);
+  cfg.blockDim = dim3(NTHREADS);
+  cfg.dynamicSmemBytes = smem;
+  cfg.numAttrs = 2;
   CQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, p));
   return CQ_OK;
 }

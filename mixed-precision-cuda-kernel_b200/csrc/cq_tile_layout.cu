@@ -219,6 +219,9 @@ extern "C" int cq_tlayer_prepare(const cq_tlayer* L, const uint8_t* qweight, con
     tprepare_cherry_kernel<<<tblocks((long long)d.n_tile * d.n_cher * 2048, T), T, 0, st>>>(
         d, (const __half*)cherry_weight, blob + L->off_stream);
   const int m = d.Kp / 8 > d.Cp ? d.Kp / 8 : d.Cp;
+  // The GEMM starts to copy weights while the kernel before it still runs (programmatic launch).  A memory node between
+  // the kernels that write them and anything launched later makes sure that they are complete by then.
+  CQ_CUDA_TRY(cudaMemsetAsync(blob + L->off_osh, 0, (size_t)(d.Kp / 8) * 4, st));
   tprepare_index_kernel<<<(m + T - 1) / T, T, 0, st>>>(d, cherry_indices, (uint32_t*)(blob + L->off_osh),
                                                        (uint16_t*)(blob + L->off_cidx));
   CQ_CUDA_TRY(cudaGetLastError());

@@ -139,3 +139,44 @@ def test_quant_cuda_ops_route_large_batches_to_the_gemm(qc, bits):
         qc.vecquant3matmul_cherryq(x[:8].contiguous(), t[0], t[1], t[2], t[3], out2, G, True)
     torch.cuda.synchronize()
     assert float((out2.float() - out[:8].float()).abs().max() / ref.abs().max()) <= 2e-3
+
+
+@pytest.mark.parametrize("K,N,bits,G,M", [
+    (512, 392, 3, 128, 1), (1024, 136, 4, 128, 31), (2048, 1024, 3, 64, 33), (384, 4096, 4, 128, 127), (8192, 1024, 3, 128, 257),
+    (2048, 2440, 4, 256, 513), (1024, 9600, 3, 128, 300), (256, 40, 4, 128, 2049)])
+def test_gemm_block_tile_and_run_edges(cabi, K, N, bits, G, M):
+    """Token blocks that end inside a step of 32, an odd number of row tiles (the pair's second CTA repeats one), units cut
+    into runs and whole ones in one call; twelve calls back to back on one workspace give the same bits."""
+    w, idx, pk, dense = make_case(K, N, bits, G, seed=K + M)
+    p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], bits, K, G)
+    x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).half()
+    y = gemm(cabi, p, x)
+    ref = x.float() @ dev(dense).float().T                                 # fp32 matmul of the dequantised weights
+    err = float((y.float() - ref).abs().max() / ref.abs().max())
+    assert err <= 2e-3, err                                                # as in test_gemm_llama7b_shapes
+    lib = cabi.lib()
+    ws = torch.empty(lib.cq_tlayer_gemm_workspace_bytes(C.byref(p.L), M), dtype=torch.uint8, device="cuda")
+    outs = [torch.full_like(y, float("nan")) for _ in range(12)]
+    for o in outs:
+        cabi.check(lib.cq_tlayer_gemm(C.byref(p.L), ptr(x), K, ptr(o), N, M, 0, ptr(ws), ptr(p.status), None), "gemm")
+    torch.cuda.synchronize()
+    assert int(p.status.item()) == 0
+    assert all(torch.equal(o, y) for o in outs)
+
+
+def test_gemm_accumulates_and_strides_unaligned(cabi):
+    """Outputs at a 2-byte aligned address with an odd row stride, whole units and cut ones, added to what is there."""
+    K, N, M = 1024, 264, 70
+    w, idx, pk, dense = make_case(K, N, 4, 128, seed=2)
+    p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], 4, K, 128)
+    lib = cabi.lib()
+    xb = torch.randn(M * (K + 1) + 1, device="cuda").half()
+    yb = torch.randn(M * (N + 3) + 1, device="cuda").half()
+    x, base = xb[1:].view(M, K + 1)[:, :K], yb[1:].view(M, N + 3).clone()
+    ws = torch.empty(lib.cq_tlayer_gemm_workspace_bytes(C.byref(p.L), M), dtype=torch.uint8, device="cuda")
+    cabi.check(lib.cq_tlayer_gemm(C.byref(p.L), xb.data_ptr() + 2, K + 1, yb.data_ptr() + 2, N + 3, M, 1, ptr(ws), ptr(p.status), None), "gemm")
+    torch.cuda.synchronize()
+    ref = x.float() @ dev(dense).float().T + base[:, :N].float()
+    got = yb[1:].view(M, N + 3)
+    assert float((got[:, :N].float() - ref).abs().max() / ref.abs().max()) <= 2e-3
+    assert torch.equal(got[:, N:], base[:, N:])
