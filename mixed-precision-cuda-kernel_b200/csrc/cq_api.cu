@@ -15,7 +15,7 @@
 
 #include "cq_common.cuh"
 
-int cq_launch_matvec_f32(int bits, const float* x, const uint8_t* q, const float* cw, const int32_t* idx,
+int cq_launch_matvec_f32(const float* x, const uint8_t* q, const float* cw, const int32_t* idx,
                          const float* sf, float* mul, int M, int K, int N, int C, int G, cudaStream_t st);
 
 namespace {
@@ -40,9 +40,8 @@ struct DeviceState {
   size_t gemm_ws_bytes = 0;
 };
 
-// From here on the tensor-core GEMM is used: measured on 4096 -> 11008 4-bit, 16 rows take 51 us on the
-// stream matvec (whose per-row activation staging grows with the batch) and 34 us on the GEMM with
-// split-K; at 8 rows 30 us against 33 us there, but 4096 -> 4096 and 11008 -> 4096 are well ahead on the GEMM.
+// Layers the row kernel does not take go to the tensor-core GEMM from here on: measured on 4096 -> 11008 4-bit, 8 rows
+// take 30 us on the stream matvec (whose per-row activation staging grows with the batch) and 19 us on the GEMM.
 constexpr int PREFILL_MIN_ROWS = 8;
 constexpr int PREFILL_CHUNK_ROWS = 4096;  // rows per GEMM call (bounds the workspace)
 
@@ -128,7 +127,7 @@ int legacy_matmul(int bits, const void* vec, const uint8_t* qweight, const void*
   const CacheKey key{dev, qweight, scales, cherry_weight, cherry_indices, bits, vec_height, width,
                      cherry_size, group_size, tag};
   // decode batches: the row-tile kernel (four activation rows per launch) up to the batch where the tile
-  // GEMM overtakes it (12 rows, 8 for layers split along K); layers the row kernel does not take: the stream kernel
+  // GEMM overtakes it (8 rows, 4 for layers split along K); layers the row kernel does not take: the stream kernel
   // below 8 rows
   int row_limit = PREFILL_MIN_ROWS - 1;
   {
@@ -244,7 +243,7 @@ extern "C" int cq_vecquant3matmul_cherryq(const void* vec, const uint8_t* qweigh
   if (!vec || !qweight || !scaling_factors || !mul || batch < 1) return CQ_ERR_BAD_ARG;
   const int Kc = vec_height - cherry_size;
   if (Kc <= 0 || Kc % 8 || height != Kc / 8 * 3 || width <= 0) return CQ_ERR_BAD_SHAPE;
-  return cq_launch_matvec_f32(3, (const float*)vec, qweight, (const float*)cherry_weight,
+  return cq_launch_matvec_f32((const float*)vec, qweight, (const float*)cherry_weight,
                               (const int32_t*)cherry_indices, (const float*)scaling_factors, (float*)mul,
                               batch, vec_height, width, cherry_size, group_size, (cudaStream_t)stream);
 }

@@ -85,3 +85,45 @@ def test_fake_quantised_weight(pkg, K, N, bits, G, C, dtype):
     g = torch.randn_like(lin.weight)
     got[0].backward(g)
     assert torch.equal(lin.weight.grad, g)
+
+
+@pytest.mark.parametrize("K,N,G,C,M", [(136, 4, 64, 8, 1), (256, 9, 128, 8, 3), (1160, 264, 64, 16, 8), (2048, 520, 256, 8, 9),
+                                       (4096, 256, 128, 72, 33), (256, 12, 256, 0, 17)])
+def test_fp32_operator(cabi, K, N, G, C, M):
+    """vecquant3matmul_cherryq with fp32 activations: exact integer sums, so only the fixed point of x (2^-31 of the largest
+    of its 128 columns), the conversion of a sum and a few fp32 additions round: 1e-6 of the result's norm is four times
+    that.  An infinite activation gives the same infinities and NaN as the plain sum."""
+    rng = np.random.default_rng(K + M)
+    _, idx = layer(K, 8, C, np.float32, K)
+    idx = np.sort(idx).astype(np.int32)
+    Kc = K - C
+    u = rng.integers(0, 8, size=(Kc, N))
+    q = O.pack_codes(u.astype(np.uint8), 3)
+    s = (rng.random(((Kc + G - 1) // G, N)) * 0.1).astype(np.float32)
+    cw = rng.normal(size=(C, N)).astype(np.float32)
+    x = rng.normal(size=(M, K)).astype(np.float32)
+    x[:, ::7] *= 1e-3
+    x[0] *= 1e-30        # steps of x below the smallest normal number (fp32 atomics flush sums below 2^-126: 1e-8 of these)
+    base = rng.normal(size=(M, N)).astype(np.float32) * (x.std(axis=1, keepdims=True))
+    dense = np.zeros((K, N))
+    dense[idx] = cw
+    dense[O.normal_columns(K, idx)] = (u - 3.5) * np.repeat(s, G, axis=0)[:Kc].astype(np.float64)
+
+    def run(x):
+        out = dev(base.copy())
+        t = [dev(a) for a in (x, q, cw, idx, s)]
+        cabi.check(cabi.lib().cq_vecquant3matmul_cherryq(ptr(t[0]), ptr(t[1]), ptr(t[2]), ptr(t[3]), ptr(t[4]), ptr(out), M, K,
+                                                         q.shape[0], N, C, G, 0, 0, None), "fp32 operator")
+        torch.cuda.synchronize()
+        return out.cpu().numpy().astype(np.float64)
+
+    ref = x.astype(np.float64) @ dense + base
+    y = run(x)
+    err = np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() <= 1e-6, err
+    x[M - 1, K // 2 + 1] = np.inf
+    with np.errstate(invalid="ignore"):
+        ref = x.astype(np.float64) @ dense + base
+    y = run(x)
+    assert np.array_equal(np.isinf(y), np.isinf(ref)) and np.array_equal(np.sign(y[np.isinf(y)]), np.sign(ref[np.isinf(ref)]))
+    assert np.array_equal(np.isnan(y), np.isnan(ref))
