@@ -1177,10 +1177,10 @@ extern "C" int cq_rlayer_preferred_rows(const cq_rlayer* L) {
   if (!L) return 0;
   const int gpw = rv_gpw_for(L);
   if (!gpw) return 0;
-  // measured on B200 through the drop-in ops against the tile GEMM: 8 rows (two launches) take 12 - 16 us
-  // against the GEMM's 25 - 33; 16 rows (four launches) 30 / 35 us on 4096 -> 4096 / 11008 against 25 / 32,
-  // so three launches are the limit; layers split along K (11008 -> 4096: 14 us per launch) stop at two
-  return L->ksplit > 1 ? 8 : 12;
+  // measured on B200 against the tile GEMM: 8 rows (two launches) take 14 / 19 / 52 us on 4096 -> 4096 / 4096 -> 11008 /
+  // 8192 -> 28672 against 14 / 19 / 52, 12 rows half as much again against the same; layers split along K stop at one
+  // launch: 11008 -> 4096 and 28672 -> 8192 take 15 / 40 us at 4 rows, 28 / 70 at 8, against 20 / 54
+  return L->ksplit > 1 ? 4 : 8;
 }
 
 extern "C" int cq_rlayer_matvec(const cq_rlayer* L, const void* x, void* y, int accumulate, uint32_t* status_word,

@@ -7,9 +7,9 @@ so a state dict written by the reference loads into it.  What runs underneath is
 different: pack and unpack are GPU kernels, and forward runs on re-packed copies of
 the buffers that the module owns (made on first use of the kernel family that needs
 them; `release_reference_buffers()` drops the originals afterwards):
-  one activation row    row-tile layout, the one-row decode kernel (where the layer fits it)
-  2..7 rows             stream layout, the stream matvec
-  8 rows or more        the drop-in op's tensor-core GEMM (tile layout, cached by the library)
+  decode batches        row-tile layout, the row kernel, up to RowLayer.preferred_rows rows
+  larger batches        tile layout, the tensor-core GEMM
+  layers the row kernel does not take: stream layout, the stream matvec, below 8 rows
 All of it needs a CUDA device.
 """
 import math
@@ -66,6 +66,7 @@ class QuantLinear(nn.Module):
         self._prepared = None        # stream layout (PreparedLayer)
         self._row = None             # row-tile layout (RowLayer)
         self._tile = None            # tile layout of the GEMM (TileLayer), only built after a release
+        self._fast = None            # PackedForward over the copies made so far
         self._row_ok = None          # None = not asked yet
         self._prepared_key = None
 
@@ -113,6 +114,7 @@ class QuantLinear(nn.Module):
         self._prepared = None
         self._row = None
         self._tile = None
+        self._fast = None
         self._row_ok = None
         self._prepared_key = None
 
@@ -166,6 +168,8 @@ class QuantLinear(nn.Module):
         row = self.row_layer() if (self._layerwise_dequantize and self.w_bits in (3, 4) and gate.dtype == torch.float16
                                    and rows <= ROW_KERNEL_MAX_ROWS) else None
         if row is None or rows > row.preferred_rows:
+            if gate.is_cuda and gate.dtype == up.dtype == torch.float16 and gate.shape == up.shape and gate.numel():
+                return self(load_quant_cuda().silu_mul(gate.contiguous(), up.contiguous()))
             return self(nn.functional.silu(gate.float()).to(gate.dtype) * up)
         g2 = gate.reshape(rows, gate.shape[-1]).contiguous()
         u2 = up.reshape(rows, up.shape[-1]).contiguous()
@@ -185,14 +189,33 @@ class QuantLinear(nn.Module):
         for name in ("qweight", "scales", "cherry_weight", "cherry_indices"):
             setattr(self, name, torch.empty(0, dtype=getattr(self, name).dtype, device=dev))
         self._prepared_key = "released"
+        self._fast = None
 
     def restore_reference_buffers(self):
         q, s, cw, ci = self._source_buffers()
         self.qweight, self.scales, self.cherry_weight, self.cherry_indices = q, s, cw, ci
         self._prepared_key = self._buffer_key()
+        self._fast = None
+
+    def tile_layer(self):
+        """The tile-layout copy of the tensor-core GEMM (built on first use)."""
+        self._sync_key()
+        if self._tile is None:
+            qc = load_quant_cuda()
+            self._require_cuda()
+            q, s, cw, ci = self._source_buffers()
+            self._tile = qc.TileLayer(q, s, cw, ci, self.w_bits, self.in_features, self.group_size)
+        return self._tile
+
+    def forward(self, x: torch.Tensor):
+        if self._fast is not None and self._layerwise_dequantize:
+            out = self._fast(x, self._buffers, self.bias)
+            if out is not None:
+                return out
+        return self._forward(x)
 
     @torch.inference_mode()
-    def forward(self, x: torch.Tensor):
+    def _forward(self, x: torch.Tensor):
         if self._layerwise_dequantize:
             if self.w_bits not in (3, 4):
                 raise NotImplementedError(f"{self.w_bits} bit kernel is not implemented yet.")
@@ -206,27 +229,17 @@ class QuantLinear(nn.Module):
             if row is not None and rows <= row.preferred_rows:
                 out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
                 row.matvec(x2, out, False)
-            elif rows >= 8 and self._prepared_key != "released":
-                # more rows: the drop-in op routes them to the tensor-core GEMM (faster from there on)
-                qc = load_quant_cuda()
-                out = torch.zeros(rows, self.out_features, dtype=torch.float16, device=x2.device)
-                if self.w_bits == 4:
-                    qc.vecquant4matmul_cherryq(x2, self.qweight, self.cherry_weight, self.cherry_indices,
-                                               self.scales, out, self.group_size)
-                else:
-                    qc.vecquant3matmul_cherryq(x2, self.qweight, self.cherry_weight, self.cherry_indices,
-                                               self.scales, out, self.group_size, True)
-            elif rows >= 8:
-                # released buffers and a large batch: the GEMM on this module's own tile-layout copy
-                if self._tile is None:
-                    qc = load_quant_cuda()
-                    q, s, cw, ci = self._source_buffers()
-                    self._tile = qc.TileLayer(q, s, cw, ci, self.w_bits, self.in_features, self.group_size)
+            elif rows >= 8 and self.w_bits == 4 and self.group_size < 128 and self._prepared_key != "released":
+                raise RuntimeError("4-bit layers with groups narrower than 128 have no kernel for large batches")
+            elif rows >= 8 or row is not None:
+                # more rows: the tensor-core GEMM on this module's tile-layout copy
                 out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
-                self._tile.gemm(x2, out, False)
+                self.tile_layer().gemm(x2, out, False)
             else:
                 out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
                 self.prepared().matvec(x2, out, False)
+            if self._row is not None or self._tile is not None:
+                self._fast = load_quant_cuda().PackedForward(self._row, self._tile, self._buffers, self._prepared_key == "released")
             out = out.reshape(out_shape).to(x.dtype)
         else:
             if not self.dequantized:
