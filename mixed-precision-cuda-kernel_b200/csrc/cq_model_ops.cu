@@ -76,56 +76,79 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const __half* __restrict_
 // Rotary embedding ("rotate half" convention) of q (T, H, D) and k (T, KV, D) in place at positions
 // pos[t], and the write of k, v rows into the caches (sequences, max_seq, KV, D): token t belongs to
 // sequence t / tokens_per_seq.
+// V = columns of each half a thread takes: 8 (16-byte accesses: half a multiple of 8 and aligned buffers, every model
+// width in use) or 1.  Scalar accesses and a 64-bit division per element cost the prefill more than the bytes.
+template <int V>
 __global__ void rope_cache_kernel(__half* __restrict__ q, __half* __restrict__ k, const __half* __restrict__ v,
                                   const float* __restrict__ cos_t, const float* __restrict__ sin_t,
                                   const long long* __restrict__ pos, __half* __restrict__ k_cache,
-                                  __half* __restrict__ v_cache, int T, int H, int KV, int D, int max_seq,
+                                  __half* __restrict__ v_cache, long long rows, int H, int KV, int D, int max_seq,
                                   int tokens_per_seq) {
   // programmatic dependent launch: let the next kernel start its prologue, then wait for our inputs
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int half = D / 2;
-  const long long total = (long long)T * (H + 2 * KV) * half;
-  for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < total;
-       id += (long long)gridDim.x * blockDim.x) {
-    const int i = (int)(id % half);
-    const int hh = (int)((id / half) % (H + 2 * KV));
-    const int t = (int)(id / ((long long)half * (H + 2 * KV)));
+  struct __align__(V * 2) Halves { __half h[V]; };
+  struct __align__(V == 8 ? 16 : 4) Floats { float f[V]; };
+  const int half = D / 2, heads = H + 2 * KV;
+  const int lanes = min(half / V, (int)blockDim.x), i0 = (int)threadIdx.x % lanes * V;    // blockDim.x is a multiple of lanes
+  const long long step = (long long)gridDim.x * (blockDim.x / lanes);
+  for (long long r = (long long)blockIdx.x * (blockDim.x / lanes) + threadIdx.x / lanes; r < rows; r += step) {
+    const int t = (int)(r / heads), hh = (int)(r - (long long)t * heads);
     const long long p = pos[t];
     if (p < 0 || p >= max_seq) continue;      // a position outside the tables and caches: nothing is read or written
     const size_t crow = (size_t)(t / tokens_per_seq) * max_seq + (size_t)p;     // row of the caches
     if (hh < H + KV) {
       __half* base = hh < H ? q + ((size_t)t * H + hh) * D : k + ((size_t)t * KV + (hh - H)) * D;
-      const float c = cos_t[p * half + i], s = sin_t[p * half + i];
-      const float x1 = __half2float(base[i]), x2 = __half2float(base[i + half]);
-      const __half o1 = __float2half(x1 * c - x2 * s), o2 = __float2half(x2 * c + x1 * s);
-      base[i] = o1;
-      base[i + half] = o2;
-      if (hh >= H) {
-        __half* kc = k_cache + (crow * KV + (hh - H)) * D;
-        kc[i] = o1;
-        kc[i + half] = o2;
+      for (int i = i0; i < half; i += lanes * V) {
+        Halves x1 = *reinterpret_cast<const Halves*>(base + i), x2 = *reinterpret_cast<const Halves*>(base + i + half);
+        const Floats c = *reinterpret_cast<const Floats*>(cos_t + p * half + i), s = *reinterpret_cast<const Floats*>(sin_t + p * half + i);
+#pragma unroll
+        for (int e = 0; e < V; ++e) {
+          const float a = __half2float(x1.h[e]), b = __half2float(x2.h[e]);
+          x1.h[e] = __float2half(a * c.f[e] - b * s.f[e]);
+          x2.h[e] = __float2half(b * c.f[e] + a * s.f[e]);
+        }
+        *reinterpret_cast<Halves*>(base + i) = x1;
+        *reinterpret_cast<Halves*>(base + i + half) = x2;
+        if (hh >= H) {
+          __half* kc = k_cache + (crow * KV + (hh - H)) * D;
+          *reinterpret_cast<Halves*>(kc + i) = x1;
+          *reinterpret_cast<Halves*>(kc + i + half) = x2;
+        }
       }
     } else {
       const int kvh = hh - H - KV;
       const __half* src = v + ((size_t)t * KV + kvh) * D;
       __half* vc = v_cache + (crow * KV + kvh) * D;
-      vc[i] = src[i];
-      vc[i + half] = src[i + half];
+      for (int i = i0; i < half; i += lanes * V) {
+        *reinterpret_cast<Halves*>(vc + i) = *reinterpret_cast<const Halves*>(src + i);
+        *reinterpret_cast<Halves*>(vc + i + half) = *reinterpret_cast<const Halves*>(src + i + half);
+      }
     }
   }
 }
 
+// V = values per access: 8 where the buffers are 16-byte aligned, 1 otherwise and for the tail.
+__device__ __forceinline__ __half silu_times(__half gate, __half up) {
+  const float g = __half2float(gate);
+  return __hmul(__float2half(g / (1.f + __expf(-g))), up);            // the silu result is an fp16 tensor
+}
+template <int V>
 __global__ void silu_mul_kernel(const __half* __restrict__ gate, const __half* __restrict__ up,
                                 __half* __restrict__ out, long long n) {
   // programmatic dependent launch: let the next kernel start its prologue, then wait for our inputs
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n; i += (long long)gridDim.x * blockDim.x) {
-    const float g = __half2float(gate[i]);
-    const __half act = __float2half(g / (1.f + __expf(-g)));          // silu result is an fp16 tensor
-    out[i] = __hmul(act, up[i]);
+  struct __align__(V * 2) Halves { __half h[V]; };
+  const long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+  for (long long i = id; i < n / V; i += step) {
+    Halves g = reinterpret_cast<const Halves*>(gate)[i];
+    const Halves u = reinterpret_cast<const Halves*>(up)[i];
+#pragma unroll
+    for (int e = 0; e < V; ++e) g.h[e] = silu_times(g.h[e], u.h[e]);
+    reinterpret_cast<Halves*>(out)[i] = g;
   }
+  if (id < n % V) out[n - 1 - id] = silu_times(gate[n - 1 - id], up[n - 1 - id]);
 }
 
 // Single-query attention over the KV cache (decode).  q and out are (sequences, H, D), the caches
@@ -268,6 +291,162 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const __half* 
       v += w * __ldcg(ps + 2 + tid);
     }
     out[(size_t)head * D + tid] = __float2half(v / l);
+  }
+  if (tid == 0) counters[hidx] = 0u;                                  // ready for the next launch
+}
+
+// One query head per CTA in one sweep over its positions, for the head widths in use (LPP = D / 8 lanes take a position
+// with 16-byte loads).  A step of short contexts is a chain of memory latencies; the kernel above has two of them (all
+// scores before the first value is fetched) and five barriers.  Here every group of lanes fetches the keys and values of
+// its next UF positions at once and keeps its own running maximum, sum and weighted values; the groups meet once, in
+// shared memory, the ranges of positions (blockIdx.z) as above.  The kernel above keeps the other head widths.
+constexpr int ONE_THREADS = 512;
+template <int LPP>
+__global__ void __launch_bounds__(ONE_THREADS) attn_decode_one_kernel(const __half* __restrict__ q,
+                                                                      const __half* __restrict__ k_cache,
+                                                                      const __half* __restrict__ v_cache,
+                                                                      const long long* __restrict__ pos,
+                                                                      __half* __restrict__ out, float* __restrict__ part,
+                                                                      unsigned int* __restrict__ counters, int H, int KV,
+                                                                      int max_seq, float scale) {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  constexpr int D = LPP * 8, GROUPS = ONE_THREADS / LPP, UF = 8, PARTS = ONE_THREADS / D, WPL = (GROUPS + 31) / 32;
+  __shared__ float s_m[GROUPS], s_l[GROUPS];
+  __shared__ __align__(16) float s_acc[GROUPS][D];
+  __shared__ float s_red[PARTS][D];
+  __shared__ int s_last;
+  const int head = blockIdx.x, kvh = head / (H / KV), seq = blockIdx.y, split = blockIdx.z, nsplit = gridDim.z;
+  const int tid = threadIdx.x, lane = tid & 31, grp = tid / LPP, l8 = (tid % LPP) * 8;
+  const long long pl = pos[seq];
+  const int n_all = pl < 0 ? 1 : (pl >= max_seq ? max_seq : (int)pl + 1);
+  const int chunk = (n_all + nsplit - 1) / nsplit;
+  const int pbeg = split * chunk;
+  const int n_pos = max(0, min(n_all - pbeg, chunk));
+  const size_t row = (size_t)KV * D;         // elements between consecutive positions of a cache
+  const size_t first = ((size_t)seq * max_seq + pbeg) * row + (size_t)kvh * D + l8;
+  const size_t hidx = (size_t)seq * H + head;
+  float qf[8];
+  {
+    const uint4 u = *reinterpret_cast<const uint4*>(q + hidx * D + l8);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const float2 f = __half22float2(reinterpret_cast<const __half2*>(&u)[i]);
+      qf[2 * i] = f.x;
+      qf[2 * i + 1] = f.y;
+    }
+  }
+  float m = -INFINITY, l = 0.f, acc[8] = {};
+  for (int base = 0; base < n_pos; base += GROUPS * UF) {
+    uint4 kk[UF], vv[UF];
+#pragma unroll
+    for (int u = 0; u < UF; ++u) {
+      const int p = base + u * GROUPS + grp;
+      kk[u] = vv[u] = make_uint4(0, 0, 0, 0);
+      if (p < n_pos) {
+        kk[u] = __ldg(reinterpret_cast<const uint4*>(k_cache + first + (size_t)p * row));
+        vv[u] = __ldg(reinterpret_cast<const uint4*>(v_cache + first + (size_t)p * row));
+      }
+    }
+    float s[UF], top = m;
+#pragma unroll
+    for (int u = 0; u < UF; ++u) {
+      s[u] = 0.f;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(reinterpret_cast<const __half2*>(&kk[u])[i]);
+        s[u] += qf[2 * i] * f.x + qf[2 * i + 1] * f.y;
+      }
+    }
+#pragma unroll
+    for (int o = LPP / 2; o; o >>= 1)
+#pragma unroll
+      for (int u = 0; u < UF; ++u) s[u] += __shfl_xor_sync(0xffffffffu, s[u], o);
+#pragma unroll
+    for (int u = 0; u < UF; ++u) {
+      s[u] = base + u * GROUPS + grp < n_pos ? s[u] * scale : -INFINITY;
+      top = fmaxf(top, s[u]);
+    }
+    if (top == -INFINITY) continue;           // none of this group's positions exists (or all scores are -infinity)
+    const float keep = __expf(m - top);
+    l *= keep;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) acc[i] *= keep;
+#pragma unroll
+    for (int u = 0; u < UF; ++u) {
+      const float w = __expf(s[u] - top);
+      l += w;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 f = __half22float2(reinterpret_cast<const __half2*>(&vv[u])[i]);
+        acc[2 * i] += w * f.x;
+        acc[2 * i + 1] += w * f.y;
+      }
+    }
+    m = top;
+  }
+  if (l8 == 0) { s_m[grp] = m; s_l[grp] = l; }
+  *reinterpret_cast<float4*>(&s_acc[grp][l8]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+  *reinterpret_cast<float4*>(&s_acc[grp][l8 + 4]) = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  __syncthreads();
+  // every warp: the groups' weights, one (or two) a lane
+  float w[WPL], top = -INFINITY, tot = 0.f;
+#pragma unroll
+  for (int i = 0; i < WPL; ++i) {
+    w[i] = lane + 32 * i < GROUPS ? s_m[lane + 32 * i] : -INFINITY;
+    top = fmaxf(top, w[i]);
+  }
+  for (int o = 16; o; o >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, o));
+#pragma unroll
+  for (int i = 0; i < WPL; ++i) {
+    w[i] = w[i] == -INFINITY ? 0.f : __expf(w[i] - top);
+    if (lane + 32 * i < GROUPS) tot += w[i] * s_l[lane + 32 * i];
+  }
+  for (int o = 16; o; o >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, o);
+  const int d = tid % D, prt = tid / D;       // (a warp lies inside one part: D is a multiple of 32)
+  float v = 0.f;
+#pragma unroll
+  for (int i = 0; i < WPL; ++i)
+#pragma unroll 8
+    for (int g = 0; g < (GROUPS < 32 ? GROUPS : 32); ++g) {
+      const float wg = __shfl_sync(0xffffffffu, w[i], g);
+      if (g % PARTS == prt) v += wg * s_acc[32 * i + g][d];
+    }
+  s_red[prt][d] = v;
+  __syncthreads();
+  if (tid < D) {
+    v = 0.f;
+#pragma unroll
+    for (int i = 0; i < PARTS; ++i) v += s_red[i][tid];
+    if (nsplit == 1) {
+      out[hidx * D + tid] = __float2half(v / tot);
+    } else {
+      float* mine = part + (hidx * nsplit + split) * (size_t)(D + 2);
+      mine[2 + tid] = v;
+      if (tid == 0) { mine[0] = top; mine[1] = tot; }
+    }
+  }
+  if (nsplit == 1) return;
+  // several ranges: the last CTA of this head merges
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) s_last = atomicAdd(&counters[hidx], 1u) == (unsigned int)(nsplit - 1);
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (tid < D) {
+    const float* all = part + hidx * nsplit * (size_t)(D + 2);
+    float mm = -INFINITY;
+    for (int s = 0; s < nsplit; ++s) mm = fmaxf(mm, __ldcg(all + (size_t)s * (D + 2)));
+    float lsum = 0.f, sum = 0.f;
+    for (int s = 0; s < nsplit; ++s) {
+      const float* ps = all + (size_t)s * (D + 2);
+      const float ms = __ldcg(ps);
+      const float ws = ms == -INFINITY ? 0.f : __expf(ms - mm);      // an empty range carries no weight
+      lsum += ws * __ldcg(ps + 1);
+      sum += ws * __ldcg(ps + 2 + tid);
+    }
+    out[hidx * D + tid] = __float2half(sum / lsum);
   }
   if (tid == 0) counters[hidx] = 0u;                                  // ready for the next launch
 }
@@ -513,16 +692,24 @@ extern "C" int cq_rope_cache(void* q, void* k, const void* v, const float* cos_t
   if (tokens_per_seq < 1 || T % tokens_per_seq) return CQ_ERR_BAD_ARG;
   if (!q || !k || !v || !cos_table || !sin_table || !positions || !k_cache || !v_cache) return CQ_ERR_BAD_ARG;
   if (T < 1 || n_heads < 1 || n_kv_heads < 1 || head_dim < 2 || (head_dim & 1) || max_seq < 1) return CQ_ERR_BAD_ARG;
-  const long long total = (long long)T * (n_heads + 2 * n_kv_heads) * (head_dim / 2);
-  CQ_CUDA_TRY(launch_pdl(rope_cache_kernel, dim3(blocks_for(total, 256, 148 * 8)), dim3(256), 0, (cudaStream_t)stream,
+  const long long rows = (long long)T * (n_heads + 2 * n_kv_heads);
+  const int half = head_dim / 2;
+  const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)cos_table | (uintptr_t)sin_table |
+                        (uintptr_t)k_cache | (uintptr_t)v_cache;
+  const int vec = half % 8 == 0 && (all & 15) == 0 ? 8 : 1;
+  const int lanes = half / vec < 256 ? half / vec : 256, threads = 256 / lanes * lanes;
+  auto kernel = vec == 8 ? rope_cache_kernel<8> : rope_cache_kernel<1>;
+  CQ_CUDA_TRY(launch_pdl(kernel, dim3(blocks_for(rows * lanes, threads, 148 * 8)), dim3(threads), 0, (cudaStream_t)stream,
                          (__half*)q, (__half*)k, (const __half*)v, cos_table, sin_table, positions, (__half*)k_cache,
-                         (__half*)v_cache, T, n_heads, n_kv_heads, head_dim, max_seq, tokens_per_seq));
+                         (__half*)v_cache, rows, n_heads, n_kv_heads, head_dim, max_seq, tokens_per_seq));
   return CQ_OK;
 }
 
 extern "C" int cq_silu_mul(const void* gate, const void* up, void* out, long long n, cq_stream_t stream) {
   if (!gate || !up || !out || n < 1) return CQ_ERR_BAD_ARG;
-  CQ_CUDA_TRY(launch_pdl(silu_mul_kernel, dim3(blocks_for(n, 256, 148 * 8)), dim3(256), 0, (cudaStream_t)stream,
+  const int vec = (((uintptr_t)gate | (uintptr_t)up | (uintptr_t)out) & 15) == 0 ? 8 : 1;
+  auto kernel = vec == 8 ? silu_mul_kernel<8> : silu_mul_kernel<1>;
+  CQ_CUDA_TRY(launch_pdl(kernel, dim3(blocks_for((n + vec - 1) / vec, 256, 148 * 8)), dim3(256), 0, (cudaStream_t)stream,
                          (const __half*)gate, (const __half*)up, (__half*)out, n));
   return CQ_OK;
 }
@@ -560,19 +747,21 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
   unsigned int* counters = (unsigned int*)workspace;
   float* part = (float*)((uint8_t*)workspace + (heads * sizeof(unsigned int) + 255) / 256 * 256);
   const int G = n_heads / n_kv_heads;
+  const bool wide = (head_dim == 64 || head_dim == 128 || head_dim == 256) &&
+                    (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
   // One CTA per KV head reads every cache row once for the query heads that share it; with several query heads
   // per KV head its per-position arithmetic is G times larger, which only pays on long caches (measured, 70B
-  // shapes: 103 us against 174 at 4000 positions, but 21 against 15 at 200): short grouped-query caches keep
-  // the per-head kernel, whose re-reads hit L2.
-  if ((head_dim == 64 || head_dim == 128 || head_dim == 256) && G <= 8 && (G == 1 || max_seq > 1024)) {
+  // shapes: 103 us against 174 at 4000 positions, but 21 against 15 at 200): short grouped-query caches take
+  // a CTA per query head, whose re-reads hit L2.
+  if (wide && G > 1 && G <= 8 && max_seq > 1024) {
     const int splits = attn_splits(sequences, n_kv_heads, max_seq);
     const int range = (max_seq + splits - 1) / splits;
-    const int gt = G <= 1 ? 1 : (G <= 2 ? 2 : (G <= 4 ? 4 : 8));
+    const int gt = G <= 2 ? 2 : (G <= 4 ? 4 : 8);
     const int words = gt * range > GQA_WARPS * gt * head_dim ? gt * range : GQA_WARPS * gt * head_dim;
     const int smem = words * (int)sizeof(float);
     if (smem > 200 * 1024) return CQ_ERR_TOO_LARGE;
     void (*fn)(const __half*, const __half*, const __half*, const long long*, __half*, float*, unsigned int*, int, int, int, int, float) =
-        gt == 1 ? attn_decode_gqa_kernel<1> : (gt == 2 ? attn_decode_gqa_kernel<2> : (gt == 4 ? attn_decode_gqa_kernel<4> : attn_decode_gqa_kernel<8>));
+        gt == 2 ? attn_decode_gqa_kernel<2> : (gt == 4 ? attn_decode_gqa_kernel<4> : attn_decode_gqa_kernel<8>);
     if (smem > 48 * 1024) CQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     CQ_CUDA_TRY(launch_pdl(fn, dim3(n_kv_heads, sequences, splits), dim3(GQA_THREADS), (size_t)smem, (cudaStream_t)stream,
                            (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, position, (__half*)out, part,
@@ -580,6 +769,13 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
     return CQ_OK;
   }
   const int splits = attn_splits(sequences, n_heads, max_seq);
+  if (wide) {
+    auto fn = head_dim == 64 ? attn_decode_one_kernel<8> : (head_dim == 128 ? attn_decode_one_kernel<16> : attn_decode_one_kernel<32>);
+    CQ_CUDA_TRY(launch_pdl(fn, dim3(n_heads, sequences, splits), dim3(ONE_THREADS), 0, (cudaStream_t)stream, (const __half*)q,
+                           (const __half*)k_cache, (const __half*)v_cache, position, (__half*)out, part, counters, n_heads,
+                           n_kv_heads, max_seq, scale));
+    return CQ_OK;
+  }
   const int range = (max_seq + splits - 1) / splits;
   const int smem = (range + ATT_THREADS) * (int)sizeof(float);
   if (smem > 200 * 1024) return CQ_ERR_TOO_LARGE;

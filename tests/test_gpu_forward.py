@@ -1,0 +1,87 @@
+"""QuantLinear.forward's native path (PackedForward): the same answers as the general path, and the general path again
+whenever the module's buffers are no longer those its copies were made from.  Decode attention at the edges of its sweep."""
+import math
+from types import SimpleNamespace
+
+import pytest
+
+torch = pytest.importorskip("torch")
+pytestmark = pytest.mark.gpu
+
+
+def packed(K, N, bits, G, seed, bias=False):
+    from cherryq_b200 import QuantLinear
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    C = math.ceil(K / 64) // 8 * 8
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.02).half()
+    idx = torch.randperm(K, device="cuda", generator=g)[:C].int()
+    b = torch.randn(N, device="cuda", generator=g).half() if bias else None
+    lin = QuantLinear(bits, G, None, 1 / 64, K, N, bias=bias).cuda()
+    lin.pack(SimpleNamespace(weight=w, bias=b, cherry_indices=idx, group_size=G))
+    return lin
+
+
+def check(lin, x, dense, bias=None):
+    ref = x.float() @ dense.float().T + (bias.float() if bias is not None else 0)
+    y = lin(x)
+    assert y.dtype == x.dtype and y.shape == x.shape[:-1] + (dense.shape[0],)
+    assert float((y.float() - ref).abs().max() / ref.abs().max()) <= 2e-3         # fp16 output, as in the parity tests
+
+
+@pytest.mark.parametrize("bits,bias", [(4, False), (3, True)])
+def test_forward_follows_the_buffers(bits, bias):
+    lin = packed(1024, 264, bits, 128, 1, bias)
+    dense = lin.unpack()
+    for shape in ((1024,), (1, 1024), (2, 3, 1024), (9, 1024), (40, 1024), (300, 1024)):
+        x = torch.randn(shape, device="cuda").half()
+        for _ in range(2):                                     # general path, then the native one
+            check(lin, x, dense, lin.bias)
+    assert lin._fast is not None
+    x = torch.randn(2, 40, 1024, device="cuda").half()
+    check(lin, x.transpose(0, 1), dense, lin.bias)             # not contiguous
+    check(lin, x.float(), dense, lin.bias)                     # another type
+    with pytest.raises(RuntimeError):
+        lin(torch.randn(3, 1016, device="cuda").half())
+    other = packed(1024, 264, bits, 128, 2, bias)
+    for name in ("qweight", "scales", "cherry_weight", "cherry_indices"):
+        setattr(lin, name, getattr(lin, name).clone())         # replaced, with tensors that keep a version
+    check(lin, torch.randn(40, 1024, device="cuda").half(), dense, lin.bias)
+    for name in ("qweight", "scales", "cherry_weight", "cherry_indices"):
+        getattr(lin, name).copy_(getattr(other, name))         # written in place
+    for m in (3, 40):
+        check(lin, torch.randn(m, 1024, device="cuda").half(), other.unpack(), lin.bias)
+    third = packed(1024, 264, bits, 128, 3, bias)
+    lin.load_state_dict(third.state_dict())
+    dense = third.unpack()
+    for m in (3, 40):
+        check(lin, torch.randn(m, 1024, device="cuda").half(), dense, lin.bias)
+    lin.release_reference_buffers()
+    for m in (3, 40, 3, 40):
+        check(lin, torch.randn(m, 1024, device="cuda").half(), dense, lin.bias)
+    lin.restore_reference_buffers()
+    for m in (3, 40):
+        check(lin, torch.randn(m, 1024, device="cuda").half(), dense, lin.bias)
+    y = lin(torch.randn(3, 1024, device="cuda").half().requires_grad_())
+    assert not y.requires_grad
+
+
+@pytest.mark.parametrize("D", [64, 128, 256])
+@pytest.mark.parametrize("H,KV,max_seq,at", [(4, 4, 2300, (0, 255, 256, 2299)), (8, 2, 600, (1, 511, 512, 599)), (3, 3, 40, (0, 7, 38, 39))])
+def test_attention_sweep_edges(D, H, KV, max_seq, at):
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    g = torch.Generator(device="cuda").manual_seed(D + H)
+    B = len(at)
+    q = torch.randn(B, H, D, device="cuda", generator=g).half()
+    k, v = (torch.randn(B, max_seq, KV, D, device="cuda", generator=g).half() for _ in range(2))
+    for b, p in enumerate(at):                                 # nothing past the position takes part
+        k[b, p + 1:] = float("nan")
+        v[b, p + 1:] = float("nan")
+    pos = torch.tensor(at, device="cuda")
+    out = qc.attn_decode(q, k, v, pos).view(B, H, D)
+    for b, p in enumerate(at):
+        kk = k[b, :p + 1].float().repeat_interleave(H // KV, dim=1)
+        vv = v[b, :p + 1].float().repeat_interleave(H // KV, dim=1)
+        s = torch.einsum("hd,phd->hp", q[b].float(), kk) / math.sqrt(D)
+        ref = torch.einsum("hp,phd->hd", s.softmax(-1), vv)
+        assert float((out[b].float() - ref).abs().max()) <= 4e-3     # fp16 output of values near 1, fast exponentials
