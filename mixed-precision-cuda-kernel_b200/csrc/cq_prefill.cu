@@ -36,8 +36,8 @@
 //               16-byte stores to y
 // Every wait is bounded and reports into the status word instead of hanging.
 //
-// Bound and state: 4096 -> 11008 4-bit, 2048 rows: 144 us = 1.28 PFLOP/s (739 us through QuantLinear and 195 us by itself
-// with lone CTAs of 128 x 256 tiles); 8192 -> 28672 3-bit, 2048 rows: 657 us = 1.46 PFLOP/s, tensor-bound.  16 rows: 18 and
+// Bound and state: 4096 -> 11008 4-bit, 2048 rows: 140 us = 1.32 PFLOP/s (739 us through QuantLinear and 195 us by itself
+// with lone CTAs of 128 x 256 tiles); 8192 -> 28672 3-bit, 2048 rows: 641 us = 1.50 PFLOP/s, tensor-bound.  16 rows: 18 and
 // 52 us (31 and 76): an item then takes about 740 cycles, the eight MMAs' reads of A from tensor memory and their issue,
 // against 365 that its weights need to arrive from HBM.
 #include <cmath>
@@ -747,13 +747,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
             float4 sum[4];
 #pragma unroll
             for (int u = 0; u < 4; ++u) sum[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-            for (uint32_t c = 0; c <= c_last - c_first; ++c) {
+            for (uint32_t c = 0; c <= c_last - c_first; c += 2) {
+              const bool two = c < c_last - c_first;
               const float4* src = parts + c * part_step + (c == 0 ? run0 * (part_floats / 2) : 0);
+              const float4* src2 = parts + (c + 1) * part_step;
+              float4 f[4], g[4];                            // two parts of four tokens in flight
 #pragma unroll
               for (int u = 0; u < 4; ++u) {
-                const int t = min(t0 + 4 * u, ntok - 1);
-                const float4 f = __ldcg(src + (size_t)t * 32);
-                sum[u].x += f.x; sum[u].y += f.y; sum[u].z += f.z; sum[u].w += f.w;
+                const size_t at = (size_t)min(t0 + 4 * u, ntok - 1) * 32;
+                f[u] = __ldcg(src + at);
+                g[u] = two ? __ldcg(src2 + at) : make_float4(0.f, 0.f, 0.f, 0.f);
+              }
+#pragma unroll
+              for (int u = 0; u < 4; ++u) {
+                sum[u].x += f[u].x; sum[u].y += f[u].y; sum[u].z += f[u].z; sum[u].w += f[u].w;
+                sum[u].x += g[u].x; sum[u].y += g[u].y; sum[u].z += g[u].z; sum[u].w += g[u].w;
               }
             }
 #pragma unroll
@@ -847,11 +855,11 @@ size_t partial_bytes_for(int M, int clusters) {
   return (size_t)clusters * 4 * part_bytes(nt);
 }
 
-// Over how many clusters the `rem` units that do not fill a wave are cut, 0 = they stay whole.  In SM cycles: an item
-// takes the tensor core 4 NT, or about 365 until its weights have come from HBM; a part costs the last arriver a read
-// of its fp32 tile, about 7 NT, and a fixed 300.
+// Over how many clusters the `rem` units that do not fill a wave are cut, 0 = they stay whole.  In SM cycles, as measured:
+// an item takes 4.5 NT, at least 740; a part costs about 20 NT and a fixed 500 (its fp32 tile is parked, and the last
+// arriver reads it in steps of four tokens a warp, each a trip to L2).
 int pick_runs(uint32_t rem, uint32_t items, int nt, int clusters) {
-  const double t_item = 4.0 * nt > 365.0 ? 4.0 * nt : 365.0, t_part = 300.0 + 7.0 * nt;
+  const double t_item = 4.5 * nt > 740.0 ? 4.5 * nt : 740.0, t_part = 500.0 + 20.0 * nt;
   double best = (double)items * t_item;
   int runs = 0;
   for (int g = (int)rem + 1; g <= clusters; ++g) {
