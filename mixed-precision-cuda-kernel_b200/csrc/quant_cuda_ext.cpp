@@ -462,18 +462,44 @@ struct TileLayer {
   }
 };
 
+// What a module's re-packed copies were made from: its four reference buffers, each by storage, address and version.
+// The address alone does not identify a buffer (the allocator hands a freed block to the next tensor of that size, whose
+// version is 0 again); the weak references keep the storages' records, so a recorded one is never taken for another.
+struct BufferGuard {
+  std::vector<c10::weak_intrusive_ptr<c10::StorageImpl>> storage;   // four entries
+  std::array<const void*, 4> ptr{};
+  std::array<uint64_t, 4> version{};
+
+  // (tensors made under torch.inference_mode keep no version counter)
+  static uint64_t version_of(const torch::Tensor& t) { return t.is_inference() ? 0u : (uint64_t)t._version(); }
+
+  BufferGuard(torch::Tensor q, torch::Tensor s, torch::Tensor cw, torch::Tensor ci) {
+    const torch::Tensor* t[4] = {&q, &s, &cw, &ci};
+    for (int i = 0; i < 4; ++i) {
+      storage.push_back(t[i]->storage().getWeakStorageImpl());
+      ptr[i] = t[i]->const_data_ptr();
+      version[i] = version_of(*t[i]);
+    }
+  }
+  bool same(int i, const torch::Tensor& t) const {
+    return t.has_storage() && t.storage().unsafeGetStorageImpl() == storage[i]._unsafe_get_target() &&
+           t.const_data_ptr() == ptr[i] && version_of(t) == version[i];
+  }
+  bool holds(const torch::Tensor& q, const torch::Tensor& s, const torch::Tensor& cw, const torch::Tensor& ci) const {
+    return same(0, q) && same(1, s) && same(2, cw) && same(3, ci);
+  }
+};
+
 // QuantLinear.forward for a layer whose re-packed copies exist: checks that the module's reference buffers are still the
 // ones the copies were made from, allocates the output and launches.  In Python these steps (four buffer look-ups, their
 // addresses and versions, shapes, output, two calls) took 9 us of a 17 us call whose kernel runs for 4.
 struct PackedForward {
-  py::object row_ref, tile_ref;                // keep the copies alive
+  py::object row_ref, tile_ref, guard_ref;     // keep the copies and the record of their buffers alive
   RowLayer* row = nullptr;
   TileLayer* tile = nullptr;
-  bool released;
+  const BufferGuard* guard = nullptr;          // null: the buffers were released and nothing is compared
   int64_t K, N, row_rows = 0;
   c10::Device device;
-  std::array<const void*, 4> ptr{};
-  std::array<uint64_t, 4> version{};
 
   static const std::array<PyObject*, 4>& names() {
     static const std::array<PyObject*, 4> n = {
@@ -485,24 +511,17 @@ struct PackedForward {
     PyObject* o = PyDict_GetItem(buffers.ptr(), names()[i]);
     return o && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
   }
-  static uint64_t version_of(const torch::Tensor& t) { return t.is_inference() ? 0u : (uint64_t)t._version(); }
 
-  // the copies belong to the buffers as they are now (released: the buffers are gone and nothing is compared)
-  PackedForward(py::object row_layer, py::object tile_layer, const py::dict& buffers, bool released_)
-      : row_ref(std::move(row_layer)), tile_ref(std::move(tile_layer)), released(released_), device(c10::kCPU) {
+  PackedForward(py::object row_layer, py::object tile_layer, py::object buffer_guard)
+      : row_ref(std::move(row_layer)), tile_ref(std::move(tile_layer)), guard_ref(std::move(buffer_guard)), device(c10::kCPU) {
     if (!row_ref.is_none()) row = row_ref.cast<RowLayer*>();
     if (!tile_ref.is_none()) tile = tile_ref.cast<TileLayer*>();
+    if (!guard_ref.is_none()) guard = guard_ref.cast<const BufferGuard*>();
     TORCH_CHECK(row || tile, "a layer without copies");
     K = row ? row->layer.K : tile->layer.K;
     N = row ? row->layer.N : tile->layer.N;
     device = (row ? row->blob : tile->blob).device();
     if (row) row_rows = cq_rlayer_preferred_rows(&row->layer);
-    for (int i = 0; i < 4 && !released; ++i) {
-      const torch::Tensor* t = buffer(buffers, i);
-      TORCH_CHECK(t, "a reference buffer is missing");
-      ptr[i] = t->data_ptr();
-      version[i] = version_of(*t);
-    }
   }
 
   // None: this call takes the general path
@@ -514,11 +533,11 @@ struct PackedForward {
     const int64_t M = x.numel() / K;
     const bool by_row = row && M <= row_rows;
     if (!by_row && !tile) return c10::nullopt;
-    for (int i = 0; i < 4 && !released; ++i) {
+    for (int i = 0; i < 4 && guard; ++i) {
       const torch::Tensor* t = buffer(buffers, i);
-      if (!t || !t->has_storage() || t->data_ptr() != ptr[i] || version_of(*t) != version[i]) return c10::nullopt;
+      if (!t || !guard->same(i, *t)) return c10::nullopt;
     }
-    c10::InferenceMode guard(true);            // as the decorated Python path
+    c10::InferenceMode inference(true);        // as the decorated Python path
     auto shape = x.sizes().vec();
     shape.back() = N;
     auto out = at::empty(shape, x.options());
@@ -721,8 +740,11 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int, int, int>())
       .def("gemm", &TileLayer::gemm)
       .def_readonly("blob", &TileLayer::blob);
+  py::class_<BufferGuard>(m, "BufferGuard")
+      .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>())
+      .def("holds", &BufferGuard::holds);
   py::class_<PackedForward>(m, "PackedForward")
-      .def(py::init<py::object, py::object, const py::dict&, bool>())
+      .def(py::init<py::object, py::object, py::object>())
       .def("__call__", &PackedForward::forward);
   py::class_<PreparedLayer>(m, "PreparedLayer")
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int, int, int>())

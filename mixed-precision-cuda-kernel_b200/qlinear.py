@@ -65,10 +65,10 @@ class QuantLinear(nn.Module):
         self.dequantized = False
         self._prepared = None        # stream layout (PreparedLayer)
         self._row = None             # row-tile layout (RowLayer)
-        self._tile = None            # tile layout of the GEMM (TileLayer), only built after a release
+        self._tile = None            # tile layout of the GEMM (TileLayer)
         self._fast = None            # PackedForward over the copies made so far
         self._row_ok = None          # None = not asked yet
-        self._prepared_key = None
+        self._prepared_key = None    # BufferGuard of the buffers the copies were made from, or "released"
 
     # ------------------------------------------------------------------ pack / unpack
     @torch.inference_mode()
@@ -105,10 +105,8 @@ class QuantLinear(nn.Module):
             raise RuntimeError("QuantLinear buffers must be on a CUDA device (there is no CPU path)")
 
     def _buffer_key(self):
-        def ver(t):   # tensors made under torch.inference_mode keep no version counter
-            return 0 if t.is_inference() else t._version
-        bufs = (self.qweight, self.scales, self.cherry_weight, self.cherry_indices)
-        return tuple(t.data_ptr() for t in bufs) + tuple(ver(t) for t in bufs)
+        """The record of the reference buffers as they are now (storages, addresses, versions)."""
+        return load_quant_cuda().BufferGuard(self.qweight, self.scales, self.cherry_weight, self.cherry_indices)
 
     def _drop_copies(self):
         self._prepared = None
@@ -122,10 +120,10 @@ class QuantLinear(nn.Module):
         """Forgets the re-packed copies when the reference buffers were replaced or written to."""
         if self._prepared_key == "released":
             return
-        key = self._buffer_key()
-        if self._prepared_key != key:
+        bufs = (self.qweight, self.scales, self.cherry_weight, self.cherry_indices)
+        if self._prepared_key is None or not self._prepared_key.holds(*bufs):
             self._drop_copies()
-            self._prepared_key = key
+            self._prepared_key = self._buffer_key()
 
     def _source_buffers(self):
         """The four reference buffers: the module's own, or rebuilt from a copy after a release."""
@@ -239,7 +237,8 @@ class QuantLinear(nn.Module):
                 out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
                 self.prepared().matvec(x2, out, False)
             if self._row is not None or self._tile is not None:
-                self._fast = load_quant_cuda().PackedForward(self._row, self._tile, self._buffers, self._prepared_key == "released")
+                guard = None if self._prepared_key == "released" else self._prepared_key
+                self._fast = load_quant_cuda().PackedForward(self._row, self._tile, guard)
             out = out.reshape(out_shape).to(x.dtype)
         else:
             if not self.dequantized:

@@ -122,3 +122,26 @@ def test_released_layer_serves_every_batch_size_from_its_own_copies():
     lin.restore_reference_buffers()
     for got, want in zip((lin.qweight, lin.scales, lin.cherry_weight, lin.cherry_indices), bufs):
         assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("rows", [1, 40])                # the row kernel, the tensor-core GEMM
+def test_quantlinear_buffers_replaced_at_the_same_addresses(qc, rows):
+    """Another checkpoint in the blocks the first one's buffers left, versions 0 as theirs were."""
+    from cherryq_b200.qlinear import QuantLinear
+    names = ("qweight", "scales", "cherry_weight", "cherry_indices")
+    x = torch.randn(rows, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).half()
+    lin = QuantLinear(BITS, G, None, 1 / 64, K, N, bias=False).cuda()
+    at = []
+    for seed in (600, 601):
+        host = [t.cpu() for t in make_layer(qc, seed)]
+        for name in names:
+            setattr(lin, name, None)
+        for name, t in zip(names, host):
+            setattr(lin, name, t.cuda())
+        at.append([getattr(lin, name).data_ptr() for name in names])
+        ref = x.cpu().numpy().astype(np.float64) @ dense(host).T
+        for _ in range(2):
+            y = lin(x).cpu().numpy().astype(np.float64)
+            assert np.abs(y - ref).max() <= 2e-3 * np.abs(ref).max()
+    if at[0] != at[1]:
+        pytest.skip("the allocator did not hand the freed blocks back")
