@@ -317,11 +317,14 @@ struct RowLayer {
   cq_rlayer layer;
   torch::Tensor blob;
 
-  // CQ_OK if the one-row kernel can run such a layer on the current device
-  static bool supported(int bits, int in_features, int out_features, int num_cherries, int group_size) {
+  // rows up to which such a layer takes the row kernel on the current device; 0 = the kernel does not take it
+  static int row_limit(int bits, int in_features, int out_features, int num_cherries, int group_size) {
     cq_rlayer L;
-    if (cq_rlayer_init(&L, bits, in_features, out_features, num_cherries, group_size, nullptr) != CQ_OK) return false;
-    return cq_rlayer_check(&L) == CQ_OK;
+    if (cq_rlayer_init(&L, bits, in_features, out_features, num_cherries, group_size, nullptr) != CQ_OK) return 0;
+    return cq_rlayer_check(&L) == CQ_OK ? cq_rlayer_preferred_rows(&L) : 0;
+  }
+  static bool supported(int bits, int in_features, int out_features, int num_cherries, int group_size) {
+    return row_limit(bits, in_features, out_features, num_cherries, group_size) > 0;
   }
 
   RowLayer(torch::Tensor qweight, torch::Tensor scales, torch::Tensor cherry_weight, torch::Tensor cherry_indices,
@@ -498,7 +501,8 @@ struct PackedForward {
   RowLayer* row = nullptr;
   TileLayer* tile = nullptr;
   const BufferGuard* guard = nullptr;          // null: the buffers were released and nothing is compared
-  int64_t K, N, row_rows = 0;
+  int64_t K, N;
+  int64_t row_rows, gemm_rows;                 // the row kernel takes 1 .. row_rows rows, the GEMM gemm_rows and more
   c10::Device device;
 
   static const std::array<PyObject*, 4>& names() {
@@ -512,8 +516,10 @@ struct PackedForward {
     return o && THPVariable_Check(o) ? &THPVariable_Unpack(o) : nullptr;
   }
 
-  PackedForward(py::object row_layer, py::object tile_layer, py::object buffer_guard)
-      : row_ref(std::move(row_layer)), tile_ref(std::move(tile_layer)), guard_ref(std::move(buffer_guard)), device(c10::kCPU) {
+  // The ranges are the layer's, whichever copies exist: a call whose kernel has no copy yet is left to the general path.
+  PackedForward(py::object row_layer, py::object tile_layer, py::object buffer_guard, int64_t row_rows_, int64_t gemm_rows_)
+      : row_ref(std::move(row_layer)), tile_ref(std::move(tile_layer)), guard_ref(std::move(buffer_guard)),
+        row_rows(row_rows_), gemm_rows(gemm_rows_), device(c10::kCPU) {
     if (!row_ref.is_none()) row = row_ref.cast<RowLayer*>();
     if (!tile_ref.is_none()) tile = tile_ref.cast<TileLayer*>();
     if (!guard_ref.is_none()) guard = guard_ref.cast<const BufferGuard*>();
@@ -521,7 +527,6 @@ struct PackedForward {
     K = row ? row->layer.K : tile->layer.K;
     N = row ? row->layer.N : tile->layer.N;
     device = (row ? row->blob : tile->blob).device();
-    if (row) row_rows = cq_rlayer_preferred_rows(&row->layer);
   }
 
   // None: this call takes the general path
@@ -531,8 +536,8 @@ struct PackedForward {
         c10::impl::TorchDispatchModeTLS::any_modes_set())
       return c10::nullopt;
     const int64_t M = x.numel() / K;
-    const bool by_row = row && M <= row_rows;
-    if (!by_row && !tile) return c10::nullopt;
+    const bool by_row = M <= row_rows;
+    if (by_row ? !row : (!tile || M < gemm_rows)) return c10::nullopt;
     for (int i = 0; i < 4 && guard; ++i) {
       const torch::Tensor* t = buffer(buffers, i);
       if (!t || !guard->same(i, *t)) return c10::nullopt;
@@ -728,6 +733,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   py::class_<RowLayer>(m, "RowLayer")
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int, int, int>())
       .def_static("supported", &RowLayer::supported)
+      .def_static("row_limit", &RowLayer::row_limit)
       .def("matvec", &RowLayer::matvec)
       .def("matvec_gather", &RowLayer::matvec_gather)
       .def("matvec_swiglu", &RowLayer::matvec_swiglu)
@@ -744,7 +750,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>())
       .def("holds", &BufferGuard::holds);
   py::class_<PackedForward>(m, "PackedForward")
-      .def(py::init<py::object, py::object, py::object>())
+      .def(py::init<py::object, py::object, py::object, int64_t, int64_t>())
       .def("__call__", &PackedForward::forward);
   py::class_<PreparedLayer>(m, "PreparedLayer")
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int, int, int>())

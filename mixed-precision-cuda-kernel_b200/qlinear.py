@@ -7,9 +7,10 @@ so a state dict written by the reference loads into it.  What runs underneath is
 different: pack and unpack are GPU kernels, and forward runs on re-packed copies of
 the buffers that the module owns (made on first use of the kernel family that needs
 them; `release_reference_buffers()` drops the originals afterwards):
-  decode batches        row-tile layout, the row kernel, up to RowLayer.preferred_rows rows
+  decode batches        row-tile layout, the row kernel, up to RowLayer.row_limit rows
   larger batches        tile layout, the tensor-core GEMM
   layers the row kernel does not take: stream layout, the stream matvec, below 8 rows
+The kernel of a call depends on the layer and the number of rows only, never on the calls before it.
 All of it needs a CUDA device.
 """
 import math
@@ -21,10 +22,7 @@ import torch.nn as nn
 from . import load_quant_cuda
 
 
-# No batch beyond this many rows goes to the row-tile decode kernel (four rows per launch, each launch
-# reads the weights once); a layer's own limit (RowLayer.preferred_rows) may be lower.  Larger batches
-# take the tensor-core GEMM.
-ROW_KERNEL_MAX_ROWS = 16
+GEMM_MIN_ROWS = 8       # layers the row kernel does not take: the stream matvec below, the tensor-core GEMM from here on
 
 
 class QuantLinear(nn.Module):
@@ -67,7 +65,7 @@ class QuantLinear(nn.Module):
         self._row = None             # row-tile layout (RowLayer)
         self._tile = None            # tile layout of the GEMM (TileLayer)
         self._fast = None            # PackedForward over the copies made so far
-        self._row_ok = None          # None = not asked yet
+        self._row_rows = None        # rows the row kernel serves, 0 = none, None = not asked yet
         self._prepared_key = None    # BufferGuard of the buffers the copies were made from, or "released"
 
     # ------------------------------------------------------------------ pack / unpack
@@ -113,7 +111,7 @@ class QuantLinear(nn.Module):
         self._row = None
         self._tile = None
         self._fast = None
-        self._row_ok = None
+        self._row_rows = None
         self._prepared_key = None
 
     def _sync_key(self):
@@ -142,18 +140,23 @@ class QuantLinear(nn.Module):
             self._prepared = qc.PreparedLayer(q, s, cw, ci, self.w_bits, self.in_features, self.group_size)
         return self._prepared
 
-    def row_layer(self):
-        """The row-tile copy for the one-row decode kernel, or None where the layer does not fit it."""
+    def _row_limit(self):
+        """Rows up to which the row kernel serves this layer, 0 where it does not take it."""
         self._sync_key()
-        if self._row_ok is None:
+        if self._row_rows is None:
             qc = load_quant_cuda()
             self._require_cuda()
-            self._row_ok = qc.RowLayer.supported(self.w_bits, self.in_features, self.out_features,
-                                                 self.num_cherries, self.group_size)
-        if self._row_ok and self._row is None:
+            self._row_rows = qc.RowLayer.row_limit(self.w_bits, self.in_features, self.out_features, self.num_cherries,
+                                                   self.group_size)
+        return self._row_rows
+
+    def row_layer(self):
+        """The row-tile copy for the decode kernel, or None where the layer does not fit it."""
+        if self._row_limit() and self._row is None:
             qc = load_quant_cuda()
             q, s, cw, ci = self._source_buffers()
             self._row = qc.RowLayer(q, s, cw, ci, self.w_bits, self.in_features, self.group_size)
+            self._fast = None
         return self._row
 
     @torch.inference_mode()
@@ -164,8 +167,8 @@ class QuantLinear(nn.Module):
         result equals forward(silu(gate) * up) bit for bit; other cases compute the product first."""
         rows = gate.numel() // gate.shape[-1]
         row = self.row_layer() if (self._layerwise_dequantize and self.w_bits in (3, 4) and gate.dtype == torch.float16
-                                   and rows <= ROW_KERNEL_MAX_ROWS) else None
-        if row is None or rows > row.preferred_rows:
+                                   and rows <= self._row_limit()) else None
+        if row is None:
             if gate.is_cuda and gate.dtype == up.dtype == torch.float16 and gate.shape == up.shape and gate.numel():
                 return self(load_quant_cuda().silu_mul(gate.contiguous(), up.contiguous()))
             return self(nn.functional.silu(gate.float()).to(gate.dtype) * up)
@@ -203,6 +206,7 @@ class QuantLinear(nn.Module):
             self._require_cuda()
             q, s, cw, ci = self._source_buffers()
             self._tile = qc.TileLayer(q, s, cw, ci, self.w_bits, self.in_features, self.group_size)
+            self._fast = None
         return self._tile
 
     def forward(self, x: torch.Tensor):
@@ -223,22 +227,21 @@ class QuantLinear(nn.Module):
                 x2 = x2.half()
             x2 = x2.contiguous()
             rows = x2.shape[0]
-            row = self.row_layer() if rows <= ROW_KERNEL_MAX_ROWS else None
-            if row is not None and rows <= row.preferred_rows:
-                out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
-                row.matvec(x2, out, False)
-            elif rows >= 8 and self.w_bits == 4 and self.group_size < 128 and self._prepared_key != "released":
-                raise RuntimeError("4-bit layers with groups narrower than 128 have no kernel for large batches")
-            elif rows >= 8 or row is not None:
-                # more rows: the tensor-core GEMM on this module's tile-layout copy
-                out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
-                self.tile_layer().gemm(x2, out, False)
-            else:
-                out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
+            limit = self._row_limit()
+            gemm_rows = limit + 1 if limit else GEMM_MIN_ROWS
+            out = torch.empty(rows, self.out_features, dtype=torch.float16, device=x2.device)
+            if rows <= limit:
+                self.row_layer().matvec(x2, out, False)
+            elif rows < gemm_rows:
                 self.prepared().matvec(x2, out, False)
-            if self._row is not None or self._tile is not None:
+            elif self.w_bits == 4 and self.group_size < 128 and self._prepared_key != "released":
+                raise RuntimeError("4-bit layers with groups narrower than 128 have no kernel for large batches")
+            else:
+                # more rows: the tensor-core GEMM on this module's tile-layout copy
+                self.tile_layer().gemm(x2, out, False)
+            if self._fast is None and (self._row is not None or self._tile is not None):
                 guard = None if self._prepared_key == "released" else self._prepared_key
-                self._fast = load_quant_cuda().PackedForward(self._row, self._tile, guard)
+                self._fast = load_quant_cuda().PackedForward(self._row, self._tile, guard, limit, gemm_rows)
             out = out.reshape(out_shape).to(x.dtype)
         else:
             if not self.dequantized:
@@ -257,8 +260,8 @@ class QuantLinear(nn.Module):
 
 def forward_shared_input(layers, x: torch.Tensor):
     """Outputs of several packed layers applied to the same input (q / k / v, gate / up of the
-    reference's LLaMA, llama/modeling_llama_quant.py): for decode batches (up to ROW_KERNEL_MAX_ROWS
-    rows) and layers that agree in bits, in_features, cherry count and group size this is ONE launch
+    reference's LLaMA, llama/modeling_llama_quant.py): for decode batches (up to the layers' row
+    limit) and layers that agree in bits, in_features, cherry count and group size this is ONE launch
     of the row-tile kernel per four rows, with the SMs divided among the layers; every other case is
     the layers' own forward, one by one.  The results are bit-identical to the separate calls."""
     layers = list(layers)
@@ -266,10 +269,9 @@ def forward_shared_input(layers, x: torch.Tensor):
     rows = x.numel() // x.shape[-1]
     same = all((l.w_bits, l.in_features, l.num_cherries, l.group_size) ==
                (first.w_bits, first.in_features, first.num_cherries, first.group_size) for l in layers)
-    if (rows <= ROW_KERNEL_MAX_ROWS and 1 < len(layers) <= 4 and same and QuantLinear._layerwise_dequantize
-            and first.w_bits in (3, 4)):
-        rls = [l.row_layer() for l in layers]
-        if all(r is not None and rows <= r.preferred_rows for r in rls):
+    if (1 < len(layers) <= 4 and same and QuantLinear._layerwise_dequantize and first.w_bits in (3, 4)):
+        if all(rows <= l._row_limit() for l in layers):
+            rls = [l.row_layer() for l in layers]
             qc = load_quant_cuda()
             x2 = x.reshape(rows, x.shape[-1])
             if x2.dtype != torch.float16:

@@ -9,14 +9,14 @@ torch = pytest.importorskip("torch")
 pytestmark = pytest.mark.gpu
 
 
-def packed(K, N, bits, G, seed, bias=False):
+def packed(K, N, bits, G, seed, bias=False, C=None):
     from cherryq_b200 import QuantLinear
     g = torch.Generator(device="cuda").manual_seed(seed)
-    C = math.ceil(K / 64) // 8 * 8
+    C = math.ceil(K / 64) // 8 * 8 if C is None else C
     w = (torch.randn(N, K, device="cuda", generator=g) * 0.02).half()
     idx = torch.randperm(K, device="cuda", generator=g)[:C].int()
     b = torch.randn(N, device="cuda", generator=g).half() if bias else None
-    lin = QuantLinear(bits, G, None, 1 / 64, K, N, bias=bias).cuda()
+    lin = QuantLinear(bits, G, None, C / K, K, N, bias=bias).cuda()
     lin.pack(SimpleNamespace(weight=w, bias=b, cherry_indices=idx, group_size=G))
     return lin
 
@@ -63,6 +63,28 @@ def test_forward_follows_the_buffers(bits, bias):
         check(lin, torch.randn(m, 1024, device="cuda").half(), dense, lin.bias)
     y = lin(torch.randn(3, 1024, device="cuda").half().requires_grad_())
     assert not y.requires_grad
+
+
+@pytest.mark.parametrize("K,C", [(2048, 16), (9216, 40), (2048, 256)])     # row kernel, the same split along K, stream matvec
+def test_kernel_does_not_depend_on_earlier_calls(K, C):
+    """A prompt first, then decode batches: the bits of a layer that never saw the prompt, through every entry point."""
+    from cherryq_b200.qlinear import forward_shared_input
+    x = torch.randn(40, K, device="cuda").half()
+    up = torch.randn(40, K, device="cuda").half()
+    old = [packed(K, 264, 4, 128, s, C=C) for s in (1, 2)]
+    for lin in old:
+        lin(x)
+        lin(x)
+    limit = old[0]._row_limit()
+    assert limit == {16: 8, 40: 4, 256: 0}[C]
+    for m in (1, 2, 4, 5, 7, 8, 9, 16, 40):
+        new = [packed(K, 264, 4, 128, s, C=C) for s in (1, 2)]
+        ref = [lin(x[:m]) for lin in new]
+        assert (new[0]._row is not None) == (m <= limit) and (new[0]._tile is not None) == (m > limit and m >= (1 if limit else 8))
+        for _ in range(2):
+            assert all(torch.equal(lin(x[:m]), r) for lin, r in zip(old, ref))
+        assert all(torch.equal(a, b) for a, b in zip(forward_shared_input(old, x[:m]), ref))
+        assert torch.equal(old[0].forward_swiglu(x[:m], up[:m]), new[0].forward_swiglu(x[:m], up[:m]))
 
 
 @pytest.mark.parametrize("D", [64, 128, 256])
