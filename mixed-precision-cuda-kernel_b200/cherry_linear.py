@@ -74,12 +74,13 @@ class QuantLinear(nn.Linear):
 
     def _one_pass(self, weight):
         """Whether the kernel takes this weight; everything else goes through the torch expressions below, which also
-        raise what they raise (one group per row or layer-wide scales are not defined for them)."""
-        return (weight.is_cuda and type(weight) in (torch.Tensor, nn.Parameter) and weight.layout == torch.strided
+        raise what they raise (one group per row or layer-wide scales are not defined for them).  _plain_eager comes
+        first: a transform's wrapper passes for a plain tensor but has no storage to ask for its address."""
+        return (_plain_eager() and weight.is_cuda and type(weight) in (torch.Tensor, nn.Parameter) and weight.layout == torch.strided
                 and weight.dtype in (torch.float16, torch.bfloat16, torch.float32) and weight.dim() == 2
                 and weight.is_contiguous() and weight.numel() > 0 and weight.shape[1] % 8 == 0 and weight.data_ptr() % 16 == 0
                 and not self.weight_layerwise and self.group_size >= 8 and weight.shape[1] < (1 << 24)
-                and weight.shape[1] // self.group_size < 12000 and self.quantizer is FullSymQuantizer and _plain_eager())
+                and weight.shape[1] // self.group_size < 12000 and self.quantizer is FullSymQuantizer)
 
     def _adjust_weight(self, weight, ste=True):
         assert not self.training or self.cherry_indices_registered, "`cherry_indices` is not registered yet."

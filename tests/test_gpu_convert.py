@@ -127,3 +127,36 @@ def test_fp32_operator(cabi, K, N, G, C, M):
     y = run(x)
     assert np.array_equal(np.isinf(y), np.isinf(ref)) and np.array_equal(np.sign(y[np.isinf(y)]), np.sign(ref[np.isinf(ref)]))
     assert np.array_equal(np.isnan(y), np.isnan(ref))
+
+
+def test_fake_quantised_weight_under_transforms(pkg):
+    """torch.func over the training layer takes the torch expressions: the values and gradients of the layer by itself."""
+    from cherryq_b200 import cherry_linear as CL
+    K, N, C = 264, 24, 16
+    w, idx = layer(K, N, C, np.float32, 3)
+    lin = CL.QuantLinear(K, N, w_bits=4, group_size=64, cherryq=True, cherry_fraction=C / K).cuda().train()
+    lin.register_cherry_indices(dev(idx.astype(np.int32)))
+    w = dev(w)
+    x = torch.randn(3, K, device="cuda")
+
+    def loss(w, x):
+        return torch.func.functional_call(lin, {"weight": w}, (x,)).square().sum()
+
+    def plain(w, x):
+        w = w.clone().requires_grad_()
+        y = loss(w, x)
+        return y.detach(), torch.autograd.grad(y, w)[0]
+
+    # fp32 sums in another order: 1e-5 of the norm is over ten times K * 2^-24
+    def same(a, b):
+        assert float((a - b).norm() / b.norm()) <= 1e-5
+
+    value, grad = plain(w, x)
+    same(torch.func.grad(loss)(w, x), grad)
+    same(torch.func.vmap(torch.func.grad(loss), (None, 0))(w, x), torch.stack([plain(w, r)[1] for r in x]))
+    t = torch.randn_like(w)
+    v, tangent = torch.func.jvp(lambda w: loss(w, x), (w,), (t,))
+    same(v, value)
+    same(tangent, (grad * t).sum())
+    ws = torch.stack([w, 2 * w])
+    same(torch.func.vmap(loss, (0, None))(ws, x), torch.stack([plain(v, x)[0] for v in ws]))
