@@ -5,13 +5,16 @@
 // (benchmark_speed.py:32).  It reads the reference's uint8 layout directly and
 // adds into `mul` with fp32 atomics like the reference.
 //
-// Products of 3-bit codes with fp32 activations on the integer tensor cores: per row of x and 128 compact columns the
-// activations become 31-bit fixed point (step 2^-29 of the power of two at the largest one, so everything down to
-// 2^-6 of it keeps all its bits), four signed-byte planes of which are B operands of mma.sync.m16n8k32; the codes are
-// the A operand.  Sums over a group are exact integers, (2 u - 7) x included, and meet the scale in fp32 - less
-// rounding than a chain of fp32 additions.  A loop of fp32 multiply-adds needs 25 us of the FMA pipe for 16 rows of
-// 4096 x 13824, before the decode of each code by the one thread that uses it.  That case: 52 us a call (93 with the
-// loop), bound by the issue rate: staging of x by every column block, byte decode and the fp32 combination share it.
+// Products of 3-bit codes with fp32 activations on the integer tensor cores: per row of x and 128 compact columns (64
+// where a scale group has 64) the activations become 31-bit fixed point (step 2^-29 of the power of two at the largest
+// one, so everything down to 2^-6 of it keeps all its bits), four signed-byte planes of which are B operands of
+// mma.sync.m16n8k32; the codes are the A operand.  Sums over a group are exact integers, (2 u - 7) x included, and meet
+// the scale in fp32.  The columns that share a step share their scale too, and no |u - 3.5| is below 1/2: half a step is
+// 2^-6 or less of what an fp32 addition rounds away beside the largest product (only activations that are smaller than
+// 2^-24 of two large ones which cancel are lost where a chain of additions in a lucky order keeps them).  A loop of fp32
+// multiply-adds needs 25 us of the FMA pipe for 16 rows of 4096 x 13824, before the decode of each code by the one
+// thread that uses it.  That case: 52 us a call (93 with the loop), bound by the issue rate: staging of x by every
+// column block, byte decode and the fp32 combination share it.
 #include "cq_common.cuh"
 
 namespace {
@@ -112,9 +115,10 @@ __global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Par
   const int b0 = blockIdx.x * p.blk_per_part, nb = min(p.blk_per_part, p.n_blk - b0);
   // [block][chunk of 32 columns][plane][token tile][lane][8 B], then per block and token: step factors, sums, flags
   uint2* planes = reinterpret_cast<uint2*>(smem);
-  float2* step = reinterpret_cast<float2*>(smem + (size_t)p.blk_per_part * 4 * NTILE * 256);    // [block][TOK]
-  int2* qsum = reinterpret_cast<int2*>(step + p.blk_per_part * TOK);                            // [block][2 halves][TOK]
-  int* bad = reinterpret_cast<int*>(qsum + p.blk_per_part * 2 * TOK);                           // [block][TOK]
+  float2* step = reinterpret_cast<float2*>(smem + (size_t)p.blk_per_part * 4 * NTILE * 256);    // [block][2 halves][TOK]
+  int2* qsum = reinterpret_cast<int2*>(step + p.blk_per_part * 2 * TOK);                        // the same
+  int* bad = reinterpret_cast<int*>(qsum + p.blk_per_part * 2 * TOK);                           // the same
+  const int halves = p.G == 64 ? 2 : 1;
   const int g = lane >> 2, c = lane & 3;
   const int n = n_cta + warp * 32 + 4 * g;                  // this thread's four columns
 
@@ -142,7 +146,9 @@ __global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Par
 #pragma unroll
       for (int e = 0; e < 8; ++e) mx = max(mx, __float_as_uint(v[e]) & 0x7FFFFFFFu);
 #pragma unroll
-      for (int d = 8; d; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+      for (int d = 4; d; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
+      const uint32_t mx2 = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
+      if (halves == 1) mx = mx2;                            // one step for the block, or one for each of its two groups
       const bool finite = mx < 0x7F800000u;
       // power of two at the largest value (subnormals count as 2^-126), less 29
       const int e2 = max((int)(mx >> 23), 1) - 127 - 29;
@@ -174,10 +180,11 @@ __global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Par
 #pragma unroll
         for (int k = 0; k < 4; ++k)
           planes[((size_t)(j * 4 + ch) * NTILE + k * TT + (t >> 3)) * 32 + dst] = make_uint2(pl[k][0], pl[k][1]);
-        if ((l16 & 7) == 0) qsum[(j * 2 + (l16 >> 3)) * TOK + t] = make_int2(hi, lo);
-        if (l16 == 0) {
-          step[j * TOK + t] = f32_pow2_pair(e2);
-          bad[j * TOK + t] = finite ? 0 : 1;
+        if ((l16 & 7) == 0) {
+          const int at = (j * 2 + (l16 >> 3)) * TOK + t;
+          qsum[at] = make_int2(hi, lo);
+          step[at] = f32_pow2_pair(e2);
+          bad[at] = finite ? 0 : 1;
         }
       }
     }
@@ -191,7 +198,6 @@ __global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Par
     uint32_t nxt[4][3];
 #pragma unroll
     for (int ch = 0; ch < 4; ++ch) f32_load_codes(p, b0 * 16 + ch * 4 + c, n, nxt[ch]);
-    const int halves = p.G == 64 ? 2 : 1;
     for (int j = 0; j < nb; ++j) {
       int acc[2][NTILE][4];
 #pragma unroll
@@ -241,13 +247,14 @@ __global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Par
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
               const int tok = 8 * t + 2 * c + e;
-              int2 qs = qsum[(j * 2 + (halves == 2 ? ch >> 1 : 0)) * TOK + tok];
+              const int at = (j * 2 + (halves == 2 ? ch >> 1 : 0)) * TOK + tok;
+              int2 qs = qsum[at];
               if (halves == 1) {
                 const int2 q2 = qsum[(j * 2 + 1) * TOK + tok];
                 qs.x += q2.x;
                 qs.y += q2.y;
               }
-              const float2 st = step[j * TOK + tok];
+              const float2 st = step[at];
               const float f1 = 0.5f * st.x;
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
@@ -257,8 +264,8 @@ __global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Par
                 const float v = __fmaf_rn((float)(2 * hi - 7 * qs.x), 65536.f, (float)(2 * lo - 7 * qs.y));
                 y[i][t][e] += v * f1 * s[i] * st.y;
               }
-              if (bad[j * TOK + tok]) {
-                // an infinite or NaN activation in this block: the plain sum over the group
+              if (bad[at]) {
+                // an infinite or NaN activation among them: the plain sum over the group
                 const int o0 = (b0 + j) * 16 + (halves == 2 ? 8 * (ch >> 1) : 0), o1 = o0 + (halves == 2 ? 8 : 16);
                 for (int i = 0; i < 4; ++i) {
                   if (n + i >= p.N) break;
@@ -330,7 +337,7 @@ int cq_launch_matvec_f32(const float* x, const uint8_t* q, const float* cw, cons
   p.aligned_q = N % 4 == 0 && ((uintptr_t)q & 3) == 0;
   p.aligned_f = N % 4 == 0 && ((uintptr_t)sf & 15) == 0 && ((uintptr_t)mul & 15) == 0;
   const int tt = M > 8 ? 2 : 1;
-  const int smem_main = per * (4 * 4 * tt * 256 + 8 * tt * (8 + 16 + 4)), smem_cherry = 64 * 8 * tt * 4;
+  const int smem_main = per * (4 * 4 * tt * 256 + 8 * tt * (16 + 16 + 8)), smem_cherry = 64 * 8 * tt * 4;
   const int smem = smem_main > smem_cherry ? smem_main : smem_cherry;
   const dim3 grid(p.n_parts + (C > 0 ? 1 : 0), ny);
   auto kernel = tt == 2 ? matvec_f32_kernel<2> : matvec_f32_kernel<1>;

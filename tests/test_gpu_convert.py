@@ -90,8 +90,8 @@ def test_fake_quantised_weight(pkg, K, N, bits, G, C, dtype):
 @pytest.mark.parametrize("K,N,G,C,M", [(136, 4, 64, 8, 1), (256, 9, 128, 8, 3), (1160, 264, 64, 16, 8), (2048, 520, 256, 8, 9),
                                        (4096, 256, 128, 72, 33), (256, 12, 256, 0, 17)])
 def test_fp32_operator(cabi, K, N, G, C, M):
-    """vecquant3matmul_cherryq with fp32 activations: exact integer sums, so only the fixed point of x (2^-31 of the largest
-    of its 128 columns), the conversion of a sum and a few fp32 additions round: 1e-6 of the result's norm is four times
+    """vecquant3matmul_cherryq with fp32 activations: exact integer sums, so only the fixed point of x (2^-30 of the power of
+    two at the largest of a group's columns, 128 at most), the conversion of a sum and a few fp32 additions round: 1e-6 of the result's norm is four times
     that.  An infinite activation gives the same infinities and NaN as the plain sum."""
     rng = np.random.default_rng(K + M)
     _, idx = layer(K, 8, C, np.float32, K)
@@ -127,6 +127,44 @@ def test_fp32_operator(cabi, K, N, G, C, M):
     y = run(x)
     assert np.array_equal(np.isinf(y), np.isinf(ref)) and np.array_equal(np.sign(y[np.isinf(y)]), np.sign(ref[np.isinf(ref)]))
     assert np.array_equal(np.isnan(y), np.isnan(ref))
+
+
+@pytest.mark.parametrize("K,N,C,M,ratio", [(1024, 264, 8, 9, 1e4), (2120, 40, 24, 3, 1e4), (1024, 264, 8, 17, 1e-5)])
+def test_fp32_operator_groups_of_unlike_magnitudes(cabi, K, N, C, M, ratio):
+    """Groups of 64 columns whose activations are `ratio` times their neighbours' and whose scales as much smaller: the
+    products have one magnitude, and those of each group keep their own bits.  Bound as in test_fp32_operator.  A NaN in
+    one group reaches every output of its row and no other row."""
+    rng = np.random.default_rng(K + M)
+    idx = np.sort(rng.permutation(K)[:C]).astype(np.int32)
+    Kc = K - C
+    u = rng.integers(0, 8, size=(Kc, N))
+    q = O.pack_codes(u.astype(np.uint8), 3)
+    big = np.arange((Kc + 63) // 64) % 2 == 0
+    s = ((rng.random((len(big), N)) + 0.1) * np.where(big, 1 / ratio, 1.0)[:, None]).astype(np.float32)
+    cw = rng.normal(size=(C, N)).astype(np.float32)
+    x = rng.normal(size=(M, K)).astype(np.float32)
+    cols = O.normal_columns(K, idx)
+    x[:, cols] *= np.repeat(np.where(big, ratio, 1.0), 64)[:Kc].astype(np.float32)
+    dense = np.zeros((K, N))
+    dense[idx] = cw
+    dense[cols] = (u - 3.5) * np.repeat(s, 64, axis=0)[:Kc].astype(np.float64)
+
+    def run(x):
+        out = torch.zeros(M, N, device="cuda")
+        t = [dev(a) for a in (x, q, cw, idx, s)]
+        cabi.check(cabi.lib().cq_vecquant3matmul_cherryq(ptr(t[0]), ptr(t[1]), ptr(t[2]), ptr(t[3]), ptr(t[4]), ptr(out), M, K,
+                                                         q.shape[0], N, C, 64, 0, 0, None), "fp32 operator")
+        torch.cuda.synchronize()
+        return out.cpu().numpy().astype(np.float64)
+
+    ref = x.astype(np.float64) @ dense
+    y = run(x)
+    err = np.linalg.norm(y - ref, axis=1) / np.linalg.norm(ref, axis=1)
+    assert err.max() <= 1e-6, err
+    x[M - 1, cols[70]] = np.nan
+    z = run(x)
+    assert np.isnan(z[M - 1]).all()
+    assert np.linalg.norm(z[:M - 1] - ref[:M - 1]) <= 1e-6 * np.linalg.norm(ref[:M - 1])
 
 
 def test_fake_quantised_weight_under_transforms(pkg):
