@@ -257,9 +257,12 @@ int cq_attn_decode(const void* q_f16, const void* k_cache_f16, const void* v_cac
                    const long long* position, void* out_f16, int sequences, int n_heads,
                    int n_kv_heads, int head_dim, int max_seq, float scale, void* workspace,
                    cq_stream_t stream);
-/* out = silu(gate) * up, n elements. */
+/* out = silu(gate) * up, n elements.  cq_silu_mul takes the fast exponential, as the row kernel's folded SwiGLU
+ * does; cq_silu_mul_full expf, as the fp32 expression. */
 int cq_silu_mul(const void* gate_f16, const void* up_f16, void* out_f16, long long n,
                 cq_stream_t stream);
+int cq_silu_mul_full(const void* gate_f16, const void* up_f16, void* out_f16, long long n,
+                     cq_stream_t stream);
 
 /* ------------------------------------------------------------------------
  * Tile-layout prepared layer: the format of the tcgen05 (UMMA + tensor memory) kernels.

@@ -128,12 +128,14 @@ __global__ void rope_cache_kernel(__half* __restrict__ q, __half* __restrict__ k
   }
 }
 
-// V = values per access: 8 where the buffers are 16-byte aligned, 1 otherwise and for the tail.
+// V = values per access: 8 where the buffers are 16-byte aligned, 1 otherwise and for the tail.  FULL: expf as in the
+// fp32 torch expression, whose fp16 result it then equals; otherwise the fast exponential, as the row kernel's staging.
+template <bool FULL>
 __device__ __forceinline__ __half silu_times(__half gate, __half up) {
   const float g = __half2float(gate);
-  return __hmul(__float2half(g / (1.f + __expf(-g))), up);            // the silu result is an fp16 tensor
+  return __hmul(__float2half(g / (1.f + (FULL ? expf(-g) : __expf(-g)))), up);            // the silu result is an fp16 tensor
 }
-template <int V>
+template <int V, bool FULL>
 __global__ void silu_mul_kernel(const __half* __restrict__ gate, const __half* __restrict__ up,
                                 __half* __restrict__ out, long long n) {
   // programmatic dependent launch: let the next kernel start its prologue, then wait for our inputs
@@ -145,10 +147,10 @@ __global__ void silu_mul_kernel(const __half* __restrict__ gate, const __half* _
     Halves g = reinterpret_cast<const Halves*>(gate)[i];
     const Halves u = reinterpret_cast<const Halves*>(up)[i];
 #pragma unroll
-    for (int e = 0; e < V; ++e) g.h[e] = silu_times(g.h[e], u.h[e]);
+    for (int e = 0; e < V; ++e) g.h[e] = silu_times<FULL>(g.h[e], u.h[e]);
     reinterpret_cast<Halves*>(out)[i] = g;
   }
-  if (id < n % V) out[n - 1 - id] = silu_times(gate[n - 1 - id], up[n - 1 - id]);
+  if (id < n % V) out[n - 1 - id] = silu_times<FULL>(gate[n - 1 - id], up[n - 1 - id]);
 }
 
 // Single-query attention over the KV cache (decode).  q and out are (sequences, H, D), the caches
@@ -705,13 +707,22 @@ extern "C" int cq_rope_cache(void* q, void* k, const void* v, const float* cos_t
   return CQ_OK;
 }
 
-extern "C" int cq_silu_mul(const void* gate, const void* up, void* out, long long n, cq_stream_t stream) {
+namespace {
+template <bool FULL> int silu_mul_launch(const void* gate, const void* up, void* out, long long n, cq_stream_t stream) {
   if (!gate || !up || !out || n < 1) return CQ_ERR_BAD_ARG;
   const int vec = (((uintptr_t)gate | (uintptr_t)up | (uintptr_t)out) & 15) == 0 ? 8 : 1;
-  auto kernel = vec == 8 ? silu_mul_kernel<8> : silu_mul_kernel<1>;
+  auto kernel = vec == 8 ? silu_mul_kernel<8, FULL> : silu_mul_kernel<1, FULL>;
   CQ_CUDA_TRY(launch_pdl(kernel, dim3(blocks_for((n + vec - 1) / vec, 256, 148 * 8)), dim3(256), 0, (cudaStream_t)stream,
                          (const __half*)gate, (const __half*)up, (__half*)out, n));
   return CQ_OK;
+}
+}  // namespace
+
+extern "C" int cq_silu_mul(const void* gate, const void* up, void* out, long long n, cq_stream_t stream) {
+  return silu_mul_launch<false>(gate, up, out, n, stream);
+}
+extern "C" int cq_silu_mul_full(const void* gate, const void* up, void* out, long long n, cq_stream_t stream) {
+  return silu_mul_launch<true>(gate, up, out, n, stream);
 }
 
 namespace {

@@ -659,14 +659,14 @@ void rope_cache(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor
                "rope_cache");
 }
 
-torch::Tensor silu_mul(torch::Tensor gate, torch::Tensor up) {
+torch::Tensor silu_mul(torch::Tensor gate, torch::Tensor up, bool full) {
   const at::cuda::OptionalCUDAGuard device_guard(device_of(gate));
   check_tensor(gate, "gate", torch::kFloat16, gate);
   check_tensor(up, "up", torch::kFloat16, gate);
   TORCH_CHECK(gate.sizes() == up.sizes(), "gate and up must have the same shape");
   auto out = torch::empty_like(gate);
-  check_status(cq_silu_mul(gate.data_ptr(), up.data_ptr(), out.data_ptr(), (long long)gate.numel(), current_stream()),
-               "silu_mul");
+  auto fn = full ? cq_silu_mul_full : cq_silu_mul;
+  check_status(fn(gate.data_ptr(), up.data_ptr(), out.data_ptr(), (long long)gate.numel(), current_stream()), "silu_mul");
   return out;
 }
 
@@ -724,7 +724,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   });
   m.def("rmsnorm", &rmsnorm, "RMSNorm with optional residual add");
   m.def("rope_cache", &rope_cache, "rotary embedding in place + KV cache write");
-  m.def("silu_mul", &silu_mul, "silu(gate) * up");
+  m.def("silu_mul", &silu_mul, "silu(gate) * up", py::arg("gate"), py::arg("up"), py::arg("full") = false);
   m.def("attn_decode", &attn_decode, "single-query attention over the KV cache");
   m.def("poll", []() { check_status(cq_poll(current_stream()), "poll"); });
   m.def("device_timed_out", &device_timed_out);

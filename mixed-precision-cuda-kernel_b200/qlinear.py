@@ -163,14 +163,15 @@ class QuantLinear(nn.Module):
     def forward_swiglu(self, gate: torch.Tensor, up: torch.Tensor):
         """This layer applied to silu(gate) * up (the down projection of the reference's LlamaMLP.forward,
         llama/modeling_llama_quant.py): for decode batches the product is formed while the kernel stages its
-        input (no separate element-wise kernel, no intermediate tensor), with the same roundings, so the
-        result equals forward(silu(gate) * up) bit for bit; other cases compute the product first."""
+        input (no separate element-wise kernel, no intermediate tensor): the result is that of
+        forward(silu_mul(gate, up)), with the fast exponential.  Other cases compute the product first, with the
+        values of the torch expression, silu in fp32."""
         rows = gate.numel() // gate.shape[-1]
         row = self.row_layer() if (self._layerwise_dequantize and self.w_bits in (3, 4) and gate.dtype == torch.float16
                                    and rows <= self._row_limit()) else None
         if row is None:
             if gate.is_cuda and gate.dtype == up.dtype == torch.float16 and gate.shape == up.shape and gate.numel():
-                return self(load_quant_cuda().silu_mul(gate.contiguous(), up.contiguous()))
+                return self(load_quant_cuda().silu_mul(gate.contiguous(), up.contiguous(), True))
             return self(nn.functional.silu(gate.float()).to(gate.dtype) * up)
         g2 = gate.reshape(rows, gate.shape[-1]).contiguous()
         u2 = up.reshape(rows, up.shape[-1]).contiguous()

@@ -87,6 +87,20 @@ def test_kernel_does_not_depend_on_earlier_calls(K, C):
         assert torch.equal(old[0].forward_swiglu(x[:m], up[:m]), new[0].forward_swiglu(x[:m], up[:m]))
 
 
+@pytest.mark.parametrize("m,C", [(9, 16), (40, 16), (3, 256)])
+def test_swiglu_beyond_the_row_kernel_is_the_torch_expression(m, C):
+    """Rows above the row kernel's limit and layers it does not take: silu in fp32, not the fast exponential.  Every fp16
+    gate value, infinities and NaN among them."""
+    lin = packed(2048, 264, 4, 128, 3, C=C)
+    gate = torch.arange(65536, device="cuda").to(torch.int16).view(torch.float16)
+    act = torch.nn.functional.silu(gate.float()).half() * torch.ones_like(gate)
+    import cherryq_b200
+    got = cherryq_b200.load_quant_cuda().silu_mul(gate, torch.ones_like(gate), True)
+    assert torch.equal(got.isnan(), act.isnan()) and torch.equal(got.nan_to_num(7.0), act.nan_to_num(7.0))
+    gate, up = (torch.randn(m, 2048, device="cuda").half() * 3 for _ in range(2))
+    assert torch.equal(lin.forward_swiglu(gate, up), lin(torch.nn.functional.silu(gate.float()).half() * up))
+
+
 @pytest.mark.parametrize("D", [64, 128, 256])
 @pytest.mark.parametrize("H,KV,max_seq,at", [(4, 4, 2300, (0, 255, 256, 2299)), (8, 2, 600, (1, 511, 512, 599)), (3, 3, 40, (0, 7, 38, 39))])
 def test_attention_sweep_edges(D, H, KV, max_seq, at):
