@@ -9,8 +9,8 @@
 //   * A operand = weights, 256 rows per tile, 128 in each CTA of a pair, dequantised to fp16 by the
 //     row's own thread (one thread = one weight row = one TENSOR MEMORY lane) and stored straight
 //     into tensor memory with tcgen05.st: exponent-trick unpack (AND-OR into the bits of 1024.0), one
-//     exact subtraction and one multiplication by the group scale per fp16 pair, which reproduces
-//     unpack()'s fp16 values bit for bit;
+//     exact multiply-add and one multiplication by the group scale per fp16 pair, which reproduces
+//     unpack()'s fp16 values bit for bit, whatever the scale;
 //   * B operand = NT tokens of activations per tile (NT = 32 .. 256 in steps of 32), half of them in each CTA,
 //     prepared once per call by a small pre-pass kernel (gather into compact column order, canonical
 //     K-major UMMA layout) so that the main kernel moves them with plain bulk async copies;
@@ -125,9 +125,9 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
-__device__ __forceinline__ uint32_t hsub2_u32(uint32_t a, uint32_t b) {
+__device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
-  asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));
+  asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
   return d;
 }
 __device__ __forceinline__ uint32_t hmul2_u32(uint32_t a, uint32_t b) {
@@ -199,45 +199,47 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t addr, uint32_t lbo16, uin
 
 // ------------------------------------------------------------------ dequantisation to fp16
 // A code field at mantissa bit p OR-ed into the bits of fp16 1024.0 is the number 1024 + 2^p u.
-// Subtracting 1024 + 2^p off is exact (the result is 2^p (u - off), a small multiple of 2^(p-1)),
-// and the product with s * 2^-p is (u - off) * s rounded once to fp16: exactly the value
-// unpack() computes as fp16(q + 0.5) * s (llama/qlinear.py:139-146 of the reference project).
+// One multiply-add, times 2^-p less (1024 * 2^-p + off), makes it u - off: every constant and the result are
+// exact.  The product with the scale s is then (u - off) * s rounded once to fp16: exactly the value unpack()
+// computes as fp16(q + 0.5) * s (llama/qlinear.py:139-146 of the reference project).  (2^-p folded into the scale
+// instead would round it where it becomes subnormal: s below 2^-8, weights of a deviation of about 0.01.)
 constexpr uint32_t MAGIC = 0x64006400u;
-__device__ __forceinline__ uint32_t dup16(uint32_t h) { return h | (h << 16); }
-// fp16 bits of 1024 + 2^p * off
+__device__ __forceinline__ constexpr uint32_t dup16(uint32_t h) { return h | (h << 16); }
+__device__ __forceinline__ constexpr uint32_t pow2_neg(int pbit) { return (uint32_t)(15 - pbit) << 10; }   // fp16 bits of 2^-p
+// fp16 bits of -(1024 * 2^-p + off)
 template <int BITS> __device__ __forceinline__ constexpr uint32_t center(int pbit) {
-  return BITS == 4 ? (pbit == 2 ? 0x641Eu : 0x65E0u)                       // 1054, 1504
-                   : (pbit == 1 ? 0x6407u : (pbit == 4 ? 0x6438u : 0x65C0u));   // 1031, 1080, 1472
+  return BITS == 4 ? (pbit == 2 ? 0xDC1Eu : 0xCDE0u)                       // -263.5, -23.5
+                   : (pbit == 1 ? 0xE007u : (pbit == 4 ? 0xD438u : 0xC9C0u));   // -515.5, -67.5, -11.5
 }
-__device__ __forceinline__ uint32_t pow2_neg(int pbit) { return (uint32_t)(15 - pbit) << 10; }   // fp16 bits of 2^-p
+// the pair of codes at mantissa bit P of `word` -> (u - off) * s
+template <int BITS, int P> __device__ __forceinline__ uint32_t code_pair(uint32_t word, uint32_t s) {
+  return hmul2_u32(hfma2_u32(word | MAGIC, dup16(pow2_neg(P)), dup16(center<BITS>(P))), s);
+}
 
-// One 4-bit word (8 codes) -> 4 fp16 pairs; sc2 / sc6 = (s * 2^-2, s * 2^-2), (s * 2^-6, s * 2^-6)
-__device__ __forceinline__ void dequant4(uint32_t w, uint32_t sc2, uint32_t sc6, uint32_t* out) {
+// One 4-bit word (8 codes) -> 4 fp16 pairs; s = the scale, twice
+__device__ __forceinline__ void dequant4(uint32_t w, uint32_t s, uint32_t* out) {
   const uint32_t v1 = w << 2, v2 = w >> 6;
-  const uint32_t c2 = dup16(center<4>(2)), c6 = dup16(center<4>(6));
-  out[0] = hmul2_u32(hsub2_u32((v1 & 0x003C003Cu) | MAGIC, c2), sc2);
-  out[1] = hmul2_u32(hsub2_u32((v1 & 0x03C003C0u) | MAGIC, c6), sc6);
-  out[2] = hmul2_u32(hsub2_u32((v2 & 0x003C003Cu) | MAGIC, c2), sc2);
-  out[3] = hmul2_u32(hsub2_u32((v2 & 0x03C003C0u) | MAGIC, c6), sc6);
+  out[0] = code_pair<4, 2>(v1 & 0x003C003Cu, s);
+  out[1] = code_pair<4, 6>(v1 & 0x03C003C0u, s);
+  out[2] = code_pair<4, 2>(v2 & 0x003C003Cu, s);
+  out[3] = code_pair<4, 6>(v2 & 0x03C003C0u, s);
 }
-// Three 3-bit words (32 codes) -> 16 fp16 pairs; sc1 / sc4 / sc7 = s * 2^-1, 2^-4, 2^-7 pairs
-__device__ __forceinline__ void dequant3(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t sc1, uint32_t sc4, uint32_t sc7,
-                                         uint32_t* out) {
-  const uint32_t c1 = dup16(center<3>(1)), c4 = dup16(center<3>(4)), c7 = dup16(center<3>(7));
+// Three 3-bit words (32 codes) -> 16 fp16 pairs
+__device__ __forceinline__ void dequant3(uint32_t w0, uint32_t w1, uint32_t w2, uint32_t s, uint32_t* out) {
   const uint32_t w[3] = {w0, w1, w2};
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     const uint32_t v = w[i] >> 6;
-    out[5 * i + 0] = hmul2_u32(hsub2_u32((w[i] & 0x000E000Eu) | MAGIC, c1), sc1);   // field at bit 1
-    out[5 * i + 1] = hmul2_u32(hsub2_u32((w[i] & 0x00700070u) | MAGIC, c4), sc4);   // bit 4
-    out[5 * i + 2] = hmul2_u32(hsub2_u32((w[i] & 0x03800380u) | MAGIC, c7), sc7);   // bit 7
-    out[5 * i + 3] = hmul2_u32(hsub2_u32((v & 0x00700070u) | MAGIC, c4), sc4);      // bit 10 -> 4
-    out[5 * i + 4] = hmul2_u32(hsub2_u32((v & 0x03800380u) | MAGIC, c7), sc7);      // bit 13 -> 7
+    out[5 * i + 0] = code_pair<3, 1>(w[i] & 0x000E000Eu, s);   // field at bit 1
+    out[5 * i + 1] = code_pair<3, 4>(w[i] & 0x00700070u, s);   // bit 4
+    out[5 * i + 2] = code_pair<3, 7>(w[i] & 0x03800380u, s);   // bit 7
+    out[5 * i + 3] = code_pair<3, 4>(v & 0x00700070u, s);      // bit 10 -> 4
+    out[5 * i + 4] = code_pair<3, 7>(v & 0x03800380u, s);      // bit 13 -> 7
   }
-  uint32_t r = ((w0 << 7) & 0x00800080u) | MAGIC;     // pair 15: one bit from each word, at bits 7..9
+  uint32_t r = (w0 << 7) & 0x00800080u;     // pair 15: one bit from each word, at bits 7..9
   r |= (w1 << 8) & 0x01000100u;
   r |= (w2 << 9) & 0x02000200u;
-  out[15] = hmul2_u32(hsub2_u32(r, c7), sc7);
+  out[15] = code_pair<3, 7>(r, s);
 }
 
 // ------------------------------------------------------------------ activation pre-pass
@@ -607,21 +609,16 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
           if constexpr (BITS == 4) {
 #pragma unroll
             for (int c4 = 0; c4 < 4; ++c4) {
-              const uint32_t s = (c4 < 2) ? s0 : s1;
-              const uint32_t sc2 = hmul2_u32(s, dup16(pow2_neg(2))), sc6 = hmul2_u32(s, dup16(pow2_neg(6)));
               uint32_t v[16];
 #pragma unroll
-              for (int e = 0; e < 4; ++e) dequant4(wds[4 * c4 + e], sc2, sc6, v + 4 * e);
+              for (int e = 0; e < 4; ++e) dequant4(wds[4 * c4 + e], (c4 < 2) ? s0 : s1, v + 4 * e);
               tmem_st16(ta + 16 * c4, v);
             }
           } else {
 #pragma unroll
             for (int t3 = 0; t3 < 4; ++t3) {
-              const uint32_t s = (t3 < 2) ? s0 : s1;
-              const uint32_t sc1 = hmul2_u32(s, dup16(pow2_neg(1))), sc4 = hmul2_u32(s, dup16(pow2_neg(4))),
-                             sc7 = hmul2_u32(s, dup16(pow2_neg(7)));
               uint32_t v[16];
-              dequant3(wds[3 * t3], wds[3 * t3 + 1], wds[3 * t3 + 2], sc1, sc4, sc7, v);
+              dequant3(wds[3 * t3], wds[3 * t3 + 1], wds[3 * t3 + 2], (t3 < 2) ? s0 : s1, v);
               tmem_st16(ta + 16 * t3, v);
             }
           }

@@ -180,3 +180,18 @@ def test_gemm_accumulates_and_strides_unaligned(cabi):
     got = yb[1:].view(M, N + 3)
     assert float((got[:, :N].float() - ref).abs().max() / ref.abs().max()) <= 2e-3
     assert torch.equal(got[:, N:], base[:, N:])
+
+
+@pytest.mark.parametrize("bits,G", [(3, 64), (3, 128), (4, 128), (4, 256)])
+def test_gemm_weights_are_unpacked_exactly_at_every_scale(cabi, bits, G):
+    """Rows of the identity read the dequantised weights back: bit for bit unpack()'s, with scales from the smallest
+    subnormal to where the largest code reaches fp16's range."""
+    K, N = 1024, 264
+    w, idx, pk, dense = make_case(K, N, bits, G, seed=bits + G)
+    rng = np.random.default_rng(G)
+    scales = np.exp2(rng.uniform(-24, 13, size=pk["scales"].shape)).astype(np.float16)
+    scales[:, :4] = np.float16(2.0 ** -24)
+    dense = O.unpack(pk["qweight"], scales, pk["cherry_weight"], pk["cherry_indices"], bits, G, K)
+    p = TilePrepared(cabi, pk["qweight"], scales, pk["cherry_weight"], pk["cherry_indices"], bits, K, G)
+    y = gemm(cabi, p, torch.eye(K, device="cuda").half())
+    assert torch.equal(y.T, dev(dense))
