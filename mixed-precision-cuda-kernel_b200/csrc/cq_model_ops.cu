@@ -369,7 +369,12 @@ __global__ void __launch_bounds__(ONE_THREADS) attn_decode_one_kernel(const __ha
       s[u] = base + u * GROUPS + grp < n_pos ? s[u] * scale : -INFINITY;
       top = fmaxf(top, s[u]);
     }
-    if (top == -INFINITY) continue;           // none of this group's positions exists (or all scores are -infinity)
+    if (top == -INFINITY) {                   // none of this group's positions exists, or their scores are -infinity
+#pragma unroll
+      for (int u = 0; u < UF; ++u)
+        if (s[u] != s[u]) l = s[u];           // (or NaN, which no maximum shows: the sum carries it)
+      continue;
+    }
     const float keep = __expf(m - top);
     l *= keep;
 #pragma unroll

@@ -121,3 +121,25 @@ def test_attention_sweep_edges(D, H, KV, max_seq, at):
         s = torch.einsum("hd,phd->hp", q[b].float(), kk) / math.sqrt(D)
         ref = torch.einsum("hp,phd->hd", s.softmax(-1), vv)
         assert float((out[b].float() - ref).abs().max()) <= 4e-3     # fp16 output of values near 1, fast exponentials
+
+
+@pytest.mark.parametrize("H,KV", [(4, 4), (8, 2)])
+@pytest.mark.parametrize("D,max_seq,at,bad", [(128, 300, 5, 3), (64, 300, 299, 299), (256, 300, 0, 0), (128, 700, 699, 300), (32, 300, 5, 3)])
+def test_attention_keeps_nan_scores(D, H, KV, max_seq, at, bad):
+    """A key of NaN makes its head's output NaN, as a softmax does, wherever it falls among the lanes and ranges; one of
+    -infinity has no weight."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    q = torch.rand(1, H, D, device="cuda").half() + 0.1
+    k, v = (torch.randn(1, max_seq, KV, D, device="cuda").half() for _ in range(2))
+    pos = torch.tensor([at], device="cuda")
+    k[0, bad, 0] = float("nan")
+    out = qc.attn_decode(q, k, v, pos).view(H, D)
+    assert out[:H // KV].isnan().all() and out[H // KV:].isfinite().all()
+    if at:
+        k[0, bad, 0] = float("-inf")
+        out = qc.attn_decode(q, k, v, pos).view(H, D)
+        keep = [p for p in range(at + 1) if p != bad]
+        s = torch.einsum("hd,pd->hp", q[0, :H // KV].float(), k[0, keep, 0].float()) / math.sqrt(D)
+        ref = s.softmax(-1) @ v[0, keep, 0].float()
+        assert float((out[:H // KV].float() - ref).abs().max()) <= 4e-3
