@@ -250,8 +250,9 @@ int cq_rope_cache(void* q_f16, void* k_f16, const void* v_f16, const float* cos_
  * divides 256 (the reference calls PyTorch's attention, llama/modeling_llama_quant.py:371-419).
  * The positions of a head are divided among several CTAs so that a decode step fills the GPU; they
  * meet in `workspace`: device memory of cq_attn_decode_workspace_bytes(...) bytes, 16-byte aligned,
- * zero-filled once before its first use (every launch leaves it ready for the next), not shared by
- * launches that can overlap on the GPU. */
+ * zero-filled before its first use and before the first call with another number of heads (sequences *
+ * n_heads: that many counters stand in front of the partial results; every launch leaves its own at zero),
+ * not shared by launches that can overlap on the GPU. */
 size_t cq_attn_decode_workspace_bytes(int sequences, int n_heads, int head_dim, int max_seq);
 int cq_attn_decode(const void* q_f16, const void* k_cache_f16, const void* v_cache_f16,
                    const long long* position, void* out_f16, int sequences, int n_heads,

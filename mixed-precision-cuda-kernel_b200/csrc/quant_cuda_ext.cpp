@@ -11,6 +11,7 @@
 //     reference's 3-bit op silently does nothing for an unsupported group size).
 // The first matmul call with a given set of weight tensors re-packs them on the GPU
 // (allocates and synchronises), so it must happen before any stream capture.
+#include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/core/InferenceMode.h>
@@ -235,7 +236,39 @@ torch::Tensor unpack_dense(torch::Tensor qweight, torch::Tensor scales, torch::T
 
 std::mutex g_mu;
 std::map<int, torch::Tensor> g_scratch;  // per device: matvec scratch followed by a status word
-std::map<int, torch::Tensor> g_attn_ws;  // per device: workspace of the decode attention
+
+// Workspace of the decode attention, per device, grow-only.  The counters of every call end at `counters` bytes, where the
+// partial results begin: calls of different numbers of heads share the buffer and none writes over the zeros that another
+// counts from.  Outgrown buffers are kept, since a captured graph may hold their addresses; sizes at least double.
+struct AttnWorkspace {
+  torch::Tensor now;
+  size_t counters = 0;
+  std::vector<torch::Tensor> outgrown;
+};
+std::map<int, AttnWorkspace> g_attn_ws;
+
+// the workspace of a call of `heads` heads (in all sequences) that needs `bytes`; `keep` holds the buffer
+void* attn_workspace(const torch::Device& dev, size_t heads, size_t bytes, torch::Tensor* keep) {
+  const size_t own = (heads * sizeof(unsigned int) + 255) / 256 * 256;
+  const auto options = torch::TensorOptions().device(dev).dtype(torch::kUInt8);
+  std::lock_guard<std::mutex> lock(g_mu);
+  auto& w = g_attn_ws[dev.index()];
+  if (w.counters < own || !w.now.defined() || (size_t)w.now.numel() < w.counters + bytes) {
+    // a buffer made under capture is the graph's own: its zeros are written when the graph runs
+    if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) {
+      *keep = torch::zeros({(int64_t)bytes}, options);
+      return keep->data_ptr();
+    }
+    const size_t counters = std::max(own, 2 * w.counters);
+    const size_t size = std::max(counters + bytes, w.now.defined() ? 2 * (size_t)w.now.numel() : 0);
+    auto t = torch::zeros({(int64_t)size}, options);
+    if (w.now.defined()) w.outgrown.push_back(w.now);
+    w.now = t;
+    w.counters = counters;
+  }
+  *keep = w.now;
+  return w.now.data_ptr<uint8_t>() + w.counters - own;
+}
 
 torch::Tensor scratch_for(const torch::Device& dev) {
   std::lock_guard<std::mutex> lock(g_mu);
@@ -685,20 +718,14 @@ torch::Tensor attn_decode(torch::Tensor q, torch::Tensor k_cache, torch::Tensor 
   TORCH_CHECK(k_cache.size(cd - 1) == q.size(2) && v_cache.sizes() == k_cache.sizes(), "caches must be ([B,] max_seq, KV, D)");
   TORCH_CHECK(position.numel() == B, "one position per sequence");
   auto out = torch::empty_like(q);
-  // the ranges of a head meet in a per-device workspace (grow-only, zero-filled when created; launches of one
-  // stream follow one another, which is how the decode harness calls this)
+  // the ranges of a head meet in a per-device workspace (launches of one stream follow one another, which is how the
+  // decode harness calls this)
   const size_t need = cq_attn_decode_workspace_bytes(B, (int)q.size(1), (int)q.size(2), (int)k_cache.size(cd - 3));
-  torch::Tensor ws;
-  {
-    std::lock_guard<std::mutex> lock(g_mu);
-    auto& slot = g_attn_ws[q.device().index()];
-    if (!slot.defined() || (size_t)slot.numel() < need)
-      slot = torch::zeros({(int64_t)need}, torch::TensorOptions().device(q.device()).dtype(torch::kUInt8));
-    ws = slot;
-  }
+  torch::Tensor keep;
+  void* ws = attn_workspace(q.device(), (size_t)B * q.size(1), need, &keep);
   check_status(cq_attn_decode(q.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), (const long long*)position.data_ptr(),
                               out.data_ptr(), B, (int)q.size(1), (int)k_cache.size(cd - 2), (int)q.size(2),
-                              (int)k_cache.size(cd - 3), 1.0f / std::sqrt((float)q.size(2)), ws.data_ptr(), current_stream()),
+                              (int)k_cache.size(cd - 3), 1.0f / std::sqrt((float)q.size(2)), ws, current_stream()),
                "attn_decode");
   return out;
 }

@@ -143,3 +143,43 @@ def test_attention_keeps_nan_scores(D, H, KV, max_seq, at, bad):
         s = torch.einsum("hd,pd->hp", q[0, :H // KV].float(), k[0, keep, 0].float()) / math.sqrt(D)
         ref = s.softmax(-1) @ v[0, keep, 0].float()
         assert float((out[:H // KV].float() - ref).abs().max()) <= 4e-3
+
+
+def test_attention_calls_of_different_sizes_share_a_workspace():
+    """Many heads after few: what the earlier calls left in the workspace is not taken for counters.  Also a call that is
+    first made under capture, and a graph that is replayed after the workspace has grown."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+
+    def case(B, H, D, max_seq, at):
+        g = torch.Generator(device="cuda").manual_seed(B + H + D)
+        q = torch.randn(B, H, D, device="cuda", generator=g).half()
+        k, v = (torch.randn(B, max_seq, H, D, device="cuda", generator=g).half() for _ in range(2))
+        s = torch.einsum("bhd,bphd->bhp", q.float(), k[:, :at + 1].float()) / math.sqrt(D)
+        ref = torch.einsum("bhp,bphd->bhd", s.softmax(-1), v[:, :at + 1].float()).half()
+        return (q, k, v, torch.full((B,), at, device="cuda")), ref
+
+    def right(out, ref):
+        assert float((out.view_as(ref) - ref).abs().max()) <= 4e-3         # as in test_attention_sweep_edges
+
+    first, ref_first = case(1, 8, 128, 1024, 1000)
+    qc.attn_decode(*first)
+    stream = torch.cuda.Stream()
+    graph, inner = torch.cuda.CUDAGraph(), torch.cuda.CUDAGraph()
+    late, ref_late = case(7, 40, 64, 4096, 4000)
+    with torch.cuda.stream(stream):
+        stream.wait_stream(torch.cuda.default_stream())
+        with torch.cuda.graph(graph, stream=stream):
+            out_first = qc.attn_decode(*first)
+        with torch.cuda.graph(inner, stream=stream):
+            out_late = qc.attn_decode(*late)
+    torch.cuda.synchronize()
+    for B, H, D, max_seq, at in ((1, 40, 128, 4096, 4000), (4, 40, 128, 512, 300), (8, 16, 64, 1024, 1000), (2, 8, 256, 700, 650),
+                                 (8, 32, 64, 600, 599), (3, 5, 32, 2000, 1999)):
+        args, ref = case(B, H, D, max_seq, at)
+        for _ in range(2):
+            right(qc.attn_decode(*args), ref)
+        for gr, out, want in ((graph, out_first, ref_first), (inner, out_late, ref_late)):
+            out.fill_(float("nan"))
+            gr.replay()
+            right(out, want)
