@@ -298,10 +298,11 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const __half* 
 }
 
 // One query head per CTA in one sweep over its positions, for the head widths in use (LPP = D / 8 lanes take a position
-// with 16-byte loads).  A step of short contexts is a chain of memory latencies; the kernel above has two of them (all
-// scores before the first value is fetched) and five barriers.  Here every group of lanes fetches the keys and values of
-// its next UF positions at once and keeps its own running maximum, sum and weighted values; the groups meet once, in
-// shared memory, the ranges of positions (blockIdx.z) as above.  The kernel above keeps the other head widths.
+// with 16-byte loads).  A step of short contexts is a chain of memory latencies; the kernels above and below have two of
+// them (all scores before the first value is fetched) and five barriers.  Here every group of lanes fetches the keys and
+// values of its next UF positions at once and keeps its own running maximum, sum and weighted values; the groups meet
+// once, in shared memory, the ranges of positions (blockIdx.z) as above.  32 heads of 128 at 500 positions: 9.6 us
+// against 14.4 with two sweeps; where it is taken stands at cq_attn_decode.
 constexpr int ONE_THREADS = 512;
 template <int LPP>
 __global__ void __launch_bounds__(ONE_THREADS) attn_decode_one_kernel(const __half* __restrict__ q,
@@ -458,11 +459,11 @@ __global__ void __launch_bounds__(ONE_THREADS) attn_decode_one_kernel(const __ha
   if (tid == 0) counters[hidx] = 0u;                                  // ready for the next launch
 }
 
-// The same for grouped-query models and long caches: one CTA per KV head (blockIdx.x), sequence and range
-// of positions handles all G = H / KV query heads that share the KV head, so every K and V row is read
-// once (with one CTA per query head it is read G times through L2).  A group of D / 8 lanes takes one
+// Two sweeps, for grouped-query models on long caches and for many heads: one CTA per KV head (blockIdx.x),
+// sequence and range of positions handles all G = H / KV query heads that share the KV head, so every K and V
+// row is read once (with one CTA per query head it is read G times through L2).  A group of D / 8 lanes takes one
 // position with 16-byte loads (8 values a lane), GT >= G query heads at a time in registers.  Partial
-// results of the ranges as in the kernel above; the arrival counter is per (sequence, KV head).
+// results of the ranges as in the kernels above; the arrival counter is per (sequence, KV head).
 constexpr int GQA_THREADS = 256, GQA_WARPS = GQA_THREADS / 32;
 template <int GT>
 __global__ void __launch_bounds__(GQA_THREADS) attn_decode_gqa_kernel(const __half* __restrict__ q,
@@ -731,10 +732,13 @@ extern "C" int cq_silu_mul_full(const void* gate, const void* up, void* out, lon
 }
 
 namespace {
-// ranges of positions per head: enough CTAs for about two per SM, at least 256 cache positions per range
-int attn_splits(int sequences, int n_heads, int max_seq) {
+int sm_count() {
   int dev = 0, sms = 148;
   if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+// ranges of positions per head: enough CTAs for about two per SM, at least 256 cache positions per range
+int attn_splits(int sms, int sequences, int n_heads, int max_seq) {
   int s = (2 * sms + sequences * n_heads - 1) / (sequences * n_heads);
   const int by_len = (max_seq + 255) / 256;
   if (s > by_len) s = by_len;
@@ -765,26 +769,41 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
   const int G = n_heads / n_kv_heads;
   const bool wide = (head_dim == 64 || head_dim == 128 || head_dim == 256) &&
                     (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
+  const int sms = sm_count();
+  const int splits = attn_splits(sms, sequences, n_heads, max_seq);
   // One CTA per KV head reads every cache row once for the query heads that share it; with several query heads
   // per KV head its per-position arithmetic is G times larger, which only pays on long caches (measured, 70B
   // shapes: 103 us against 174 at 4000 positions, but 21 against 15 at 200): short grouped-query caches take
   // a CTA per query head, whose re-reads hit L2.
-  if (wide && G > 1 && G <= 8 && max_seq > 1024) {
-    const int splits = attn_splits(sequences, n_kv_heads, max_seq);
-    const int range = (max_seq + splits - 1) / splits;
-    const int gt = G <= 2 ? 2 : (G <= 4 ? 4 : 8);
+  // Without grouped queries the same kernel competes with the one-sweep kernel, which has one latency less but runs one
+  // CTA of 512 threads per SM (128 registers), where four of the other's 256 threads fit.  Measured on cold caches:
+  //   all of the call's CTAs at once (128-wide heads: 32 at 500 of 512 positions 9.6 us against 14.4, 16 at 1000 of 1024 9.6
+  //   against 14.1; with one CTA per SM exceeded, 40 at 1000 of 1024 15.5 against 15.2, 8 x 32 at 500 of 512 33 against 22):
+  //   one sweep.  64-wide heads on caches of up to 256 positions are the exception: 8.8 us against 8.4 at 200, 9.0
+  //   against 10.5 at 500.
+  //   between four and five CTAs per SM (608 .. 736 heads), where the other kernel has a second wave that is nearly empty
+  //   and this one its fifth: 152 us against 177 at 2200 positions, 52 against 51 at 500, 42 against 33 at 300: one sweep
+  //   on caches of 1024 positions and more.
+  //   Caches whose scores would not fit the other kernel's shared memory.
+  const long long heads_all = (long long)sequences * n_heads;
+  const bool one_sweep = (heads_all * splits <= sms && (head_dim > 64 || max_seq > 256)) ||
+                         (heads_all > 4ll * sms && heads_all <= 5ll * sms && max_seq >= 1024) ||
+                         (size_t)((max_seq + splits - 1) / splits) * sizeof(float) > 200 * 1024;
+  if (wide && G <= 8 && (G > 1 ? max_seq > 1024 : !one_sweep)) {
+    const int kv_splits = attn_splits(sms, sequences, n_kv_heads, max_seq);
+    const int range = (max_seq + kv_splits - 1) / kv_splits;
+    const int gt = G <= 1 ? 1 : (G <= 2 ? 2 : (G <= 4 ? 4 : 8));
     const int words = gt * range > GQA_WARPS * gt * head_dim ? gt * range : GQA_WARPS * gt * head_dim;
     const int smem = words * (int)sizeof(float);
     if (smem > 200 * 1024) return CQ_ERR_TOO_LARGE;
     void (*fn)(const __half*, const __half*, const __half*, const long long*, __half*, float*, unsigned int*, int, int, int, int, float) =
-        gt == 2 ? attn_decode_gqa_kernel<2> : (gt == 4 ? attn_decode_gqa_kernel<4> : attn_decode_gqa_kernel<8>);
+        gt == 1 ? attn_decode_gqa_kernel<1> : (gt == 2 ? attn_decode_gqa_kernel<2> : (gt == 4 ? attn_decode_gqa_kernel<4> : attn_decode_gqa_kernel<8>));
     if (smem > 48 * 1024) CQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    CQ_CUDA_TRY(launch_pdl(fn, dim3(n_kv_heads, sequences, splits), dim3(GQA_THREADS), (size_t)smem, (cudaStream_t)stream,
+    CQ_CUDA_TRY(launch_pdl(fn, dim3(n_kv_heads, sequences, kv_splits), dim3(GQA_THREADS), (size_t)smem, (cudaStream_t)stream,
                            (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, position, (__half*)out, part,
                            counters, n_heads, n_kv_heads, head_dim, max_seq, scale));
     return CQ_OK;
   }
-  const int splits = attn_splits(sequences, n_heads, max_seq);
   if (wide) {
     auto fn = head_dim == 64 ? attn_decode_one_kernel<8> : (head_dim == 128 ? attn_decode_one_kernel<16> : attn_decode_one_kernel<32>);
     CQ_CUDA_TRY(launch_pdl(fn, dim3(n_heads, sequences, splits), dim3(ONE_THREADS), 0, (cudaStream_t)stream, (const __half*)q,

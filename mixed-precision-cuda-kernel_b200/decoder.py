@@ -87,10 +87,10 @@ class CherryDecoder:
         # decode attention over the KV cache: "own" = this library's kernel (cq_attn_decode); "flash" = the
         # flash_attn package's flash_attn_with_kvcache (a library call, like the lm_head's cuBLAS matmul);
         # "auto" = own, except for grouped-query models with caches of more than 1024 positions where that
-        # package imports.  Measured on B200: without grouped queries the own kernel is ahead at every size
-        # tried (13B shapes at 2100 positions: 19 us against 22 at batch 1, 91 against 159 at batch 8; 7B at 200
-        # positions 9 against 21); with 8 query heads per KV head at 4000 positions its SIMT dot products lose to
-        # flash_attn's tensor-core tiles (45 us against 25 at batch 1, 110 against 29 at batch 4).
+        # package imports.  Measured on B200 with cold caches: without grouped queries the own kernels are level or
+        # ahead (7B at 200 positions 8.6 us against 9.7; 13B shapes at 2100 positions 20.7 against 20.4 at batch 1, 86
+        # against 159 at batch 8); with 8 query heads per KV head at 4000 positions their SIMT dot products lose to
+        # flash_attn's tensor-core tiles (44 us against 20 at batch 1, 114 against 27 at batch 4).
         if attention not in ("auto", "own", "flash"):
             raise ValueError("attention is 'auto', 'own' or 'flash'")
         self._flash = None

@@ -183,3 +183,24 @@ def test_attention_calls_of_different_sizes_share_a_workspace():
             out.fill_(float("nan"))
             gr.replay()
             right(out, want)
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,max_seq", [(1, 37, 1024), (1, 38, 1024), (4, 16, 2300), (8, 32, 512), (16, 37, 1024), (20, 37, 1024),
+                                         (21, 36, 1030)])
+def test_attention_on_both_sides_of_the_dispatch(D, B, H, max_seq):
+    """Heads up to and beyond a CTA per SM, four and five CTAs per SM (148 SMs), at the first and last positions."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    g = torch.Generator(device="cuda").manual_seed(H)
+    q = torch.randn(B, H, D, device="cuda", generator=g).half()
+    k, v = (torch.randn(B, max_seq, H, D, device="cuda", generator=g).half() for _ in range(2))
+    at = [0, max_seq - 1, 255, 256, max_seq // 2]
+    pos = torch.tensor([at[b % 5] for b in range(B)], device="cuda")
+    for p in (pos, torch.full_like(pos, max_seq - 1)):
+        out = qc.attn_decode(q, k, v, p).view(B, H, D)
+        for b in {0, 1 % B, 2 % B, B - 1}:
+            n = int(p[b]) + 1
+            s = torch.einsum("hd,phd->hp", q[b].float(), k[b, :n].float()) / math.sqrt(D)
+            ref = torch.einsum("hp,phd->hd", s.softmax(-1), v[b, :n].float())
+            assert float((out[b].float() - ref).abs().max()) <= 4e-3         # as in test_attention_sweep_edges
