@@ -34,7 +34,10 @@
 //               a few hundred cycles, so they are two and keep their addresses and phases without a division
 //   warps 19-22 epilogue: tcgen05.ld of a finished tile into shared memory (which frees the accumulator), then
 //               16-byte stores to y
-// Every wait is bounded and reports into the status word instead of hanging.
+// Every wait is bounded and reports into the status word instead of hanging.  The kernel may be resident while kernels
+// before the pre-pass still run (an exchange that waits for a late rank for seconds, say), so a role starts to wait for
+// anything that depends on the activations only once it has passed the dependency wait; what comes before that are the
+// weights, which depend on nothing.
 //
 // Bound and state: 4096 -> 11008 4-bit, 2048 rows: 140 us = 1.32 PFLOP/s (739 us through QuantLinear and 195 us by itself
 // with lone CTAs of 128 x 256 tiles); 8192 -> 28672 3-bit, 2048 rows: 641 us = 1.50 PFLOP/s, tensor-bound.  16 rows: 18 and
@@ -125,6 +128,8 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
                ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
 }
+// until the kernels before this one have finished and their writes are visible
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ uint32_t hfma2_u32(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t d;
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(d) : "r"(a), "r"(b), "r"(c));
@@ -463,7 +468,10 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         const uint8_t* src = p.stream + (size_t)tile * p.tile_bytes + (size_t)c0 * CQT_CHER_BYTES + (size_t)(w.j0 - c0) * p.gran_bytes;
         for (uint32_t j = w.j0; j < w.j1; ++j) {
           const uint32_t bytes = j < NCH ? (uint32_t)CQT_CHER_BYTES : (uint32_t)p.gran_bytes;
-          if (ring.round) mbar_wait(B_WEMPTY(ring.slot), ring.phase ^ 1, &s_abort, p.status, 1u);
+          if (ring.round) {
+            if (ring.round == 1 && ring.slot == 0) dependency_wait();      // the ring is full: it drains with the activations
+            mbar_wait(B_WEMPTY(ring.slot), ring.phase ^ 1, &s_abort, p.status, 1u);
+          }
           if (*(volatile int*)&s_abort) break;
           mbar_expect_tx(B_WFULL(ring.slot), bytes);
           bulk_g2s(wring + ring.slot * (uint32_t)p.wstage_bytes, src, bytes, B_WFULL(ring.slot));
@@ -479,7 +487,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     // ================================================================ activation producer
     if (lane == 0) {
       // the staged activations are written by the kernel launched just before this one
-      asm volatile("griddepcontrol.wait;" ::: "memory");
+      dependency_wait();
       const uint32_t bring = smem_u32(smem + p.off_bring);
       Ring ring;
       WorkList wl(p, cluster, n_clusters, IPT);
@@ -515,6 +523,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
   } else if (warp == W_MMA) {
     if (rank == 0) {
       // ================================================================ MMA issuer (leader CTA)
+      dependency_wait();
       // The whole warp walks the list and one elected lane issues: addresses and descriptors then stay in uniform
       // registers, where the MMA takes them (all of tensor memory is allocated, so its base is column 0).
       // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = NT, M = 256
@@ -597,6 +606,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(B_WEMPTY(sw));
+        if (turn == 1) dependency_wait();
         if (turn) mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_abort, p.status, 64u);
         ++turn;
         tc_fence_after();
@@ -629,13 +639,19 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         if (lane == 0) {
           // The group's first warp also answers for the activation tile.  (No wait by parity comes a round early: the
           // MMAs of item n - 4 are done, so the slot's last tile, of an item n - SB <= n - 4, has landed.)
-          if ((warp & 3) == 0) mbar_wait(B_BFULL(sb), bphase, &s_abort, p.status, 16u);
+          if ((warp & 3) == 0) {
+            if (turn == 1) dependency_wait();
+            mbar_wait(B_BFULL(sb), bphase, &s_abort, p.status, 16u);
+          }
           if (rank == 0) mbar_arrive(ready);
           else mbar_arrive_cluster(ready);
         }
       }
     }
-    if (turn) mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_abort, p.status, 64u);
+    if (turn) {
+      dependency_wait();
+      mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_abort, p.status, 64u);
+    }
   } else {
     // ================================================================ epilogue (last four warps)
     const int quad = warp & 3;                              // the tensor-memory lanes this warp may read
@@ -645,7 +661,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     const int ewarp = etid >> 5;
     __half* stage = reinterpret_cast<__half*>(smem + p.off_stage);      // [token][128 rows]
     auto epi_sync = [&]() { asm volatile("bar.sync 2, 128;" ::: "memory"); };
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    dependency_wait();
     uint32_t lu = 0;
     WorkList wl(p, cluster, n_clusters, IPT);
     Work w;

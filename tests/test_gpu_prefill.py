@@ -195,3 +195,36 @@ def test_gemm_weights_are_unpacked_exactly_at_every_scale(cabi, bits, G):
     p = TilePrepared(cabi, pk["qweight"], scales, pk["cherry_weight"], pk["cherry_indices"], bits, K, G)
     y = gemm(cabi, p, torch.eye(K, device="cuda").half())
     assert torch.equal(y.T, dev(dense))
+
+
+@pytest.mark.parametrize("M", [16, 300])
+def test_gemm_behind_a_kernel_that_waits_for_long(cabi, M):
+    """Programmatic launches let the GEMM start while an exchange two kernels before it still waits, here for a rank that
+    does not exist and 1.5 s long: longer than the GEMM's own waits may last, which only begin afterwards."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    lib = cabi.lib()
+    K, N = 2048, 1024
+    w, idx, pk, dense = make_case(K, N, 4, 128, seed=M)
+    p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], 4, K, 128)
+    h = torch.randn(M, K, device="cuda").half()
+    ones = torch.ones(K, dtype=torch.float16, device="cuda")
+    want = gemm(cabi, p, qc.rmsnorm(h, None, ones, 1e-5, False)[0])
+    region = C.c_void_p()
+    cabi.check(lib.cq_peer_region_create(1 << 20, C.byref(region)), "create")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    x = torch.randn(1, 256, device="cuda").half()
+    out = torch.zeros(1, 512, dtype=torch.float16, device="cuda")
+    y = torch.zeros_like(want)
+    ws = torch.empty(lib.cq_tlayer_gemm_workspace_bytes(C.byref(p.L), M), dtype=torch.uint8, device="cuda")
+    torch.cuda.synchronize()
+    stream = C.c_void_p(torch.cuda.current_stream().cuda_stream)
+    regions = (C.c_void_p * 2)(region.value, region.value)
+    cabi.check(lib.cq_peer_allgather(regions, 2, 0, 1 << 20, ptr(x), ptr(out), 1, 256, 1500, ptr(status), stream), "exchange")
+    xn = qc.rmsnorm(h, None, ones, 1e-5, False)[0]
+    cabi.check(lib.cq_tlayer_gemm(C.byref(p.L), ptr(xn), K, ptr(y), N, M, 0, ptr(ws), ptr(p.status), stream), "gemm")
+    torch.cuda.synchronize()
+    cabi.check(lib.cq_peer_region_destroy(region), "destroy")
+    assert int(status.item()) & 8                                  # the exchange ran into its limit
+    assert int(p.status.item()) == 0
+    assert torch.equal(y, want)
