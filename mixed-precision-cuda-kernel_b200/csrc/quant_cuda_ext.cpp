@@ -11,6 +11,7 @@
 //     reference's 3-bit op silently does nothing for an unsupported group size).
 // The first matmul call with a given set of weight tensors re-packs them on the GPU
 // (allocates and synchronises), so it must happen before any stream capture.
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -280,10 +281,32 @@ torch::Tensor scratch_for(const torch::Device& dev) {
   return it->second;
 }
 
+// The device memory of a re-packed layer, and the stream that it was allocated on.  Launches on any stream read it.  Those
+// on its own need no record (the allocator gives a freed block out in that stream's order); one on another stream is
+// recorded, so that the block is not given out before it ends.
+struct LayerBlob {
+  torch::Tensor t;
+  c10::optional<c10::cuda::CUDAStream> home;
+
+  // A re-pack is finished before the first launch (which reads weights ahead of stream order, or runs on another stream),
+  // and a captured one would only run with the graph: neither can happen under capture.
+  void allocate(uint64_t bytes, const torch::TensorOptions& options, const char* what) {
+    TORCH_CHECK(c10::cuda::currentStreamCaptureStatusMayInitCtx() == c10::cuda::CaptureStatus::None, what,
+                ": the first call of a layer re-packs its weights and cannot be captured; call it once before the capture");
+    home = c10::cuda::getCurrentCUDAStream();
+    t = torch::empty({(int64_t)bytes}, options);
+  }
+  void finish() const { home->synchronize(); }
+  void use() const {
+    const auto now = c10::cuda::getCurrentCUDAStream(t.device().index());
+    if (!home || now != *home) c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), now);
+  }
+};
+
 // A layer re-packed into the stream layout; owns its device blob.
 struct PreparedLayer {
   cq_layer layer;
-  torch::Tensor blob;
+  LayerBlob blob;
 
   PreparedLayer(torch::Tensor qweight, torch::Tensor scales, torch::Tensor cherry_weight,
                 torch::Tensor cherry_indices, int bits, int in_features, int group_size) {
@@ -297,13 +320,12 @@ struct PreparedLayer {
     TORCH_CHECK(qweight.size(0) == layer.Kc / 8 * bits, "qweight has ", qweight.size(0), " rows, expected ",
                 layer.Kc / 8 * bits);
     TORCH_CHECK(scales.size(0) == (layer.Kc + layer.G - 1) / layer.G && scales.size(1) == N, "scales must be (ceil(K'/G), N)");
-    blob = torch::empty({(int64_t)layer.blob_bytes}, qweight.options());
-    layer.blob = blob.data_ptr();
+    blob.allocate(layer.blob_bytes, qweight.options(), "PreparedLayer");
+    layer.blob = blob.t.data_ptr();
     check_status(cq_layer_prepare(&layer, qweight.data_ptr<uint8_t>(), scales.data_ptr(), cherry_weight.data_ptr(),
                                   (const int16_t*)cherry_indices.data_ptr(), current_stream()),
                  "PreparedLayer");
-    // the matvec prefetches weights ahead of stream order: finish the re-pack first
-    c10::cuda::getCurrentCUDAStream().synchronize();
+    blob.finish();
   }
 
   // A layer rebuilt around an existing blob (e.g. loaded from a file or sliced from a shard).
@@ -312,18 +334,19 @@ struct PreparedLayer {
     check_status(cq_layer_init(&layer, bits, in_features, out_features, num_cherries, group_size, nullptr), "PreparedLayer");
     TORCH_CHECK((uint64_t)blob_.numel() == layer.blob_bytes, "blob has ", blob_.numel(), " bytes, expected ", layer.blob_bytes);
     TORCH_CHECK(((uintptr_t)blob_.data_ptr() & 255) == 0, "blob must be 256-byte aligned");
-    blob = blob_;
-    layer.blob = blob.data_ptr();
+    blob.t = blob_;
+    layer.blob = blob.t.data_ptr();
   }
 
   // out (M, N) fp16 = [out +] x (M, K) fp16 . W^T
   void matvec(torch::Tensor x, torch::Tensor out, bool accumulate) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
-    check_tensor(x, "x", torch::kFloat16, blob);
-    check_tensor(out, "out", torch::kFloat16, blob);
+    check_tensor(x, "x", torch::kFloat16, blob.t);
+    check_tensor(out, "out", torch::kFloat16, blob.t);
     TORCH_CHECK(x.dim() == 2 && x.size(1) == layer.K, "x must be (M, ", layer.K, ")");
     TORCH_CHECK(out.dim() == 2 && out.size(0) == x.size(0) && out.size(1) == layer.N, "out must be (M, ", layer.N, ")");
     auto scratch = scratch_for(x.device());
+    blob.use();
     uint8_t* sp = scratch.data_ptr<uint8_t>();
     check_status(cq_layer_matvec(&layer, x.data_ptr(), layer.K, out.data_ptr(), layer.N, (int)x.size(0),
                                  accumulate ? 1 : 0, sp, (uint32_t*)(sp + cq_scratch_bytes()), current_stream()),
@@ -332,8 +355,9 @@ struct PreparedLayer {
 
   // Back to the reference's four buffers: (qweight, scales, cherry_weight, cherry_indices).
   std::vector<torch::Tensor> unprepare() {
-    const at::cuda::OptionalCUDAGuard device_guard(device_of(blob));
-    auto o = blob.options();
+    const at::cuda::OptionalCUDAGuard device_guard(device_of(blob.t));
+    auto o = blob.t.options();
+    blob.use();
     auto qweight = torch::empty({layer.Kc / 8 * layer.bits, layer.N}, o);
     auto scales = torch::empty({(layer.Kc + layer.G - 1) / layer.G, layer.N}, o.dtype(torch::kFloat16));
     auto cw = torch::empty({layer.C, layer.N}, o.dtype(torch::kFloat16));
@@ -348,7 +372,7 @@ struct PreparedLayer {
 // A layer re-packed into the row-tile layout of the one-row decode kernel; owns its device blob.
 struct RowLayer {
   cq_rlayer layer;
-  torch::Tensor blob;
+  LayerBlob blob;
 
   // rows up to which such a layer takes the row kernel on the current device; 0 = the kernel does not take it
   static int row_limit(int bits, int in_features, int out_features, int num_cherries, int group_size) {
@@ -373,24 +397,24 @@ struct RowLayer {
     TORCH_CHECK(qweight.size(0) == layer.Kc / 8 * bits, "qweight has ", qweight.size(0), " rows, expected ",
                 layer.Kc / 8 * bits);
     TORCH_CHECK(scales.size(0) == (layer.Kc + layer.G - 1) / layer.G && scales.size(1) == N, "scales must be (ceil(K'/G), N)");
-    blob = torch::empty({(int64_t)layer.blob_bytes}, qweight.options());
-    layer.blob = blob.data_ptr();
+    blob.allocate(layer.blob_bytes, qweight.options(), "RowLayer");
+    layer.blob = blob.t.data_ptr();
     check_status(cq_rlayer_prepare(&layer, qweight.data_ptr<uint8_t>(), scales.data_ptr(), cherry_weight.data_ptr(),
                                    (const int16_t*)cherry_indices.data_ptr(), current_stream()),
                  "RowLayer");
-    // the kernel copies weights ahead of stream order: finish the re-pack first
-    c10::cuda::getCurrentCUDAStream().synchronize();
+    blob.finish();
   }
 
   // out (M, N) fp16 = [out +] x (M, K) fp16 . W^T; four rows per launch
   void matvec(torch::Tensor x, torch::Tensor out, bool accumulate) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
-    check_tensor(x, "x", torch::kFloat16, blob);
-    check_tensor(out, "out", torch::kFloat16, blob);
+    check_tensor(x, "x", torch::kFloat16, blob.t);
+    check_tensor(out, "out", torch::kFloat16, blob.t);
     TORCH_CHECK(x.numel() % layer.K == 0 && x.numel() > 0, "x must hold rows of ", layer.K, " activations");
     const int M = (int)(x.numel() / layer.K);
     TORCH_CHECK(out.numel() == (int64_t)M * layer.N, "out must hold ", M, " rows of ", layer.N, " values");
     auto scratch = scratch_for(x.device());
+    blob.use();
     uint8_t* sp = scratch.data_ptr<uint8_t>();
     const cq_rlayer* lp = &layer;
     void* yp = out.data_ptr();
@@ -402,14 +426,15 @@ struct RowLayer {
   // out (M, N) fp16 = (silu(gate) * up) (M, K) . W^T: the SwiGLU of a gated MLP folded into the down projection
   void matvec_swiglu(torch::Tensor gate, torch::Tensor up, torch::Tensor out) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(gate));
-    check_tensor(gate, "gate", torch::kFloat16, blob);
-    check_tensor(up, "up", torch::kFloat16, blob);
-    check_tensor(out, "out", torch::kFloat16, blob);
+    check_tensor(gate, "gate", torch::kFloat16, blob.t);
+    check_tensor(up, "up", torch::kFloat16, blob.t);
+    check_tensor(out, "out", torch::kFloat16, blob.t);
     TORCH_CHECK(gate.sizes() == up.sizes() && gate.numel() % layer.K == 0 && gate.numel() > 0,
                 "gate and up must hold the same rows of ", layer.K, " values");
     const int M = (int)(gate.numel() / layer.K);
     TORCH_CHECK(out.numel() == (int64_t)M * layer.N, "out must hold ", M, " rows of ", layer.N, " values");
     auto scratch = scratch_for(gate.device());
+    blob.use();
     uint8_t* sp = scratch.data_ptr<uint8_t>();
     check_status(cq_rlayer_matvec_swiglu(&layer, gate.data_ptr(), up.data_ptr(), layer.K, out.data_ptr(), layer.N, M,
                                          (uint32_t*)(sp + cq_scratch_bytes()), current_stream()),
@@ -421,15 +446,16 @@ struct RowLayer {
   void matvec_gather(torch::Tensor x, torch::Tensor y_local, torch::Tensor y_all, std::vector<int64_t> regions, int rank,
                      int64_t capacity, int timeout_ms, torch::Tensor status) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
-    check_tensor(x, "x", torch::kFloat16, blob);
-    check_tensor(y_local, "y_local", torch::kFloat16, blob);
-    check_tensor(y_all, "y_all", torch::kFloat16, blob);
-    check_tensor(status, "status", torch::kInt32, blob);
+    check_tensor(x, "x", torch::kFloat16, blob.t);
+    check_tensor(y_local, "y_local", torch::kFloat16, blob.t);
+    check_tensor(y_all, "y_all", torch::kFloat16, blob.t);
+    check_tensor(status, "status", torch::kInt32, blob.t);
     TORCH_CHECK(x.numel() % layer.K == 0 && x.numel() > 0, "x must hold rows of ", layer.K, " activations");
     const int M = (int)(x.numel() / layer.K), P = (int)regions.size();
     TORCH_CHECK(y_local.numel() == (int64_t)M * layer.N && y_all.numel() == (int64_t)M * layer.N * P,
                 "y_local must be (M, N) and y_all (M, P * N)");
     std::vector<void*> rp(P);
+    blob.use();
     for (int i = 0; i < P; ++i) rp[i] = (void*)(uintptr_t)regions[i];
     check_status(cq_rlayer_matvec_gather(&layer, x.data_ptr(), layer.K, y_local.data_ptr(), M, rp.data(), P, rank,
                                          (size_t)capacity, y_all.data_ptr(), timeout_ms, (uint32_t*)status.data_ptr(),
@@ -439,8 +465,9 @@ struct RowLayer {
 
   // Back to the reference's four buffers: (qweight, scales, cherry_weight, cherry_indices).
   std::vector<torch::Tensor> unprepare() {
-    const at::cuda::OptionalCUDAGuard device_guard(device_of(blob));
-    auto o = blob.options();
+    const at::cuda::OptionalCUDAGuard device_guard(device_of(blob.t));
+    auto o = blob.t.options();
+    blob.use();
     auto qweight = torch::empty({layer.Kc / 8 * layer.bits, layer.N}, o);
     auto scales = torch::empty({(layer.Kc + layer.G - 1) / layer.G, layer.N}, o.dtype(torch::kFloat16));
     auto cw = torch::empty({layer.C, layer.N}, o.dtype(torch::kFloat16));
@@ -455,7 +482,7 @@ struct RowLayer {
 // A layer re-packed into the tile layout of the tensor-core GEMM (prefill and large batches); owns its blob.
 struct TileLayer {
   cq_tlayer layer;
-  torch::Tensor blob;
+  LayerBlob blob;
 
   TileLayer(torch::Tensor qweight, torch::Tensor scales, torch::Tensor cherry_weight, torch::Tensor cherry_indices,
             int bits, int in_features, int group_size) {
@@ -468,24 +495,26 @@ struct TileLayer {
     check_status(cq_tlayer_init(&layer, bits, in_features, N, C, group_size, nullptr), "TileLayer");
     TORCH_CHECK(qweight.size(0) == (in_features - C) / 8 * bits, "qweight has ", qweight.size(0), " rows, expected ",
                 (in_features - C) / 8 * bits);
-    blob = torch::empty({(int64_t)layer.blob_bytes}, qweight.options());
-    layer.blob = blob.data_ptr();
+    blob.allocate(layer.blob_bytes, qweight.options(), "TileLayer");
+    layer.blob = blob.t.data_ptr();
     check_status(cq_tlayer_prepare(&layer, qweight.data_ptr<uint8_t>(), scales.data_ptr(), cherry_weight.data_ptr(),
                                    (const int16_t*)cherry_indices.data_ptr(), current_stream()),
                  "TileLayer");
+    blob.finish();
   }
 
   // out (M, N) fp16 = [out +] x (M, K) fp16 . W^T, walked in slices of 4096 rows (bounds the workspace)
   void gemm(torch::Tensor x, torch::Tensor out, bool accumulate) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
-    check_tensor(x, "x", torch::kFloat16, blob);
-    check_tensor(out, "out", torch::kFloat16, blob);
+    check_tensor(x, "x", torch::kFloat16, blob.t);
+    check_tensor(out, "out", torch::kFloat16, blob.t);
     TORCH_CHECK(x.dim() == 2 && x.size(1) == layer.K, "x must be (M, ", layer.K, ")");
     TORCH_CHECK(out.dim() == 2 && out.size(0) == x.size(0) && out.size(1) == layer.N, "out must be (M, ", layer.N, ")");
     const int M = (int)x.size(0), CH = 4096;
     const int chunk = M < CH ? M : CH;
-    auto ws = torch::empty({(int64_t)cq_tlayer_gemm_workspace_bytes(&layer, chunk)}, blob.options());
+    auto ws = torch::empty({(int64_t)cq_tlayer_gemm_workspace_bytes(&layer, chunk)}, blob.t.options());
     auto scratch = scratch_for(x.device());
+    blob.use();
     uint8_t* sp = scratch.data_ptr<uint8_t>();
     const uint16_t* xp = (const uint16_t*)x.data_ptr();      // fp16 elements
     uint16_t* yp = (uint16_t*)out.data_ptr();
@@ -559,7 +588,7 @@ struct PackedForward {
     TORCH_CHECK(row || tile, "a layer without copies");
     K = row ? row->layer.K : tile->layer.K;
     N = row ? row->layer.N : tile->layer.N;
-    device = (row ? row->blob : tile->blob).device();
+    device = (row ? row->blob : tile->blob).t.device();
   }
 
   // None: this call takes the general path
@@ -595,7 +624,7 @@ struct PackedForward {
 void row_layers_matvec(std::vector<RowLayer*> layers, torch::Tensor x, std::vector<torch::Tensor> outs, bool accumulate) {
   TORCH_CHECK(!layers.empty() && layers.size() <= 4 && layers.size() == outs.size(), "1 to 4 layers, one output each");
   const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
-  check_tensor(x, "x", torch::kFloat16, layers[0]->blob);
+  check_tensor(x, "x", torch::kFloat16, layers[0]->blob.t);
   const int K = layers[0]->layer.K;
   TORCH_CHECK(x.numel() % K == 0 && x.numel() > 0, "x must hold rows of ", K, " activations");
   const int M = (int)(x.numel() / K);
@@ -616,6 +645,7 @@ void row_layers_matvec(std::vector<RowLayer*> layers, torch::Tensor x, std::vect
     ls[i] = &layers[i]->layer;
     ys[i] = o.data_ptr();
   }
+  for (const auto* l : layers) l->blob.use();
   auto scratch = scratch_for(x.device());
   uint8_t* sp = scratch.data_ptr<uint8_t>();
   check_status(cq_rlayers_matvec(ls, (int)layers.size(), x.data_ptr(), K, ys, (int)ldy, M, accumulate ? 1 : 0,
@@ -765,14 +795,14 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def("matvec_gather", &RowLayer::matvec_gather)
       .def("matvec_swiglu", &RowLayer::matvec_swiglu)
       .def("unprepare", &RowLayer::unprepare)
-      .def_readonly("blob", &RowLayer::blob)
+      .def_property_readonly("blob", [](const RowLayer& p) { return p.blob.t; })
       .def_property_readonly("preferred_rows", [](const RowLayer& p) { return cq_rlayer_preferred_rows(&p.layer); })
       .def_property_readonly("out_features", [](const RowLayer& p) { return p.layer.N; })
       .def_property_readonly("in_features", [](const RowLayer& p) { return p.layer.K; });
   py::class_<TileLayer>(m, "TileLayer")
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int, int, int>())
       .def("gemm", &TileLayer::gemm)
-      .def_readonly("blob", &TileLayer::blob);
+      .def_property_readonly("blob", [](const TileLayer& p) { return p.blob.t; });
   py::class_<BufferGuard>(m, "BufferGuard")
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor>())
       .def("holds", &BufferGuard::holds);
@@ -784,7 +814,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
       .def(py::init<torch::Tensor, int, int, int, int, int>())
       .def("matvec", &PreparedLayer::matvec)
       .def("unprepare", &PreparedLayer::unprepare)
-      .def_readonly("blob", &PreparedLayer::blob)
+      .def_property_readonly("blob", [](const PreparedLayer& p) { return p.blob.t; })
       .def_property_readonly("bits", [](const PreparedLayer& p) { return p.layer.bits; })
       .def_property_readonly("in_features", [](const PreparedLayer& p) { return p.layer.K; })
       .def_property_readonly("out_features", [](const PreparedLayer& p) { return p.layer.N; })

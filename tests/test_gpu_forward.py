@@ -204,3 +204,49 @@ def test_attention_on_both_sides_of_the_dispatch(D, B, H, max_seq):
             s = torch.einsum("hd,phd->hp", q[b].float(), k[b, :n].float()) / math.sqrt(D)
             ref = torch.einsum("hp,phd->hd", s.softmax(-1), v[b, :n].float())
             assert float((out[b].float() - ref).abs().max()) <= 4e-3         # as in test_attention_sweep_edges
+
+
+@pytest.mark.parametrize("m,C", [(1, 16), (40, 16), (3, 256)])     # row kernel, GEMM, stream matvec
+def test_copies_dropped_while_another_stream_uses_them(m, C):
+    """The block of a dropped copy is not given out before the launches that read it have finished, and is afterwards."""
+    lin = packed(2048, 520, 4, 128, 1, C=C)
+    x = torch.randn(m, 2048, device="cuda").half()
+    want = lin(x)
+    blob = (lin._row or lin._tile or lin._prepared).blob
+    ptr, size = blob.data_ptr(), blob.numel()
+    del blob
+    torch.cuda.synchronize()
+    side = torch.cuda.Stream()
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(400_000_000)                             # about 0.2 s
+        y = lin(x)
+    lin._drop_copies()
+    held = [torch.empty(size, dtype=torch.uint8, device="cuda").fill_(0xFF) for _ in range(4)]
+    assert not side.query(), "the test must look while the launch is pending"
+    assert all(t.data_ptr() != ptr for t in held)
+    torch.cuda.synchronize()
+    assert torch.equal(y, want)
+    del held
+    torch.cuda.empty_cache()
+    later = [torch.empty(size, dtype=torch.uint8, device="cuda") for _ in range(8)]
+    assert len(later) == 8 and torch.equal(lin(x), want)
+
+
+@pytest.mark.parametrize("m,C", [(1, 16), (40, 16), (3, 256)])
+def test_first_call_is_refused_under_capture(m, C):
+    """A captured re-pack would run with the graph only; the refusal leaves the capture and the layer usable."""
+    lin = packed(2048, 264, 4, 128, 2, C=C)
+    x = torch.randn(m, 2048, device="cuda").half()
+    dense = lin.unpack()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        z = x + 1
+        with pytest.raises(RuntimeError, match="before the capture"):
+            lin(x)
+    graph.replay()
+    assert torch.equal(z, x + 1)
+    check(lin, x, dense)
+    with torch.cuda.graph(graph := torch.cuda.CUDAGraph()):
+        y = lin(x)
+    graph.replay()
+    assert torch.equal(y, lin(x))
