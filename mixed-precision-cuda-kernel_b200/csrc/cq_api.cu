@@ -8,9 +8,11 @@
 // tensor-core GEMM.  A layer only pays for the layouts it is actually called with.
 // cq_cache_evict drops the copies of one buffer set (the torch shim calls it when
 // the tensors behind a cached address have been freed).
+#include <atomic>
 #include <map>
 #include <mutex>
 #include <tuple>
+#include <utility>
 #include <vector>
 
 #include "cq_common.cuh"
@@ -192,6 +194,31 @@ int legacy_matmul(int bits, const void* vec, const uint8_t* qweight, const void*
 }  // namespace
 
 void cq_set_cuda_error(int err) { g_last_cuda_error = err; }
+
+cudaError_t cq_grant_smem(const void* fn, int bytes) {
+  static std::mutex mu;
+  static std::map<std::pair<const void*, int>, int> granted;
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  std::lock_guard<std::mutex> lock(mu);
+  int& have = granted[{fn, dev}];
+  if (bytes > have) {
+    e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess) have = bytes;
+  }
+  return e;
+}
+
+int cq_sm_count() {
+  static std::atomic<int> count[64];
+  int dev = 0, sms = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+  if ((sms = count[dev].load(std::memory_order_relaxed)) > 0) return sms;
+  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms < 1) return 148;
+  count[dev].store(sms, std::memory_order_relaxed);
+  return sms;
+}
 
 extern "C" int cq_last_cuda_error(void) { return g_last_cuda_error; }
 extern "C" int cq_abi_version(void) { return 3; }

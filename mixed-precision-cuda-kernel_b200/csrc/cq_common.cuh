@@ -48,6 +48,12 @@
 // thread-local record of the last CUDA error (defined in cq_api.cu)
 void cq_set_cuda_error(int err);
 
+// Opts a kernel in to `bytes` of dynamic shared memory on the current device.  The limit belongs to the kernel, not to a
+// launch: it is only ever raised, or a thread with a smaller call would take it from another between its set and launch.
+cudaError_t cq_grant_smem(const void* fn, int bytes);
+// SMs of the current device
+int cq_sm_count();
+
 #define CQ_CUDA_TRY(expr)                       \
   do {                                          \
     cudaError_t _e = (expr);                    \

@@ -322,11 +322,12 @@ int cq_launch_matvec_f32(const float* x, const uint8_t* q, const float* cw, cons
   // Blocks per CTA: the split whose waves of two CTAs per SM take the fewest block times (a CTA's fixed part, x staging
   // set-up and the atomics, counts as one).  4096 x 13824, 16 rows: 8 blocks, one wave of 270.
   const int ny = (N + F32_COLS - 1) / F32_COLS;
+  const int slots = 2 * cq_sm_count();
   int per = 1;
   long long best = 0;
   for (int b = 1; b <= F32_MAX_BLOCKS; ++b) {
     const long long ctas = (long long)ny * ((p.n_blk + b - 1) / b + (C > 0 ? 1 : 0));
-    const long long t = (ctas + 2 * 148 - 1) / (2 * 148) * (b + 1);
+    const long long t = (ctas + slots - 1) / slots * (b + 1);
     if (b == 1 || t < best) {
       best = t;
       per = b;
@@ -341,7 +342,7 @@ int cq_launch_matvec_f32(const float* x, const uint8_t* q, const float* cw, cons
   const int smem = smem_main > smem_cherry ? smem_main : smem_cherry;
   const dim3 grid(p.n_parts + (C > 0 ? 1 : 0), ny);
   auto kernel = tt == 2 ? matvec_f32_kernel<2> : matvec_f32_kernel<1>;
-  CQ_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  CQ_CUDA_TRY(cq_grant_smem((const void*)kernel, smem));
   kernel<<<grid, F32_THREADS, smem, st>>>(p);
   CQ_CUDA_TRY(cudaGetLastError());
   return CQ_OK;

@@ -892,7 +892,7 @@ int plan_smem(const cq_layer* L, int M, int grid, int max_smem, int ncw, int tar
 // Opt in to the dynamic shared memory the plan needs, and ask for the largest shared-memory
 // carve-out so that a second CTA (the next launch in the stream) fits beside this one.
 cudaError_t prepare_kernel(KernelFn fn, int smem) {
-  cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  cudaError_t e = cq_grant_smem((const void*)fn, smem);
   if (e != cudaSuccess) return e;
   return cudaFuncSetAttribute(fn, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
 }

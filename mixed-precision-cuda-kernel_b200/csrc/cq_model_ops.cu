@@ -732,11 +732,6 @@ extern "C" int cq_silu_mul_full(const void* gate, const void* up, void* out, lon
 }
 
 namespace {
-int sm_count() {
-  int dev = 0, sms = 148;
-  if (cudaGetDevice(&dev) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  return sms;
-}
 // ranges of positions per head: enough CTAs for about two per SM, at least 256 cache positions per range
 int attn_splits(int sms, int sequences, int n_heads, int max_seq) {
   int s = (2 * sms + sequences * n_heads - 1) / (sequences * n_heads);
@@ -769,7 +764,7 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
   const int G = n_heads / n_kv_heads;
   const bool wide = (head_dim == 64 || head_dim == 128 || head_dim == 256) &&
                     (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
-  const int sms = sm_count();
+  const int sms = cq_sm_count();
   const int splits = attn_splits(sms, sequences, n_heads, max_seq);
   // One CTA per KV head reads every cache row once for the query heads that share it; with several query heads
   // per KV head its per-position arithmetic is G times larger, which only pays on long caches (measured, 70B
@@ -798,7 +793,7 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
     if (smem > 200 * 1024) return CQ_ERR_TOO_LARGE;
     void (*fn)(const __half*, const __half*, const __half*, const long long*, __half*, float*, unsigned int*, int, int, int, int, float) =
         gt == 1 ? attn_decode_gqa_kernel<1> : (gt == 2 ? attn_decode_gqa_kernel<2> : (gt == 4 ? attn_decode_gqa_kernel<4> : attn_decode_gqa_kernel<8>));
-    if (smem > 48 * 1024) CQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    CQ_CUDA_TRY(cq_grant_smem((const void*)fn, smem));
     CQ_CUDA_TRY(launch_pdl(fn, dim3(n_kv_heads, sequences, kv_splits), dim3(GQA_THREADS), (size_t)smem, (cudaStream_t)stream,
                            (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, position, (__half*)out, part,
                            counters, n_heads, n_kv_heads, head_dim, max_seq, scale));
@@ -814,8 +809,7 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
   const int range = (max_seq + splits - 1) / splits;
   const int smem = (range + ATT_THREADS) * (int)sizeof(float);
   if (smem > 200 * 1024) return CQ_ERR_TOO_LARGE;
-  if (smem > 48 * 1024)
-    CQ_CUDA_TRY(cudaFuncSetAttribute(attn_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  CQ_CUDA_TRY(cq_grant_smem((const void*)attn_decode_kernel, smem));
   CQ_CUDA_TRY(launch_pdl(attn_decode_kernel, dim3(n_heads, sequences, splits), dim3(ATT_THREADS), (size_t)smem,
                          (cudaStream_t)stream, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, position,
                          (__half*)out, part, counters, n_heads, n_kv_heads, head_dim, max_seq, scale));

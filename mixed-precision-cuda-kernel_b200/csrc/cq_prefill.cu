@@ -971,7 +971,7 @@ extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* 
   const int smem = off + p.sw * p.wstage_bytes;
 
   PKernelFn fn = ppick(L->bits, L->sets);
-  CQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+  CQ_CUDA_TRY(cq_grant_smem((const void*)fn, smem));
   cfg.gridDim = dim3(2 * used);
   cfg.blockDim = dim3(NTHREADS);
   cfg.dynamicSmemBytes = smem;

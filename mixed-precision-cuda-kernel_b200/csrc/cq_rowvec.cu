@@ -27,8 +27,6 @@
 //     cherry columns are one fp16 mma.sync.m16n8k16 per tile;
 //   * the warps' partial sums of a tile meet in shared memory and are added in a fixed order:
 //     no atomics, no scratch, no cross-CTA traffic, bit-identical runs.
-#include <map>
-#include <mutex>
 #include <utility>
 
 #include "cq_common.cuh"
@@ -1006,17 +1004,7 @@ int rv_launch(RowvecFn fn, int W, int GPW, const cq_rlayer* const* Ls, int n, co
   p.accumulate = accumulate;
   p.gather = peer ? 1 : 0;
   if (peer) p.peer = *peer; else p.peer = cq_peer::PeerGatherParams{};
-  {
-    // opt in to the dynamic shared memory this launch needs (remembered per kernel and device)
-    static std::mutex mu;
-    static std::map<std::pair<const void*, int>, int> granted;
-    std::lock_guard<std::mutex> lk(mu);
-    int& have = granted[{(const void*)fn, dev}];
-    if (smem > have) {
-      CQ_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-      have = smem;
-    }
-  }
+  CQ_CUDA_TRY(cq_grant_smem((const void*)fn, smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid);
   cfg.blockDim = dim3((W + 1) * 32);
