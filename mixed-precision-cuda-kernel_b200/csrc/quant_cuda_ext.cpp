@@ -303,6 +303,20 @@ struct LayerBlob {
   }
 };
 
+// The four reference buffers of a layer of which the re-pack kernels read Kc / 8 * bits x N codes, ceil(Kc / G) x N scales
+// and C x N cherry weights.
+void check_buffers(const torch::Tensor& qweight, const torch::Tensor& scales, const torch::Tensor& cherry_weight,
+                   const torch::Tensor& cherry_indices, int bits, int Kc, int G) {
+  check_tensor(qweight, "qweight", torch::kUInt8, qweight);
+  check_tensor(scales, "scales", torch::kFloat16, qweight);
+  check_tensor(cherry_weight, "cherry_weight", torch::kFloat16, qweight);
+  check_tensor(cherry_indices, "cherry_indices", torch::kInt16, qweight);
+  TORCH_CHECK(qweight.dim() == 2 && qweight.size(0) == Kc / 8 * bits, "qweight must be (", Kc / 8 * bits, ", N)");
+  const int64_t N = qweight.size(1);
+  TORCH_CHECK(scales.dim() == 2 && scales.size(0) == (Kc + G - 1) / G && scales.size(1) == N, "scales must be (ceil(K'/G), N)");
+  TORCH_CHECK(cherry_weight.numel() == cherry_indices.numel() * N, "cherry_weight must be (C, N)");
+}
+
 // A layer re-packed into the stream layout; owns its device blob.
 struct PreparedLayer {
   cq_layer layer;
@@ -311,15 +325,10 @@ struct PreparedLayer {
   PreparedLayer(torch::Tensor qweight, torch::Tensor scales, torch::Tensor cherry_weight,
                 torch::Tensor cherry_indices, int bits, int in_features, int group_size) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(qweight));
-    check_tensor(qweight, "qweight", torch::kUInt8, qweight);
-    check_tensor(scales, "scales", torch::kFloat16, qweight);
-    check_tensor(cherry_weight, "cherry_weight", torch::kFloat16, qweight);
-    check_tensor(cherry_indices, "cherry_indices", torch::kInt16, qweight);
+    TORCH_CHECK(qweight.dim() == 2, "qweight must be 2-D");
     const int N = (int)qweight.size(1), C = (int)cherry_indices.numel();
     check_status(cq_layer_init(&layer, bits, in_features, N, C, group_size, nullptr), "PreparedLayer");
-    TORCH_CHECK(qweight.size(0) == layer.Kc / 8 * bits, "qweight has ", qweight.size(0), " rows, expected ",
-                layer.Kc / 8 * bits);
-    TORCH_CHECK(scales.size(0) == (layer.Kc + layer.G - 1) / layer.G && scales.size(1) == N, "scales must be (ceil(K'/G), N)");
+    check_buffers(qweight, scales, cherry_weight, cherry_indices, bits, layer.Kc, layer.G);
     blob.allocate(layer.blob_bytes, qweight.options(), "PreparedLayer");
     layer.blob = blob.t.data_ptr();
     check_status(cq_layer_prepare(&layer, qweight.data_ptr<uint8_t>(), scales.data_ptr(), cherry_weight.data_ptr(),
@@ -387,16 +396,11 @@ struct RowLayer {
   RowLayer(torch::Tensor qweight, torch::Tensor scales, torch::Tensor cherry_weight, torch::Tensor cherry_indices,
            int bits, int in_features, int group_size) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(qweight));
-    check_tensor(qweight, "qweight", torch::kUInt8, qweight);
-    check_tensor(scales, "scales", torch::kFloat16, qweight);
-    check_tensor(cherry_weight, "cherry_weight", torch::kFloat16, qweight);
-    check_tensor(cherry_indices, "cherry_indices", torch::kInt16, qweight);
+    TORCH_CHECK(qweight.dim() == 2, "qweight must be 2-D");
     const int N = (int)qweight.size(1), C = (int)cherry_indices.numel();
     check_status(cq_rlayer_init(&layer, bits, in_features, N, C, group_size, nullptr), "RowLayer");
     check_status(cq_rlayer_check(&layer), "RowLayer");
-    TORCH_CHECK(qweight.size(0) == layer.Kc / 8 * bits, "qweight has ", qweight.size(0), " rows, expected ",
-                layer.Kc / 8 * bits);
-    TORCH_CHECK(scales.size(0) == (layer.Kc + layer.G - 1) / layer.G && scales.size(1) == N, "scales must be (ceil(K'/G), N)");
+    check_buffers(qweight, scales, cherry_weight, cherry_indices, bits, layer.Kc, layer.G);
     blob.allocate(layer.blob_bytes, qweight.options(), "RowLayer");
     layer.blob = blob.t.data_ptr();
     check_status(cq_rlayer_prepare(&layer, qweight.data_ptr<uint8_t>(), scales.data_ptr(), cherry_weight.data_ptr(),
@@ -487,14 +491,10 @@ struct TileLayer {
   TileLayer(torch::Tensor qweight, torch::Tensor scales, torch::Tensor cherry_weight, torch::Tensor cherry_indices,
             int bits, int in_features, int group_size) {
     const at::cuda::OptionalCUDAGuard device_guard(device_of(qweight));
-    check_tensor(qweight, "qweight", torch::kUInt8, qweight);
-    check_tensor(scales, "scales", torch::kFloat16, qweight);
-    check_tensor(cherry_weight, "cherry_weight", torch::kFloat16, qweight);
-    check_tensor(cherry_indices, "cherry_indices", torch::kInt16, qweight);
+    TORCH_CHECK(qweight.dim() == 2, "qweight must be 2-D");
     const int N = (int)qweight.size(1), C = (int)cherry_indices.numel();
     check_status(cq_tlayer_init(&layer, bits, in_features, N, C, group_size, nullptr), "TileLayer");
-    TORCH_CHECK(qweight.size(0) == (in_features - C) / 8 * bits, "qweight has ", qweight.size(0), " rows, expected ",
-                (in_features - C) / 8 * bits);
+    check_buffers(qweight, scales, cherry_weight, cherry_indices, bits, layer.Kc, layer.G);
     blob.allocate(layer.blob_bytes, qweight.options(), "TileLayer");
     layer.blob = blob.t.data_ptr();
     check_status(cq_tlayer_prepare(&layer, qweight.data_ptr<uint8_t>(), scales.data_ptr(), cherry_weight.data_ptr(),

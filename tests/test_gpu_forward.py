@@ -250,3 +250,12 @@ def test_first_call_is_refused_under_capture(m, C):
         y = lin(x)
     graph.replay()
     assert torch.equal(y, lin(x))
+
+
+@pytest.mark.parametrize("m,C", [(1, 16), (40, 16), (3, 256)])     # row kernel, GEMM, stream matvec
+@pytest.mark.parametrize("name", ["qweight", "scales", "cherry_weight"])
+def test_buffers_of_the_wrong_size_are_refused(m, C, name):
+    lin = packed(2048, 264, 4, 128, 3, C=C)
+    setattr(lin, name, getattr(lin, name)[:-2].clone())
+    with pytest.raises(RuntimeError, match=name):
+        lin(torch.zeros(m, 2048, device="cuda").half())
