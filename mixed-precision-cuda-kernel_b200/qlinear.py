@@ -114,6 +114,14 @@ class QuantLinear(nn.Module):
         self._row_rows = None
         self._prepared_key = None
 
+    def __getstate__(self):
+        """For copy and pickle: without the re-packed copies, which the other module makes again on first use.  (After a
+        release they are all there is of the weights, and cannot be pickled: restore the reference buffers first.)"""
+        state = self.__dict__.copy()
+        if self._prepared_key != "released":
+            state.update(_prepared=None, _row=None, _tile=None, _fast=None, _row_rows=None, _prepared_key=None)
+        return state
+
     def _sync_key(self):
         """Forgets the re-packed copies when the reference buffers were replaced or written to."""
         if self._prepared_key == "released":

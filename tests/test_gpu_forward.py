@@ -259,3 +259,19 @@ def test_buffers_of_the_wrong_size_are_refused(m, C, name):
     setattr(lin, name, getattr(lin, name)[:-2].clone())
     with pytest.raises(RuntimeError, match=name):
         lin(torch.zeros(m, 2048, device="cuda").half())
+
+
+@pytest.mark.parametrize("m", [1, 40])
+def test_forward_of_modules_with_parameters_and_of_copies(m):
+    """A reference buffer turned into a parameter, a deep copy made after a call: the same answers."""
+    import copy
+    lin = packed(1024, 264, 4, 128, 4)
+    x = torch.randn(m, 1024, device="cuda").half()
+    want = lin(x)
+    other = copy.deepcopy(lin)
+    assert torch.equal(other(x), want) and torch.equal(other(x), want)
+    lin.qweight = torch.nn.Parameter(lin.qweight.clone(), requires_grad=False)
+    for _ in range(3):
+        assert torch.equal(lin(x), want)
+    lin.qweight = torch.nn.Parameter(torch.zeros_like(lin.qweight), requires_grad=False)
+    assert not torch.equal(lin(x), want)

@@ -43,3 +43,23 @@ def test_copies_go_with_a_buffer_replaced_at_the_same_address(name):
         pytest.skip("the allocator did not hand the freed block back")
     lin._sync_key()
     assert lin._row is None and lin._tile is None
+
+
+def test_copy_and_pickle_leave_the_copies_behind():
+    """A module that has answered calls copies and pickles like one that has not; a released one is refused."""
+    import copy
+    import io
+    lin = layer()
+    lin._fast = lin._prepared = lock = __import__("threading").Lock()          # not to be pickled, like a copy on the GPU
+    lin.scales.fill_(2)
+    buf = io.BytesIO()
+    torch.save(lin, buf)
+    buf.seek(0)
+    for other in (copy.deepcopy(lin), copy.copy(lin), torch.load(buf, weights_only=False)):
+        assert all(torch.equal(getattr(other, n), getattr(lin, n)) for n in NAMES)
+        assert other._row is other._tile is other._fast is other._prepared is other._prepared_key is None
+        other._sync_key()
+    assert lin._tile == "copy" and lin._fast is lock
+    lin._prepared_key = "released"
+    with pytest.raises(TypeError):
+        copy.deepcopy(lin)
