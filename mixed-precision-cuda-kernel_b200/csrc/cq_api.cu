@@ -2,10 +2,10 @@
 // (csrc/quant_cuda.cpp:41-69 of the reference project) on top of the prepared
 // layer interfaces: the first call with a given set of reference buffers re-packs
 // them on the GPU into the layout of the kernel that serves the call's batch size
-// and caches the result.  One activation row: row-tile layout (cq_rlayer) when the
-// layer fits that kernel; 2..7 rows (and the layers it does not fit): stream layout
-// (cq_layer); 8 rows or more (large decode batches, prefill): tile layout and the
-// tensor-core GEMM.  A layer only pays for the layouts it is actually called with.
+// and caches the result.  Up to cq_rlayer_preferred_rows rows: row-tile layout (cq_rlayer);
+// larger batches and prefill: tile layout and the tensor-core GEMM (cq_tlayer).  Layers that
+// the row kernel does not take run on the stream layout (cq_layer) below 8 rows.  A layer only
+// pays for the layouts it is actually called with.
 // cq_cache_evict drops the copies of one buffer set (the torch shim calls it when
 // the tensors behind a cached address have been freed).
 #include <atomic>
@@ -129,7 +129,7 @@ int legacy_matmul(int bits, const void* vec, const uint8_t* qweight, const void*
   const CacheKey key{dev, qweight, scales, cherry_weight, cherry_indices, bits, vec_height, width,
                      cherry_size, group_size, tag};
   // decode batches: the row-tile kernel (four activation rows per launch) up to the batch where the tile
-  // GEMM overtakes it (8 rows, 4 for layers split along K); layers the row kernel does not take: the stream kernel
+  // GEMM overtakes it (cq_rlayer_preferred_rows); layers the row kernel does not take: the stream kernel
   // below 8 rows
   int row_limit = PREFILL_MIN_ROWS - 1;
   {

@@ -1165,10 +1165,13 @@ extern "C" int cq_rlayer_preferred_rows(const cq_rlayer* L) {
   if (!L) return 0;
   const int gpw = rv_gpw_for(L);
   if (!gpw) return 0;
-  // measured on B200 against the tile GEMM: 8 rows (two launches) take 14 / 19 / 52 us on 4096 -> 4096 / 4096 -> 11008 /
-  // 8192 -> 28672 against 14 / 19 / 52, 12 rows half as much again against the same; layers split along K stop at one
-  // launch: 11008 -> 4096 and 28672 -> 8192 take 15 / 40 us at 4 rows, 28 / 70 at 8, against 20 / 54
-  return L->ksplit > 1 ? 4 : 8;
+  // measured on B200 against the tile GEMM: 8 rows (two launches) take 15 / 19 / 54 us on 4096 -> 4096 / 4096 -> 11008 /
+  // 8192 -> 28672 against 14 / 19 / 54, 9 rows a quarter more against the same; layers split along K stop at one launch:
+  // 11008 -> 4096 takes 14 us at 4 rows, 23 at 5, against 19.  Of these the large 3-bit ones go on to 6 rows, since the
+  // GEMM's decode grows with the layer: 28672 -> 8192 52 us at 5 rows, 53 at 6, against 55; 16384 -> 16384 57 / 59
+  // against 61 (16384 -> 8192 36 / 38 against 36; 4 bits 58 / 62 against 57).
+  if (L->ksplit > 1) return L->bits == 3 && (long long)L->K * L->N >= 200000000ll ? 6 : 4;
+  return 8;
 }
 
 extern "C" int cq_rlayer_matvec(const cq_rlayer* L, const void* x, void* y, int accumulate, uint32_t* status_word,

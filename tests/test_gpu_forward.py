@@ -65,6 +65,15 @@ def test_forward_follows_the_buffers(bits, bias):
     assert not y.requires_grad
 
 
+def test_row_limits():
+    import cherryq_b200
+    limit = cherryq_b200.load_quant_cuda().RowLayer.row_limit
+    for args, rows in (((4, 4096, 4096, 16, 128), 8), ((3, 8192, 28672, 32, 128), 8), ((4, 11008, 4096, 40, 128), 4),
+                       ((3, 28672, 8192, 112, 128), 6), ((4, 28672, 8192, 112, 128), 4), ((3, 16384, 8192, 64, 128), 4),
+                       ((3, 16384, 16384, 64, 128), 6), ((4, 4096, 4096, 256, 128), 0), ((4, 4096, 4096, 16, 64), 0)):
+        assert limit(*args) == rows, args
+
+
 @pytest.mark.parametrize("K,C", [(2048, 16), (9216, 40), (2048, 256)])     # row kernel, the same split along K, stream matvec
 def test_kernel_does_not_depend_on_earlier_calls(K, C):
     """A prompt first, then decode batches: the bits of a layer that never saw the prompt, through every entry point."""
