@@ -145,8 +145,8 @@ def test_quant_cuda_ops_route_large_batches_to_the_gemm(qc, bits):
     (512, 392, 3, 128, 1), (1024, 136, 4, 128, 31), (2048, 1024, 3, 64, 33), (384, 4096, 4, 128, 127), (8192, 1024, 3, 128, 257),
     (2048, 2440, 4, 256, 513), (1024, 9600, 3, 128, 300), (256, 40, 4, 128, 2049)])
 def test_gemm_block_tile_and_run_edges(cabi, K, N, bits, G, M):
-    """Token blocks that end inside a step of 32, an odd number of row tiles (the pair's second CTA repeats one), units cut
-    into runs and whole ones in one call; twelve calls back to back on one workspace give the same bits."""
+    """Token blocks that end inside a step of 32, an odd number of row tiles (the pair's second CTA repeats one), calls of
+    whole units and calls whose units are all cut into runs; twelve calls back to back on one workspace give the same bits."""
     w, idx, pk, dense = make_case(K, N, bits, G, seed=K + M)
     p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], bits, K, G)
     x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).half()
@@ -165,7 +165,7 @@ def test_gemm_block_tile_and_run_edges(cabi, K, N, bits, G, M):
 
 
 def test_gemm_accumulates_and_strides_unaligned(cabi):
-    """Outputs at a 2-byte aligned address with an odd row stride, whole units and cut ones, added to what is there."""
+    """Outputs at a 2-byte aligned address with an odd row stride, whole units, added to what is there."""
     K, N, M = 1024, 264, 70
     w, idx, pk, dense = make_case(K, N, 4, 128, seed=2)
     p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], 4, K, 128)
@@ -180,6 +180,29 @@ def test_gemm_accumulates_and_strides_unaligned(cabi):
     got = yb[1:].view(M, N + 3)
     assert float((got[:, :N].float() - ref).abs().max() / ref.abs().max()) <= 2e-3
     assert torch.equal(got[:, N:], base[:, N:])
+
+
+@pytest.mark.parametrize("M", [70, 9599])
+def test_gemm_units_cut_into_runs(cabi, M):
+    """On 148 SMs: 70 rows are two units of 33 items, both cut; 9599 rows are 74 whole units and two cut ones in one call.
+    Plain, several times, and added to outputs at a 2-byte aligned address with an odd row stride."""
+    K, N = 4096, 264
+    w, idx, pk, dense = make_case(K, N, 3, 128, seed=3)
+    p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], 3, K, 128)
+    x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).half()
+    ref = x.float() @ dev(dense).float().T
+    y = gemm(cabi, p, x)
+    assert float((y.float() - ref).abs().max() / ref.abs().max()) <= 2e-3          # as in test_gemm_llama7b_shapes
+    for _ in range(4):
+        assert torch.equal(gemm(cabi, p, x), y)
+    yb = torch.randn(M * (N + 3) + 1, device="cuda").half()
+    base = yb[1:].view(M, N + 3).clone()
+    ws = torch.empty(cabi.lib().cq_tlayer_gemm_workspace_bytes(C.byref(p.L), M), dtype=torch.uint8, device="cuda")
+    cabi.check(cabi.lib().cq_tlayer_gemm(C.byref(p.L), ptr(x), K, yb.data_ptr() + 2, N + 3, M, 1, ptr(ws), ptr(p.status), None), "gemm")
+    torch.cuda.synchronize()
+    got, want = yb[1:].view(M, N + 3), ref + base[:, :N].float()
+    assert float((got[:, :N].float() - want).abs().max() / want.abs().max()) <= 2e-3
+    assert torch.equal(got[:, N:], base[:, N:]) and int(p.status.item()) == 0
 
 
 @pytest.mark.parametrize("bits,G", [(3, 64), (3, 128), (4, 128), (4, 256)])
