@@ -77,7 +77,8 @@ __global__ void __launch_bounds__(1024) rmsnorm_kernel(const __half* __restrict_
 // pos[t], and the write of k, v rows into the caches (sequences, max_seq, KV, D): token t belongs to
 // sequence t / tokens_per_seq.
 // V = columns of each half a thread takes: 8 (16-byte accesses: half a multiple of 8 and aligned buffers, every model
-// width in use) or 1.  Scalar accesses and a 64-bit division per element cost the prefill more than the bytes.
+// width in use) or 1.  Scalar accesses and a 64-bit division per element cost the prefill more than the bytes.  The
+// divisions of a thread's first row come before the dependency wait: one row of 96 heads 1.95 us with them after it, 1.90.
 template <int V>
 __global__ void rope_cache_kernel(__half* __restrict__ q, __half* __restrict__ k, const __half* __restrict__ v,
                                   const float* __restrict__ cos_t, const float* __restrict__ sin_t,
@@ -86,14 +87,17 @@ __global__ void rope_cache_kernel(__half* __restrict__ q, __half* __restrict__ k
                                   int tokens_per_seq) {
   // programmatic dependent launch: let the next kernel start its prologue, then wait for our inputs
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
   struct __align__(V * 2) Halves { __half h[V]; };
   struct __align__(V == 8 ? 16 : 4) Floats { float f[V]; };
   const int half = D / 2, heads = H + 2 * KV;
-  const int lanes = min(half / V, (int)blockDim.x), i0 = (int)threadIdx.x % lanes * V;    // blockDim.x is a multiple of lanes
-  const long long step = (long long)gridDim.x * (blockDim.x / lanes);
-  for (long long r = (long long)blockIdx.x * (blockDim.x / lanes) + threadIdx.x / lanes; r < rows; r += step) {
-    const int t = (int)(r / heads), hh = (int)(r - (long long)t * heads);
+  const int lanes = min(half / V, (int)blockDim.x), group = (int)threadIdx.x / lanes;     // blockDim.x is a multiple of lanes
+  const int i0 = ((int)threadIdx.x - group * lanes) * V, groups = (int)blockDim.x / lanes;
+  const long long step = (long long)gridDim.x * groups;
+  long long r = (long long)blockIdx.x * groups + group;
+  int t = (int)(r / heads);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  for (; r < rows; r += step, t = (int)(r / heads)) {
+    const int hh = (int)(r - (long long)t * heads);
     const long long p = pos[t];
     if (p < 0 || p >= max_seq) continue;      // a position outside the tables and caches: nothing is read or written
     const size_t crow = (size_t)(t / tokens_per_seq) * max_seq + (size_t)p;     // row of the caches
@@ -128,8 +132,10 @@ __global__ void rope_cache_kernel(__half* __restrict__ q, __half* __restrict__ k
   }
 }
 
-// V = values per access: 8 where the buffers are 16-byte aligned, 1 otherwise and for the tail.  FULL: expf as in the
+// V = values per access: 8 where the buffers are 16-byte aligned, 1 otherwise, for few values (11008: 1.16 us against
+// 1.65, 55296: 1.44 and 1.68, 88064: 1.84 and 1.68) and for the tail.  FULL: expf as in the
 // fp32 torch expression, whose fp16 result it then equals; otherwise the fast exponential, as the row kernel's staging.
+constexpr long long WIDE_MIN_VALUES = 65536;
 template <bool FULL>
 __device__ __forceinline__ __half silu_times(__half gate, __half up) {
   const float g = __half2float(gate);
@@ -716,7 +722,7 @@ extern "C" int cq_rope_cache(void* q, void* k, const void* v, const float* cos_t
 namespace {
 template <bool FULL> int silu_mul_launch(const void* gate, const void* up, void* out, long long n, cq_stream_t stream) {
   if (!gate || !up || !out || n < 1) return CQ_ERR_BAD_ARG;
-  const int vec = (((uintptr_t)gate | (uintptr_t)up | (uintptr_t)out) & 15) == 0 ? 8 : 1;
+  const int vec = (((uintptr_t)gate | (uintptr_t)up | (uintptr_t)out) & 15) == 0 && n >= WIDE_MIN_VALUES ? 8 : 1;
   auto kernel = vec == 8 ? silu_mul_kernel<8, FULL> : silu_mul_kernel<1, FULL>;
   CQ_CUDA_TRY(launch_pdl(kernel, dim3(blocks_for((n + vec - 1) / vec, 256, 148 * 8)), dim3(256), 0, (cudaStream_t)stream,
                          (const __half*)gate, (const __half*)up, (__half*)out, n));
