@@ -158,9 +158,12 @@ class QuantLinear(nn.Module):
                                                    self.group_size)
         return self._row_rows
 
-    def row_layer(self):
-        """The row-tile copy for the decode kernel, or None where the layer does not fit it."""
-        if self._row_limit() and self._row is None:
+    def row_layer(self, rows=1):
+        """The row-tile copy for the decode kernel (built on first use), or None where the kernel does not take the layer
+        or that many rows."""
+        if rows > self._row_limit():
+            return None
+        if self._row is None:
             qc = load_quant_cuda()
             q, s, cw, ci = self._source_buffers()
             self._row = qc.RowLayer(q, s, cw, ci, self.w_bits, self.in_features, self.group_size)
@@ -175,8 +178,8 @@ class QuantLinear(nn.Module):
         forward(silu_mul(gate, up)), with the fast exponential.  Other cases compute the product first, with the
         values of the torch expression, silu in fp32."""
         rows = gate.numel() // gate.shape[-1]
-        row = self.row_layer() if (self._layerwise_dequantize and self.w_bits in (3, 4) and gate.dtype == torch.float16
-                                   and rows <= self._row_limit()) else None
+        row = self.row_layer(rows) if (self._layerwise_dequantize and self.w_bits in (3, 4)
+                                       and gate.dtype == torch.float16) else None
         if row is None:
             if gate.is_cuda and gate.dtype == up.dtype == torch.float16 and gate.shape == up.shape and gate.numel():
                 return self(load_quant_cuda().silu_mul(gate.contiguous(), up.contiguous(), True))
@@ -279,8 +282,8 @@ def forward_shared_input(layers, x: torch.Tensor):
     same = all((l.w_bits, l.in_features, l.num_cherries, l.group_size) ==
                (first.w_bits, first.in_features, first.num_cherries, first.group_size) for l in layers)
     if (1 < len(layers) <= 4 and same and QuantLinear._layerwise_dequantize and first.w_bits in (3, 4)):
-        if all(rows <= l._row_limit() for l in layers):
-            rls = [l.row_layer() for l in layers]
+        rls = [l.row_layer(rows) for l in layers]
+        if all(r is not None for r in rls):
             qc = load_quant_cuda()
             x2 = x.reshape(rows, x.shape[-1])
             if x2.dtype != torch.float16:
