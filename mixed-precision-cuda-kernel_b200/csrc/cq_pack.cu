@@ -109,8 +109,8 @@ __global__ void pack_codes_kernel(const void* __restrict__ w, int is_f32, const 
 // apart, and divides per weight.  The loads are 2 bytes a lane, 64 contiguous bytes a warp, because the removed
 // cherry columns leave the compact columns at any alignment; the tile turns them so that a thread quantises 32
 // columns of one row and the byte stores have 32 consecutive rows a warp.  Groups of more than one chunk are read
-// a second time for the codes (mostly from L2).  4096 x 11008 4-bit: 58 us (114 MB, bound by the issue rate: about 25
-// instructions per weight), 415 us for sort, cherries, scales and codes in four kernels.
+// a second time for the codes (mostly from L2).  4096 x 11008 4-bit: 57 us (114 MB, bound by the issue rate: about 25 instructions per weight), 415 us for sort, cherries, scales
+// and codes in four kernels.
 constexpr int PK_ROWS = 64, PK_COLS = 128, PK_THREADS = 256;
 
 template <typename T> struct PackTile;
@@ -258,12 +258,13 @@ __global__ void __launch_bounds__(PK_THREADS, sizeof(T) == 2 ? 5 : 3) pack_fused
 // ------------------------------------------------------------------ dense unpack
 // llama/qlinear.py:120-162: dense[n, k] = cherry ? cherry_weight : fp16((q + 0.5) * s).
 // A block writes 64 rows x 128 columns: a thread makes one octet of 8 original columns of four consecutive rows.
-// Without a cherry column or a group boundary inside, the octet's codes are 8 consecutive compact columns: the bytes
-// of two compact octets (one 32-bit load per byte row covers the four rows), shifted by the position inside the first.
-// Pairs of codes become the low mantissa bits of 1024 + u, minus (1024 + off), times the scale: each step but the
-// last exact, so the product is rounded once as in the reference.  The tile in shared memory (16-byte slots, slot
-// number XOR row quad against bank conflicts) turns the octets into rows of 256 contiguous bytes.  11008 x 4096 3-bit:
-// 52 us (108 MB), 296 us with a binary search, a byte-wise code fetch and two divisions per element.
+// The octet's codes are consecutive compact columns: the bytes of two compact octets (one 32-bit load per byte row covers
+// the four rows), shifted by the position inside the first; a cherry column inside leaves a gap in the word, and its
+// values go over the finished octet.  Pairs of codes become the low mantissa bits of 1024 + u, minus (1024 + off), times
+// the scale: each step but the last exact, so the product is rounded once as in the reference.  The tile in shared memory
+// (16-byte slots, slot number XOR row quad against bank conflicts) turns the octets into rows of 256 contiguous bytes.
+// 11008 x 4096 3-bit: 36 us (108 MB), 290 with a binary search, a byte-wise code fetch and two divisions per element; 512 x
+// 512: 3.6 us and 4.3.
 constexpr int UP_ROWS = 64, UP_COLS = 128;
 
 __device__ __forceinline__ uint32_t load_quad(const uint8_t* p, bool aligned) {
@@ -282,7 +283,8 @@ template <int BITS> __device__ __forceinline__ __half2 code_pair(uint32_t word, 
   return __hsub2(d, *reinterpret_cast<const __half2*>(&half));
 }
 
-template <int BITS>
+// CHERRY = the layer has cherry columns
+template <int BITS, bool CHERRY>
 __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
     const uint8_t* __restrict__ q, const __half* __restrict__ scales, const __half* __restrict__ cw,
     const int16_t* __restrict__ idx, int K, int N, int C, int G, int g_shift, __half* __restrict__ dense, int aligned) {
@@ -292,7 +294,7 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
   const int k0 = blockIdx.x * UP_COLS, n0 = blockIdx.y * UP_ROWS;
   const int k = k0 + 8 * oct, n = n0 + 4 * nq;
   const int Kc = K - C, n_oct = Kc / 8;
-  if (tid <= UP_COLS / 8) {
+  if (CHERRY && tid <= UP_COLS / 8) {
     const int kk = k0 + 8 * tid;
     int low = 0, high = C;
     while (low < high) {
@@ -303,8 +305,9 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
   }
   __syncthreads();
   if (k < K && n < N) {
-    const int low = before[oct], kc = k - low, o = kc >> 3, r = kc & 7;
-    const bool cherry = before[oct + 1] != low;
+    const int low = CHERRY ? before[oct] : 0;
+    const int cnt = CHERRY ? max(0, min(8, before[oct + 1] - low)) : 0, n_codes = 8 - cnt;      // cherry columns and codes
+    const int kc = max(k - low, 0), o = kc >> 3, r = kc & 7;
     // the bytes of compact octets o and o + 1, four rows in each word
     uint32_t b[2][BITS];
     const uint8_t* src = q + (size_t)o * BITS * N + n;
@@ -315,17 +318,19 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
         b[h][i] = (o + h < n_oct && (h == 0 || r)) ? load_quad(src + (size_t)(h * BITS + i) * N, aligned & 1) : 0u;
     auto group_of = [&](int c) { return g_shift >= 0 ? c >> g_shift : c / G; };
     const int g = group_of(kc), split = (g + 1) * G - kc;       // codes 0 .. split - 1 belong to group g
+    const bool whole = split >= n_codes;
     unsigned long long s0 = 0, s1 = 0;                          // the four rows' scales of groups g and g + 1
-    const bool whole = split >= 8;
-    if (!cherry) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        s0 |= (unsigned long long)__half_as_ushort(scales[(size_t)g * N + n + j]) << (16 * j);
-        if (!whole) s1 |= (unsigned long long)__half_as_ushort(scales[(size_t)(g + 1) * N + n + j]) << (16 * j);
-      }
+    for (int j = 0; j < 4; ++j) {
+      if (n_codes > 0) s0 |= (unsigned long long)__half_as_ushort(scales[(size_t)g * N + n + j]) << (16 * j);
+      if (!whole) s1 |= (unsigned long long)__half_as_ushort(scales[(size_t)(g + 1) * N + n + j]) << (16 * j);
     }
-    // (groups narrower than 8 columns can put more than two into an octet: the general path below)
-    const bool general = cherry || (!whole && G < 8);
+    uint32_t own = 0, second = 0;                               // columns that are cherries; that belong to group g + 1
+    for (int t = 0; t < cnt; ++t) own |= 1u << (((int)idx[low + t] - k) & 7);
+    if (!whole) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) second |= (e - __popc(own & ((1u << e) - 1)) >= split ? 1u : 0u) << e;
+    }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       uint32_t w[2];
@@ -342,35 +347,38 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
         word = __funnelshift_r(w[0], w[1], 4 * r);
       else
         word = ((w[0] & 0xFFFFFFu) >> (3 * r)) | (r ? w[1] << (24 - 3 * r) : 0u);
-      if (!general) {
-        const uint32_t sa = (uint32_t)(s0 >> (16 * j)) & 0xFFFFu, sb = (uint32_t)(s1 >> (16 * j)) & 0xFFFFu;
-        uint32_t p[4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t sc = whole ? (sa | (sa << 16)) : ((2 * i < split ? sa : sb) | ((2 * i + 1 < split ? sa : sb) << 16));
-          const __half2 v = __hmul2(code_pair<BITS>(word, i), *reinterpret_cast<const __half2*>(&sc));
-          p[i] = *reinterpret_cast<const uint32_t*>(&v);
-        }
-        tile[(4 * nq + j) * 16 + (oct ^ nq)] = make_uint4(p[0], p[1], p[2], p[3]);
+      for (uint32_t m = own; m; m &= m - 1) {                   // a gap at each cherry column
+        const int at = BITS * (__ffs(m) - 1);
+        const uint32_t below = (1u << at) - 1;
+        word = (word & below) | ((word & ~below) << BITS);
       }
+      const uint32_t sa = (uint32_t)(s0 >> (16 * j)) & 0xFFFFu, sb = (uint32_t)(s1 >> (16 * j)) & 0xFFFFu;
+      uint32_t p[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t sc = whole ? (sa | (sa << 16))
+                                  : (((second >> (2 * i)) & 1u ? sb : sa) | (((second >> (2 * i + 1)) & 1u ? sb : sa) << 16));
+        const __half2 v = __hmul2(code_pair<BITS>(word, i), *reinterpret_cast<const __half2*>(&sc));
+        p[i] = *reinterpret_cast<const uint32_t*>(&v);
+      }
+      tile[(4 * nq + j) * 16 + (oct ^ nq)] = make_uint4(p[0], p[1], p[2], p[3]);
     }
-    if (general) {
-      // column by column
+    for (int t = 0; t < cnt; ++t) {
+      const int e = ((int)idx[low + t] - k) & 7;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) reinterpret_cast<__half*>(&tile[(4 * nq + j) * 16 + (oct ^ nq)])[e] = cw[(size_t)(low + t) * N + n + j];
+    }
+    if (!whole && G < 8) {
+      // groups narrower than 8 columns can put more than two into an octet: column by column
 #pragma unroll 1
-      for (int j = 0; j < 4; ++j) {
-        __half* dst = reinterpret_cast<__half*>(&tile[(4 * nq + j) * 16 + (oct ^ nq)]);
-        int m = low;
-#pragma unroll 1
-        for (int e = 0; e < 8; ++e) {
-          while (m < C && (int)idx[m] < k + e) ++m;
-          if (m < C && (int)idx[m] == k + e) {
-            dst[e] = cw[(size_t)m * N + n + j];
-          } else {
-            const int c = k + e - m;
-            const uint32_t u = cq_ref_code(q, BITS, c, n + j, N);
-            const float a = (float)((int)u - (1 << (BITS - 1))) + 0.5f;
-            dst[e] = __float2half_rn(__fmul_rn(a, __half2float(scales[(size_t)group_of(c) * N + n + j])));
-          }
+      for (int e = 0, m = low; e < 8; ++e) {
+        if ((own >> e) & 1u) { ++m; continue; }
+        const int c = k + e - m;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const float a = (float)((int)cq_ref_code(q, BITS, c, n + j, N) - (1 << (BITS - 1))) + 0.5f;
+          reinterpret_cast<__half*>(&tile[(4 * nq + j) * 16 + (oct ^ nq)])[e] =
+              __float2half_rn(__fmul_rn(a, __half2float(scales[(size_t)group_of(c) * N + n + j])));
         }
       }
     }
@@ -478,7 +486,8 @@ extern "C" int cq_unpack_dense(const uint8_t* qweight, const void* scales, const
   int g_shift = -1;
   if ((G & (G - 1)) == 0)
     for (g_shift = 0; (1 << g_shift) < G;) ++g_shift;
-  auto kernel = bits == 4 ? unpack_dense_kernel<4> : unpack_dense_kernel<3>;
+  auto kernel = bits == 4 ? (C > 0 ? unpack_dense_kernel<4, true> : unpack_dense_kernel<4, false>)
+                          : (C > 0 ? unpack_dense_kernel<3, true> : unpack_dense_kernel<3, false>);
   kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(qweight, (const __half*)scales, (const __half*)cherry_weight,
                                                  cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
   CQ_CUDA_TRY(cudaGetLastError());

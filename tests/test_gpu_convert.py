@@ -51,6 +51,20 @@ def test_pack_and_unpack(cabi, K, N, bits, G, C, dtype):
     assert np.array_equal(gpu_unpack(cabi, ref, bits, K, G).view(np.uint16), dense.view(np.uint16))
 
 
+@pytest.mark.parametrize("bits", [3, 4])
+@pytest.mark.parametrize("K,N,G,C", [(264, 72, 1, 24), (264, 72, 4, 24), (264, 8, 12, 16), (520, 136, 20, 64), (1032, 64, 24, 1016),
+                                     (128, 64, 64, 120)])
+def test_pack_and_unpack_of_narrow_groups_and_many_cherries(cabi, K, N, G, C, bits):
+    """Octets with several cherry columns, with group boundaries among them, with no code at all; groups inside an octet."""
+    w, idx = layer(K, N, C, np.float16, K + G)
+    ref = O.pack(w, idx, bits, G)
+    got = gpu_pack(cabi, w, idx, bits, G)
+    for key in ("qweight", "scales", "cherry_weight", "cherry_indices"):
+        assert np.array_equal(got[key].view(np.uint8), ref[key].view(np.uint8)), key
+    dense = O.unpack(ref["qweight"], ref["scales"], ref["cherry_weight"], ref["cherry_indices"], bits, G, K)
+    assert np.array_equal(gpu_unpack(cabi, ref, bits, K, G).view(np.uint16), dense.view(np.uint16))
+
+
 def test_unpack_into_unaligned_buffers(cabi):
     K, N, bits, G, C = 264, 72, 3, 128, 8
     w, idx = layer(K, N, C, np.float16, 5)
