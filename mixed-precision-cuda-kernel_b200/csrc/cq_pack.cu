@@ -109,7 +109,8 @@ __global__ void pack_codes_kernel(const void* __restrict__ w, int is_f32, const 
 // apart, and divides per weight.  The loads are 2 bytes a lane, 64 contiguous bytes a warp, because the removed
 // cherry columns leave the compact columns at any alignment; the tile turns them so that a thread quantises 32
 // columns of one row and the byte stores have 32 consecutive rows a warp.  Groups of more than one chunk are read
-// a second time for the codes (mostly from L2).  4096 x 11008 4-bit: 57 us (114 MB, bound by the issue rate: about 25 instructions per weight), 415 us for sort, cherries, scales
+// a second time for the codes (mostly from L2); cq_pack leaves those of few rows to the general pair.  4096 x 11008
+// 4-bit: 57 us (114 MB, bound by the issue rate: about 25 instructions per weight), 415 us for sort, cherries, scales
 // and codes in four kernels.
 constexpr int PK_ROWS = 64, PK_COLS = 128, PK_THREADS = 256;
 
@@ -446,8 +447,16 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
   const int T = 256;
   if (C > 0) pack_sort_kernel<<<nblocks(C, T), T, 0, st>>>(cherry_unsorted, C, cherry_indices);
   const int ng = (K - C + G - 1) / G;
-  if (G == 64 || G % PK_COLS == 0 || ng == 1) {
-    const int span = G == 64 ? PK_COLS : (ng == 1 ? (K - C) : G);         // compact columns a block owns
+  const int span = G == 64 ? PK_COLS : (ng == 1 ? (K - C) : G);           // compact columns a block owns
+  // A block walks a group of several chunks from end to end, twice, while the general pair spreads it over the chip: on
+  // matrices of few rows the pair is faster.  Microseconds as measured over 256 .. 11008 columns, 64 .. 16384 rows (one
+  // group per row, 4096 columns with cherries: 64 rows 65 and 98, 1024 rows 86 and 99, 2048 rows 111 and 100, 8192 rows
+  // 301 and 112; without cherries 1024 rows 27 and 83, 8192 rows 155 and 85).
+  const int chunks = (span + PK_COLS - 1) / PK_COLS;
+  const double weights = (double)K * N;
+  const double pair_us = C > 0 ? 8.0 + 0.0138 * span + 6.0e-6 * weights : 4.8 + 0.0013 * span + 4.4e-6 * weights;
+  const double one_us = C > 0 ? (weight_is_f32 ? 4.0 + 3.7 * chunks : 3.0 + 3.0 * chunks) : 1.5 + (weight_is_f32 ? 3.3 : 2.6) * chunks;
+  if ((G == 64 || G % PK_COLS == 0 || ng == 1) && (chunks == 1 || one_us <= pair_us)) {
     const int n_tiles = (N + PK_ROWS - 1) / PK_ROWS, n_spans = (K - C + span - 1) / span;
     const long long blocks = (long long)n_tiles * (n_spans + (C > 0));
     if (blocks <= 0x7fffffffll) {

@@ -51,6 +51,18 @@ def test_pack_and_unpack(cabi, K, N, bits, G, C, dtype):
     assert np.array_equal(gpu_unpack(cabi, ref, bits, K, G).view(np.uint16), dense.view(np.uint16))
 
 
+@pytest.mark.parametrize("dtype", [np.float16, np.float32])
+@pytest.mark.parametrize("K,N,G,C", [(1040, 2056, 1040, 16), (1040, 200, 1040, 16), (520, 4104, 520, 0), (520, 1000, 520, 0),
+                                     (1552, 1544, 512, 8)])
+def test_pack_of_long_groups(cabi, K, N, G, C, dtype):
+    """Groups of several chunks, on both sides of the rule between the one-pass kernel and the general pair."""
+    w, idx = layer(K, N, C, dtype, K + N)
+    ref = O.pack(w, idx, 3, G)
+    got = gpu_pack(cabi, w, idx, 3, G)
+    for key in ("qweight", "scales", "cherry_weight", "cherry_indices"):
+        assert np.array_equal(got[key].view(np.uint8), ref[key].view(np.uint8)), key
+
+
 @pytest.mark.parametrize("bits", [3, 4])
 @pytest.mark.parametrize("K,N,G,C", [(264, 72, 1, 24), (264, 72, 4, 24), (264, 8, 12, 16), (520, 136, 20, 64), (1032, 64, 24, 1016),
                                      (128, 64, 64, 120)])
