@@ -310,7 +310,7 @@ int cq_tlayer_gemm(const cq_tlayer* layer, const void* x_f16, int ldx, void* y_f
  * The re-packed layer is cached inside the library, keyed by the four buffer
  * addresses, the dimensions and version_tag (pass any value that changes when
  * the buffers' contents change, e.g. a sum of tensor version counters); a copy
- * is made per kernel family actually used (1 row / 2..7 rows / 8 rows and more).
+ * is made per kernel family actually used (row kernel / GEMM / stream matvec, by the number of rows).
  * Addresses alone do not identify a buffer for ever: call cq_cache_evict when the
  * buffers are freed or re-filled.
  * ---------------------------------------------------------------------- */
