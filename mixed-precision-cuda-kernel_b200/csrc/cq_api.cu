@@ -38,7 +38,7 @@ struct CacheKey {
 struct DeviceState {
   void* scratch = nullptr;
   uint32_t* status = nullptr;
-  void* gemm_ws = nullptr;        // staged activations of the prefill GEMM (grow-only)
+  void* gemm_ws = nullptr;        // staged activations of the GEMM (grow-only, sizes at least double)
   size_t gemm_ws_bytes = 0;
 };
 
@@ -52,6 +52,7 @@ std::map<CacheKey, cq_layer> g_cache;
 std::map<CacheKey, cq_tlayer> g_tcache;
 std::map<CacheKey, cq_rlayer> g_rcache;
 std::map<int, DeviceState> g_dev;
+std::map<int, std::vector<void*>> g_outgrown;   // workspaces kept until the cache is cleared: a graph may hold their addresses
 
 int device_state(int dev, DeviceState* out) {
   auto it = g_dev.find(dev);
@@ -91,14 +92,12 @@ int legacy_gemm(const CacheKey& key, int dev, const void* vec, const uint8_t* qw
   const int chunk = batch < PREFILL_CHUNK_ROWS ? batch : PREFILL_CHUNK_ROWS;
   const size_t need = cq_tlayer_gemm_workspace_bytes(&L, chunk);
   if (need > ds.gemm_ws_bytes) {
-    if (ds.gemm_ws) {
-      CQ_CUDA_TRY(cudaStreamSynchronize(st));   // earlier GEMMs may still read the old buffer
-      CQ_CUDA_TRY(cudaFree(ds.gemm_ws));
-      ds.gemm_ws = nullptr;
-      ds.gemm_ws_bytes = 0;
-    }
-    CQ_CUDA_TRY(cudaMalloc(&ds.gemm_ws, need));
-    ds.gemm_ws_bytes = need;
+    const size_t bytes = need > 2 * ds.gemm_ws_bytes ? need : 2 * ds.gemm_ws_bytes;
+    void* ws = nullptr;
+    CQ_CUDA_TRY(cudaMalloc(&ws, bytes));
+    if (ds.gemm_ws) g_outgrown[dev].push_back(ds.gemm_ws);
+    ds.gemm_ws = ws;
+    ds.gemm_ws_bytes = bytes;
   }
   const __half* xp = (const __half*)vec;
   __half* yp = (__half*)mul;
@@ -302,6 +301,14 @@ extern "C" int cq_cache_clear(void) {
     if (cur != kv.first.dev) cudaSetDevice(cur);
   }
   g_rcache.clear();
+  for (auto& kv : g_outgrown) {
+    int cur = 0;
+    cudaGetDevice(&cur);
+    if (cur != kv.first) cudaSetDevice(kv.first);
+    for (void* p : kv.second) cudaFree(p);
+    if (cur != kv.first) cudaSetDevice(cur);
+  }
+  g_outgrown.clear();
   return CQ_OK;
 }
 

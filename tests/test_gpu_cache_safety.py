@@ -145,3 +145,26 @@ def test_quantlinear_buffers_replaced_at_the_same_addresses(qc, rows):
             assert np.abs(y - ref).max() <= 2e-3 * np.abs(ref).max()
     if at[0] != at[1]:
         pytest.skip("the allocator did not hand the freed blocks back")
+
+
+def test_captured_call_after_the_workspace_has_grown(qc):
+    """A graph holds the address of the GEMM's workspace; a larger call afterwards must not take it away."""
+    qc.cache_clear()
+    a = make_layer(qc, 700)
+    ref = dense(a)
+    xs = {rows: torch.randn(rows, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(rows)).half()
+          for rows in (64, 900, 4000)}
+    call(qc, xs[64], a)
+    graph = torch.cuda.CUDAGraph()
+    y = torch.zeros(64, N, dtype=torch.float16, device="cuda")
+    with torch.cuda.graph(graph):
+        y.zero_()
+        qc.vecquant4matmul_cherryq(xs[64], a[0], a[2], a[3], a[1], y, G)
+    for rows in (900, 4000):
+        out = call(qc, xs[rows], a)
+        want = xs[rows].cpu().numpy().astype(np.float64) @ ref.T
+        assert np.abs(out - want).max() <= 2e-3 * np.abs(want).max()
+        graph.replay()
+        torch.cuda.synchronize()
+        want = xs[64].cpu().numpy().astype(np.float64) @ ref.T
+        assert np.abs(y.cpu().numpy().astype(np.float64) - want).max() <= 2e-3 * np.abs(want).max()
