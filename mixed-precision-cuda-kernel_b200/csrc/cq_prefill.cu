@@ -35,9 +35,9 @@
 //   warps 19-22 epilogue: tcgen05.ld of a finished tile into shared memory (which frees the accumulator), then
 //               16-byte stores to y
 // Every wait is bounded and reports into the status word instead of hanging.  The kernel may be resident while kernels
-// before the pre-pass still run (an exchange that waits for a late rank for seconds, say), so a role starts to wait for
-// anything that depends on the activations only once it has passed the dependency wait; what comes before that are the
-// weights, which depend on nothing.
+// before the pre-pass still run (an exchange that waits for a late rank for seconds, say): the bounds only count once the
+// activation producer has passed the dependency wait, which it notes in the CTA's state.  (A dependency wait in every
+// role did the same and cost a call of 16 rows 0.3 us.)
 //
 // Bound and state: 4096 -> 11008 4-bit, 2048 rows: 140 us = 1.32 PFLOP/s (739 us through QuantLinear and 195 us by itself
 // with lone CTAs of 128 x 256 tiles); 8192 -> 28672 3-bit, 2048 rows: 641 us = 1.50 PFLOP/s, tensor-bound.  16 rows: 18 and
@@ -99,30 +99,33 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
       : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
   return ok != 0;
 }
-// Bounded wait: gives up after WAIT_LIMIT polls (at once when the CTA already gave up), records
-// which wait failed in the status word and lets the caller run on to the common exit.
-__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* abort_flag,
+// State of a CTA: whether the kernels before this one have finished, and whether a wait ran out.
+constexpr int RUNNING = 0, ABORTED = 1, PENDING = 2;
+// Bounded wait: gives up after WAIT_LIMIT polls or about one second of the device's nanosecond timer (read once some polls
+// have failed), at once when the CTA already gave up, records which wait failed in the status word and lets the caller run
+// on to the common exit.  While the CTA is PENDING nothing counts: that time belongs to the kernels before.
+__device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volatile int* state,
                                             uint32_t* status, uint32_t code) {
-  // bounded in polls and in time (about one second of the device's nanosecond timer, read once some polls have failed)
-  const uint32_t limit = *abort_flag ? 1u : WAIT_LIMIT;
+  const uint32_t limit = *state == ABORTED ? 1u : WAIT_LIMIT;
   unsigned long long t0 = 0;
-  for (uint32_t it = 0; it < limit; ++it) {
+  for (uint32_t it = 0; it < limit;) {
     if (mbar_try_wait(bar, parity)) return true;
-    if ((it & 255u) == 255u) {
+    if (*state == PENDING) continue;
+    if ((++it & 255u) == 0u) {
       unsigned long long t1;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
       if (t0 == 0) t0 = t1;
       else if (t1 - t0 > 1000000000ull) break;
     }
   }
-  *abort_flag = 1;
+  *state = ABORTED;
   if (status) atomicOr(status, code);
   return false;
 }
-__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, uint32_t* status,
+__device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* state, uint32_t* status,
                                           uint32_t code) {
   if (mbar_try_wait(bar, parity)) return true;
-  return mbar_wait_slow(bar, parity, abort_flag, status, code);
+  return mbar_wait_slow(bar, parity, state, status, code);
 }
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
@@ -403,7 +406,7 @@ template <int BITS, int SETS>
 __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillParams p) {
   constexpr int W_MMA = NGRP * 4, W_PROD_W = NGRP * 4 + 1, W_PROD_B = NGRP * 4 + 2;
   extern __shared__ __align__(128) uint8_t smem[];
-  __shared__ int s_abort;
+  __shared__ int s_state;
   __shared__ uint32_t s_tmem;
   __shared__ int s_last;
 
@@ -431,7 +434,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
   auto B_DEMPTY = [&](uint32_t d) { return bar0 + 8 * (2 * SW_MAX + 2 * SB_MAX + 2 * NA + 2 + d); };
 
   if (tid == 0) {
-    s_abort = 0;
+    s_state = PENDING;
     for (uint32_t s = 0; s < SW; ++s) { mbar_init(B_WFULL(s), 1); mbar_init(B_WEMPTY(s), 4); }
     for (uint32_t s = 0; s < SB; ++s) {
       mbar_init(B_BFULL(s), 1);
@@ -468,11 +471,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         const uint8_t* src = p.stream + (size_t)tile * p.tile_bytes + (size_t)c0 * CQT_CHER_BYTES + (size_t)(w.j0 - c0) * p.gran_bytes;
         for (uint32_t j = w.j0; j < w.j1; ++j) {
           const uint32_t bytes = j < NCH ? (uint32_t)CQT_CHER_BYTES : (uint32_t)p.gran_bytes;
-          if (ring.round) {
-            if (ring.round == 1 && ring.slot == 0) dependency_wait();      // the ring is full: it drains with the activations
-            mbar_wait(B_WEMPTY(ring.slot), ring.phase ^ 1, &s_abort, p.status, 1u);
-          }
-          if (*(volatile int*)&s_abort) break;
+          if (ring.round) mbar_wait(B_WEMPTY(ring.slot), ring.phase ^ 1, &s_state, p.status, 1u);
+          if (*(volatile int*)&s_state == ABORTED) break;
           mbar_expect_tx(B_WFULL(ring.slot), bytes);
           bulk_g2s(wring + ring.slot * (uint32_t)p.wstage_bytes, src, bytes, B_WFULL(ring.slot));
           src += bytes;
@@ -488,6 +488,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     if (lane == 0) {
       // the staged activations are written by the kernel launched just before this one
       dependency_wait();
+      atomicCAS(&s_state, PENDING, RUNNING);
       const uint32_t bring = smem_u32(smem + p.off_bring);
       Ring ring;
       WorkList wl(p, cluster, n_clusters, IPT);
@@ -500,8 +501,8 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
                              (size_t)(w.j0 - c0) * B_GRAN_BYTES;
         for (uint32_t j = w.j0; j < w.j1; ++j) {
           const uint32_t bytes = j < NCH ? B_CHER_BYTES : B_GRAN_BYTES;
-          if (ring.round) mbar_wait(B_BEMPTY(ring.slot), ring.phase ^ 1, &s_abort, p.status, 2u);
-          if (*(volatile int*)&s_abort) break;
+          if (ring.round) mbar_wait(B_BEMPTY(ring.slot), ring.phase ^ 1, &s_state, p.status, 2u);
+          if (*(volatile int*)&s_state == ABORTED) break;
           if (real) {
             mbar_expect_tx(B_BFULL(ring.slot), bytes);
             bulk_g2s(bring + ring.slot * B_GRAN_BYTES, src, bytes, B_BFULL(ring.slot));
@@ -523,14 +524,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
   } else if (warp == W_MMA) {
     if (rank == 0) {
       // ================================================================ MMA issuer (leader CTA)
-      dependency_wait();
       // The whole warp walks the list and one elected lane issues: addresses and descriptors then stay in uniform
       // registers, where the MMA takes them (all of tensor memory is allocated, so its base is column 0).
       // instruction descriptor: fp32 accumulate, fp16 A and B, both K-major, N = NT, M = 256
       const uint32_t IDESC = (1u << 4) | ((NT >> 3) << 17) | (16u << 24);
       const uint32_t bring = smem_u32(smem + p.off_bring);
       if (tmem != 0) {
-        s_abort = 1;
+        s_state = ABORTED;
         if (p.status && lane == 0) atomicOr(p.status, 1024u);
       }
       __syncwarp();
@@ -541,11 +541,11 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
       for (; wl.next(w); ++lu) {
         const uint32_t dbuf = lu % ND;
         const uint32_t td = D_BASE + dbuf * NT;
-        if (lu >= ND) mbar_wait(B_DEMPTY(dbuf), ((lu / ND) - 1) & 1, &s_abort, p.status, 4u);
+        if (lu >= ND) mbar_wait(B_DEMPTY(dbuf), ((lu / ND) - 1) & 1, &s_state, p.status, 4u);
         tc_fence_after();
         for (uint32_t j = w.j0; j < w.j1; ++j) {
           // one wait an item: everything that stands between two items idles the tensor core
-          const bool ok = mbar_wait(B_READY(ra.slot), ra.phase, &s_abort, p.status, 8u);
+          const bool ok = mbar_wait(B_READY(ra.slot), ra.phase, &s_state, p.status, 8u);
           if (!__all_sync(0xffffffffu, ok)) break;           // nothing is issued on operands that never came
           tc_fence_after();
           const uint64_t bdesc = smem_desc(bring + rb.slot * B_GRAN_BYTES, 8, 16);
@@ -568,7 +568,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         if (elect_one()) tc_commit_pair(B_DFULL(dbuf));
         __syncwarp();
       }
-      if (*(volatile int*)&s_abort) __nanosleep(100000);     // (after a wait that ran out: let issued MMAs finish)
+      if (*(volatile int*)&s_state == ABORTED) __nanosleep(100000);     // (after a wait that ran out: let issued MMAs finish)
     }
   } else if (warp < W_MMA) {
     // ================================================================ decode groups
@@ -589,7 +589,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         ring.advance(SW);
         rb.advance(SB);
         if ((int)(n % NGRP) != grp) continue;
-        mbar_wait(B_WFULL(sw), wphase, &s_abort, p.status, 32u);
+        mbar_wait(B_WFULL(sw), wphase, &s_state, p.status, 32u);
         const uint8_t* item = wring + (size_t)sw * p.wstage_bytes;
         const bool cherry = j < NCH;
         uint4 raw[BITS];
@@ -606,8 +606,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         }
         __syncwarp();
         if (lane == 0) mbar_arrive(B_WEMPTY(sw));
-        if (turn == 1) dependency_wait();
-        if (turn) mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_abort, p.status, 64u);
+        if (turn) mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_state, p.status, 64u);
         ++turn;
         tc_fence_after();
         const uint32_t ta = tmem + lane_addr + a * A_COLS;
@@ -639,19 +638,13 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         if (lane == 0) {
           // The group's first warp also answers for the activation tile.  (No wait by parity comes a round early: the
           // MMAs of item n - 4 are done, so the slot's last tile, of an item n - SB <= n - 4, has landed.)
-          if ((warp & 3) == 0) {
-            if (turn == 1) dependency_wait();
-            mbar_wait(B_BFULL(sb), bphase, &s_abort, p.status, 16u);
-          }
+          if ((warp & 3) == 0) mbar_wait(B_BFULL(sb), bphase, &s_state, p.status, 16u);
           if (rank == 0) mbar_arrive(ready);
           else mbar_arrive_cluster(ready);
         }
       }
     }
-    if (turn) {
-      dependency_wait();
-      mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_abort, p.status, 64u);
-    }
+    if (turn) mbar_wait(B_AEMPTY(a), (turn - 1) & 1, &s_state, p.status, 64u);
   } else {
     // ================================================================ epilogue (last four warps)
     const int quad = warp & 3;                              // the tensor-memory lanes this warp may read
@@ -688,7 +681,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
           }
           epi_sync();
         }
-        mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_abort, p.status, 128u);
+        mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_state, p.status, 128u);
         tc_fence_after();
         // (NT is a multiple of 32: a 32-column step may read padding, never past the accumulator)
 #pragma unroll 1
@@ -728,7 +721,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         // stores the outputs
         const size_t part_floats = (size_t)NT * 128;
         float* mine = p.partial + ((size_t)(cluster * 2 + w.run) * 2 + rank) * part_floats;
-        mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_abort, p.status, 128u);
+        mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_state, p.status, 128u);
         tc_fence_after();
 #pragma unroll 1
         for (int c = 0; c < ntok; c += 32) {
