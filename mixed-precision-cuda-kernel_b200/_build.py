@@ -20,7 +20,7 @@ ROOT = os.path.dirname(HERE)
 
 LIB = os.path.join(HERE, "libcherryq.so")
 CUDA_SOURCES = ["cq_api.cu", "cq_layout.cu", "cq_matvec.cu", "cq_rowvec.cu", "cq_pack.cu", "cq_fakequant.cu", "cq_legacy_f32.cu",
-                "cq_tile_layout.cu", "cq_prefill.cu", "cq_model_ops.cu", "cq_peer.cu"]
+                "cq_tile_layout.cu", "cq_prefill.cu", "cq_model_ops.cu", "cq_attn.cu", "cq_peer.cu"]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "--shared", "-Xcompiler", "-fPIC", "-Xptxas", "-v", "--fmad=true",
@@ -47,7 +47,7 @@ def cuda_sources():
 
 def build_lib(force: bool = False, verbose: bool = False) -> str:
     srcs = cuda_sources()
-    deps = srcs + [os.path.join(CSRC, "cq_common.cuh"), os.path.join(CSRC, "cq_tile.cuh"),
+    deps = srcs + [os.path.join(CSRC, "cq_common.cuh"), os.path.join(CSRC, "cq_tile.cuh"), os.path.join(CSRC, "cq_attn.cuh"),
                    os.path.join(ROOT, "include", "cherryq.h")]
     if not force and _newer(LIB, deps):
         return LIB

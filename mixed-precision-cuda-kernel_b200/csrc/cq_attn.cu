@@ -1,0 +1,320 @@
+// Single-query attention over the KV cache (decode) for 64- and 128-wide heads and up to 8 query heads per KV head, on
+// mma.sync; in the reference a part of its vendored LLaMA (llama/modeling_llama_quant.py:371-419 of the reference project).
+//
+// The bound is the cache itself, read once.  With fp32 dot products a step of 8 query heads per KV head was bound by its
+// arithmetic, one head per KV head by latencies and registers; here the arithmetic is small beside the loads in either
+// case (32 MMAs per 8 KB of cache and warp), so one kernel serves both:
+//   * scores S (heads x positions) = Q . K^T, m16n8k16: rows 0-7 of A are the query heads.  A lane's share of a
+//     position's key is two or four 16-byte pieces, loaded straight from the cache: the order of the columns inside a
+//     step is free as long as both operands agree;
+//   * the sums land where P . V needs its A operand.  Rows 0-7 take the upper 11 bits of the weights, rows 8-15, which
+//     the heads leave empty, the next 11: weights keep the precision of fp32 sums at no cost;
+//   * V is the B operand, two positions' 16-byte pieces interleaved in registers (which columns of the head an MMA
+//     covers is free, too).
+// A warp takes 16 positions a turn with all of their keys and values in flight, and keeps its own running maximum, sum
+// and weighted values; the warps meet once in shared memory, the ranges of positions (blockIdx.z) in the workspace, where
+// the CTA that arrives last merges them.
+#include "cq_attn.cuh"
+
+namespace {
+
+constexpr int AM_SM_WARPS = 12;              // warps an SM holds (168 registers a thread)
+constexpr int AM_HEADS = 8;                  // query heads of a CTA
+constexpr int AM_POS = 16;                   // positions of a turn
+constexpr int AM_MAX_SPLITS = 32;            // (a lane per range in the merge)
+
+__device__ __forceinline__ void am_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+}
+__device__ __forceinline__ float ex2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+// the upper 11 bits of two weights, and what is left of them
+__device__ __forceinline__ uint2 split_weights(float a, float b) {
+  const __half2 hi = __floats2half2_rn(a, b);
+  const float2 f = __half22float2(hi);
+  const __half2 lo = __floats2half2_rn(a - f.x, b - f.y);
+  return make_uint2(*reinterpret_cast<const uint32_t*>(&hi), *reinterpret_cast<const uint32_t*>(&lo));
+}
+
+template <int D, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_mma_kernel(
+    const __half* __restrict__ q, const __half* __restrict__ k_cache, const __half* __restrict__ v_cache,
+    const long long* __restrict__ pos, __half* __restrict__ out, float* __restrict__ part,
+    unsigned int* __restrict__ counters, int H, int KV, int max_seq, float scale) {
+  constexpr int THREADS = WARPS * 32;
+  constexpr int KP = D / 32;                 // 16-byte pieces of a position's key per lane (four lanes a position)
+  constexpr int VS = D / 64;                 // of a position's value (eight lanes a position)
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  extern __shared__ __align__(16) float am_sum[];          // [warp][head][D]
+  __shared__ __align__(16) __half s_q[AM_HEADS][D + 32];
+  __shared__ float s_m[WARPS][AM_HEADS], s_l[WARPS][AM_HEADS];
+  __shared__ float s_f[AM_HEADS][AM_MAX_SPLITS], s_r[AM_HEADS][AM_MAX_SPLITS], s_tot[AM_HEADS];
+  __shared__ int s_last;
+  const int kvh = blockIdx.x, seq = blockIdx.y, split = blockIdx.z, nsplit = gridDim.z;
+  const int G = H / KV, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const long long pl = pos[seq];
+  const int n_all = pl < 0 ? 1 : (pl >= max_seq ? max_seq : (int)pl + 1);
+  const int chunk = (n_all + nsplit - 1) / nsplit;
+  const int pbeg = split * chunk;
+  const int n_pos = max(0, min(n_all - pbeg, chunk));
+  const size_t row = (size_t)KV * D;         // elements between consecutive positions of a cache
+  const size_t first = ((size_t)seq * max_seq + pbeg) * row + (size_t)kvh * D;
+  const size_t head0 = (size_t)seq * H + (size_t)kvh * G;
+
+  // queries in shared memory (in registers they would spill): a lane's pieces 8 t4 + 32 i of head g8
+  for (int i = tid; i < AM_HEADS * D / 8; i += THREADS) {
+    const int g = i / (D / 8), c = 8 * (i - g * (D / 8));
+    *reinterpret_cast<uint4*>(&s_q[g][c]) = g < G ? *reinterpret_cast<const uint4*>(q + (head0 + g) * D + c) : make_uint4(0, 0, 0, 0);
+  }
+  __syncthreads();
+  const __half* mine_q = &s_q[g8][8 * t4];
+
+  const float scale2 = scale * 1.4426950408889634f;        // scores in powers of two
+  float m = -INFINITY, l = 0.f;
+  float o[8 * VS][4];                        // MMA j + 8 s: its column n is column 64 s + 8 n + j of the head
+#pragma unroll
+  for (int i = 0; i < 8 * VS; ++i)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
+
+#pragma unroll 1
+  for (int base = warp * AM_POS; base < n_pos; base += WARPS * AM_POS) {
+    uint4 kk[2][KP], vv[4][VS];
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      const int p = base + 8 * h + g8;
+#pragma unroll
+      for (int i = 0; i < KP; ++i)
+        kk[h][i] = p < n_pos ? __ldg(reinterpret_cast<const uint4*>(k_cache + first + (size_t)p * row + 8 * t4 + 32 * i)) : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int p = base + 8 * (u >> 1) + 2 * t4 + (u & 1);
+#pragma unroll
+      for (int i = 0; i < VS; ++i)
+        vv[u][i] = p < n_pos ? __ldg(reinterpret_cast<const uint4*>(v_cache + first + (size_t)p * row + 8 * g8 + 64 * i)) : make_uint4(0, 0, 0, 0);
+    }
+    float s[2][4];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) s[h][e] = 0.f;
+#pragma unroll
+    for (int i = 0; i < KP; ++i) {
+      const uint4 qa = *reinterpret_cast<const uint4*>(mine_q + 32 * i);
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        am_mma(s[h], qa.x, 0u, qa.y, 0u, kk[h][i].x, kk[h][i].y);
+        am_mma(s[h], qa.z, 0u, qa.w, 0u, kk[h][i].z, kk[h][i].w);
+      }
+    }
+    // this lane: head g8, positions base + 8 h + 2 t4 + e
+    float top = m;
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        s[h][e] = base + 8 * h + 2 * t4 + e < n_pos ? s[h][e] * scale2 : -INFINITY;
+        top = fmaxf(top, s[h][e]);
+      }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    // (no finite score so far: weights 0, or NaN where a score is NaN, which no maximum shows)
+    const float ref = top == -INFINITY ? 0.f : top;
+    const float keep = ex2(m - ref);         // (m = -infinity: 0)
+    m = top;
+    // weights times 2^15: the halves of their split then reach down to 2^-39 of the largest
+    float w[2][2];
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) w[h][e] = ex2(s[h][e] - ref + 15.f);
+    l = l * keep + ((w[0][0] + w[0][1]) + (w[1][0] + w[1][1]));
+    if (__any_sync(0xffffffffu, keep != 1.f)) {
+#pragma unroll
+      for (int i = 0; i < 8 * VS; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) o[i][e] *= keep;
+    }
+    const uint2 w0 = split_weights(w[0][0], w[0][1]), w1 = split_weights(w[1][0], w[1][1]);
+#pragma unroll
+    for (int i = 0; i < VS; ++i) {
+      const uint32_t* v0 = reinterpret_cast<const uint32_t*>(&vv[0][i]);
+      const uint32_t* v1 = reinterpret_cast<const uint32_t*>(&vv[1][i]);
+      const uint32_t* v2 = reinterpret_cast<const uint32_t*>(&vv[2][i]);
+      const uint32_t* v3 = reinterpret_cast<const uint32_t*>(&vv[3][i]);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
+        am_mma(o[8 * i + j], w0.x, w0.y, w1.x, w1.y, __byte_perm(v0[j >> 1], v1[j >> 1], sel), __byte_perm(v2[j >> 1], v3[j >> 1], sel));
+      }
+    }
+  }
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  if (t4 == 0) {
+    s_m[warp][g8] = m;
+    s_l[warp][g8] = l;
+  }
+  if (g8 < G) {
+    float* to = am_sum + (warp * AM_HEADS + g8) * D;
+#pragma unroll
+    for (int i = 0; i < VS; ++i)
+#pragma unroll
+      for (int c = 0; c < 2; ++c)            // columns n = 2 t4 + c
+#pragma unroll
+        for (int j = 0; j < 8; j += 4)
+          *reinterpret_cast<float4*>(to + 64 * i + 8 * (2 * t4 + c) + j) =
+              make_float4(o[8 * i + j][c] + o[8 * i + j][2 + c], o[8 * i + j + 1][c] + o[8 * i + j + 1][2 + c],
+                          o[8 * i + j + 2][c] + o[8 * i + j + 2][2 + c], o[8 * i + j + 3][c] + o[8 * i + j + 3][2 + c]);
+  }
+  __syncthreads();
+  for (int e = tid; e < G * D; e += THREADS) {
+    const int g = e / D, d = e - g * D;
+    float top = -INFINITY;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) top = fmaxf(top, s_m[w][g]);
+    float sum = 0.f, tot = 0.f;
+#pragma unroll
+    for (int w = 0; w < WARPS; ++w) {
+      // a warp without a finite score adds nothing, unless its sum is NaN
+      const float lw = s_l[w][g], f = s_m[w][g] == -INFINITY ? (lw == 0.f ? 0.f : 1.f) : ex2(s_m[w][g] - top);
+      if (f != 0.f) {
+        sum += f * am_sum[(w * AM_HEADS + g) * D + d];
+        tot += f * lw;
+      }
+    }
+    if (!(fabsf(sum) <= 3.0e38f) && tot == tot) {
+      // An infinite or NaN value takes part.  The two halves of a weight turn infinity into NaN where the product does
+      // not: this column is added again, weight by weight.
+      sum = 0.f;
+      const __half* qh = q + (head0 + g) * D;
+      for (int p = 0; p < n_pos; ++p) {
+        const __half* kr = k_cache + first + (size_t)p * row;
+        float dot = 0.f;
+        for (int c = 0; c < D; ++c) dot += __half2float(qh[c]) * __half2float(kr[c]);
+        sum += ex2(dot * scale2 - (top == -INFINITY ? 0.f : top) + 15.f) * __half2float(v_cache[first + (size_t)p * row + d]);
+      }
+    }
+    if (nsplit == 1) {
+      out[(head0 + g) * D + d] = __float2half(sum / tot);
+    } else {
+      float* mine = part + ((head0 + g) * nsplit + split) * (size_t)(D + 2);
+      mine[2 + d] = sum;
+      if (d == 0) { mine[0] = top; mine[1] = tot; }
+    }
+  }
+  if (nsplit == 1) return;
+  // several ranges: the last CTA of these heads merges
+  __threadfence();
+  __syncthreads();
+  const size_t cidx = (size_t)seq * KV + kvh;
+  if (tid == 0) s_last = atomicAdd(&counters[cidx], 1u) == (unsigned int)(nsplit - 1);
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  // the ranges' weights, then two columns a thread
+  const float* all = part + head0 * nsplit * (size_t)(D + 2);
+  for (int e = tid; e < G * nsplit; e += THREADS) {
+    const int g = e / nsplit, r = e - g * nsplit;
+    const float2 ml = __ldcg(reinterpret_cast<const float2*>(all + (size_t)e * (D + 2)));
+    s_f[g][r] = ml.x;
+    s_r[g][r] = ml.y;
+  }
+  __syncthreads();
+  for (int g = warp; g < G; g += WARPS) {
+    const float mr = lane < nsplit ? s_f[g][lane] : -INFINITY, lr = lane < nsplit ? s_r[g][lane] : 0.f;
+    float top = mr;
+    for (int d = 16; d; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
+    const float f = mr == -INFINITY ? (lr == 0.f ? 0.f : 1.f) : ex2(mr - top);      // an empty range carries no weight
+    float tot = f == 0.f ? 0.f : f * lr;
+    for (int d = 16; d; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
+    if (lane < nsplit) s_f[g][lane] = f;
+    if (lane == 0) s_tot[g] = tot;
+  }
+  __syncthreads();
+  for (int e = tid; e < G * D / 2; e += THREADS) {
+    const int g = e / (D / 2), d = 2 * (e - g * (D / 2));
+    const float* src = all + (size_t)g * nsplit * (D + 2) + 2 + d;
+    float2 v = make_float2(0.f, 0.f);
+#pragma unroll 8
+    for (int r = 0; r < nsplit; ++r) {
+      const float2 x = __ldcg(reinterpret_cast<const float2*>(src + (size_t)r * (D + 2)));
+      const float f = s_f[g][r];
+      if (f != 0.f) {
+        v.x += f * x.x;
+        v.y += f * x.y;
+      }
+    }
+    *reinterpret_cast<__half2*>(out + (head0 + g) * D + d) = __floats2half2_rn(v.x / s_tot[g], v.y / s_tot[g]);
+  }
+  if (tid == 0) counters[cidx] = 0u;                       // ready for the next launch
+}
+
+}  // namespace
+
+bool cq_attn_mma_takes(int sequences, int n_heads, int n_kv_heads, int head_dim, int max_seq) {
+  const int G = n_heads / n_kv_heads;
+  if ((head_dim != 64 && head_dim != 128) || G > AM_HEADS) return false;
+  // Without grouped queries the two-sweep kernel has four CTAs of 256 threads on an SM against three of 128 here.  Up to one
+  // wave of those, and for well-filled waves on short caches, this kernel is faster (128-wide heads on cold caches: 32 at
+  // 256 positions 5.8 us against 7.1, at 2100 13.5 and 17.7; 256 at 200 10.5 and 12.9; 320 at 2100 70 and 81; 1280 at 200
+  // 32 and 37), beyond it is not (480 at 700 47 and 37, 1024 at 3900 331 and 322).
+  const long long tasks = (long long)sequences * n_kv_heads, slots = 3ll * cq_sm_count();
+  const long long waves = (tasks + slots - 1) / slots;
+  return G > 1 || waves == 1 || (max_seq <= 512 && 10 * tasks >= 8 * waves * slots);
+}
+
+int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, const long long* position, void* out, int sequences,
+                       int n_heads, int n_kv_heads, int head_dim, int max_seq, float scale, int most, unsigned int* counters,
+                       float* part, cudaStream_t stream) {
+  // Twelve warps a CTA, one CTA an SM, and the ranges that cost the fewest turns in a row: a wave's turn brings 192
+  // positions to every SM; a range's start and its warps' meeting count as 1.2 turns, the merge of the ranges as one and
+  // more with the heads it is for.  (64 query heads on 8 KV heads at 4000 positions: 1 sequence 14 us, 4 24, 16 53, 32 101;
+  // the fp32 dot products took 47, 112, 283 and 457, flash_attn 20, 27, 64 and 194.)  Without grouped queries: more heads
+  // than SMs take CTAs of four warps, three on an SM (256 heads at 200 positions 10.5 us against 13.5, 320 at 2100 70 and
+  // 78), and so do few heads on short caches, one turn for each range of 64 positions (32 heads at 500 positions 7.3 us
+  // against 8.3).
+  const int sms = cq_sm_count(), G = n_heads / n_kv_heads;
+  const long long tasks = (long long)sequences * n_kv_heads;
+  const bool few = G == 1 && max_seq > 256 && max_seq <= 512 && tasks * 8 <= 3ll * sms;
+  const int warps = few || (G == 1 && tasks > sms) ? 4 : 12;
+  if (most > AM_MAX_SPLITS) most = AM_MAX_SPLITS;
+  int splits = few ? 8 : 1;
+  if (warps == 12) {
+    double best = 0;
+    for (int n = 1; n <= most; ++n) {
+      const long long waves = (tasks * n + sms - 1) / sms;
+      const int turns = ((max_seq + n - 1) / n + 12 * AM_POS - 1) / (12 * AM_POS);
+      const double t = (double)waves * (turns + 1.2) + (n > 1 ? 1.0 + 0.15 * G + 0.05 * n : 0.0);
+      if (n == 1 || t < best) {
+        best = t;
+        splits = n;
+      }
+    }
+  }
+  auto fn = head_dim == 64 ? (warps == 4 ? attn_decode_mma_kernel<64, 4> : attn_decode_mma_kernel<64, 12>)
+                           : (warps == 4 ? attn_decode_mma_kernel<128, 4> : attn_decode_mma_kernel<128, 12>);
+  const int smem = warps * AM_HEADS * head_dim * (int)sizeof(float);
+  CQ_CUDA_TRY(cq_grant_smem((const void*)fn, smem));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(n_kv_heads, sequences, splits);
+  cfg.blockDim = dim3(warps * 32);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, position, (__half*)out,
+                                 part, counters, n_heads, n_kv_heads, max_seq, scale));
+  return CQ_OK;
+}

@@ -1,0 +1,11 @@
+// The decode attention on mma.sync (cq_attn.cu), called by cq_attn_decode for the calls it takes.
+#pragma once
+
+#include "cq_common.cuh"
+
+// Whether the kernel takes such a call (on 16-byte aligned buffers).
+bool cq_attn_mma_takes(int sequences, int n_heads, int n_kv_heads, int head_dim, int max_seq);
+// counters, part: the workspace as cq_attn_decode lays it out, partial results of up to `most` ranges per head.
+int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, const long long* position, void* out, int sequences,
+                       int n_heads, int n_kv_heads, int head_dim, int max_seq, float scale, int most, unsigned int* counters,
+                       float* part, cudaStream_t stream);

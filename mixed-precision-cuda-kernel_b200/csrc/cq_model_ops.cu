@@ -4,6 +4,7 @@
 // apply_rotary_pos_emb, LlamaMLP.forward of the reference project); at batch 1 each of them is a
 // launch-latency-bound kernel, so the harness fuses them to keep the step dominated by the
 // projections.  fp16 in / out, fp32 arithmetic.
+#include "cq_attn.cuh"
 #include "cq_common.cuh"
 
 namespace {
@@ -303,7 +304,7 @@ __global__ void __launch_bounds__(ATT_THREADS) attn_decode_kernel(const __half* 
   if (tid == 0) counters[hidx] = 0u;                                  // ready for the next launch
 }
 
-// One query head per CTA in one sweep over its positions, for the head widths in use (LPP = D / 8 lanes take a position
+// One query head per CTA in one sweep over its positions, where the kernel of cq_attn.cu is not taken (LPP = D / 8 lanes take a position
 // with 16-byte loads).  A step of short contexts is a chain of memory latencies; the kernels above and below have two of
 // them (all scores before the first value is fetched) and five barriers.  Here every group of lanes fetches the keys and
 // values of its next UF positions at once and keeps its own running maximum, sum and weighted values; the groups meet
@@ -465,7 +466,7 @@ __global__ void __launch_bounds__(ONE_THREADS) attn_decode_one_kernel(const __ha
   if (tid == 0) counters[hidx] = 0u;                                  // ready for the next launch
 }
 
-// Two sweeps, for grouped-query models on long caches and for many heads: one CTA per KV head (blockIdx.x),
+// Two sweeps, for 256-wide grouped-query heads on long caches and for many heads: one CTA per KV head (blockIdx.x),
 // sequence and range of positions handles all G = H / KV query heads that share the KV head, so every K and V
 // row is read once (with one CTA per query head it is read G times through L2).  A group of D / 8 lanes takes one
 // position with 16-byte loads (8 values a lane), GT >= G query heads at a time in registers.  Partial
@@ -770,24 +771,25 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
   const int G = n_heads / n_kv_heads;
   const bool wide = (head_dim == 64 || head_dim == 128 || head_dim == 256) &&
                     (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
+  if (wide && ((uintptr_t)out & 3) == 0 && cq_attn_mma_takes(sequences, n_heads, n_kv_heads, head_dim, max_seq))
+    return cq_attn_mma_launch(q, k_cache, v_cache, position, out, sequences, n_heads, n_kv_heads, head_dim, max_seq, scale,
+                              ATT_MAX_SPLITS, counters, part, (cudaStream_t)stream);
   const int sms = cq_sm_count();
   const int splits = attn_splits(sms, sequences, n_heads, max_seq);
+  // What is left: 256-wide heads, more than 8 query heads per KV head, and many heads without grouped queries.
   // One CTA per KV head reads every cache row once for the query heads that share it; with several query heads
-  // per KV head its per-position arithmetic is G times larger, which only pays on long caches (measured, 70B
-  // shapes: 103 us against 174 at 4000 positions, but 21 against 15 at 200): short grouped-query caches take
+  // per KV head its per-position arithmetic is G times larger, which only pays on long caches (measured on 128-wide heads,
+  // 8 per KV head: 103 us against 174 at 4000 positions, but 21 against 15 at 200): short grouped-query caches take
   // a CTA per query head, whose re-reads hit L2.
   // Without grouped queries the same kernel competes with the one-sweep kernel, which has one latency less but runs one
   // CTA of 512 threads per SM (128 registers), where four of the other's 256 threads fit.  Measured on cold caches:
-  //   all of the call's CTAs at once (128-wide heads: 32 at 500 of 512 positions 9.6 us against 14.4, 16 at 1000 of 1024 9.6
-  //   against 14.1; with one CTA per SM exceeded, 40 at 1000 of 1024 15.5 against 15.2, 8 x 32 at 500 of 512 33 against 22):
-  //   one sweep.  64-wide heads on caches of up to 256 positions are the exception: 8.8 us against 8.4 at 200, 9.0
-  //   against 10.5 at 500.
+  //   all of the call's CTAs at once (128-wide heads: 32 at 500 of 512 positions 9.6 us against 14.4): one sweep.
   //   between four and five CTAs per SM (608 .. 736 heads), where the other kernel has a second wave that is nearly empty
   //   and this one its fifth: 152 us against 177 at 2200 positions, 52 against 51 at 500, 42 against 33 at 300: one sweep
   //   on caches of 1024 positions and more.
   //   Caches whose scores would not fit the other kernel's shared memory.
   const long long heads_all = (long long)sequences * n_heads;
-  const bool one_sweep = (heads_all * splits <= sms && (head_dim > 64 || max_seq > 256)) ||
+  const bool one_sweep = heads_all * splits <= sms ||
                          (heads_all > 4ll * sms && heads_all <= 5ll * sms && max_seq >= 1024) ||
                          (size_t)((max_seq + splits - 1) / splits) * sizeof(float) > 200 * 1024;
   if (wide && G <= 8 && (G > 1 ? max_seq > 1024 : !one_sweep)) {

@@ -84,17 +84,18 @@ class CherryDecoder:
             raise ValueError("batch must be at least 1")
         self.cfg, self.dev, self.dense = cfg, torch.device(device), dense
         self.batch = batch          # sequences decoded in lockstep (same prompt length, one position counter)
-        # decode attention over the KV cache: "own" = this library's kernel (cq_attn_decode); "flash" = the
+        # decode attention over the KV cache: "own" = this library's kernels (cq_attn_decode); "flash" = the
         # flash_attn package's flash_attn_with_kvcache (a library call, like the lm_head's cuBLAS matmul);
-        # "auto" = own, except for grouped-query models with caches of more than 1024 positions where that
-        # package imports.  Measured on B200 with cold caches: without grouped queries the own kernels are level or
-        # ahead (7B at 200 positions 8.6 us against 9.7; 13B shapes at 2100 positions 20.7 against 20.4 at batch 1, 86
-        # against 159 at batch 8); with 8 query heads per KV head at 4000 positions their SIMT dot products lose to
-        # flash_attn's tensor-core tiles (44 us against 20 at batch 1, 114 against 27 at batch 4).
+        # "auto" = own, except for grouped-query models with caches of more than 1024 positions whose heads the tensor-core
+        # kernel does not take, where that package imports.  Measured on B200 with cold caches, own against flash_attn:
+        # 7B at 256 positions 5.8 us and 9.5; 13B shapes at 2100 positions, batch 8, 70 and 159; 8 query heads per KV head
+        # at 4000 positions 14 and 20 at batch 1, 24 and 27 at 4, 53 and 64 at 16, 101 and 194 at 32.
         if attention not in ("auto", "own", "flash"):
             raise ValueError("attention is 'auto', 'own' or 'flash'")
         self._flash = None
-        if attention == "flash" or (attention == "auto" and cfg.max_seq > 1024 and cfg.n_kv_heads < cfg.n_heads):
+        grouped = cfg.n_heads // cfg.n_kv_heads
+        if attention == "flash" or (attention == "auto" and cfg.max_seq > 1024 and
+                                    grouped > (8 if cfg.head_dim in (64, 128) else 1)):
             try:
                 from flash_attn import flash_attn_with_kvcache
                 self._flash = flash_attn_with_kvcache

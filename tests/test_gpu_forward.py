@@ -215,6 +215,39 @@ def test_attention_on_both_sides_of_the_dispatch(D, B, H, max_seq):
             assert float((out[b].float() - ref).abs().max()) <= 4e-3         # as in test_attention_sweep_edges
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,KV,max_seq", [(5, 8, 1, 193), (5, 6, 2, 700), (20, 64, 8, 400), (1, 64, 8, 4100), (5, 40, 40, 300),
+                                            (9, 50, 50, 500)])
+def test_attention_on_tensor_cores(D, B, H, KV, max_seq):
+    """Turns of 16 positions a warp (64 and 192 a CTA), one to eight heads per KV head, one and several ranges, CTAs of 4 and
+    12 warps.  Weights beside the largest that an 11-bit weight would lose, and infinite values: of weight 0 and not."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    g = torch.Generator(device="cuda").manual_seed(H + max_seq)
+    G = H // KV
+    q = torch.randn(B, H, D, device="cuda", generator=g).half()
+    k, v = (torch.randn(B, max_seq, KV, D, device="cuda", generator=g).half() for _ in range(2))
+    at = [0, 15, 16, 63, 64, 191, 192, max_seq - 1, max_seq // 2]
+    pos = torch.tensor([min(at[b % 9], max_seq - 1) for b in range(B)], device="cuda")
+    v[:, 1:, 0] *= 0.02
+    v[:, 0, 0] = 300.                                           # one large value: the others show in the last bits
+    k[:, 0, 0] *= 0.5
+
+    def reference(b, vv):
+        n = int(pos[b]) + 1
+        s = torch.einsum("gd,pd->gp", q[b, :G].double(), k[b, :n, 0].double()) / math.sqrt(D)
+        return s.softmax(-1) @ vv[b, :n, 0].double()
+    out = qc.attn_decode(q, k, v, pos).view(B, H, D)
+    for b in range(B):
+        ref = reference(b, v)
+        # half an fp16 step of the result, and 2^-16 for the exponentials and fp32 sums
+        assert bool(((out[b, :G].double() - ref).abs() <= (2.0 ** -11 + 2.0 ** -16) * ref.abs() + 1e-6).all())
+    v[:, 0, 0, 1], v[:, 0, 0, 2] = float("inf"), float("-inf")
+    out = qc.attn_decode(q, k, v, pos).view(B, H, D)
+    assert bool((out[:, :G, 1] == float("inf")).all() and (out[:, :G, 2] == float("-inf")).all())
+    assert bool(out[:, :G, 3:].isfinite().all() and out[:, :G, 0].isfinite().all() and out[:, G:].isfinite().all())
+
+
 @pytest.mark.parametrize("m,C", [(1, 16), (40, 16), (3, 256)])     # row kernel, GEMM, stream matvec
 def test_copies_dropped_while_another_stream_uses_them(m, C):
     """The block of a dropped copy is not given out before the launches that read it have finished, and is afterwards."""
