@@ -4,12 +4,14 @@
 // the weight's type as the element-wise torch expressions round it.  With `ste` the result is (real - w) + w, the
 // value of the straight-through expression.
 //
-// Bound: HBM, one read and one write of the matrix; the chain of torch operations moves it about twenty times.  A
-// block owns a row: the first sweep takes the group maxima (warp reduction, one shared-memory maximum per warp and
-// group), the second re-reads the row from L1 and writes.  The order of the columns never changes, so there is no
-// gather: a table made once per call gives every octet of columns its position in the compact order and its
-// quantised columns.  A training step of a 4096 -> 11008 layer on 2048 tokens in bf16: 2150 us with the torch chain,
-// 552 us with this kernel, of which the three products take about 450.
+// Bound: HBM, one read and one write of the matrix; the chain of torch operations moves it about twenty times.  The order of
+// the columns never changes, so there is no gather: a table made once per call gives every octet of columns its group, the
+// columns of it that are quantised, and those of them that belong to the next group.
+//   16-bit weights: a block goes down the rows.  One sweep takes the group maxima, the second re-reads the row from L1 and
+//   writes.  Both run on packed pairs, rounded as the expressions round, and treat every octet as one whole group's; the
+//   few others (a cherry column or a group's end inside) are on a list and are done apart, so that they do not hold up
+//   the warps.  4096 x 11008 bf16: 111 us element by element (73 instructions a weight, bound by the issue rate).
+//   fp32 weights: element by element, a block a row.
 #include <cuda_bf16.h>
 
 #include <type_traits>
@@ -20,8 +22,9 @@ namespace {
 
 constexpr int FQ_THREADS = 256;
 
-// table[o] = quantised columns before octet o << 8 | mask of the quantised columns inside it
-__global__ void __launch_bounds__(1024) fq_table_kernel(const uint8_t* __restrict__ quantised, int n_oct,
+// table[o] = group of octet o's first quantised column << 16 | mask of the columns of the next group << 8 | mask of all
+// quantised columns (G >= 8: an octet has two groups at most)
+__global__ void __launch_bounds__(1024) fq_table_kernel(const uint8_t* __restrict__ quantised, int n_oct, int G, int ng,
                                                         uint32_t* __restrict__ table) {
   __shared__ uint32_t warp_sum[32];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -45,50 +48,43 @@ __global__ void __launch_bounds__(1024) fq_table_kernel(const uint8_t* __restric
   for (int w = 0; w < warp; ++w) rank += warp_sum[w];
   for (int o = o0; o < o1; ++o) {
     const uint32_t m = mask_of(o);
-    table[o] = (rank << 8) | m;
+    const uint32_t g = min(rank / (uint32_t)G, (uint32_t)(ng - 1)), rest = (g + 1) * G - rank;
+    uint32_t next = rest < 8 ? m : 0u;
+    for (uint32_t i = 0; i < rest && next; ++i) next &= next - 1;
+    table[o] = (g << 16) | (next << 8) | m;
     rank += __popc(m);
   }
 }
 
-template <typename T> struct FqType;
-template <> struct FqType<float> {
-  static __device__ __forceinline__ void load(const float* p, float* v) {
-    const float4 a = *reinterpret_cast<const float4*>(p), b = *reinterpret_cast<const float4*>(p + 4);
-    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+// ------------------------------------------------------------------ 16-bit weights, in packed pairs
+// (explicit roundings: nothing is contracted into a fused multiply-add)
+#define FQ_OP2(name, instr)                                                       \
+  static __device__ __forceinline__ uint32_t name(uint32_t a, uint32_t b) {      \
+    uint32_t d;                                                                   \
+    asm(instr " %0, %1, %2;" : "=r"(d) : "r"(a), "r"(b));                         \
+    return d;                                                                     \
   }
-  static __device__ __forceinline__ void store(float* p, const float* v) {
-    *reinterpret_cast<float4*>(p) = make_float4(v[0], v[1], v[2], v[3]);
-    *reinterpret_cast<float4*>(p + 4) = make_float4(v[4], v[5], v[6], v[7]);
-  }
-  static __device__ __forceinline__ float2 round2(float a, float b) { return make_float2(a, b); }
-  static __device__ __forceinline__ float div(float w, float s, float) { return __fdiv_rn(w, s); }
-};
-template <> struct FqType<__half> {
-  static __device__ __forceinline__ void load(const __half* p, float* v) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&w[i]));
-      v[2 * i] = f.x;
-      v[2 * i + 1] = f.y;
-    }
-  }
-  static __device__ __forceinline__ void store(__half* p, const float* v) {
-    __half2 h[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = __floats2half2_rn(v[2 * i], v[2 * i + 1]);
-    *reinterpret_cast<uint4*>(p) = *reinterpret_cast<const uint4*>(h);
-  }
-  static __device__ __forceinline__ float2 round2(float a, float b) { return __half22float2(__floats2half2_rn(a, b)); }
-  // close enough to w / s that its fp16 rounding is the quotient's (Markstein's residual step; two 11-bit
-  // significands never have a quotient within 2^-23 of a midpoint); an infinite s gives 0 or NaN as the division does
-  static __device__ __forceinline__ float div(float w, float s, float r) {
-    const float q = __fmul_rn(w, r);
-    return s < 65536.f ? __fmaf_rn(__fmaf_rn(-q, s, w), r, q) : q;
+template <typename T> struct FqPair;
+template <> struct FqPair<__half> {
+  static constexpr uint32_t HALF = 0x38003800u, MAGIC = 0x66006600u;     // 0.5; 1536: a sum up to 8.5 away is an integer
+  FQ_OP2(add, "add.rn.f16x2")
+  FQ_OP2(sub, "sub.rn.f16x2")
+  FQ_OP2(mul, "mul.rn.f16x2")
+  FQ_OP2(max, "max.NaN.f16x2")
+  FQ_OP2(min, "min.NaN.f16x2")
+  static __device__ __forceinline__ float2 widen(uint32_t u) { return __half22float2(*reinterpret_cast<const __half2*>(&u)); }
+  static __device__ __forceinline__ uint32_t narrow(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
   }
 };
-template <> struct FqType<__nv_bfloat16> {
+template <> struct FqPair<__nv_bfloat16> {
+  static constexpr uint32_t HALF = 0x3F003F00u, MAGIC = 0x43404340u;     // 0.5; 192
+  FQ_OP2(add, "add.rn.bf16x2")
+  FQ_OP2(sub, "sub.rn.bf16x2")
+  FQ_OP2(mul, "mul.rn.bf16x2")
+  FQ_OP2(max, "max.NaN.bf16x2")
+  FQ_OP2(min, "min.NaN.bf16x2")
   static __device__ __forceinline__ float2 widen(uint32_t u) {
     return make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xFFFF0000u));
   }
@@ -96,27 +92,166 @@ template <> struct FqType<__nv_bfloat16> {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
   }
-  static __device__ __forceinline__ void load(const __nv_bfloat16* p, float* v) {
-    const uint4 u = *reinterpret_cast<const uint4*>(p);
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 f = widen(w[i]);
-      v[2 * i] = f.x;
-      v[2 * i + 1] = f.y;
-    }
-  }
-  static __device__ __forceinline__ void store(__nv_bfloat16* p, const float* v) {
-    uint32_t h[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) h[i] = narrow(v[2 * i], v[2 * i + 1]);
-    *reinterpret_cast<uint4*>(p) = make_uint4(h[0], h[1], h[2], h[3]);
-  }
-  static __device__ __forceinline__ float2 round2(float a, float b) { return widen(narrow(a, b)); }
-  // two 8-bit significands never have a quotient within 2^-17 of a bf16 midpoint: one product is enough
-  static __device__ __forceinline__ float div(float w, float, float r) { return __fmul_rn(w, r); }
 };
+#undef FQ_OP2
 
+// A pair of weights quantised with a scale (twice in s2; r = RN(1 / s)), before the straight-through expression.  The
+// quotients: an fp32 product with r is within 2^-23 of the quotient, and no quotient of two 11-bit (8-bit) significands
+// is that close to a midpoint of two normal numbers of the type; quotients below the normal numbers leave -0.5 or what is
+// next to it after the subtraction, either way.  Every other step is one rounding of an exact sum or product, as in the
+// expressions (fp32 holds the exact result of each; differences so wide apart that it does not are no midpoints).
+template <typename T> __device__ __forceinline__ uint32_t fq_pair(uint32_t w, float r, uint32_t s2, uint32_t lim2) {
+  using F = FqPair<T>;
+  const float2 v = F::widen(w);
+  uint32_t q = F::narrow(__fmul_rn(v.x, r), __fmul_rn(v.y, r));
+  q = F::min(F::max(q, lim2 ^ 0x80008000u), lim2);
+  q = F::sub(q, F::HALF);
+  q = F::sub(F::add(q, F::MAGIC), F::MAGIC);
+  return F::mul(F::add(q, F::HALF), s2);
+}
+template <typename T> __device__ __forceinline__ uint32_t fq_through(uint32_t q, uint32_t w, int ste) {
+  return ste ? FqPair<T>::add(FqPair<T>::sub(q, w), w) : q;
+}
+// bits e and e + 1 of m as halves of ones
+__device__ __forceinline__ uint32_t fq_halves(uint32_t m, int e) {
+  return ((m >> e) & 1u ? 0xFFFFu : 0u) | ((m >> e) & 2u ? 0xFFFF0000u : 0u);
+}
+// the larger half as the bits of an fp32 number (NaN above all)
+template <typename T> __device__ __forceinline__ uint32_t fq_larger(uint32_t u) {
+  const float2 f = FqPair<T>::widen(u);
+  return max(__float_as_uint(f.x), __float_as_uint(f.y));
+}
+
+constexpr int FQ_LIST = 1024;                // octets on the list; more are looked for again on each turn
+
+// FQ_ROWS rows a turn: one look at the table for all, their loads in flight together.
+template <typename T, int FQ_ROWS>
+__global__ void __launch_bounds__(FQ_THREADS, 4) fake_quant_pairs_kernel(const T* __restrict__ w, const uint32_t* __restrict__ table,
+                                                                         int bits, int K, int N, int ng, int ste, T* __restrict__ out) {
+  using F = FqPair<T>;
+  extern __shared__ __align__(8) uint32_t fq_smem[];
+  uint2* scale = reinterpret_cast<uint2*>(fq_smem);           // [FQ_ROWS][ng] scale as a pair, 1 / scale
+  uint32_t* gmax = fq_smem + 2 * FQ_ROWS * ng;                // [FQ_ROWS][ng] bits of the group maxima; zero between turns
+  __shared__ int list[FQ_LIST], s_n;
+  const int tid = threadIdx.x, lane = tid & 31, n_oct = K >> 3;
+  auto whole = [](uint32_t t) { return (t & 0xFFFFu) == 0xFFu; };
+  if (tid == 0) s_n = 0;
+  for (int g = tid; g < FQ_ROWS * ng; g += FQ_THREADS) gmax[g] = 0u;
+  __syncthreads();
+  for (int o = tid; o < n_oct; o += FQ_THREADS)
+    if (!whole(table[o])) {
+      const int at = atomicAdd(&s_n, 1);
+      if (at < FQ_LIST) list[at] = o;
+    }
+  __syncthreads();
+  const bool listed = s_n <= FQ_LIST;
+  const int n_list = listed ? s_n : n_oct;
+  const float inv = 1.f / (float)(1 << (bits - 1));           // a power of two: the product is the quotient
+  const uint32_t lim2 = F::narrow((float)((double)(1 << (bits - 1)) - 1e-2), (float)((double)(1 << (bits - 1)) - 1e-2));
+  constexpr uint32_t ABS = 0x7FFF7FFFu;
+
+  for (int n = blockIdx.x * FQ_ROWS; n < N; n += gridDim.x * FQ_ROWS) {
+    const int rows = min(FQ_ROWS, N - n);
+    const uint4* row[FQ_ROWS];                                // (rows past the matrix repeat its last one)
+#pragma unroll
+    for (int r = 0; r < FQ_ROWS; ++r) row[r] = reinterpret_cast<const uint4*>(w + (size_t)(n + min(r, rows - 1)) * K);
+    // f(row, octet, table entry) for the octets that are not one whole group's
+    auto others = [&](auto f) {
+      for (int i = tid; i < n_list * FQ_ROWS; i += FQ_THREADS) {
+        const int o = listed ? list[i / FQ_ROWS] : i / FQ_ROWS, r = i % FQ_ROWS;
+        const uint32_t t = table[o];
+        if (!whole(t) && r < rows) f(r, o, t);
+      }
+    };
+    // ---- group maxima
+    for (int o0 = tid & ~31; o0 < n_oct; o0 += FQ_THREADS) {
+      const int o = o0 + lane;
+      uint32_t m[FQ_ROWS] = {};
+      int g = 0x7fffffff;
+      if (o < n_oct) {
+        const uint32_t t = table[o];
+        uint4 v[FQ_ROWS];
+#pragma unroll
+        for (int r = 0; r < FQ_ROWS; ++r) v[r] = row[r][o];
+        if (whole(t)) {
+          g = (int)(t >> 16);
+#pragma unroll
+          for (int r = 0; r < FQ_ROWS; ++r)
+            m[r] = fq_larger<T>(F::max(F::max(v[r].x & ABS, v[r].y & ABS), F::max(v[r].z & ABS, v[r].w & ABS)));
+        }
+      }
+      // one maximum per group and warp
+      const int g_lo = __reduce_min_sync(0xffffffffu, g), g_hi = __reduce_max_sync(0xffffffffu, g == 0x7fffffff ? -1 : g);
+      for (int q = g_lo; q <= g_hi; ++q) {
+        uint32_t top = 0;                                     // lane r: row r's
+#pragma unroll
+        for (int r = 0; r < FQ_ROWS; ++r) {
+          const uint32_t x = __reduce_max_sync(0xffffffffu, g == q ? m[r] : 0u);
+          if (lane == r) top = x;
+        }
+        if (lane < FQ_ROWS && top) atomicMax(&gmax[lane * ng + q], top);
+      }
+    }
+    others([&](int r, int o, uint32_t t) {
+      const uint4 v = reinterpret_cast<const uint4*>(w + (size_t)(n + r) * K)[o];
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w}, next = (t >> 8) & 0xFFu, own = t & 0xFFu & ~next;
+      uint32_t a = 0, b = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a = F::max(a, u[i] & ABS & fq_halves(own, 2 * i));
+        b = F::max(b, u[i] & ABS & fq_halves(next, 2 * i));
+      }
+      if (own) atomicMax(&gmax[r * ng + (t >> 16)], fq_larger<T>(a));
+      if (next) atomicMax(&gmax[r * ng + (t >> 16) + 1], fq_larger<T>(b));
+    });
+    __syncthreads();
+    // ---- scales
+    for (int g = tid; g < FQ_ROWS * ng; g += FQ_THREADS) {
+      const float a = F::widen(F::narrow(__fadd_rn(__uint_as_float(gmax[g]), 1e-6f), 0.f)).x;
+      const uint32_t s2 = F::narrow(__fmul_rn(a, inv), __fmul_rn(a, inv));
+      scale[g] = make_uint2(s2, __float_as_uint(__frcp_rn(F::widen(s2).x)));
+      gmax[g] = 0u;
+    }
+    __syncthreads();
+    // ---- weights
+    for (int o = tid; o < n_oct; o += FQ_THREADS) {
+      const uint32_t t = table[o];
+      if (!whole(t)) continue;
+      uint4 v[FQ_ROWS];
+#pragma unroll
+      for (int r = 0; r < FQ_ROWS; ++r) v[r] = row[r][o];
+      uint4* dst = reinterpret_cast<uint4*>(out + (size_t)n * K) + o;
+#pragma unroll
+      for (int r = 0; r < FQ_ROWS; ++r) {
+        const uint2 sc = scale[r * ng + (t >> 16)];
+        const float x = __uint_as_float(sc.y);
+        v[r].x = fq_through<T>(fq_pair<T>(v[r].x, x, sc.x, lim2), v[r].x, ste);
+        v[r].y = fq_through<T>(fq_pair<T>(v[r].y, x, sc.x, lim2), v[r].y, ste);
+        v[r].z = fq_through<T>(fq_pair<T>(v[r].z, x, sc.x, lim2), v[r].z, ste);
+        v[r].w = fq_through<T>(fq_pair<T>(v[r].w, x, sc.x, lim2), v[r].w, ste);
+        if (r < rows) *dst = v[r];
+        dst += n_oct;
+      }
+    }
+    others([&](int r, int o, uint32_t t) {
+      const uint4 v = reinterpret_cast<const uint4*>(w + (size_t)(n + r) * K)[o];
+      const uint32_t next = (t >> 8) & 0xFFu, own = t & 0xFFu & ~next;
+      const uint2 s0 = scale[r * ng + (t >> 16)], s1 = next ? scale[r * ng + (t >> 16) + 1] : s0;
+      uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t a = fq_halves(own, 2 * i), b = fq_halves(next, 2 * i);
+        uint32_t q = u[i] & ~(a | b);                             // cherry columns keep their value
+        q |= fq_pair<T>(u[i], __uint_as_float(s0.y), s0.x, lim2) & a;
+        q |= fq_pair<T>(u[i], __uint_as_float(s1.y), s1.x, lim2) & b;
+        u[i] = fq_through<T>(q, u[i], ste);
+      }
+      reinterpret_cast<uint4*>(out + (size_t)(n + r) * K)[o] = make_uint4(u[0], u[1], u[2], u[3]);
+    });
+  }
+}
+
+// ------------------------------------------------------------------ fp32 weights
 // minimum and maximum that keep NaN, as torch.clamp does
 __device__ __forceinline__ float clamp_nan(float v, float lim) {
   float r;
@@ -126,21 +261,17 @@ __device__ __forceinline__ float clamp_nan(float v, float lim) {
 // nearest integer, ties to even, of |v| <= 2^21 (NaN stays NaN)
 __device__ __forceinline__ float nearest(float v) { return __fsub_rn(__fadd_rn(v, 12582912.f), 12582912.f); }
 
-template <typename T>
-__global__ void __launch_bounds__(FQ_THREADS) fake_quant_kernel(const T* __restrict__ w, const uint32_t* __restrict__ table,
-                                                                int bits, int K, int G, int ste, T* __restrict__ out) {
+__global__ void __launch_bounds__(FQ_THREADS) fake_quant_kernel(const float* __restrict__ w, const uint32_t* __restrict__ table,
+                                                                int bits, int K, int ng, int ste, float* __restrict__ out) {
   extern __shared__ uint32_t gmax[];          // bits of the group maxima, then of the scales
-  using F = FqType<T>;
-  const int tid = threadIdx.x, lane = tid & 31, n_oct = K >> 3, ng = (K + G - 1) / G;
-  const T* row = w + (size_t)blockIdx.x * K;
-  T* dst = out + (size_t)blockIdx.x * K;
+  const int tid = threadIdx.x, lane = tid & 31, n_oct = K >> 3;
+  const float* row = w + (size_t)blockIdx.x * K;
+  float* dst = out + (size_t)blockIdx.x * K;
   for (int g = tid; g < ng; g += FQ_THREADS) gmax[g] = 0u;
   __syncthreads();
-  // octet o's quantised columns belong to group g, from the rem-th on to group g + 1 (G >= 8)
-  auto second = [&](uint32_t m, int rem) {
-    if (rem >= 8) return 0u;
-    for (int i = 0; i < rem; ++i) m &= m - 1;
-    return m;
+  auto load = [&](int o, float* v) {
+    const float4 a = *reinterpret_cast<const float4*>(row + 8 * o), b = *reinterpret_cast<const float4*>(row + 8 * o + 4);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
   };
   for (int o0 = (tid >> 5) * 32; o0 < n_oct; o0 += FQ_THREADS) {
     const int o = o0 + lane;
@@ -148,16 +279,14 @@ __global__ void __launch_bounds__(FQ_THREADS) fake_quant_kernel(const T* __restr
     int g = 0x7fffffff;
     if (o < n_oct) {
       float v[8];
-      F::load(row + 8 * o, v);
-      const uint32_t t = table[o], m = t & 0xFFu;
-      const int rank = (int)(t >> 8);
-      g = rank / G;
-      const uint32_t sec = second(m, (g + 1) * G - rank);
+      load(o, v);
+      const uint32_t t = table[o];
+      g = (int)(t >> 16);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const uint32_t a = __float_as_uint(v[e]) & 0x7FFFFFFFu;
-        if ((sec >> e) & 1u) m1 = max(m1, a);
-        else if ((m >> e) & 1u) m0 = max(m0, a);
+        if ((t >> (8 + e)) & 1u) m1 = max(m1, a);
+        else if ((t >> e) & 1u) m0 = max(m0, a);
       }
     }
     // one maximum per group and warp
@@ -170,39 +299,24 @@ __global__ void __launch_bounds__(FQ_THREADS) fake_quant_kernel(const T* __restr
   }
   __syncthreads();
   const float inv = 1.f / (float)(1 << (bits - 1));           // a power of two: the product is the quotient
-  for (int g = tid; g < ng; g += FQ_THREADS) {
-    const float a = F::round2(__fadd_rn(__uint_as_float(gmax[g]), 1e-6f), 0.f).x;
-    gmax[g] = __float_as_uint(F::round2(__fmul_rn(a, inv), 0.f).x);
-  }
+  for (int g = tid; g < ng; g += FQ_THREADS) gmax[g] = __float_as_uint(__fmul_rn(__fadd_rn(__uint_as_float(gmax[g]), 1e-6f), inv));
   __syncthreads();
-  const float lim = F::round2((float)((double)(1 << (bits - 1)) - 1e-2), 0.f).x;
+  const float lim = (float)((double)(1 << (bits - 1)) - 1e-2);
   for (int o = tid; o < n_oct; o += FQ_THREADS) {
     float v[8];
-    F::load(row + 8 * o, v);
-    const uint32_t t = table[o], m = t & 0xFFu;
-    const int rank = (int)(t >> 8), g = min(rank / G, ng - 1);
-    const uint32_t sec = second(m, (g + 1) * G - rank);
-    const float s0 = __uint_as_float(gmax[g]), s1 = sec ? __uint_as_float(gmax[g + 1]) : s0;
-    const float r0 = __frcp_rn(s0), r1 = sec ? __frcp_rn(s1) : r0;
+    load(o, v);
+    const uint32_t t = table[o], sec = (t >> 8) & 0xFFu;
+    const float s0 = __uint_as_float(gmax[t >> 16]), s1 = sec ? __uint_as_float(gmax[(t >> 16) + 1]) : s0;
 #pragma unroll
-    for (int e = 0; e < 8; e += 2) {
-      const bool b0 = (sec >> e) & 1u, b1 = (sec >> e) & 2u;
-      const float sa = b0 ? s1 : s0, sb = b1 ? s1 : s0;
-      float2 q = F::round2(F::div(v[e], sa, b0 ? r1 : r0), F::div(v[e + 1], sb, b1 ? r1 : r0));
-      q.x = clamp_nan(q.x, lim);
-      q.y = clamp_nan(q.y, lim);
-      q = F::round2(__fsub_rn(q.x, 0.5f), __fsub_rn(q.y, 0.5f));
-      q = F::round2(__fmul_rn(__fadd_rn(nearest(q.x), 0.5f), sa), __fmul_rn(__fadd_rn(nearest(q.y), 0.5f), sb));
-      if (!((m >> e) & 1u)) q.x = v[e];
-      if (!((m >> e) & 2u)) q.y = v[e + 1];
-      if (ste) {
-        q = F::round2(__fsub_rn(q.x, v[e]), __fsub_rn(q.y, v[e + 1]));
-        q = make_float2(__fadd_rn(q.x, v[e]), __fadd_rn(q.y, v[e + 1]));
-      }
-      v[e] = q.x;
-      v[e + 1] = q.y;
+    for (int e = 0; e < 8; ++e) {
+      const float s = (sec >> e) & 1u ? s1 : s0;
+      float q = __fsub_rn(clamp_nan(__fdiv_rn(v[e], s), lim), 0.5f);
+      q = __fmul_rn(__fadd_rn(nearest(q), 0.5f), s);
+      if (!((t >> e) & 1u)) q = v[e];
+      v[e] = ste ? __fadd_rn(__fsub_rn(q, v[e]), v[e]) : q;
     }
-    F::store(dst + 8 * o, v);
+    *reinterpret_cast<float4*>(dst + 8 * o) = make_float4(v[0], v[1], v[2], v[3]);
+    *reinterpret_cast<float4*>(dst + 8 * o + 4) = make_float4(v[4], v[5], v[6], v[7]);
   }
 }
 
@@ -216,19 +330,29 @@ extern "C" int cq_fake_quant(const void* weight, int dtype, const uint8_t* quant
   if (K <= 0 || N <= 0 || K % 8 || K >= (1 << 24)) return CQ_ERR_BAD_SHAPE;
   if (G < 8) return CQ_ERR_BAD_GROUP;
   if (G > K) G = K;
-  const size_t smem = (size_t)((K + G - 1) / G) * 4;
-  if (smem > 48 * 1024) return CQ_ERR_TOO_LARGE;
+  const int ng = (K + G - 1) / G;
+  if ((size_t)ng * 4 > 48 * 1024) return CQ_ERR_TOO_LARGE;
   cudaStream_t st = (cudaStream_t)stream;
-  fq_table_kernel<<<1, 1024, 0, st>>>(quantised, K / 8, table);
-  auto launch = [&](auto* wp, auto* op) {
-    using T = std::remove_pointer_t<decltype(op)>;
-    fake_quant_kernel<T><<<N, FQ_THREADS, smem, st>>>(wp, table, bits, K, G, ste, op);
-  };
-  switch (dtype) {
-    case 0: launch((const __half*)weight, (__half*)out); break;
-    case 1: launch((const float*)weight, (float*)out); break;
-    case 2: launch((const __nv_bfloat16*)weight, (__nv_bfloat16*)out); break;
-    default: return CQ_ERR_BAD_ARG;
+  if (dtype < 0 || dtype > 2) return CQ_ERR_BAD_ARG;
+  fq_table_kernel<<<1, 1024, 0, st>>>(quantised, K / 8, G, ng, table);
+  if (dtype == 1) {
+    fake_quant_kernel<<<N, FQ_THREADS, (size_t)ng * 4, st>>>((const float*)weight, table, bits, K, ng, ste, (float*)out);
+  } else {
+    // Four rows a turn where the matrix has a turn for every block that the chip holds and the groups of four rows fit
+    // shared memory comfortably; two waves of blocks, each of which makes its list once and goes down the rows.
+    const int blocks = 8 * cq_sm_count(), rows = N >= 2 * blocks && ng <= 1000 ? 4 : 1;
+    const int smem = rows * ng * 12, turns = (N + rows - 1) / rows;
+    auto launch = [&](auto kernel, auto* wp, auto* op) -> int {
+      CQ_CUDA_TRY(cq_grant_smem((const void*)kernel, smem));
+      kernel<<<turns < blocks ? turns : blocks, FQ_THREADS, smem, st>>>(wp, table, bits, K, N, ng, ste, op);
+      return CQ_OK;
+    };
+    auto pick = [&](auto* wp, auto* op) {
+      using T = std::remove_pointer_t<decltype(op)>;
+      return rows == 4 ? launch(fake_quant_pairs_kernel<T, 4>, wp, op) : launch(fake_quant_pairs_kernel<T, 1>, wp, op);
+    };
+    const int rc = dtype == 0 ? pick((const __half*)weight, (__half*)out) : pick((const __nv_bfloat16*)weight, (__nv_bfloat16*)out);
+    if (rc != CQ_OK) return rc;
   }
   CQ_CUDA_TRY(cudaGetLastError());
   return CQ_OK;
