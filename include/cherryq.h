@@ -258,6 +258,12 @@ int cq_attn_decode(const void* q_f16, const void* k_cache_f16, const void* v_cac
                    const long long* position, void* out_f16, int sequences, int n_heads,
                    int n_kv_heads, int head_dim, int max_seq, float scale, void* workspace,
                    cq_stream_t stream);
+/* One decode step of attention: cq_rope_cache of one token per sequence (q, k, v as there, T = sequences), then
+ * cq_attn_decode, in one launch where the kernels allow.  q and k may or may not be left rotated. */
+int cq_attn_decode_step(void* q_f16, void* k_f16, const void* v_f16, const float* cos_table,
+                        const float* sin_table, const long long* position, void* k_cache_f16,
+                        void* v_cache_f16, void* out_f16, int sequences, int n_heads, int n_kv_heads,
+                        int head_dim, int max_seq, float scale, void* workspace, cq_stream_t stream);
 /* out = silu(gate) * up, n elements.  cq_silu_mul takes the fast exponential, as the row kernel's folded SwiGLU
  * does; cq_silu_mul_full expf, as the fp32 expression. */
 int cq_silu_mul(const void* gate_f16, const void* up_f16, void* out_f16, long long n,

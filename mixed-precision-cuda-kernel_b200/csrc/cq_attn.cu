@@ -14,6 +14,11 @@
 // A warp takes 16 positions a turn with all of their keys and values in flight, and keeps its own running maximum, sum
 // and weighted values; the warps meet once in shared memory, the ranges of positions (blockIdx.z) in the workspace, where
 // the CTA that arrives last merges them.
+//
+// ROPE: the step's rotary embedding and cache write ride along (one launch less a layer): queries are rotated on their way
+// into shared memory, the new position's key and value go into the caches by the CTA whose range ends with it.
+#include <type_traits>
+
 #include "cq_attn.cuh"
 
 namespace {
@@ -34,6 +39,13 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// 16 bytes of a cache; not as read-only data where the launch itself writes a row of it
+template <bool WRITTEN> __device__ __forceinline__ uint4 ld_cache(const __half* p) {
+  if (!WRITTEN) return __ldg(reinterpret_cast<const uint4*>(p));
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p) : "memory");
+  return v;
+}
 // the upper 11 bits of two weights, and what is left of them
 __device__ __forceinline__ uint2 split_weights(float a, float b) {
   const __half2 hi = __floats2half2_rn(a, b);
@@ -42,9 +54,28 @@ __device__ __forceinline__ uint2 split_weights(float a, float b) {
   return make_uint2(*reinterpret_cast<const uint32_t*>(&hi), *reinterpret_cast<const uint32_t*>(&lo));
 }
 
-template <int D, int WARPS>
+struct RopeStep {
+  const __half* k;            // [sequence][KV][D], not rotated
+  const __half* v;
+  const float* cos_t;         // [max_seq][D / 2]
+  const float* sin_t;
+};
+
+// eight columns of the lower half of a head (x1) and the same of the upper half (x2), rotated as rope_cache_kernel does
+__device__ __forceinline__ void rotate8(uint4& x1, uint4& x2, const float* __restrict__ cos_p, const float* __restrict__ sin_p) {
+  __half* h1 = reinterpret_cast<__half*>(&x1);
+  __half* h2 = reinterpret_cast<__half*>(&x2);
+#pragma unroll
+  for (int e = 0; e < 8; ++e) {
+    const float a = __half2float(h1[e]), b = __half2float(h2[e]), c = cos_p[e], s = sin_p[e];
+    h1[e] = __float2half(a * c - b * s);
+    h2[e] = __float2half(b * c + a * s);
+  }
+}
+
+template <int D, int WARPS, bool ROPE>
 __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_mma_kernel(
-    const __half* __restrict__ q, const __half* __restrict__ k_cache, const __half* __restrict__ v_cache,
+    const __half* __restrict__ q, __half* k_cache, __half* v_cache, const RopeStep rope,
     const long long* __restrict__ pos, __half* __restrict__ out, float* __restrict__ part,
     unsigned int* __restrict__ counters, int H, int KV, int max_seq, float scale) {
   constexpr int THREADS = WARPS * 32;
@@ -69,9 +100,38 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
   const size_t head0 = (size_t)seq * H + (size_t)kvh * G;
 
   // queries in shared memory (in registers they would spill): a lane's pieces 8 t4 + 32 i of head g8
-  for (int i = tid; i < AM_HEADS * D / 8; i += THREADS) {
-    const int g = i / (D / 8), c = 8 * (i - g * (D / 8));
-    *reinterpret_cast<uint4*>(&s_q[g][c]) = g < G ? *reinterpret_cast<const uint4*>(q + (head0 + g) * D + c) : make_uint4(0, 0, 0, 0);
+  const bool step = ROPE && pl >= 0 && pl < max_seq;       // (a position outside the tables and caches: as it is, nothing is written)
+  if (ROPE) {
+    const float* cos_p = rope.cos_t + (step ? pl : 0) * (D / 2);
+    const float* sin_p = rope.sin_t + (step ? pl : 0) * (D / 2);
+    constexpr int PIECES = D / 16;
+    for (int i = tid; i < AM_HEADS * PIECES; i += THREADS) {
+      const int g = i / PIECES, c = 8 * (i - g * PIECES);
+      uint4 x1 = make_uint4(0, 0, 0, 0), x2 = x1;
+      if (g < G) {
+        x1 = *reinterpret_cast<const uint4*>(q + (head0 + g) * D + c);
+        x2 = *reinterpret_cast<const uint4*>(q + (head0 + g) * D + c + D / 2);
+        if (step) rotate8(x1, x2, cos_p + c, sin_p + c);
+      }
+      *reinterpret_cast<uint4*>(&s_q[g][c]) = x1;
+      *reinterpret_cast<uint4*>(&s_q[g][c + D / 2]) = x2;
+    }
+    if (step && n_pos > 0 && pbeg + n_pos == n_all && tid < 2 * PIECES) {
+      const size_t from = ((size_t)seq * KV + kvh) * D, to = first + (size_t)(n_pos - 1) * row;
+      const int c = 8 * (tid % PIECES);
+      const bool value = tid >= PIECES;
+      const __half* src = (value ? rope.v : rope.k) + from + c;
+      __half* dst = (value ? v_cache : k_cache) + to + c;
+      uint4 x1 = *reinterpret_cast<const uint4*>(src), x2 = *reinterpret_cast<const uint4*>(src + D / 2);
+      if (!value) rotate8(x1, x2, cos_p + c, sin_p + c);
+      *reinterpret_cast<uint4*>(dst) = x1;
+      *reinterpret_cast<uint4*>(dst + D / 2) = x2;
+    }
+  } else {
+    for (int i = tid; i < AM_HEADS * D / 8; i += THREADS) {
+      const int g = i / (D / 8), c = 8 * (i - g * (D / 8));
+      *reinterpret_cast<uint4*>(&s_q[g][c]) = g < G ? *reinterpret_cast<const uint4*>(q + (head0 + g) * D + c) : make_uint4(0, 0, 0, 0);
+    }
   }
   __syncthreads();
   const __half* mine_q = &s_q[g8][8 * t4];
@@ -92,14 +152,14 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
       const int p = base + 8 * h + g8;
 #pragma unroll
       for (int i = 0; i < KP; ++i)
-        kk[h][i] = p < n_pos ? __ldg(reinterpret_cast<const uint4*>(k_cache + first + (size_t)p * row + 8 * t4 + 32 * i)) : make_uint4(0, 0, 0, 0);
+        kk[h][i] = p < n_pos ? ld_cache<ROPE>(k_cache + first + (size_t)p * row + 8 * t4 + 32 * i) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
       const int p = base + 8 * (u >> 1) + 2 * t4 + (u & 1);
 #pragma unroll
       for (int i = 0; i < VS; ++i)
-        vv[u][i] = p < n_pos ? __ldg(reinterpret_cast<const uint4*>(v_cache + first + (size_t)p * row + 8 * g8 + 64 * i)) : make_uint4(0, 0, 0, 0);
+        vv[u][i] = p < n_pos ? ld_cache<ROPE>(v_cache + first + (size_t)p * row + 8 * g8 + 64 * i) : make_uint4(0, 0, 0, 0);
     }
     float s[2][4];
 #pragma unroll
@@ -195,11 +255,10 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
       // An infinite or NaN value takes part.  The two halves of a weight turn infinity into NaN where the product does
       // not: this column is added again, weight by weight.
       sum = 0.f;
-      const __half* qh = q + (head0 + g) * D;
       for (int p = 0; p < n_pos; ++p) {
         const __half* kr = k_cache + first + (size_t)p * row;
         float dot = 0.f;
-        for (int c = 0; c < D; ++c) dot += __half2float(qh[c]) * __half2float(kr[c]);
+        for (int c = 0; c < D; ++c) dot += __half2float(s_q[g][c]) * __half2float(kr[c]);
         sum += ex2(dot * scale2 - (top == -INFINITY ? 0.f : top) + 15.f) * __half2float(v_cache[first + (size_t)p * row + d]);
       }
     }
@@ -274,7 +333,8 @@ bool cq_attn_mma_takes(int sequences, int n_heads, int n_kv_heads, int head_dim,
 
 int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, const long long* position, void* out, int sequences,
                        int n_heads, int n_kv_heads, int head_dim, int max_seq, float scale, int most, unsigned int* counters,
-                       float* part, cudaStream_t stream) {
+                       float* part, cudaStream_t stream, const void* k_new, const void* v_new, const float* cos_table,
+                       const float* sin_table) {
   // Twelve warps a CTA, one CTA an SM, and the ranges that cost the fewest turns in a row: a wave's turn brings 192
   // positions to every SM; a range's start and its warps' meeting count as 1.2 turns, the merge of the ranges as one and
   // more with the heads it is for.  (64 query heads on 8 KV heads at 4000 positions: 1 sequence 14 us, 4 24, 16 53, 32 101;
@@ -300,8 +360,12 @@ int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, 
       }
     }
   }
-  auto fn = head_dim == 64 ? (warps == 4 ? attn_decode_mma_kernel<64, 4> : attn_decode_mma_kernel<64, 12>)
-                           : (warps == 4 ? attn_decode_mma_kernel<128, 4> : attn_decode_mma_kernel<128, 12>);
+  auto pick = [&](auto rope) {
+    constexpr bool R = decltype(rope)::value;
+    return head_dim == 64 ? (warps == 4 ? attn_decode_mma_kernel<64, 4, R> : attn_decode_mma_kernel<64, 12, R>)
+                          : (warps == 4 ? attn_decode_mma_kernel<128, 4, R> : attn_decode_mma_kernel<128, 12, R>);
+  };
+  auto fn = k_new ? pick(std::true_type()) : pick(std::false_type());
   const int smem = warps * AM_HEADS * head_dim * (int)sizeof(float);
   CQ_CUDA_TRY(cq_grant_smem((const void*)fn, smem));
   cudaLaunchConfig_t cfg = {};
@@ -314,7 +378,8 @@ int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, 
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  CQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, (const __half*)q, (const __half*)k_cache, (const __half*)v_cache, position, (__half*)out,
-                                 part, counters, n_heads, n_kv_heads, max_seq, scale));
+  CQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, fn, (const __half*)q, (__half*)k_cache, (__half*)v_cache,
+                                 RopeStep{(const __half*)k_new, (const __half*)v_new, cos_table, sin_table}, position, (__half*)out, part,
+                                 counters, n_heads, n_kv_heads, max_seq, scale));
   return CQ_OK;
 }

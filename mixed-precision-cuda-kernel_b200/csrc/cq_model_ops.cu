@@ -823,3 +823,26 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
                          (__half*)out, part, counters, n_heads, n_kv_heads, head_dim, max_seq, scale));
   return CQ_OK;
 }
+
+extern "C" int cq_attn_decode_step(void* q, void* k, const void* v, const float* cos_table, const float* sin_table,
+                                   const long long* position, void* k_cache, void* v_cache, void* out, int sequences,
+                                   int n_heads, int n_kv_heads, int head_dim, int max_seq, float scale, void* workspace,
+                                   cq_stream_t stream) {
+  if (!q || !k || !v || !cos_table || !sin_table || !position || !k_cache || !v_cache || !out || !workspace) return CQ_ERR_BAD_ARG;
+  if (sequences < 1 || sequences > 65535 || ((uintptr_t)workspace & 15)) return CQ_ERR_BAD_ARG;
+  if (n_heads < 1 || n_kv_heads < 1 || n_heads % n_kv_heads || head_dim < 2 || head_dim > 256 || (head_dim & 1) ||
+      256 % head_dim || max_seq < 1 || max_seq > 65536)
+    return CQ_ERR_BAD_SHAPE;
+  const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)cos_table | (uintptr_t)sin_table |
+                        (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out;
+  if ((all & 15) == 0 && cq_attn_mma_takes(sequences, n_heads, n_kv_heads, head_dim, max_seq)) {
+    const size_t heads = (size_t)sequences * n_heads;
+    float* part = (float*)((uint8_t*)workspace + (heads * sizeof(unsigned int) + 255) / 256 * 256);
+    return cq_attn_mma_launch(q, k_cache, v_cache, position, out, sequences, n_heads, n_kv_heads, head_dim, max_seq, scale,
+                              ATT_MAX_SPLITS, (unsigned int*)workspace, part, (cudaStream_t)stream, k, v, cos_table, sin_table);
+  }
+  const int rc = cq_rope_cache(q, k, v, cos_table, sin_table, position, k_cache, v_cache, sequences, n_heads, n_kv_heads, head_dim,
+                               max_seq, 1, stream);
+  if (rc != CQ_OK) return rc;
+  return cq_attn_decode(q, k_cache, v_cache, position, out, sequences, n_heads, n_kv_heads, head_dim, max_seq, scale, workspace, stream);
+}

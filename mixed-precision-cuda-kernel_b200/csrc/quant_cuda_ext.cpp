@@ -760,6 +760,37 @@ torch::Tensor attn_decode(torch::Tensor q, torch::Tensor k_cache, torch::Tensor 
   return out;
 }
 
+// A decode step: rope_cache of one token per sequence, then attn_decode (q and k may or may not be left rotated).
+torch::Tensor attn_decode_step(torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor cos_table, torch::Tensor sin_table,
+                               torch::Tensor position, torch::Tensor k_cache, torch::Tensor v_cache) {
+  const at::cuda::OptionalCUDAGuard device_guard(device_of(q));
+  check_tensor(q, "q", torch::kFloat16, q);
+  check_tensor(k, "k", torch::kFloat16, q);
+  check_tensor(v, "v", torch::kFloat16, q);
+  check_tensor(cos_table, "cos", torch::kFloat32, q);
+  check_tensor(sin_table, "sin", torch::kFloat32, q);
+  check_tensor(position, "position", torch::kInt64, q);
+  check_tensor(k_cache, "k_cache", torch::kFloat16, q);
+  check_tensor(v_cache, "v_cache", torch::kFloat16, q);
+  TORCH_CHECK(q.dim() == 3 && k.dim() == 3 && v.sizes() == k.sizes() && q.size(0) == k.size(0) && q.size(2) == k.size(2),
+              "q must be (B, H, D), k and v (B, KV, D)");
+  const int B = (int)q.size(0), H = (int)q.size(1), KV = (int)k.size(1), D = (int)q.size(2);
+  TORCH_CHECK(position.numel() == B, "one position per sequence");
+  TORCH_CHECK(k_cache.dim() == 4 && k_cache.size(0) == B && k_cache.size(2) == KV && k_cache.size(3) == D && v_cache.sizes() == k_cache.sizes(),
+              "caches must be (B, max_seq, KV, D)");
+  const int S = (int)k_cache.size(1);
+  TORCH_CHECK(cos_table.dim() == 2 && cos_table.size(1) == D / 2 && cos_table.size(0) >= S && sin_table.sizes() == cos_table.sizes(),
+              "cos / sin tables must be (at least max_seq, D / 2)");
+  auto out = torch::empty_like(q);
+  torch::Tensor keep;
+  void* ws = attn_workspace(q.device(), (size_t)B * H, cq_attn_decode_workspace_bytes(B, H, D, S), &keep);
+  check_status(cq_attn_decode_step(q.data_ptr(), k.data_ptr(), v.data_ptr(), cos_table.data_ptr<float>(), sin_table.data_ptr<float>(),
+                                   (const long long*)position.data_ptr(), k_cache.data_ptr(), v_cache.data_ptr(), out.data_ptr(), B, H,
+                                   KV, D, S, 1.0f / std::sqrt((float)D), ws, current_stream()),
+               "attn_decode_step");
+  return out;
+}
+
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("vecquant3matmul_cherryq", &vecquant3matmul_cherryq, "a 3-bit version");
   m.def("vecquant4matmul_cherryq", &vecquant4matmul_cherryq, "a 4-bit version");
@@ -782,6 +813,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("rmsnorm", &rmsnorm, "RMSNorm with optional residual add");
   m.def("rope_cache", &rope_cache, "rotary embedding in place + KV cache write");
   m.def("silu_mul", &silu_mul, "silu(gate) * up", py::arg("gate"), py::arg("up"), py::arg("full") = false);
+  m.def("attn_decode_step", &attn_decode_step, "rotary embedding, KV cache write and attention of a decode step");
   m.def("attn_decode", &attn_decode, "single-query attention over the KV cache");
   m.def("poll", []() { check_status(cq_poll(current_stream()), "poll"); });
   m.def("device_timed_out", &device_timed_out);

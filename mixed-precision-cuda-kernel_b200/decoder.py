@@ -228,18 +228,18 @@ class CherryDecoder:
         xn, h = self._norm(h, delta, lay["norm1"])
         q, k, v = self._lins(lay, ("q", "k", "v"), xn)
         q, k, v = q.view(t, nh, hd), k.view(t, kv, hd), v.view(t, kv, hd)
-        self.qc.rope_cache(q, k, v, self.cos, self.sin, pos, self.k_cache[li], self.v_cache[li])
-        if decode:
-            if self._flash is not None:
+        if decode and self._flash is None:
+            a = self.qc.attn_decode_step(q, k, v, self.cos, self.sin, pos, self.k_cache[li], self.v_cache[li]).view(t, nh * hd)
+        else:
+            self.qc.rope_cache(q, k, v, self.cos, self.sin, pos, self.k_cache[li], self.v_cache[li])
+            if decode:
                 a = self._flash(q.view(t, 1, nh, hd), self.k_cache[li], self.v_cache[li],
                                 cache_seqlens=(pos + 1).to(torch.int32), causal=True).view(t, nh * hd)
             else:
-                a = self.qc.attn_decode(q, self.k_cache[li], self.v_cache[li], pos).view(t, nh * hd)
-        else:
-            ts = t // nb              # tokens per sequence; rows are (sequence, token)
-            a = F.scaled_dot_product_attention(q.view(nb, ts, nh, hd).transpose(1, 2), k.view(nb, ts, kv, hd).transpose(1, 2),
-                                               v.view(nb, ts, kv, hd).transpose(1, 2), is_causal=True, enable_gqa=(kv != nh))
-            a = a.transpose(1, 2).reshape(t, nh * hd)
+                ts = t // nb              # tokens per sequence; rows are (sequence, token)
+                a = F.scaled_dot_product_attention(q.view(nb, ts, nh, hd).transpose(1, 2), k.view(nb, ts, kv, hd).transpose(1, 2),
+                                                   v.view(nb, ts, kv, hd).transpose(1, 2), is_causal=True, enable_gqa=(kv != nh))
+                a = a.transpose(1, 2).reshape(t, nh * hd)
         xn, h = self._norm(h, self._lin_gather(lay["o"], self._gather(a)), lay["norm2"])
         gate, up = self._lins(lay, ("gate", "up"), xn)
         if self.tp == 1 and not self.dense and t <= 16:

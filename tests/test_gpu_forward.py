@@ -248,6 +248,32 @@ def test_attention_on_tensor_cores(D, B, H, KV, max_seq):
     assert bool(out[:, :G, 3:].isfinite().all() and out[:, :G, 0].isfinite().all() and out[:, G:].isfinite().all())
 
 
+@pytest.mark.parametrize("B,H,KV,D,max_seq", [(3, 4, 4, 128, 40), (2, 8, 1, 64, 700), (17, 64, 8, 128, 400), (2, 8, 2, 256, 40), (3, 6, 6, 32, 300)])
+def test_attention_step_is_rotation_cache_write_and_attention(B, H, KV, D, max_seq):
+    """One launch and the two kernels, at the first and last positions of ranges and caches and at positions outside, which
+    read and write nothing of the new token."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    g = torch.Generator(device="cuda").manual_seed(B + D)
+    at = [0, max_seq - 1, 15, 16, -1, max_seq, 63, 64]
+    pos = torch.tensor([at[b % 8] for b in range(B)], device="cuda")
+    q = torch.randn(B, H, D, device="cuda", generator=g).half()
+    k, v = (torch.randn(B, KV, D, device="cuda", generator=g).half() for _ in range(2))
+    caches = [torch.randn(B, max_seq, KV, D, device="cuda", generator=g).half() for _ in range(2)]
+    ang = torch.outer(torch.arange(max_seq, device="cuda", dtype=torch.float32), torch.rand(D // 2, device="cuda", generator=g))
+    cos, sin = ang.cos(), ang.sin()
+    q1, k1, mine = q.clone(), k.clone(), [c.clone() for c in caches]
+    out = qc.attn_decode_step(q1, k1, v, cos, sin, pos, *mine)
+    qc.rope_cache(q, k, v, cos, sin, pos, *caches)
+    want = qc.attn_decode(q, caches[0], caches[1], pos)
+    assert torch.equal(mine[1], caches[1])
+    # (a rotation may contract its products otherwise: one step of fp16)
+    assert float((mine[0].float() - caches[0].float()).abs().max()) <= 4e-3
+    changed = (mine[0] != caches[0]).any(-1).any(-1)
+    assert int(changed.sum()) <= B and not bool(changed[pos < 0].any()) and not bool(changed[pos >= max_seq].any())
+    assert float((out.float() - want.float()).abs().max()) <= 4e-3           # as in test_attention_sweep_edges
+
+
 @pytest.mark.parametrize("m,C", [(1, 16), (40, 16), (3, 256)])     # row kernel, GEMM, stream matvec
 def test_copies_dropped_while_another_stream_uses_them(m, C):
     """The block of a dropped copy is not given out before the launches that read it have finished, and is afterwards."""
