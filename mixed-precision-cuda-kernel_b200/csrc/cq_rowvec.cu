@@ -60,6 +60,12 @@ struct RowvecParams {
   const __half* x;
   const __half* x2;         // not null: the activations are silu(x) * x2, element by element (the SwiGLU of a gated MLP
                             // computed while the down projection stages its input); same shape and stride as x
+  // NORM: the activations are the RMS norm of x (+ delta), which every CTA takes for itself; the first one also stores the
+  // sum x + delta
+  const __half* norm_w;
+  const __half* delta;      // may be null
+  __half* sum_out;          // may be null
+  float eps;
   int M, ldx, ldy;          // activation rows of the call (1..4) and the row strides of x and y, in elements
   uint32_t* status;         // may be null
   int K, C, NG, ncb;        // common to the layers of a launch; ncb = cherry blocks of 16 columns
@@ -144,6 +150,25 @@ __device__ __forceinline__ uint4 rv_swiglu8(uint4 g, uint4 u) {
   for (int i = 0; i < 8; ++i) rh[i] = rv_swiglu(gh[i], uh[i]);
   return r;
 }
+// x + delta as an fp16 tensor
+__device__ __forceinline__ uint4 rv_add8(uint4 x, uint4 d) {
+  __half2* a = reinterpret_cast<__half2*>(&x);
+  const __half2* b = reinterpret_cast<const __half2*>(&d);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) a[i] = __hadd2(a[i], b[i]);
+  return x;
+}
+// fp16(x * inv) * w, the roundings of rmsnorm_kernel
+__device__ __forceinline__ uint4 rv_norm8(uint4 x, float inv, uint4 w) {
+  __half2* a = reinterpret_cast<__half2*>(&x);
+  const __half2* b = reinterpret_cast<const __half2*>(&w);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const float2 f = __half22float2(a[i]);
+    a[i] = __hmul2(__floats2half2_rn(f.x * inv, f.y * inv), b[i]);
+  }
+  return x;
+}
 // D (16 x 8, s32) += A (16 x 32, u8) . B (32 x 8, s8)
 __device__ __forceinline__ void rv_imma(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile(
@@ -199,10 +224,12 @@ __device__ __forceinline__ void issue_tile(const RowvecParams& p, const uint8_t*
 // the copy queue is full, i.e. for most of the streaming time: that thread must not have other
 // work); GPW groups of 128 columns a warp can own (its activations stay in 8 * GPW registers).
 // MR = 1: one activation row (the row loop below collapses); MR = 4: p.M rows, 1..4.
-template <int BITS, int SETS, int W, int GPW, int MR>
+// NORM: an RMS norm in front (decode harness: it saves the norm kernel's launch, whose latency is about that of the sums here).
+template <int BITS, int SETS, int W, int GPW, int MR, bool NORM>
 __global__ void __launch_bounds__((W + 1) * 32, 1) cq_rowvec_kernel(const RowvecParams p) {
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_abort, s_last;
+  __shared__ float s_ss[NORM ? RV_MAX_ROWS : 1][W];          // a warp's share of a row's sum of squares
   constexpr int NTHR = (W + 1) * 32;
   constexpr int GRP_BYTES = 256 * BITS;      // 16 rows x 128 codes
   constexpr int PVW = (GPW + 1) / 2;         // octets of activations a lane stages (16 per group, 32 lanes)
@@ -301,20 +328,64 @@ __global__ void __launch_bounds__((W + 1) * 32, 1) cq_rowvec_kernel(const Rowvec
   const bool owns_tail = ngw > 0 && g0 + ngw == p.NG;       // the warp whose last group may hold padding columns
   int ccol = -1;
   if (has_cherry && lane < 16 && warp * 16 + lane < p.C) ccol = sg.cidx[warp * 16 + lane];
-  const bool gated = p.x2 != nullptr;
+  const bool gated = !NORM && p.x2 != nullptr;
   const bool x_aligned = ((reinterpret_cast<uintptr_t>(p.x) | reinterpret_cast<uintptr_t>(p.x2) | (uintptr_t)(p.ldx * 2)) & 15) == 0;
-  // 16 bytes / one element of the activations at element offset `at` of the matrix
-  auto ld8 = [&](size_t at) {
-    const uint4 v = __ldcg(reinterpret_cast<const uint4*>(p.x + at));
-    return gated ? rv_swiglu8(v, __ldcg(reinterpret_cast<const uint4*>(p.x2 + at))) : v;
-  };
-  auto ld1 = [&](size_t at) {
-    const __half v = __ldcg(p.x + at);
-    return gated ? rv_swiglu(v, __ldcg(p.x2 + at)) : v;
-  };
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
+
+  const int Mrows = MR == 1 ? 1 : p.M;
+  constexpr bool normed = NORM;                              // (buffers 16-byte aligned, one launch: the host's rule)
+  if (normed) {
+    // sums of squares of whole rows: every CTA reads them (they are in L2), one barrier among the working warps
+#pragma unroll 1
+    for (int m = 0; m < Mrows; ++m) {
+      float ss = 0.f;
+      for (int i = tid; i < p.K / 8; i += W * 32) {
+        const size_t at = (size_t)m * p.ldx + 8 * i;
+        uint4 v = __ldcg(reinterpret_cast<const uint4*>(p.x + at));
+        if (p.delta) v = rv_add8(v, __ldcg(reinterpret_cast<const uint4*>(p.delta + at)));
+        if (p.sum_out && blockIdx.x == 0) *reinterpret_cast<uint4*>(p.sum_out + at) = v;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 f = __half22float2(reinterpret_cast<const __half2*>(&v)[e]);
+          ss += f.x * f.x + f.y * f.y;
+        }
+      }
+      for (int d = 16; d > 0; d >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, d);
+      if (lane == 0) s_ss[m][warp] = ss;
+    }
+    asm volatile("bar.sync 1, %0;" ::"n"(W * 32) : "memory");
+  }
+  float inv = 0.f;
+  auto take_inv = [&](int m) {
+    if (!normed) return;
+    float tot = 0.f;
+#pragma unroll
+    for (int w = 0; w < W; ++w) tot += s_ss[m][w];
+    inv = rsqrtf(tot / (float)p.K + p.eps);
+  };
+  // 16 bytes / one element of the activations at column `col` of row m
+  auto ld8 = [&](int m, int col) {
+    const size_t at = (size_t)m * p.ldx + col;
+    uint4 v = __ldcg(reinterpret_cast<const uint4*>(p.x + at));
+    if (gated) return rv_swiglu8(v, __ldcg(reinterpret_cast<const uint4*>(p.x2 + at)));
+    if (normed) {
+      if (p.delta) v = rv_add8(v, __ldcg(reinterpret_cast<const uint4*>(p.delta + at)));
+      v = rv_norm8(v, inv, __ldg(reinterpret_cast<const uint4*>(p.norm_w + col)));
+    }
+    return v;
+  };
+  auto ld1 = [&](int m, int col) {
+    const size_t at = (size_t)m * p.ldx + col;
+    __half v = __ldcg(p.x + at);
+    if (gated) return rv_swiglu(v, __ldcg(p.x2 + at));
+    if (normed) {
+      if (p.delta) v = __hadd(v, __ldcg(p.delta + at));
+      v = __hmul(__float2half(__half2float(v) * inv), __ldg(p.norm_w + col));
+    }
+    return v;
+  };
 
   // What a lane keeps of the activations.  The integer MMA's B operand has 8 columns: column 2 m holds
   // the high plane of activation row m, column 2 m + 1 its low plane, so up to four rows ride in the MMAs
@@ -332,20 +403,20 @@ __global__ void __launch_bounds__((W + 1) * 32, 1) cq_rowvec_kernel(const Rowvec
     for (int e = 0; e < 8; ++e) xb[gi][e] = 0u;
   }
 
-  const int Mrows = MR == 1 ? 1 : p.M;
   // ---- the warp's slice of row m -> its shared-memory slice (coalesced 16-byte loads), cherry activations.
   // The loads of row m + 1 are in flight while row m is gathered and quantised.
   uint4 xv[XCH];
   uint32_t xcv_next = 0;
+  take_inv(0);
   if (x_aligned) {
 #pragma unroll
     for (int c = 0; c < XCH; ++c) {
       const int ch = lane + 32 * c;
       xv[c] = make_uint4(0, 0, 0, 0);
-      if (ch < nchunk) xv[c] = ld8((size_t)lo8 + 8 * ch);
+      if (ch < nchunk) xv[c] = ld8(0, lo8 + 8 * ch);
     }
   }
-  if (ccol >= 0) xcv_next = (uint32_t)__half_as_ushort(ld1((size_t)ccol));
+  if (ccol >= 0) xcv_next = (uint32_t)__half_as_ushort(ld1(0, ccol));
 #pragma unroll 1
   for (int m = 0; m < Mrows; ++m) {
   const uint32_t xcv = xcv_next;
@@ -356,19 +427,18 @@ __global__ void __launch_bounds__((W + 1) * 32, 1) cq_rowvec_kernel(const Rowvec
       if (ch < nchunk) reinterpret_cast<uint4*>(slice)[ch] = xv[c];
     }
   } else {
-    const size_t xr = (size_t)m * p.ldx + lo8;
-    for (int i = lane; i < nchunk * 8; i += 32) slice[i] = ld1(xr + i);
+    for (int i = lane; i < nchunk * 8; i += 32) slice[i] = ld1(m, lo8 + i);
   }
   if (MR > 1 && m + 1 < Mrows) {
-    const size_t xn = (size_t)(m + 1) * p.ldx;
+    take_inv(m + 1);
     if (x_aligned) {
 #pragma unroll
       for (int c = 0; c < XCH; ++c) {
         const int ch = lane + 32 * c;
-        if (ch < nchunk) xv[c] = ld8(xn + lo8 + 8 * ch);
+        if (ch < nchunk) xv[c] = ld8(m + 1, lo8 + 8 * ch);
       }
     }
-    if (ccol >= 0) xcv_next = (uint32_t)__half_as_ushort(ld1(xn + ccol));
+    if (ccol >= 0) xcv_next = (uint32_t)__half_as_ushort(ld1(m + 1, ccol));
   }
   if (owns_tail && lane == 0) slice[p.K - lo8] = __float2half(0.f);   // zero slot for padding columns
   __syncwarp();
@@ -871,14 +941,14 @@ inline int rv_gpw_for(const cq_rlayer* L) {
   return need <= 2 ? 2 : (need <= 4 ? 4 : 0);
 }
 
-template <int W, int GPW>
+template <int W, int GPW, bool NORM = false>
 RowvecFn rv_pick(int bits, int sets, int M = 1) {
   if (M == 1) {
-    if (bits == 4) return cq_rowvec_kernel<4, 1, W, GPW, 1>;
-    return sets == 1 ? cq_rowvec_kernel<3, 1, W, GPW, 1> : cq_rowvec_kernel<3, 2, W, GPW, 1>;
+    if (bits == 4) return cq_rowvec_kernel<4, 1, W, GPW, 1, NORM>;
+    return sets == 1 ? cq_rowvec_kernel<3, 1, W, GPW, 1, NORM> : cq_rowvec_kernel<3, 2, W, GPW, 1, NORM>;
   }
-  if (bits == 4) return cq_rowvec_kernel<4, 1, W, GPW, RV_MAX_ROWS>;
-  return sets == 1 ? cq_rowvec_kernel<3, 1, W, GPW, RV_MAX_ROWS> : cq_rowvec_kernel<3, 2, W, GPW, RV_MAX_ROWS>;
+  if (bits == 4) return cq_rowvec_kernel<4, 1, W, GPW, RV_MAX_ROWS, NORM>;
+  return sets == 1 ? cq_rowvec_kernel<3, 1, W, GPW, RV_MAX_ROWS, NORM> : cq_rowvec_kernel<3, 2, W, GPW, RV_MAX_ROWS, NORM>;
 }
 
 // Plan of one launch over `n` layers that share the activation row (same bits, K, cherry count and
@@ -975,11 +1045,19 @@ int rv_plan(int W, int GPW, const cq_rlayer* const* Ls, int n, int M, const RvDe
   return CQ_OK;
 }
 
+// An RMS norm in front of the layers: of x (+ delta), weight w; the sum x + delta is stored to sum_out if not null.
+struct RvNorm {
+  const __half* w = nullptr;
+  const __half* delta = nullptr;
+  __half* sum_out = nullptr;
+  float eps = 0.f;
+};
+
 // One launch of a kernel whose warp count is W and whose warps can own GPW groups, over `n` layers
 // that take the same activation row x; ys[i] receives layer i's output.
 int rv_launch(RowvecFn fn, int W, int GPW, const cq_rlayer* const* Ls, int n, const __half* x, int ldx,
               __half* const* ys, int ldy, int M, int accumulate, uint32_t* status, cudaStream_t st,
-              const cq_peer::PeerGatherParams* peer = nullptr, const __half* x2 = nullptr) {
+              const cq_peer::PeerGatherParams* peer = nullptr, const __half* x2 = nullptr, const RvNorm& norm = RvNorm()) {
   int dev = 0;
   CQ_CUDA_TRY(cudaGetDevice(&dev));
   const RvDevice di = rv_device(dev);
@@ -1000,6 +1078,7 @@ int rv_launch(RowvecFn fn, int W, int GPW, const cq_rlayer* const* Ls, int n, co
     if (i >= n) { p.seg[i].N = 0; p.seg[i].cta0 = grid; p.seg[i].tiles_q = 0; p.seg[i].tiles_r = 0; }
   }
   p.x = x; p.x2 = x2; p.status = status;
+  p.norm_w = norm.w; p.delta = norm.delta; p.sum_out = norm.sum_out; p.eps = norm.eps;
   p.M = M; p.ldx = ldx; p.ldy = ldy;
   p.accumulate = accumulate;
   p.gather = peer ? 1 : 0;
@@ -1119,6 +1198,33 @@ extern "C" int cq_rlayers_matvec(const cq_rlayer* const* layers, int n_layers, c
     if (rc != CQ_OK) return rc;
   }
   return CQ_OK;
+}
+
+extern "C" int cq_rlayers_matvec_norm(const cq_rlayer* const* layers, int n_layers, const void* x, const void* delta,
+                                      const void* norm_weight, float eps, void* sum_out, int ldx, void* const* ys, int ldy, int M,
+                                      uint32_t* status_word, cq_stream_t stream) {
+  if (!layers || !ys || !x || !norm_weight || n_layers < 1 || n_layers > RV_MAX_SEG || M < 1) return CQ_ERR_BAD_ARG;
+  if (M > RV_MAX_ROWS) return CQ_ERR_UNSUPPORTED;
+  __half* yp[RV_MAX_SEG];
+  int nmax = 0;
+  for (int i = 0; i < n_layers; ++i) {
+    if (!layers[i] || !layers[i]->blob || !ys[i] || ((uintptr_t)ys[i] & 1)) return CQ_ERR_BAD_ARG;
+    if (layers[i]->N > nmax) nmax = layers[i]->N;
+    yp[i] = (__half*)ys[i];
+  }
+  const cq_rlayer* L = layers[0];
+  if (ldx < L->K || ldy < nmax || ldx % 8) return CQ_ERR_BAD_ARG;
+  if (((uintptr_t)x | (uintptr_t)delta | (uintptr_t)norm_weight | (uintptr_t)sum_out) & 15) return CQ_ERR_BAD_ARG;
+  RvNorm norm;
+  norm.w = (const __half*)norm_weight;
+  norm.delta = (const __half*)delta;
+  norm.sum_out = (__half*)sum_out;
+  norm.eps = eps;
+  switch (rv_gpw_for(L)) {
+    case 2: return rv_launch(rv_pick<RV_W, 2, true>(L->bits, L->sets, M), RV_W, 2, layers, n_layers, (const __half*)x, ldx, yp, ldy, M, 0, status_word, (cudaStream_t)stream, nullptr, nullptr, norm);
+    case 4: return rv_launch(rv_pick<RV_W, 4, true>(L->bits, L->sets, M), RV_W, 4, layers, n_layers, (const __half*)x, ldx, yp, ldy, M, 0, status_word, (cudaStream_t)stream, nullptr, nullptr, norm);
+    default: return CQ_ERR_UNSUPPORTED;
+  }
 }
 
 extern "C" int cq_rlayer_matvec_gather(const cq_rlayer* L, const void* x, int ldx, void* y_local, int M, void* const* regions,

@@ -621,7 +621,10 @@ struct PackedForward {
 // One launch (per four activation rows) for several row-tile layers that take the same activations
 // (q / k / v, gate / up): outs[i] = [outs[i] +] x (M, K) fp16 . W_i^T.  The outputs are rows of `ldy`
 // elements each: views into one (M, ldy) buffer, or separate (M, N_i) tensors when every N_i == ldy.
-void row_layers_matvec(std::vector<RowLayer*> layers, torch::Tensor x, std::vector<torch::Tensor> outs, bool accumulate) {
+// norm_weight: the layers' input is the RMS norm of x (+ delta); the sum goes to `sum` (the last three may be undefined).
+void row_layers_launch(const std::vector<RowLayer*>& layers, const torch::Tensor& x, const std::vector<torch::Tensor>& outs,
+                       bool accumulate, const torch::Tensor& norm_weight, const torch::Tensor& delta, const torch::Tensor& sum,
+                       double eps) {
   TORCH_CHECK(!layers.empty() && layers.size() <= 4 && layers.size() == outs.size(), "1 to 4 layers, one output each");
   const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
   check_tensor(x, "x", torch::kFloat16, layers[0]->blob.t);
@@ -647,10 +650,38 @@ void row_layers_matvec(std::vector<RowLayer*> layers, torch::Tensor x, std::vect
   }
   for (const auto* l : layers) l->blob.use();
   auto scratch = scratch_for(x.device());
-  uint8_t* sp = scratch.data_ptr<uint8_t>();
-  check_status(cq_rlayers_matvec(ls, (int)layers.size(), x.data_ptr(), K, ys, (int)ldy, M, accumulate ? 1 : 0,
-                                 (uint32_t*)(sp + cq_scratch_bytes()), current_stream()),
+  uint32_t* status = (uint32_t*)(scratch.data_ptr<uint8_t>() + cq_scratch_bytes());
+  if (norm_weight.defined()) {
+    check_tensor(norm_weight, "norm_weight", torch::kFloat16, x);
+    TORCH_CHECK(norm_weight.numel() == K, "norm_weight must hold ", K, " values");
+    for (const auto* t : {&delta, &sum}) {
+      if (!t->defined()) continue;
+      check_tensor(*t, "delta / sum", torch::kFloat16, x);
+      TORCH_CHECK(t->numel() == x.numel(), "delta and sum must have the shape of x");
+    }
+    check_status(cq_rlayers_matvec_norm(ls, (int)layers.size(), x.data_ptr(), delta.defined() ? delta.data_ptr() : nullptr,
+                                        norm_weight.data_ptr(), (float)eps, sum.defined() ? sum.data_ptr() : nullptr, K, ys, (int)ldy, M,
+                                        status, current_stream()),
+                 "row_layers_matvec_norm");
+    return;
+  }
+  check_status(cq_rlayers_matvec(ls, (int)layers.size(), x.data_ptr(), K, ys, (int)ldy, M, accumulate ? 1 : 0, status, current_stream()),
                "row_layers_matvec");
+}
+void row_layers_matvec(std::vector<RowLayer*> layers, torch::Tensor x, std::vector<torch::Tensor> outs, bool accumulate) {
+  row_layers_launch(layers, x, outs, accumulate, torch::Tensor(), torch::Tensor(), torch::Tensor(), 0.0);
+}
+// The same on the RMS norm of x (+ delta), up to four rows; returns the sum x + delta (x itself without a delta).
+torch::Tensor row_layers_matvec_norm(std::vector<RowLayer*> layers, torch::Tensor x, c10::optional<torch::Tensor> delta,
+                                     torch::Tensor norm_weight, double eps, std::vector<torch::Tensor> outs) {
+  torch::Tensor d, sum;
+  if (delta.has_value()) {
+    const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
+    d = *delta;
+    sum = torch::empty_like(x);
+  }
+  row_layers_launch(layers, x, outs, false, norm_weight, d, sum, eps);
+  return sum.defined() ? sum : x;
 }
 
 // Reads and clears the status word the PreparedLayer launches report into.
@@ -818,6 +849,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("poll", []() { check_status(cq_poll(current_stream()), "poll"); });
   m.def("device_timed_out", &device_timed_out);
   m.def("row_layers_matvec", &row_layers_matvec, "one launch for row-tile layers sharing an activation row");
+  m.def("row_layers_matvec_norm", &row_layers_matvec_norm, "row_layers_matvec on the RMS norm of its input");
   m.def("abi_version", &cq_abi_version);
   py::class_<RowLayer>(m, "RowLayer")
       .def(py::init<torch::Tensor, torch::Tensor, torch::Tensor, torch::Tensor, int, int, int>())

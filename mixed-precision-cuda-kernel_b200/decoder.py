@@ -37,7 +37,7 @@ import torch
 import torch.nn.functional as F
 
 from . import load_quant_cuda
-from .qlinear import QuantLinear, forward_shared_input
+from .qlinear import QuantLinear, forward_normed_input, forward_shared_input
 
 
 @dataclass
@@ -220,13 +220,19 @@ class CherryDecoder:
         y, hs = self.qc.rmsnorm(h, delta, w, self.cfg.eps, True)
         return y, hs
 
+    def _norm_lins(self, lay, names, h: torch.Tensor, delta, w: torch.Tensor):
+        """The projections `names` of rmsnorm(h + delta) * w, and h + delta: up to four rows in one launch."""
+        if self.dense:
+            xn, h = self._norm(h, delta, w)
+            return self._lins(lay, names, xn), h
+        return forward_normed_input([lay[n] for n in names], h, delta, w, self.cfg.eps)
+
     def _layer(self, li: int, h: torch.Tensor, delta, pos: torch.Tensor, decode: bool):
         """One decoder layer on the residual stream h with the previous layer's MLP output `delta`
         still to be added; returns (h, delta) in the same form."""
         cfg, lay = self.cfg, self.layers[li]
         t, nh, kv, hd, nb = h.shape[0], self.h_local, self.kv_local, cfg.head_dim, self.batch
-        xn, h = self._norm(h, delta, lay["norm1"])
-        q, k, v = self._lins(lay, ("q", "k", "v"), xn)
+        (q, k, v), h = self._norm_lins(lay, ("q", "k", "v"), h, delta, lay["norm1"])
         q, k, v = q.view(t, nh, hd), k.view(t, kv, hd), v.view(t, kv, hd)
         if decode and self._flash is None:
             a = self.qc.attn_decode_step(q, k, v, self.cos, self.sin, pos, self.k_cache[li], self.v_cache[li]).view(t, nh * hd)
@@ -240,8 +246,7 @@ class CherryDecoder:
                 a = F.scaled_dot_product_attention(q.view(nb, ts, nh, hd).transpose(1, 2), k.view(nb, ts, kv, hd).transpose(1, 2),
                                                    v.view(nb, ts, kv, hd).transpose(1, 2), is_causal=True, enable_gqa=(kv != nh))
                 a = a.transpose(1, 2).reshape(t, nh * hd)
-        xn, h = self._norm(h, self._lin_gather(lay["o"], self._gather(a)), lay["norm2"])
-        gate, up = self._lins(lay, ("gate", "up"), xn)
+        (gate, up), h = self._norm_lins(lay, ("gate", "up"), h, self._lin_gather(lay["o"], self._gather(a)), lay["norm2"])
         if self.tp == 1 and not self.dense and t <= 16:
             # one GPU, decode batch: the SwiGLU rides in the down projection's input staging
             return h, lay["down"].forward_swiglu(gate, up)

@@ -270,6 +270,32 @@ class QuantLinear(nn.Module):
         return out
 
 
+def _row_copies(layers, rows):
+    """The row-tile copies of layers that one launch of the row kernel can serve for that many rows, or None."""
+    first = layers[0]
+    same = all((l.w_bits, l.in_features, l.num_cherries, l.group_size) ==
+               (first.w_bits, first.in_features, first.num_cherries, first.group_size) for l in layers)
+    if not (1 < len(layers) <= 4 and same and QuantLinear._layerwise_dequantize and first.w_bits in (3, 4)):
+        return None
+    rls = [l.row_layer(rows) for l in layers]
+    return rls if all(r is not None for r in rls) else None
+
+
+def _row_outputs(layers, shape, dtype, rows, device, launch):
+    """Outputs of `layers` as views of one buffer, filled by launch(outs)."""
+    widths = [l.out_features for l in layers]
+    buf = torch.empty(rows, sum(widths), dtype=torch.float16, device=device)
+    outs = list(buf.split(widths, dim=1))                       # views of one buffer: one row stride
+    launch(outs)
+    res = []
+    for l, o in zip(layers, outs):
+        o = o.contiguous().reshape(shape[:-1] + (l.out_features,)).to(dtype)
+        if l.bias is not None:
+            o += l.bias
+        res.append(o)
+    return res
+
+
 def forward_shared_input(layers, x: torch.Tensor):
     """Outputs of several packed layers applied to the same input (q / k / v, gate / up of the
     reference's LLaMA, llama/modeling_llama_quant.py): for decode batches (up to the layers' row
@@ -277,27 +303,33 @@ def forward_shared_input(layers, x: torch.Tensor):
     of the row-tile kernel per four rows, with the SMs divided among the layers; every other case is
     the layers' own forward, one by one.  The results are bit-identical to the separate calls."""
     layers = list(layers)
-    first = layers[0]
     rows = x.numel() // x.shape[-1]
-    same = all((l.w_bits, l.in_features, l.num_cherries, l.group_size) ==
-               (first.w_bits, first.in_features, first.num_cherries, first.group_size) for l in layers)
-    if (1 < len(layers) <= 4 and same and QuantLinear._layerwise_dequantize and first.w_bits in (3, 4)):
-        rls = [l.row_layer(rows) for l in layers]
-        if all(r is not None for r in rls):
-            qc = load_quant_cuda()
-            x2 = x.reshape(rows, x.shape[-1])
-            if x2.dtype != torch.float16:
-                x2 = x2.half()
-            x2 = x2.contiguous()
-            widths = [l.out_features for l in layers]
-            buf = torch.empty(rows, sum(widths), dtype=torch.float16, device=x2.device)
-            outs = list(buf.split(widths, dim=1))               # views of one buffer: one row stride
-            qc.row_layers_matvec(rls, x2, outs, False)
-            res = []
-            for l, o in zip(layers, outs):
-                o = o.contiguous().reshape(x.shape[:-1] + (l.out_features,)).to(x.dtype)
-                if l.bias is not None:
-                    o += l.bias
-                res.append(o)
-            return res
-    return [l(x) for l in layers]
+    rls = _row_copies(layers, rows)
+    if rls is None:
+        return [l(x) for l in layers]
+    x2 = x.reshape(rows, x.shape[-1])
+    if x2.dtype != torch.float16:
+        x2 = x2.half()
+    x2 = x2.contiguous()
+    return _row_outputs(layers, x.shape, x.dtype, rows, x2.device,
+                        lambda outs: load_quant_cuda().row_layers_matvec(rls, x2, outs, False))
+
+
+def forward_normed_input(layers, h: torch.Tensor, delta, weight: torch.Tensor, eps: float):
+    """(outputs, h + delta): the layers applied to the RMS norm of h + delta (delta may be None), the residual stream of the
+    reference's decoder layer (llama/modeling_llama_quant.py:724-785).  Up to four fp16 rows: the norm rides in the
+    launch of forward_shared_input; everything else is the norm kernel and that function."""
+    layers = list(layers)
+    qc = load_quant_cuda()
+    rows = h.numel() // h.shape[-1]
+    plain = all(t is None or (t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in (h, delta, weight))
+    rls = _row_copies(layers, rows) if rows <= 4 and plain and h.dim() == 2 else None
+    if rls is None:
+        if delta is None:
+            return forward_shared_input(layers, qc.rmsnorm(h, None, weight, eps, False)[0]), h
+        y, h = qc.rmsnorm(h, delta, weight, eps, True)
+        return forward_shared_input(layers, y), h
+    sums = []
+    outs = _row_outputs(layers, h.shape, h.dtype, rows, h.device,
+                        lambda o: sums.append(qc.row_layers_matvec_norm(rls, h, delta, weight, eps, o)))
+    return outs, sums[0]

@@ -96,6 +96,29 @@ def test_kernel_does_not_depend_on_earlier_calls(K, C):
         assert torch.equal(old[0].forward_swiglu(x[:m], up[:m]), new[0].forward_swiglu(x[:m], up[:m]))
 
 
+@pytest.mark.parametrize("K,bits,G", [(2048, 4, 128), (1032, 3, 64), (9216, 3, 128)])      # whole rows, a ragged group, split along K
+@pytest.mark.parametrize("m,with_delta", [(1, True), (1, False), (4, True), (5, True)])
+def test_norm_in_front_of_a_shared_input(K, bits, G, m, with_delta):
+    """The norm kernel and the layers' own forward against both in one launch (up to four rows)."""
+    import cherryq_b200
+    from cherryq_b200.qlinear import forward_normed_input
+    qc = cherryq_b200.load_quant_cuda()
+    lins = [packed(K, n, bits, G, s) for s, n in ((1, 264), (2, 520))]
+    h = torch.randn(m, K, device="cuda").half() * 3
+    delta = torch.randn(m, K, device="cuda").half() if with_delta else None
+    w = (torch.randn(K, device="cuda") * 0.1 + 1).half()
+    outs, total = forward_normed_input(lins, h, delta, w, 1e-5)
+    if with_delta:
+        y, want = qc.rmsnorm(h, delta, w, 1e-5, True)
+    else:
+        y, want = qc.rmsnorm(h, None, w, 1e-5, False)[0], h
+    assert torch.equal(total, want)
+    for lin, out in zip(lins, outs):
+        ref = lin(y).float()
+        # the sum of squares is added in another order: a few of the norm's values move by one fp16 step
+        assert float((out.float() - ref).norm()) <= 3e-4 * float(ref.norm()) and out.shape == (m, lin.out_features)
+
+
 @pytest.mark.parametrize("m,C", [(9, 16), (40, 16), (3, 256)])
 def test_swiglu_beyond_the_row_kernel_is_the_torch_expression(m, C):
     """Rows above the row kernel's limit and layers it does not take: silu in fp32, not the fast exponential.  Every fp16
