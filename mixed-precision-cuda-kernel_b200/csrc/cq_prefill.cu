@@ -41,8 +41,10 @@
 //
 // Bound and state: 4096 -> 11008 4-bit, 2048 rows: 140 us = 1.32 PFLOP/s (739 us through QuantLinear and 195 us by itself
 // with lone CTAs of 128 x 256 tiles); 8192 -> 28672 3-bit, 2048 rows: 641 us = 1.50 PFLOP/s, tensor-bound.  16 rows: 18 and
-// 52 us (31 and 76): an item then takes about 740 cycles, the eight MMAs' reads of A from tensor memory and their issue,
-// against 365 that its weights need to arrive from HBM.
+// 49 us (31 and 76): an item then takes about 700 cycles, most of them the decode groups' instructions and waits, against
+// 365 that its weights need to arrive from HBM.  (54 us while every decode warp walked over all items, polled without a
+// hint and took every fourth; the hint without the stepping was slower, 61.  With six groups, or with lone CTAs that leave
+// room for seven A slots, it was no faster.)
 #include <cmath>
 
 #include "cq_tile.cuh"
@@ -50,6 +52,9 @@
 namespace {
 
 constexpr uint32_t WAIT_LIMIT = 1u << 22;
+// How long one try of a wait may suspend its thread.  Every role but the decode groups mostly waits, and a call of few
+// rows is bound by what the decode groups issue; without the hint its polls come back after some tens of cycles each.
+constexpr uint32_t WAIT_HINT_NS = 20000;
 constexpr int NGRP = 4;                 // decode groups of four warps
 constexpr int NA = 4;                   // A slots in tensor memory (64 columns each), one per decode group
 constexpr int A_COLS = 64;
@@ -94,9 +99,9 @@ __device__ __forceinline__ bool mbar_try_wait(uint32_t bar, uint32_t parity) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+      : "=r"(ok) : "r"(bar), "r"(parity), "r"(WAIT_HINT_NS) : "memory");
   return ok != 0;
 }
 // State of a CTA: whether the kernels before this one have finished, and whether a wait ran out.
@@ -111,7 +116,7 @@ __device__ __noinline__ bool mbar_wait_slow(uint32_t bar, uint32_t parity, volat
   for (uint32_t it = 0; it < limit;) {
     if (mbar_try_wait(bar, parity)) return true;
     if (*state == PENDING) continue;
-    if ((++it & 255u) == 0u) {
+    if ((++it & 15u) == 0u) {
       unsigned long long t1;
       asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t1));
       if (t0 == 0) t0 = t1;
@@ -392,6 +397,14 @@ struct Ring {
       ++round;
     }
   }
+  // `n` at once, at most the number of stages
+  __device__ __forceinline__ void skip(uint32_t n, uint32_t stages) {
+    if ((slot += n) >= stages) {
+      slot -= stages;
+      phase ^= 1;
+      ++round;
+    }
+  }
   // the last use of every slot used so far
   template <typename F> __device__ __forceinline__ void each_last(uint32_t stages, F f) const {
     for (uint32_t s = 0; s < stages; ++s) {
@@ -577,18 +590,21 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     const uint32_t lane_addr = (uint32_t)((warp & 3) * 32) << 16;
     const uint8_t* wring = smem + p.off_wring;
     static_assert(NA == NGRP, "a decode group owns one A slot");
-    uint32_t n = 0, turn = 0;                               // items so far; items of this group so far
+    uint32_t n = 0, turn = 0;                               // items before this piece modulo NGRP; items of this group so far
     const uint32_t a = grp;
+    // the group steps from one of its items to the next, every NGRP-th, in the rings too (both have NGRP stages and more)
     Ring ring, rb;
+    ring.slot = rb.slot = grp;
     const uint32_t ready = rank == 0 ? B_READY(a) : cluster_addr(B_READY(a), 0);
     WorkList wl(p, cluster, n_clusters, IPT);
     Work w;
     while (wl.next(w)) {
-      for (uint32_t j = w.j0; j < w.j1; ++j, ++n) {
+      const uint32_t first = w.j0 + (grp >= (int)n ? grp - n : grp + NGRP - n);
+      n = (n + w.j1 - w.j0) % NGRP;
+      for (uint32_t j = first; j < w.j1; j += NGRP) {
         const uint32_t sw = ring.slot, wphase = ring.phase, sb = rb.slot, bphase = rb.phase;
-        ring.advance(SW);
-        rb.advance(SB);
-        if ((int)(n % NGRP) != grp) continue;
+        ring.skip(NGRP, SW);
+        rb.skip(NGRP, SB);
         mbar_wait(B_WFULL(sw), wphase, &s_state, p.status, 32u);
         const uint8_t* item = wring + (size_t)sw * p.wstage_bytes;
         const bool cherry = j < NCH;

@@ -205,6 +205,20 @@ def test_gemm_units_cut_into_runs(cabi, M):
     assert torch.equal(got[:, N:], base[:, N:]) and int(p.status.item()) == 0
 
 
+@pytest.mark.parametrize("K", [128, 256, 384, 512, 640, 896])
+def test_gemm_every_fourth_item_of_a_group(cabi, K):
+    """Units of 1 to 8 items (a decode group takes every fourth, counted over the units): 20 token blocks x 5 pairs of row
+    tiles are whole units and cut ones in one call of 148 SMs."""
+    N, M = 1160, 5000
+    w, idx, pk, dense = make_case(K, N, 4, 128, seed=K)
+    p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], 4, K, 128)
+    x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(K)).half()
+    ref = x.float() @ dev(dense).float().T
+    y = gemm(cabi, p, x)
+    assert float((y.float() - ref).abs().max() / ref.abs().max()) <= 2e-3          # as in test_gemm_llama7b_shapes
+    assert torch.equal(gemm(cabi, p, x), y)
+
+
 @pytest.mark.parametrize("bits,G", [(3, 64), (3, 128), (4, 128), (4, 256)])
 def test_gemm_weights_are_unpacked_exactly_at_every_scale(cabi, bits, G):
     """Rows of the identity read the dequantised weights back: bit for bit unpack()'s, with scales from the smallest
