@@ -103,15 +103,13 @@ __global__ void pack_codes_kernel(const void* __restrict__ w, int is_f32, const 
   }
 }
 
-// One pass over the weights for the group sizes in use (64, multiples of 128, one group per row): a block owns
-// PK_ROWS output rows of one group (two 64-wide ones), reads them once in chunks of 128 compact columns, reduces
+// One pass over the weights for groups of several chunks of 128 compact columns (multiples of 128, one group per row) and
+// for fp32 weights: a block owns PK_ROWS output rows of one group (two 64-wide ones), reads them once in chunks, reduces
 // the maxima and writes scales and codes.  The general pair of kernels above reads the matrix twice, lanes a row
 // apart, and divides per weight.  The loads are 2 bytes a lane, 64 contiguous bytes a warp, because the removed
 // cherry columns leave the compact columns at any alignment; the tile turns them so that a thread quantises 32
 // columns of one row and the byte stores have 32 consecutive rows a warp.  Groups of more than one chunk are read
-// a second time for the codes (mostly from L2); cq_pack leaves those of few rows to the general pair.  4096 x 11008
-// 4-bit: 57 us (114 MB, bound by the issue rate: about 25 instructions per weight), 415 us for sort, cherries, scales
-// and codes in four kernels.
+// a second time for the codes (mostly from L2); cq_pack leaves those of few rows to the general pair.
 constexpr int PK_ROWS = 64, PK_COLS = 128, PK_THREADS = 256;
 
 template <typename T> struct PackTile;
@@ -253,6 +251,255 @@ __global__ void __launch_bounds__(PK_THREADS, sizeof(T) == 2 ? 5 : 3) pack_fused
         for (int b = 0; b < BITS; ++b) dst[(size_t)b * N] = (uint8_t)(word >> (8 * b));
       }
     }
+  }
+}
+
+// fp16 weights of large matrices in groups of one chunk: a block keeps 128 compact columns, one group (two 64-wide ones); each
+// of its warps goes down the rows, 32 at a time, a lane a row, without a barrier.
+//   * Bound by the issue rate: the kernel above executes 31 instructions a weight, much of it set-up per 32 weights.  Here
+//     the rows come in with 16-byte copies, in their original order; the removed cherry columns only show when a lane takes
+//     32 compact columns of its row from shared memory, at some position (the same for the whole warp: each position has
+//     its own straight code): those after a cherry column move up.  (Picked one by one where a cherry column lay among
+//     them, such blocks were the last to end: 57 us for 11008 x 4096 3-bit with 40, 36 without.)  Maxima, clamps and
+//     roundings run on packed pairs.  Four rows' bytes are turned into words for the stores.
+//   * The 128 columns go in four turns of one loop, twice, instead of 64 registers a lane: unrolled, a fourth of the issue
+//     slots waited for instructions.  What depends on the columns alone is done once per block.
+// 4096 x 11008 4-bit: 46 us (58 with the kernel above), 16384 x 28672: 342 (542).
+constexpr int PG_WARPS = 4, PG_ROWS = 32, PG_BLOCKS = 4;        // warps of a block, rows of a warp's turn, blocks of an SM
+constexpr int PG_SPAN = 160;                          // original columns that fit the tile
+constexpr int PG_STRIDE = PG_SPAN + 8;                // an odd number of 16-byte pieces: those of 8 rows hit 8 different bank groups
+
+// The 32 values from position OFF on of the 16-byte pieces at `u`, as pairs.
+template <int OFF> __device__ __forceinline__ void take32(const uint4* u, uint32_t (&raw)[16]) {
+  constexpr int N = OFF ? 5 : 4;
+  uint32_t w[4 * N];
+#pragma unroll
+  for (int i = 0; i < N; ++i) {
+    const uint4 v = u[i];
+    w[4 * i] = v.x; w[4 * i + 1] = v.y; w[4 * i + 2] = v.z; w[4 * i + 3] = v.w;
+  }
+#pragma unroll
+  for (int i = 0; i < 16; ++i) raw[i] = (OFF & 1) ? __funnelshift_r(w[OFF / 2 + i], w[OFF / 2 + i + (OFF & 1)], 16) : w[OFF / 2 + i];
+}
+// rint(r - 0.5) + 2^(BITS-1) of both halves, in the low bytes.  The difference of an fp16 number and 0.5 is exact in fp32;
+// adding 1.5 * 2^23 (+ the code offset) rounds it to the nearest integer, ties to even.
+template <int BITS> __device__ __forceinline__ void codes_of(uint32_t h, uint32_t& c0, uint32_t& c1) {
+  const float magic = 12582912.f + (float)(1 << (BITS - 1));
+  float a, b;
+  asm("{\n\t.reg .f16 l, h;\n\tmov.b32 {l, h}, %2;\n\tadd.rn.f32.f16 %0, l, %3;\n\tadd.rn.f32.f16 %1, h, %3;\n\t}"
+      : "=f"(a), "=f"(b) : "r"(h), "f"(-0.5f));
+  c0 = __float_as_uint(__fadd_rn(a, magic));
+  c1 = __float_as_uint(__fadd_rn(b, magic));
+}
+
+template <int BITS>
+__global__ void __launch_bounds__(PG_WARPS * 32, PG_BLOCKS) pack_group_kernel(
+    const __half* __restrict__ w, const int16_t* __restrict__ idx, int K, int N, int C, int G,
+    __half* __restrict__ scales, uint8_t* __restrict__ q, __half* __restrict__ cw) {
+  __shared__ __align__(16) __half tiles[PG_WARPS][PG_ROWS * PG_STRIDE + 32];      // (+ 32: reads of 32 columns where fewer are left)
+  __shared__ int source[PK_COLS], s_at[4], s_gaps[4], s_gap[4], s_end;
+  __shared__ __align__(16) uint32_t turned[PG_WARPS][4][32];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int Kc = K - C, k0 = blockIdx.x * PK_COLS, cols = min(PK_COLS, Kc - k0);
+  const bool two = G == 64;                                       // two groups in the block's 128 columns
+
+  // ---- where the columns are
+  static_assert(PG_WARPS * 32 == PK_COLS, "a thread a column");
+  source[tid] = tid < cols ? k0 + tid + cherry_shift(idx, C, k0 + tid) : -1;
+  if (tid == 0) s_end = k0 + PK_COLS >= Kc ? C : cherry_shift(idx, C, k0 + PK_COLS);
+  __syncthreads();
+  // the cherry columns before the next block's first column are this block's to copy
+  const int c_begin = blockIdx.x == 0 ? 0 : source[0] - k0, c_end = s_end;
+  const int first = c_begin < c_end ? min(idx[c_begin], source[0]) : source[0];
+  const int last = c_begin < c_end ? max(idx[c_end - 1], source[cols - 1]) : source[cols - 1];
+  const int base = first & ~7, pieces = (last - base) / 8 + 1;
+  const bool wide = (reinterpret_cast<uintptr_t>(w) & 15) == 0 && pieces * 8 <= PG_SPAN;      // (K is a multiple of 8)
+  // of each 32 columns: where the first is in the tile, how many cherry columns lie among them, the first of these
+  const int parts = (cols + 31) / 32;
+  if (tid < parts) {
+    const int j = 32 * tid, from = source[j], to = source[min(j + 31, cols - 1)];
+    s_at[tid] = wide ? from - base : j;
+    s_gaps[tid] = wide ? to - from - min(31, cols - 1 - j) : 0;
+    s_gap[tid] = from - (k0 + j);
+  }
+  __syncthreads();
+  // this lane's first piece, and how far its next one is: rows, pieces
+  const int piece_r = lane / pieces, piece_c = lane - piece_r * pieces, step_r = 32 / pieces, step_c = 32 - step_r * pieces;
+  __half* tile = tiles[warp];
+  const uint32_t tile_s = (uint32_t)__cvta_generic_to_shared(tile);
+  auto copy = [&](int n0) {
+    const int rows = min(PG_ROWS, N - n0);
+    if (wide) {
+      const __half* src = w + (size_t)(n0 + piece_r) * K + base + 8 * piece_c;
+      uint32_t dst = tile_s + (piece_r * PG_STRIDE + 8 * piece_c) * 2;
+      int c = piece_c;
+      for (int r = piece_r; r < rows;) {
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
+        const bool wrap = c + step_c >= pieces;
+        const int dr = step_r + wrap, dc = step_c - (wrap ? pieces : 0);
+        r += dr;
+        c += dc;
+        src += dr * K + 8 * dc;
+        dst += (dr * PG_STRIDE + 8 * dc) * 2;
+      }
+    } else {
+      // unaligned weights, or so many cherry columns inside the chunk that it does not fit: compact columns one by one
+      for (int j = lane; j < cols; j += 32) {
+        const __half* src = w + (size_t)n0 * K + source[j];
+#pragma unroll 16
+        for (int r = 0; r < rows; ++r) tile[r * PG_STRIDE + j] = src[(size_t)r * K];
+      }
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+
+  const int step = gridDim.y * PG_WARPS * PG_ROWS;
+  int n0 = (blockIdx.y * PG_WARPS + warp) * PG_ROWS;
+  if (n0 < N) copy(n0);
+  for (; n0 < N; n0 += step) {
+    const bool live = n0 + lane < N;
+    const int n = live ? n0 + lane : N - 1;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncwarp();
+    uint32_t raw[16];
+    const __half* t = tile + lane * PG_STRIDE;
+    // cherry_weight[c, n] = W[n, idx[c]]
+    if (wide) {
+      for (int c = c_begin; c < c_end; ++c) {
+        const __half v = t[idx[c] - base];
+        if (live) cw[(size_t)c * N + n] = v;
+      }
+    } else {
+      // not in the tile, but the 32 columns after the 128 are free
+      const int rows = min(PG_ROWS, N - n0);
+      for (int c0 = c_begin; c0 < c_end; c0 += 32) {
+        if (c0 + lane < c_end) {
+          const __half* src = w + (size_t)n0 * K + idx[c0 + lane];
+#pragma unroll 16
+          for (int r = 0; r < rows; ++r) tile[r * PG_STRIDE + PK_COLS + lane] = src[(size_t)r * K];
+        }
+        __syncwarp();
+        for (int c = c0; c < min(c_end, c0 + 32); ++c)
+          if (live) cw[(size_t)c * N + n] = t[PK_COLS + c - c0];
+        __syncwarp();
+      }
+    }
+    auto take = [&](int p) {                                      // this lane's columns 32 p .. 32 p + 31
+      const int at = s_at[p], gaps = s_gaps[p], left = cols - 32 * p;
+      const uint4* u = reinterpret_cast<const uint4*>(t + (at & ~7));
+      switch (at & 7) {                                           // the same for the whole warp
+        case 0: take32<0>(u, raw); break;
+        case 1: take32<1>(u, raw); break;
+        case 2: take32<2>(u, raw); break;
+        case 3: take32<3>(u, raw); break;
+        case 4: take32<4>(u, raw); break;
+        case 5: take32<5>(u, raw); break;
+        case 6: take32<6>(u, raw); break;
+        default: take32<7>(u, raw); break;
+      }
+#pragma unroll 1
+      for (int g = 0; g < gaps; ++g) {                            // a cherry column goes, those after it move up
+        const int pos = idx[s_gap[p] + g] - base - at - g;
+        const uint32_t next = reinterpret_cast<const unsigned short*>(t)[min(at + 32 + g, PG_SPAN)];
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const uint32_t follow = i < 15 ? raw[i + 1 < 16 ? i + 1 : 15] : next;
+          if (2 * i + 1 >= pos) raw[i] = __byte_perm(raw[i], follow, 2 * i + 1 == pos ? 0x5410 : 0x5432);
+        }
+      }
+      if (left < 32) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) raw[i] = 2 * i + 1 < left ? raw[i] : (2 * i < left ? raw[i] & 0xffffu : 0u);
+      }
+    };
+    // ---- scales of the two 64-column halves (of one group: the same)
+    float s[2];
+    __half2 m2[2] = {__float2half2_rn(0.f), __float2half2_rn(0.f)};       // (the maximum leaves NaN out, as fmaxf does)
+#pragma unroll 1
+    for (int p = 0; p < parts; ++p) {
+      take(p);
+      __half2 m = __float2half2_rn(0.f);
+#pragma unroll
+      for (int i = 0; i < 16; ++i) m = __hmax2(m, __habs2(*reinterpret_cast<const __half2*>(&raw[i])));
+      if (p < 2) m2[0] = __hmax2(m2[0], m);
+      else m2[1] = __hmax2(m2[1], m);
+    }
+    if (!two) m2[0] = m2[1] = __hmax2(m2[0], m2[1]);
+#pragma unroll
+    for (int h = 0; h < 2; ++h) {
+      if (h == 1 && !two) { s[1] = s[0]; break; }
+      const float mx = fmaxf(__low2float(m2[h]), __high2float(m2[h]));
+      // fp16 add and fp16 divide (by a power of two: the product is the quotient), each rounded once
+      const __half sh = __float2half_rn(__fmul_rn(__half2float(__float2half_rn(__fadd_rn(mx, 1e-6f))), 1.f / (1 << (BITS - 1))));
+      const int grp = k0 / G + h;
+      if (live && grp < (Kc + G - 1) / G) scales[(size_t)grp * N + n] = sh;
+      s[h] = __half2float(sh);
+    }
+    // ---- quotients fp16(w / s) from the product with r = RN(1 / s): the product's relative error is below 2^-23; a quotient
+    // of two 11-bit significands is farther than 2^-23 (1 + 2^-12) from a midpoint of two normal fp16 numbers, so the fp16
+    // rounding is that of the quotient.  Quotients below 2^-14 may lie on a midpoint; of those only -2^-25, between -0 and
+    // the first number that gets another code, matters, and w = -2^-25 s needs s >= 2.  Such scales (and infinite ones)
+    // take the residual step of div_fp16.
+    const bool large = __any_sync(0xffffffffu, !(s[0] < 2.f && s[1] < 2.f));
+    const __half2 top = __float2half2_rn(BITS == 4 ? 7.98828125f : 3.98828125f), bottom = __hneg2(top);
+#pragma unroll 1
+    for (int p = 0; p < parts; ++p) {
+      take(p);
+      const float sp = p < 2 ? s[0] : s[1], rs = __frcp_rn(sp);
+      if (large) {
+        const float s_residual = sp < 65536.f ? sp : 0.f;
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&raw[i]));
+          const __half2 h = __floats2half2_rn(div_fp16(f.x, s_residual, rs), div_fp16(f.y, s_residual, rs));
+          raw[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) {
+          const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&raw[i]));
+          const __half2 h = __floats2half2_rn(__fmul_rn(f.x, rs), __fmul_rn(f.y, rs));
+          raw[i] = *reinterpret_cast<const uint32_t*>(&h);
+        }
+      }
+      // ---- codes, clamped at an fp16 number just below 2^(BITS-1) - 0.01: the same code, whose middle is half a code away
+#pragma unroll
+      for (int o = 0; o < 4; ++o) {
+        uint32_t code[8];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const __half2 h = __hmin2(__hmax2(*reinterpret_cast<const __half2*>(&raw[4 * o + i]), bottom), top);
+          codes_of<BITS>(*reinterpret_cast<const uint32_t*>(&h), code[2 * i], code[2 * i + 1]);
+        }
+        // bytes 0, 2, 4, 6 and 1, 3, 5, 7
+        const uint32_t even = __byte_perm(__byte_perm(code[0], code[2], 0x0040), __byte_perm(code[4], code[6], 0x0040), 0x5410);
+        const uint32_t odd = __byte_perm(__byte_perm(code[1], code[3], 0x0040), __byte_perm(code[5], code[7], 0x0040), 0x5410);
+        uint32_t word = even | (odd << BITS);
+        if (BITS == 3) word = (word & 0x3Fu) | ((word >> 2) & 0xFC0u) | ((word >> 4) & 0x3F000u) | ((word >> 6) & 0xFC0000u);
+        turned[warp][o][lane] = word;
+      }
+      __syncwarp();
+      {
+        // this lane: octet lane / 8 of the four, rows 4 (lane & 7) .. + 3 of the 32: four words to BITS rows of four bytes
+        const int o = lane >> 3, m = n0 + 4 * (lane & 7);
+        const uint4 v = *reinterpret_cast<const uint4*>(&turned[warp][o][4 * (lane & 7)]);
+        if (m < N && 32 * p + 8 * o < cols) {                     // (N is a multiple of 8)
+          const uint32_t p0 = __byte_perm(v.x, v.y, 0x5140), p1 = __byte_perm(v.x, v.y, 0x7362);
+          const uint32_t p2 = __byte_perm(v.z, v.w, 0x5140), p3 = __byte_perm(v.z, v.w, 0x7362);
+          const uint32_t b[4] = {__byte_perm(p0, p2, 0x5410), __byte_perm(p0, p2, 0x7632), __byte_perm(p1, p3, 0x5410), __byte_perm(p1, p3, 0x7632)};
+          uint8_t* dst = q + (size_t)((k0 >> 3) + 4 * p + o) * BITS * N + m;
+          if ((reinterpret_cast<uintptr_t>(q) & 3) == 0) {
+#pragma unroll
+            for (int i = 0; i < BITS; ++i) *reinterpret_cast<uint32_t*>(dst + (size_t)i * N) = b[i];
+          } else {
+            for (int i = 0; i < BITS; ++i)
+              for (int e = 0; e < 4; ++e) dst[(size_t)i * N + e] = (uint8_t)(b[i] >> (8 * e));
+          }
+        }
+      }
+      __syncwarp();
+    }
+    if (n0 + step < N) copy(n0 + step);                           // (every lane is done with the tile)
   }
 }
 
@@ -423,6 +670,14 @@ int nblocks(long long total, int threads) {
   return (int)b;
 }
 
+// Blocks over the rows for kernels whose blocks keep their columns and go down the rows, `per_sm` of them on an SM at once:
+// about four waves, so that a last one that is nearly empty costs little (one wave and a bit took twice the time).
+int row_blocks(int n_x, int n_tiles, int per_sm) {
+  long long n = 4ll * per_sm * cq_sm_count() / n_x;
+  if (n > n_tiles) n = n_tiles;
+  return n < 1 ? 1 : (n > 65535 ? 65535 : (int)n);
+}
+
 int check_dims(int bits, int K, int N, int C, int* G) {
   if (bits != 3 && bits != 4) return CQ_ERR_BAD_BITS;
   if (*G == -1) *G = K;
@@ -447,6 +702,17 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
   const int T = 256;
   if (C > 0) pack_sort_kernel<<<nblocks(C, T), T, 0, st>>>(cherry_unsorted, C, cherry_indices);
   const int ng = (K - C + G - 1) / G;
+  // From 12 million weights on a warp of pack_group_kernel has rows enough to go down (4096 x 11008 4-bit: 48.0 and 58.8 us;
+  // 16384 x 28672 342 and 542; 4096 x 4096 22.9 and 24.9; 16384 x 1024 25.6 and 27.5; 4096 x 2048 16.5 and 16.5; 2048 x 1024
+  // 12.3 and 10.3; 1032 x 1000 12.3 and 9.6).
+  if (!weight_is_f32 && (G == 64 || G == PK_COLS) && (long long)K * N >= (3ll << 22)) {
+    const int n_x = (K - C + PK_COLS - 1) / PK_COLS, rows = PG_WARPS * PG_ROWS;
+    auto kernel = bits == 4 ? pack_group_kernel<4> : pack_group_kernel<3>;
+    kernel<<<dim3(n_x, row_blocks(n_x, (N + rows - 1) / rows, PG_BLOCKS)), PG_WARPS * 32, 0, st>>>(
+        (const __half*)weight, cherry_indices, K, N, C, G, (__half*)scales, qweight, (__half*)cherry_weight);
+    CQ_CUDA_TRY(cudaGetLastError());
+    return CQ_OK;
+  }
   const int span = G == 64 ? PK_COLS : (ng == 1 ? (K - C) : G);           // compact columns a block owns
   // A block walks a group of several chunks from end to end, twice, while the general pair spreads it over the chip: on
   // matrices of few rows the pair is faster.  Microseconds as measured over 256 .. 11008 columns, 64 .. 16384 rows (one

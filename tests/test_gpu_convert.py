@@ -77,6 +77,28 @@ def test_pack_and_unpack_of_narrow_groups_and_many_cherries(cabi, K, N, G, C, bi
     assert np.array_equal(gpu_unpack(cabi, ref, bits, K, G).view(np.uint16), dense.view(np.uint16))
 
 
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("K,N,bits,G,C", [(1032, 12296, 4, 128, 16), (1160, 10856, 3, 64, 8), (4096, 3080, 3, 128, 2056),
+                                          (2048, 6152, 4, 128, 520)])
+def test_pack_of_large_matrices(cabi, K, N, bits, G, C, offset):
+    """From 12 million fp16 weights on: rows that end inside a warp's 32, columns inside a block's 128, cherry columns among
+    32 columns and so many that a block's columns do not fit the tile; weights and codes off their alignment."""
+    w, idx = layer(K, N, C, np.float16, K + N)
+    if C == 520:
+        idx = np.concatenate([np.arange(1000, 1500), np.arange(2028, 2048)])            # side by side, and at the end
+    ref = O.pack(w, idx, bits, G)
+    wd = torch.zeros(N * K + offset, dtype=torch.float16, device="cuda")
+    wd[offset:] = dev(w).flatten()
+    q = torch.zeros(ref["qweight"].size + offset, dtype=torch.uint8, device="cuda")
+    t = [dev(np.zeros_like(ref[k])) for k in ("scales", "cherry_weight", "cherry_indices")]
+    cabi.check(cabi.lib().cq_pack(wd.data_ptr() + 2 * offset, 0, ptr(dev(idx.astype(np.int32))), bits, K, N, C, G,
+                                  q.data_ptr() + offset, *[ptr(a) for a in t], None, None), "pack")
+    torch.cuda.synchronize()
+    assert np.array_equal(q[offset:].cpu().numpy(), ref["qweight"].ravel())
+    for a, key in zip(t, ("scales", "cherry_weight", "cherry_indices")):
+        assert np.array_equal(a.cpu().numpy().view(np.uint8), ref[key].view(np.uint8)), key
+
+
 def test_unpack_into_unaligned_buffers(cabi):
     K, N, bits, G, C = 264, 72, 3, 128, 8
     w, idx = layer(K, N, C, np.float16, 5)
