@@ -505,21 +505,63 @@ __global__ void __launch_bounds__(PG_WARPS * 32, PG_BLOCKS) pack_group_kernel(
 
 // ------------------------------------------------------------------ dense unpack
 // llama/qlinear.py:120-162: dense[n, k] = cherry ? cherry_weight : fp16((q + 0.5) * s).
-// A block writes 64 rows x 128 columns: a thread makes one octet of 8 original columns of four consecutive rows.
-// The octet's codes are consecutive compact columns: the bytes of two compact octets (one 32-bit load per byte row covers
-// the four rows), shifted by the position inside the first; a cherry column inside leaves a gap in the word, and its
-// values go over the finished octet.  Pairs of codes become the low mantissa bits of 1024 + u, minus (1024 + off), times
-// the scale: each step but the last exact, so the product is rounded once as in the reference.  The tile in shared memory
-// (16-byte slots, slot number XOR row quad against bank conflicts) turns the octets into rows of 256 contiguous bytes.
-// 11008 x 4096 3-bit: 36 us (108 MB), 290 with a binary search, a byte-wise code fetch and two divisions per element; 512 x
-// 512: 3.6 us and 4.3.
-constexpr int UP_ROWS = 64, UP_COLS = 128;
+// A block keeps 128 original columns and goes down the rows, 64 at a time: what depends on the columns alone (the search for
+// the cherry columns among it) is done once, the next rows' codes are on their way while these are written.  A thread makes
+// one octet of 8 columns of four consecutive rows.  The octet's codes are consecutive compact columns: the bytes of two
+// compact octets (one 32-bit load per byte row covers the four rows), shifted by the position inside the first.  Pairs of
+// codes become mantissa bits of 1024; one exact multiply-add and the product with the scale, rounded once as in the
+// reference, make the values.  Warps whose octets have a cherry column or a group's end inside take a general path: a gap
+// in the word for each cherry column, whose values go over the finished octet, and a scale for each column.  The tile in
+// shared memory (16-byte slots, slot number XOR row quad against bank conflicts) turns the octets into rows of 256
+// contiguous bytes.  Bound by the issue rate: 11008 x 4096 3-bit 35.6 us (108 MB), 38.9 with the kernel above; 4096 x 11008
+// 4-bit 36.9 and 40.6; 16384 x 28672 335 and 360.
+constexpr int UP_ROWS = 64, UP_COLS = 128, UP_BLOCKS = 4;       // blocks of an SM
 
 __device__ __forceinline__ uint32_t load_quad(const uint8_t* p, bool aligned) {
   if (aligned) return __ldg(reinterpret_cast<const uint32_t*>(p));
   return (uint32_t)p[0] | ((uint32_t)p[1] << 8) | ((uint32_t)p[2] << 16) | ((uint32_t)p[3] << 24);
 }
+// four consecutive scales
+__device__ __forceinline__ uint2 load_scales(const __half* p, bool aligned) {
+  if (aligned) return __ldg(reinterpret_cast<const uint2*>(p));
+  const unsigned short* u = reinterpret_cast<const unsigned short*>(p);
+  return make_uint2((uint32_t)u[0] | ((uint32_t)u[1] << 16), (uint32_t)u[2] | ((uint32_t)u[3] << 16));
+}
 
+// the codes of a word, 2 i and 2 i + 1 in field bits P_i of the halves of t[i], into (u - off) * s with the pair's scales
+template <int BITS, int P> __device__ __forceinline__ uint32_t scaled_pair(uint32_t t, uint32_t s2) {
+  constexpr uint32_t FIELD = (uint32_t)(((1 << BITS) - 1) << P), ONE = (uint32_t)(15 - P) << 10;      // 2^-P
+  // -(1024 * 2^-P + off)
+  constexpr uint32_t CENTER = BITS == 4 ? 0xD478u : (P == 1 ? 0xE007u : 0xC9C0u);       // -71.5; -515.5, -11.5
+  static_assert(BITS == 4 ? P == 4 : (P == 1 || P == 7), "no other fields are used");
+  uint32_t d;
+  asm("{\n\t.reg .b32 v;\n\tfma.rn.f16x2 v, %1, %2, %3;\n\tmul.rn.f16x2 %0, v, %4;\n\t}"
+      : "=r"(d) : "r"((t & (FIELD | (FIELD << 16))) | 0x64006400u), "r"(ONE | (ONE << 16)), "r"(CENTER | (CENTER << 16)), "r"(s2));
+  return d;
+}
+// eight codes (consecutive fields of `word`) times the scales of each pair
+template <int BITS> __device__ __forceinline__ uint4 scaled_octet(uint32_t word, const uint32_t (&s2)[4]) {
+  uint4 v;
+  if constexpr (BITS == 4) {
+    const uint32_t up = word << 4;            // byte i of `up` has code 2 i above, byte i of `word` code 2 i + 1
+    v.x = scaled_pair<4, 4>(__byte_perm(up, word, 0x4400), s2[0]);
+    v.y = scaled_pair<4, 4>(__byte_perm(up, word, 0x5511), s2[1]);
+    v.z = scaled_pair<4, 4>(__byte_perm(up, word, 0x6622), s2[2]);
+    v.w = scaled_pair<4, 4>(__byte_perm(up, word, 0x7733), s2[3]);
+  } else {
+    // low half: codes 0 .. 4 from bit 1 on, high half: codes 1 .. 5
+    const uint32_t a = ((word << 1) & 0xFFFFu) | ((word << 14) & 0xFFFF0000u);
+    const uint32_t b = ((word >> 11) & 0xFFFFu) | ((word << 2) & 0xFFFF0000u);      // the same from code 4 on
+    v.x = scaled_pair<3, 1>(a, s2[0]);
+    v.y = scaled_pair<3, 7>(a, s2[1]);
+    v.z = scaled_pair<3, 1>(b, s2[2]);
+    v.w = scaled_pair<3, 7>(b, s2[3]);
+  }
+  return v;
+}
+
+// For layers with many cherry columns: a block makes one tile of 64 rows x 128 columns, each value by itself, gaps and groups
+// included.  (4096 x 11008 4-bit, 512 cherry columns: 54.5 us, the kernel below 62.4; 256: 48.4 and 50.5.)
 // codes 2 i, 2 i + 1 of a word as fp16 (u - off)
 template <int BITS> __device__ __forceinline__ __half2 code_pair(uint32_t word, int i) {
   const uint32_t x = word >> (2 * BITS * i);
@@ -531,7 +573,6 @@ template <int BITS> __device__ __forceinline__ __half2 code_pair(uint32_t word, 
   return __hsub2(d, *reinterpret_cast<const __half2*>(&half));
 }
 
-// CHERRY = the layer has cherry columns
 template <int BITS, bool CHERRY>
 __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
     const uint8_t* __restrict__ q, const __half* __restrict__ scales, const __half* __restrict__ cw,
@@ -650,6 +691,160 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
   }
 }
 
+
+// CHERRY = the layer has cherry columns
+template <int BITS, bool CHERRY>
+__global__ void __launch_bounds__(256, UP_BLOCKS) unpack_rows_kernel(
+    const uint8_t* __restrict__ q, const __half* __restrict__ scales, const __half* __restrict__ cw,
+    const int16_t* __restrict__ idx, int K, int N, int C, int G, int g_shift, __half* __restrict__ dense, int aligned) {
+  __shared__ __align__(16) uint4 tiles[2][UP_ROWS * (UP_COLS / 8)];
+  const int tid = threadIdx.x, nq = tid & 15, oct = tid >> 4, lane = tid & 31;
+  const int k0 = blockIdx.x * UP_COLS, k = k0 + 8 * oct, k_warp = k0 + 8 * (oct & ~1);       // a warp has two octets
+  const int Kc = K - C, n_oct = Kc / 8;
+  int low = 0, cnt = 0;                                         // cherry columns before the octet and inside it
+  if (CHERRY) {
+    int before[3] = {0, 0, 0};                                  // ... before the warp's first, second and the next octet
+    for (int c = lane; c - lane < C; c += 32) {
+      const int col = c < C ? (int)idx[c] : 0x7fffffff;
+#pragma unroll
+      for (int i = 0; i < 3; ++i) before[i] += __popc(__ballot_sync(0xffffffffu, col < k_warp + 8 * i));
+    }
+    low = before[oct & 1];
+    cnt = max(0, min(8, before[(oct & 1) + 1] - low));
+  }
+  const int n_codes = 8 - cnt;
+  const int kc = max(k - low, 0), o = kc >> 3, r = kc & 7;
+  auto group_of = [&](int c) { return g_shift >= 0 ? c >> g_shift : c / G; };
+  const int g = group_of(kc), split = (g + 1) * G - kc;         // codes 0 .. split - 1 belong to group g
+  const bool whole = split >= n_codes;
+  const bool plain = __all_sync(0xffffffffu, whole && cnt == 0);        // the whole warp's octets: eight codes of one group
+  uint32_t own = 0, second = 0;                                 // columns that are cherries; that belong to group g + 1
+  if (!plain && k < K) {
+    for (int t = 0; t < cnt; ++t) own |= 1u << (((int)idx[low + t] - k) & 7);
+    if (!whole) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) second |= (e - __popc(own & ((1u << e) - 1)) >= split ? 1u : 0u) << e;
+    }
+  }
+  const bool in = k < K, more = r && o + 1 < n_oct, first = o < n_oct;
+  // the bytes of compact octets o and o + 1, four rows in each word
+  uint32_t b[2][BITS];
+  uint2 ahead = make_uint2(0, 0);                               // the four rows' scales of group g
+  const uint8_t* src = q + (size_t)o * BITS * N;
+  const __half* own_scales = scales + (size_t)g * N;
+  auto load = [&](int n) {
+    const uint8_t* p = src + n;
+    if (in && n < N && n_codes > 0) ahead = load_scales(own_scales + n, aligned & 4);
+#pragma unroll
+    for (int h = 0; h < 2; ++h)
+#pragma unroll
+      for (int i = 0; i < BITS; ++i) {
+        b[h][i] = (in && n < N && (h ? more : first)) ? load_quad(p, aligned & 1) : 0u;
+        p += N;
+      }
+  };
+  load(blockIdx.y * UP_ROWS + 4 * nq);
+  uint4* tile = tiles[0];
+  uint4* slot = tile + 64 * nq + (oct ^ nq);                    // rows 4 nq + j: 16 j slots on
+  int other = UP_ROWS * (UP_COLS / 8);
+  for (int n0 = blockIdx.y * UP_ROWS; n0 < N; n0 += gridDim.y * UP_ROWS) {
+    const int n = n0 + 4 * nq;
+    if (in && n < N) {
+      const uint2 sc = ahead;
+      // the four rows' words of both octets (a 4 x 4 transpose of bytes), then the eight codes from column kc on
+      uint32_t words[4];
+      {
+        uint32_t w[2][4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const uint32_t b3 = BITS == 4 ? b[h][BITS - 1] : 0u;
+          const uint32_t p0 = __byte_perm(b[h][0], b[h][1], 0x5140), p1 = __byte_perm(b[h][0], b[h][1], 0x7362);
+          const uint32_t p2 = __byte_perm(b[h][2], b3, 0x5140), p3 = __byte_perm(b[h][2], b3, 0x7362);
+          w[h][0] = __byte_perm(p0, p2, 0x5410);
+          w[h][1] = __byte_perm(p0, p2, 0x7632);
+          w[h][2] = __byte_perm(p1, p3, 0x5410);
+          w[h][3] = __byte_perm(p1, p3, 0x7632);
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (BITS == 4)
+            words[j] = __funnelshift_r(w[0][j], w[1][j], 4 * r);
+          else
+            words[j] = (w[0][j] >> (3 * r)) | (r ? w[1][j] << (24 - 3 * r) : 0u);
+        }
+      }
+      load(n + (int)gridDim.y * UP_ROWS);
+      if (plain) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const uint32_t s = __byte_perm(j < 2 ? sc.x : sc.y, 0, (j & 1) ? 0x3232 : 0x1010);
+          const uint32_t s2[4] = {s, s, s, s};
+          slot[16 * j] = scaled_octet<BITS>(words[j], s2);
+        }
+      } else {
+        const uint2 sd = whole ? sc : load_scales(scales + (size_t)(g + 1) * N + n, aligned & 4);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          uint32_t word = words[j];
+          for (uint32_t m = own; m; m &= m - 1) {               // a gap at each cherry column
+            const int at = BITS * (__ffs(m) - 1);
+            const uint32_t below = (1u << at) - 1;
+            word = (word & below) | ((word & ~below) << BITS);
+          }
+          const uint32_t sa = __byte_perm(j < 2 ? sc.x : sc.y, 0, (j & 1) ? 0x4432 : 0x4410);
+          const uint32_t sb = __byte_perm(j < 2 ? sd.x : sd.y, 0, (j & 1) ? 0x4432 : 0x4410);
+          uint32_t s2[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i)
+            s2[i] = ((second >> (2 * i)) & 1u ? sb : sa) | (((second >> (2 * i + 1)) & 1u ? sb : sa) << 16);
+          slot[16 * j] = scaled_octet<BITS>(word, s2);
+        }
+        for (int t = 0; t < cnt; ++t) {
+          const int e = ((int)idx[low + t] - k) & 7;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) reinterpret_cast<__half*>(slot + 16 * j)[e] = cw[(size_t)(low + t) * N + n + j];
+        }
+        if (!whole && G < 8) {
+          // groups narrower than 8 columns can put more than two into an octet: column by column
+#pragma unroll 1
+          for (int e = 0, m = low; e < 8; ++e) {
+            if ((own >> e) & 1u) { ++m; continue; }
+            const int c = k + e - m;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+              const float a = (float)((int)cq_ref_code(q, BITS, c, n + j, N) - (1 << (BITS - 1))) + 0.5f;
+              reinterpret_cast<__half*>(slot + 16 * j)[e] =
+                  __float2half_rn(__fmul_rn(a, __half2float(scales[(size_t)group_of(c) * N + n + j])));
+            }
+          }
+        }
+      }
+    }
+    __syncthreads();                                            // (the other tile was read before this barrier)
+    const int rr = tid >> 4, oo = tid & 15, kk = k0 + 8 * oo;
+    if (kk < K) {
+      __half* dst = dense + (size_t)(n0 + rr) * K + kk;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {                             // rows rr + 16 i
+        if (n0 + rr + 16 * i < N) {
+          const uint4 v = tile[(rr + 16 * i) * 16 + (oo ^ ((rr >> 2) + 4 * i))];
+          if (aligned & 2) {
+            *reinterpret_cast<uint4*>(dst) = v;
+          } else {
+            const uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+            for (int e = 0; e < 8; ++e) dst[e] = __ushort_as_half((unsigned short)(u[e >> 1] >> (16 * (e & 1))));
+          }
+        }
+        dst += 16 * (size_t)K;
+      }
+    }
+    tile += other;
+    slot += other;
+    other = -other;
+  }
+}
+
 // ------------------------------------------------------------------ Dequantize{3,4}Normal
 __global__ void dequant_normal_kernel(const uint8_t* __restrict__ q, const float* __restrict__ sf,
                                       float* __restrict__ out, int bits, int Kc, int N, int G) {
@@ -756,15 +951,26 @@ extern "C" int cq_unpack_dense(const uint8_t* qweight, const void* scales, const
   if (C > 0 && (!cherry_weight || !cherry_indices)) return CQ_ERR_BAD_ARG;
   const int rc = check_dims(bits, K, N, C, &G);
   if (rc) return rc;
-  dim3 grid((K + UP_COLS - 1) / UP_COLS, (N + UP_ROWS - 1) / UP_ROWS);
-  const int aligned = (((uintptr_t)qweight & 3) == 0 ? 1 : 0) | (((uintptr_t)dense & 15) == 0 ? 2 : 0);
+  const int aligned = (((uintptr_t)qweight & 3) == 0 ? 1 : 0) | (((uintptr_t)dense & 15) == 0 ? 2 : 0) | (((uintptr_t)scales & 7) == 0 ? 4 : 0);
   int g_shift = -1;
   if ((G & (G - 1)) == 0)
     for (g_shift = 0; (1 << g_shift) < G;) ++g_shift;
-  auto kernel = bits == 4 ? (C > 0 ? unpack_dense_kernel<4, true> : unpack_dense_kernel<4, false>)
-                          : (C > 0 ? unpack_dense_kernel<3, true> : unpack_dense_kernel<3, false>);
-  kernel<<<grid, 256, 0, (cudaStream_t)stream>>>(qweight, (const __half*)scales, (const __half*)cherry_weight,
-                                                 cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
+  const int n_cols = (K + UP_COLS - 1) / UP_COLS, n_tiles = (N + UP_ROWS - 1) / UP_ROWS;
+  auto launch = [&](auto kernel, int n_y) {
+    kernel<<<dim3(n_cols, n_y), 256, 0, (cudaStream_t)stream>>>(qweight, (const __half*)scales, (const __half*)cherry_weight,
+                                                               cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
+  };
+  // Up to a cherry column in 32, so that most octets have none (4096 x 11008 4-bit, new and old kernel: 16 cherry columns 36.9
+  // and 40.6 us, 64 40.2 and 43.9, 128 44.6 and 46.2, then see the old kernel).  Matrices of few columns have no columns to
+  // spread over the chip but rows: 128 x 65536 13.4 and 12.2.
+  if ((long long)C * 32 <= K && n_cols >= 8) {
+    const int n_y = row_blocks(n_cols, n_tiles, UP_BLOCKS);
+    bits == 4 ? (C > 0 ? launch(unpack_rows_kernel<4, true>, n_y) : launch(unpack_rows_kernel<4, false>, n_y))
+              : (C > 0 ? launch(unpack_rows_kernel<3, true>, n_y) : launch(unpack_rows_kernel<3, false>, n_y));
+  } else {
+    bits == 4 ? (C > 0 ? launch(unpack_dense_kernel<4, true>, n_tiles) : launch(unpack_dense_kernel<4, false>, n_tiles))
+              : (C > 0 ? launch(unpack_dense_kernel<3, true>, n_tiles) : launch(unpack_dense_kernel<3, false>, n_tiles));
+  }
   CQ_CUDA_TRY(cudaGetLastError());
   return CQ_OK;
 }

@@ -99,6 +99,24 @@ def test_pack_of_large_matrices(cabi, K, N, bits, G, C, offset):
         assert np.array_equal(a.cpu().numpy().view(np.uint8), ref[key].view(np.uint8)), key
 
 
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("K,N,bits,G,C", [(904, 8, 3, 1, 8), (1032, 72, 4, 4, 24), (1160, 136, 3, 12, 32), (2048, 520, 4, 96, 64),
+                                          (1024, 3208, 3, 64, 0)])
+def test_unpack_going_down_the_rows(cabi, K, N, bits, G, C, offset):
+    """Eight and more blocks of columns, few cherry columns: octets with one inside, with group boundaries, of groups narrower
+    than an octet; rows that end inside a tile; codes and outputs off their alignment."""
+    w, idx = layer(K, N, C, np.float16, K + G)
+    ref = O.pack(w, idx, bits, G)
+    t = [dev(ref[k]) for k in ("scales", "cherry_weight", "cherry_indices")]
+    q = torch.zeros(ref["qweight"].size + offset, dtype=torch.uint8, device="cuda")
+    q[offset:] = dev(ref["qweight"]).flatten()
+    out = torch.zeros(N * K + offset, dtype=torch.float16, device="cuda")
+    cabi.check(cabi.lib().cq_unpack_dense(q.data_ptr() + offset, *[ptr(a) for a in t], bits, K, N, C, G,
+                                          out.data_ptr() + 2 * offset, None), "unpack")
+    dense = O.unpack(ref["qweight"], ref["scales"], ref["cherry_weight"], ref["cherry_indices"], bits, G, K)
+    assert np.array_equal(out[offset:].cpu().numpy().view(np.uint16), dense.view(np.uint16).ravel())
+
+
 def test_unpack_into_unaligned_buffers(cabi):
     K, N, bits, G, C = 264, 72, 3, 128, 8
     w, idx = layer(K, N, C, np.float16, 5)
