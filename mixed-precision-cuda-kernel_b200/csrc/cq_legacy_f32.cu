@@ -13,15 +13,22 @@
 // 2^-6 or less of what an fp32 addition rounds away beside the largest product (only activations that are smaller than
 // 2^-24 of two large ones which cancel are lost where a chain of additions in a lucky order keeps them).  A loop of fp32
 // multiply-adds needs 25 us of the FMA pipe for 16 rows of 4096 x 13824, before the decode of each code by the one
-// thread that uses it.  That case: 52 us a call (93 with the loop), bound by the issue rate: staging of x by every
-// column block, byte decode and the fp32 combination share it.
+// thread that uses it.  That case: 32 us a call (93 with the loop; 52 while every 256 columns staged x for themselves, with a
+// search for each octet's columns and a digit at a time, and codes were spread to bytes column by column: 1640 instructions
+// a warp and block of 128 columns).  Bound by the issue rate still.  512 columns share the staging, the columns are searched
+// once, the four digits of a value are one addition and one exclusive or, codes are taken out for four columns at once and
+// turned.  Other sizes, before and now: 1 row 33 and 21 us, 64 rows 190 and 103, 16384 x 28672 317 and 208, 1024 x 1024
+// 8.8 and 8.7.
+#include <algorithm>
+
 #include "cq_common.cuh"
 
 namespace {
 
-constexpr int F32_THREADS = 256;       // 8 warps, 32 output columns each
-constexpr int F32_COLS = 256;
-constexpr int F32_MAX_BLOCKS = 10;     // 128-column blocks a CTA stages
+constexpr int F32_THREADS = 512;       // 16 warps, 32 output columns each
+constexpr int F32_COLS = 512;
+constexpr int F32_MAX_BLOCKS = 16;     // 128-column blocks a CTA stages
+constexpr int F32_DIGITS = 0x808080;   // added to a value, then exclusive or: its bytes are signed digits
 
 struct F32Params {
   const float* x;
@@ -30,7 +37,7 @@ struct F32Params {
   const int32_t* idx;
   const float* sf;
   float* mul;
-  int M, K, N, C, G, Kc, n_blk, blk_per_part, n_parts, aligned_q, aligned_f;
+  int M, K, N, C, G, Kc, n_blk, blk_per_part, n_parts, cherry_parts, aligned_q, aligned_f;
 };
 
 __device__ __forceinline__ int f32_source_col(const F32Params& p, int kc) {
@@ -48,7 +55,13 @@ __device__ __forceinline__ float2 f32_pow2_pair(int e) {
   return make_float2(__int_as_float((a + 127) << 23), __int_as_float((b + 127) << 23));
 }
 
-__device__ __forceinline__ void imma(int (&d)[4], const uint32_t (&a)[4], uint2 b) {
+template <bool FIRST> __device__ __forceinline__ void imma(int (&d)[4], const uint32_t (&a)[4], uint2 b) {
+  if (FIRST) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y), "r"(0));
+    return;
+  }
   asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.u8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
                : "+r"(d[0]), "+r"(d[1]), "+r"(d[2]), "+r"(d[3])
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b.x), "r"(b.y));
@@ -72,223 +85,210 @@ __device__ __forceinline__ void f32_load_codes(const F32Params& p, int o, int n,
   }
 }
 
-// TT = token tiles of 8 rows of x per sweep over the weights
-template <int TT>
-__global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Params p) {
+// four words with a byte of each of four columns -> a word of each column
+__device__ __forceinline__ void f32_turn(const uint32_t* r, uint32_t (&v)[4]) {
+  const uint32_t p0 = __byte_perm(r[0], r[1], 0x5140), p1 = __byte_perm(r[0], r[1], 0x7362);
+  const uint32_t p2 = __byte_perm(r[2], r[3], 0x5140), p3 = __byte_perm(r[2], r[3], 0x7362);
+  v[0] = __byte_perm(p0, p2, 0x5410);
+  v[1] = __byte_perm(p0, p2, 0x7632);
+  v[2] = __byte_perm(p1, p3, 0x5410);
+  v[3] = __byte_perm(p1, p3, 0x7632);
+}
+
+// The plain sum of column n over octets o0 .. o1 of row m, whose columns are at source[0 ..]: where an activation among
+// them is infinite or NaN.
+__device__ __noinline__ float f32_plain_sum(const F32Params& p, int n, int m, int o0, int o1, const int* source) {
+  float part = 0.f;
+  for (int o = o0; o < o1 && 8 * o < p.Kc; ++o, source += 8) {
+    const uint8_t* src = p.q + (size_t)o * 3 * p.N + n;
+    const uint32_t w = src[0] | ((uint32_t)src[p.N] << 8) | ((uint32_t)src[2 * (size_t)p.N] << 16);
+#pragma unroll
+    for (int b = 0; b < 8; ++b) part += ((float)((w >> (3 * b)) & 7u) - 3.5f) * p.x[(size_t)m * p.K + source[b]];
+  }
+  return part;
+}
+
+// TT = token tiles of 8 rows of x per sweep over the weights, HALVES = scale groups of a 128-column block (2: G = 64)
+template <int TT, int HALVES>
+__global__ void __launch_bounds__(F32_THREADS, 1) matvec_f32_kernel(const __grid_constant__ F32Params p) {
   constexpr int TOK = 8 * TT, NTILE = 4 * TT;
   extern __shared__ __align__(16) uint8_t smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int n_cta = blockIdx.y * F32_COLS;
-
-  if ((int)blockIdx.x >= p.n_parts) {
-    // cherry columns: one output column per thread
-    float* xs = reinterpret_cast<float*>(smem);             // [64 cherry columns][TOK]
-    const int n = n_cta + tid;
-    for (int m0 = 0; m0 < p.M; m0 += TOK) {
-      float acc[TOK];
-#pragma unroll
-      for (int t = 0; t < TOK; ++t) acc[t] = 0.f;
-      for (int c0 = 0; c0 < p.C; c0 += 64) {
-        const int len = min(64, p.C - c0);
-        __syncthreads();
-        for (int i = tid; i < len * TOK; i += F32_THREADS) {
-          const int t = i / len, c = i - t * len;
-          xs[c * TOK + t] = m0 + t < p.M ? p.x[(size_t)(m0 + t) * p.K + p.idx[c0 + c]] : 0.f;
-        }
-        __syncthreads();
-        if (n < p.N)
-          for (int c = 0; c < len; ++c) {
-            const float wv = __ldg(p.cw + (size_t)(c0 + c) * p.N + n);
-#pragma unroll
-            for (int t = 0; t < TOK; ++t) acc[t] += wv * xs[c * TOK + t];
-          }
-      }
-      if (n < p.N) {
-#pragma unroll
-        for (int t = 0; t < TOK; ++t)
-          if (m0 + t < p.M) atomicAdd(p.mul + (size_t)(m0 + t) * p.N + n, acc[t]);
-      }
-    }
-    return;
-  }
-
   const int b0 = blockIdx.x * p.blk_per_part, nb = min(p.blk_per_part, p.n_blk - b0);
-  // [block][chunk of 32 columns][plane][token tile][lane][8 B], then per block and token: step factors, sums, flags
+  // [block][chunk of 32 columns][plane][token tile][lane][8 B]
   uint2* planes = reinterpret_cast<uint2*>(smem);
-  float2* step = reinterpret_cast<float2*>(smem + (size_t)p.blk_per_part * 4 * NTILE * 256);    // [block][2 halves][TOK]
-  int2* qsum = reinterpret_cast<int2*>(step + p.blk_per_part * 2 * TOK);                        // the same
-  int* bad = reinterpret_cast<int*>(qsum + p.blk_per_part * 2 * TOK);                           // the same
-  const int halves = p.G == 64 ? 2 : 1;
+  // per block, half and token: -7 times the sums of the upper and lower two digits, half the first step factor, the second
+  // (a first factor of 0: an activation is not finite)
+  int4* meta = reinterpret_cast<int4*>(smem + (size_t)p.blk_per_part * 4 * NTILE * 256);
+  int* source = reinterpret_cast<int*>(meta + p.blk_per_part * HALVES * TOK);                   // [block][128]
+  int* bad = source + p.blk_per_part * 128;                                                     // [block]
   const int g = lane >> 2, c = lane & 3;
   const int n = n_cta + warp * 32 + 4 * g;                  // this thread's four columns
 
+  for (int i = tid; i < nb * 128; i += F32_THREADS) source[i] = b0 * 128 + i < p.Kc ? f32_source_col(p, b0 * 128 + i) : 0;
+
   for (int m0 = 0; m0 < p.M; m0 += TOK) {
+    if (tid < nb) bad[tid] = 0;
     __syncthreads();
+    uint32_t nxt[4][3];
+#pragma unroll
+    for (int ch = 0; ch < 4; ++ch) f32_load_codes(p, b0 * 16 + ch * 4 + c, n, nxt[ch]);
     // ---- staging: a half-warp per (token, block), a lane per octet
     const int l16 = lane & 15;
-    for (int it = warp * 2 + (lane >> 4); it < ((nb * TOK + 15) & ~15); it += F32_THREADS / 16) {
+    for (int it = warp * 2 + (lane >> 4); it < ((nb * TOK + 1) & ~1); it += F32_THREADS / 16) {
       const int j = it / TOK, t = it - j * TOK;
       const bool live = it < nb * TOK;
-      const int kc = (b0 + j) * 128 + 8 * l16;
       float v[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) v[e] = 0.f;
-      if (live && m0 + t < p.M && kc < p.Kc) {
+      if (live && m0 + t < p.M && (b0 + j) * 128 + 8 * l16 < p.Kc) {
         const float* xr = p.x + (size_t)(m0 + t) * p.K;
-        int low = f32_source_col(p, kc) - kc;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          while (low < p.C && p.idx[low] - low <= kc + e) ++low;
-          v[e] = __ldg(xr + kc + e + low);
-        }
+        const int4* at = reinterpret_cast<const int4*>(source + j * 128 + 8 * l16);
+        const int4 s0 = at[0], s1 = at[1];
+        v[0] = __ldg(xr + s0.x); v[1] = __ldg(xr + s0.y); v[2] = __ldg(xr + s0.z); v[3] = __ldg(xr + s0.w);
+        v[4] = __ldg(xr + s1.x); v[5] = __ldg(xr + s1.y); v[6] = __ldg(xr + s1.z); v[7] = __ldg(xr + s1.w);
       }
       uint32_t mx = 0;
 #pragma unroll
       for (int e = 0; e < 8; ++e) mx = max(mx, __float_as_uint(v[e]) & 0x7FFFFFFFu);
 #pragma unroll
-      for (int d = 4; d; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
-      const uint32_t mx2 = max(mx, __shfl_xor_sync(0xffffffffu, mx, 8));
-      if (halves == 1) mx = mx2;                            // one step for the block, or one for each of its two groups
+      for (int d = 8 / HALVES; d; d >>= 1) mx = max(mx, __shfl_xor_sync(0xffffffffu, mx, d));
       const bool finite = mx < 0x7F800000u;
       // power of two at the largest value (subnormals count as 2^-126), less 29
       const int e2 = max((int)(mx >> 23), 1) - 127 - 29;
       const float2 up = f32_pow2_pair(-e2);
-      int qv[8], hi = 0, lo = 0;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) qv[e] = finite ? __float2int_rn(v[e] * up.x * up.y) : 0;
-      uint32_t pl[4][2] = {};
+      // |value| <= 2^30: four signed digits, the bytes of (value + F32_DIGITS) ^ F32_DIGITS
+      uint32_t r[8];
+      int hi = 0, lo = 0;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
-        int r = qv[e];
-        int d[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-          d[k] = k < 3 ? (int)(signed char)(r & 0xFF) : r;
-          r = (r - d[k]) >> 8;
-          pl[k][e >> 2] |= (uint32_t)(d[k] & 0xFF) << (8 * (e & 3));
-        }
-        hi += d[3] * 256 + d[2];
-        lo += d[1] * 256 + d[0];
+        r[e] = (uint32_t)((finite ? __float2int_rn(v[e] * up.x * up.y) : 0) + F32_DIGITS);
+        hi += (int)r[e] >> 16;
+        lo += (int)(r[e] & 0xFFFFu);
+        r[e] ^= (uint32_t)F32_DIGITS;
       }
+      hi -= 8 * (F32_DIGITS >> 16);
+      lo -= 8 * (F32_DIGITS & 0xFFFF);
 #pragma unroll
-      for (int d = 4; d; d >>= 1) {
+      for (int d = 8 / HALVES; d; d >>= 1) {
         hi += __shfl_xor_sync(0xffffffffu, hi, d);
         lo += __shfl_xor_sync(0xffffffffu, lo, d);
       }
       if (live) {
+        uint32_t pl[2][4];
+        f32_turn(r, pl[0]);
+        f32_turn(r + 4, pl[1]);
         const int ch = l16 >> 2, dst = 4 * (t & 7) + (l16 & 3);
 #pragma unroll
         for (int k = 0; k < 4; ++k)
-          planes[((size_t)(j * 4 + ch) * NTILE + k * TT + (t >> 3)) * 32 + dst] = make_uint2(pl[k][0], pl[k][1]);
-        if ((l16 & 7) == 0) {
-          const int at = (j * 2 + (l16 >> 3)) * TOK + t;
-          qsum[at] = make_int2(hi, lo);
-          step[at] = f32_pow2_pair(e2);
-          bad[at] = finite ? 0 : 1;
+          planes[((size_t)(j * 4 + ch) * NTILE + k * TT + (t >> 3)) * 32 + dst] = make_uint2(pl[0][k], pl[1][k]);
+        if ((l16 & (16 / HALVES - 1)) == 0) {
+          const float2 st = f32_pow2_pair(e2);
+          meta[(j * HALVES + (HALVES == 2 ? l16 >> 3 : 0)) * TOK + t] =
+              make_int4(-7 * hi, -7 * lo, finite ? __float_as_int(0.5f * st.x) : 0, __float_as_int(st.y));
+          if (!finite) bad[j] = 1;
         }
       }
     }
-    __syncthreads();
 
     float y[4][TT][2];                                      // [column][token tile][token 2c, 2c + 1]
 #pragma unroll
     for (int j = 0; j < 4; ++j)
 #pragma unroll
       for (int t = 0; t < TT; ++t) y[j][t][0] = y[j][t][1] = 0.f;
-    uint32_t nxt[4][3];
+    auto load4 = [&](const float* row, float (&f)[4]) {     // row[n .. n + 3], zero past the matrix
+      if (p.aligned_f) {
+        const float4 v = n < p.N ? __ldg(reinterpret_cast<const float4*>(row + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+        f[0] = v.x; f[1] = v.y; f[2] = v.z; f[3] = v.w;
+      } else {
 #pragma unroll
-    for (int ch = 0; ch < 4; ++ch) f32_load_codes(p, b0 * 16 + ch * 4 + c, n, nxt[ch]);
+        for (int i = 0; i < 4; ++i) f[i] = n + i < p.N ? __ldg(row + n + i) : 0.f;
+      }
+    };
+    // ---- this part's share of the cherry columns
+    const int share = (int)blockIdx.x - (int)gridDim.x + p.cherry_parts;
+    const int c_end = share < 0 ? 0 : (int)((long long)p.C * (share + 1) / p.cherry_parts);
+#pragma unroll 4
+    for (int ci = share < 0 ? 0 : (int)((long long)p.C * share / p.cherry_parts); ci < c_end; ++ci) {
+      const float* xr = p.x + p.idx[ci];
+      float w[4];
+      load4(p.cw + (size_t)ci * p.N, w);
+#pragma unroll
+      for (int t = 0; t < TT; ++t)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          const int m = m0 + 8 * t + 2 * c + e;
+          const float xv = m < p.M ? __ldg(xr + (size_t)m * p.K) : 0.f;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) y[i][t][e] = __fmaf_rn(w[i], xv, y[i][t][e]);
+        }
+    }
+    __syncthreads();
+
     for (int j = 0; j < nb; ++j) {
       int acc[2][NTILE][4];
+      float s[HALVES][4];
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int k = 0; k < NTILE; ++k)
-#pragma unroll
-          for (int e = 0; e < 4; ++e) acc[i][k][e] = 0;
+      for (int h = 0; h < HALVES; ++h) {
+        const int k = (b0 + j) * 128 + 64 * h;
+        if (k < p.Kc) load4(p.sf + (size_t)(k / p.G) * p.N, s[h]);
+        else s[h][0] = s[h][1] = s[h][2] = s[h][3] = 0.f;
+      }
 #pragma unroll
       for (int ch = 0; ch < 4; ++ch) {
-        uint32_t r[3] = {nxt[ch][0], nxt[ch][1], nxt[ch][2]};
+        // codes 0 .. 3 and 4 .. 7 of the octets of four columns
+        const uint32_t r0 = nxt[ch][0], r1 = nxt[ch][1], r2 = nxt[ch][2];
+        const uint32_t code[8] = {r0 & 0x07070707u, (r0 >> 3) & 0x07070707u, ((r0 >> 6) & 0x03030303u) | ((r1 << 2) & 0x04040404u),
+                                  (r1 >> 1) & 0x07070707u, (r1 >> 4) & 0x07070707u,
+                                  ((r1 >> 7) & 0x01010101u) | ((r2 << 1) & 0x06060606u), (r2 >> 2) & 0x07070707u, (r2 >> 5) & 0x07070707u};
+        uint32_t front[4], back[4];
+        f32_turn(code, front);
+        f32_turn(code + 4, back);
         if (j + 1 < nb) f32_load_codes(p, (b0 + j + 1) * 16 + ch * 4 + c, n, nxt[ch]);
-        uint32_t a[2][4];
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          // the 24 bits of column i's octet, codes 0..3 and 4..7 spread to bytes
-          const uint32_t two = __byte_perm(r[0], r[1], (uint32_t)i | ((uint32_t)(4 + i) << 4));
-          const uint32_t w = __byte_perm(two, r[2], 0x0010u | ((uint32_t)(4 + i) << 8) | 0x3000u);
-          a[i >> 1][i & 1] = (w & 0x7u) | ((w << 5) & 0x700u) | ((w << 10) & 0x70000u) | ((w << 15) & 0x7000000u);
-          a[i >> 1][2 + (i & 1)] = ((w >> 12) & 0x7u) | ((w >> 7) & 0x700u) | ((w >> 2) & 0x70000u) | ((w << 3) & 0x7000000u);
-        }
+        const uint32_t a[2][4] = {{front[0], front[1], back[0], back[1]}, {front[2], front[3], back[2], back[3]}};
 #pragma unroll
         for (int k = 0; k < NTILE; ++k) {
           const uint2 b = planes[((size_t)(j * 4 + ch) * NTILE + k) * 32 + lane];
-          imma(acc[0][k], a[0], b);
-          imma(acc[1][k], a[1], b);
-        }
-        if (ch == 3 || (ch == 1 && halves == 2)) {
-          // end of a scale group (or of the block): exact integer sums -> fp32
-          const int grp = ((b0 + j) * 128 + (halves == 2 ? 64 * (ch >> 1) : 0)) / p.G;
-          float s[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) s[i] = 0.f;
-          if ((size_t)grp * p.G < (size_t)p.Kc) {
-            const float* sp = p.sf + (size_t)grp * p.N + n;
-            if (p.aligned_f && n < p.N) {
-              const float4 f = __ldg(reinterpret_cast<const float4*>(sp));
-              s[0] = f.x; s[1] = f.y; s[2] = f.z; s[3] = f.w;
-            } else {
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (n + i < p.N) s[i] = __ldg(sp + i);
-            }
+          for (int i = 0; i < 2; ++i) {
+            if (ch % (4 / HALVES) == 0) imma<true>(acc[i][k], a[i], b);
+            else imma<false>(acc[i][k], a[i], b);
           }
+        }
+        if (ch % (4 / HALVES) == 4 / HALVES - 1) {
+          // end of a scale group (or of the block): exact integer sums -> fp32
+          constexpr int LAST = HALVES - 1;
+          const int h = ch == 3 ? LAST : 0;
 #pragma unroll
           for (int t = 0; t < TT; ++t)
 #pragma unroll
             for (int e = 0; e < 2; ++e) {
-              const int tok = 8 * t + 2 * c + e;
-              const int at = (j * 2 + (halves == 2 ? ch >> 1 : 0)) * TOK + tok;
-              int2 qs = qsum[at];
-              if (halves == 1) {
-                const int2 q2 = qsum[(j * 2 + 1) * TOK + tok];
-                qs.x += q2.x;
-                qs.y += q2.y;
-              }
-              const float2 st = step[at];
-              const float f1 = 0.5f * st.x;
+              const int4 mt = meta[(j * HALVES + h) * TOK + 8 * t + 2 * c + e];
 #pragma unroll
               for (int i = 0; i < 4; ++i) {
                 const int ei = 2 * (i & 1) + e;
-                const int hi = acc[i >> 1][3 * TT + t][ei] * 256 + acc[i >> 1][2 * TT + t][ei];
-                const int lo = acc[i >> 1][TT + t][ei] * 256 + acc[i >> 1][t][ei];
-                const float v = __fmaf_rn((float)(2 * hi - 7 * qs.x), 65536.f, (float)(2 * lo - 7 * qs.y));
-                y[i][t][e] += v * f1 * s[i] * st.y;
-              }
-              if (bad[at]) {
-                // an infinite or NaN activation among them: the plain sum over the group
-                const int o0 = (b0 + j) * 16 + (halves == 2 ? 8 * (ch >> 1) : 0), o1 = o0 + (halves == 2 ? 8 : 16);
-                for (int i = 0; i < 4; ++i) {
-                  if (n + i >= p.N) break;
-                  float part = 0.f;
-                  for (int o = o0; o < o1 && 8 * o < p.Kc; ++o) {
-                    const uint8_t* src = p.q + (size_t)o * 3 * p.N + n + i;
-                    const uint32_t w = src[0] | ((uint32_t)src[p.N] << 8) | ((uint32_t)src[2 * (size_t)p.N] << 16);
-                    for (int b = 0; b < 8; ++b)
-                      part += ((float)((w >> (3 * b)) & 7u) - 3.5f) * p.x[(size_t)(m0 + tok) * p.K + f32_source_col(p, 8 * o + b)];
-                  }
-                  y[i][t][e] += s[i] * part;
-                }
+                const int hi = acc[i >> 1][3 * TT + t][ei] * 512 + (acc[i >> 1][2 * TT + t][ei] * 2 + mt.x);
+                const int lo = acc[i >> 1][TT + t][ei] * 512 + (acc[i >> 1][t][ei] * 2 + mt.y);
+                const float v = __fmaf_rn((float)hi, 65536.f, (float)lo);
+                y[i][t][e] += v * __int_as_float(mt.z) * s[h][i] * __int_as_float(mt.w);
               }
             }
-          if (halves == 2 && ch == 1) {
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-#pragma unroll
-              for (int k = 0; k < NTILE; ++k)
-#pragma unroll
-                for (int e = 0; e < 4; ++e) acc[i][k][e] = 0;
-          }
         }
+      }
+      if (bad[j]) {
+#pragma unroll
+        for (int h = 0; h < HALVES; ++h)
+#pragma unroll
+          for (int t = 0; t < TT; ++t)
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int tok = 8 * t + 2 * c + e, o = (b0 + j) * 16 + 8 * h;
+              if (meta[(j * HALVES + h) * TOK + tok].z != 0) continue;
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (n + i < p.N) y[i][t][e] += s[h][i] * f32_plain_sum(p, n + i, m0 + tok, o, o + 16 / HALVES, source + j * 128 + 64 * h);
+            }
       }
     }
 #pragma unroll
@@ -307,6 +307,7 @@ __global__ void __launch_bounds__(F32_THREADS, 2) matvec_f32_kernel(const F32Par
           }
         }
       }
+    __syncthreads();
   }
 }
 
@@ -319,14 +320,14 @@ int cq_launch_matvec_f32(const float* x, const uint8_t* q, const float* cw, cons
   p.x = x; p.q = q; p.cw = cw; p.idx = idx; p.sf = sf; p.mul = mul;
   p.M = M; p.K = K; p.N = N; p.C = C; p.G = G; p.Kc = K - C;
   p.n_blk = (p.Kc + 127) / 128;
-  // Blocks per CTA: the split whose waves of two CTAs per SM take the fewest block times (a CTA's fixed part, x staging
-  // set-up and the atomics, counts as one).  4096 x 13824, 16 rows: 8 blocks, one wave of 270.
+  // Blocks per CTA: the split whose waves of a CTA per SM take the fewest block times (a CTA's fixed part, x staging
+  // set-up and the atomics, counts as one).  4096 x 13824, 16 rows: 7 blocks, one wave of 135.
   const int ny = (N + F32_COLS - 1) / F32_COLS;
-  const int slots = 2 * cq_sm_count();
+  const int slots = cq_sm_count();
   int per = 1;
   long long best = 0;
   for (int b = 1; b <= F32_MAX_BLOCKS; ++b) {
-    const long long ctas = (long long)ny * ((p.n_blk + b - 1) / b + (C > 0 ? 1 : 0));
+    const long long ctas = (long long)ny * ((p.n_blk + b - 1) / b);
     const long long t = (ctas + slots - 1) / slots * (b + 1);
     if (b == 1 || t < best) {
       best = t;
@@ -335,13 +336,18 @@ int cq_launch_matvec_f32(const float* x, const uint8_t* q, const float* cw, cons
   }
   p.blk_per_part = per;
   p.n_parts = (p.n_blk + per - 1) / per;
+  // Cherry columns (18 take a warp as long as a block): parts of their own where SMs are left, four columns each; else the
+  // last part, which may be shorter, or more of the last ones where they are many.  (In every part they cost each one more
+  // rounding: 3 % more error at 1024 x 1024.  All in the last part there: 10.9 us and 8.8.)
+  const int spare = C > 0 ? std::min(slots / ny - p.n_parts, (C + 3) / 4) : 0, extra = spare > 0 ? spare : 0;
+  p.cherry_parts = extra > 0 ? extra : (C <= 16 ? 1 : std::min(p.n_parts, C / per + 1));
   p.aligned_q = N % 4 == 0 && ((uintptr_t)q & 3) == 0;
-  p.aligned_f = N % 4 == 0 && ((uintptr_t)sf & 15) == 0 && ((uintptr_t)mul & 15) == 0;
-  const int tt = M > 8 ? 2 : 1;
-  const int smem_main = per * (4 * 4 * tt * 256 + 8 * tt * (16 + 16 + 8)), smem_cherry = 64 * 8 * tt * 4;
-  const int smem = smem_main > smem_cherry ? smem_main : smem_cherry;
-  const dim3 grid(p.n_parts + (C > 0 ? 1 : 0), ny);
-  auto kernel = tt == 2 ? matvec_f32_kernel<2> : matvec_f32_kernel<1>;
+  p.aligned_f = N % 4 == 0 && ((uintptr_t)sf & 15) == 0 && ((uintptr_t)cw & 15) == 0 && ((uintptr_t)mul & 15) == 0;
+  const int tt = M > 8 ? 2 : 1, halves = G == 64 ? 2 : 1;
+  const int smem = per * (4 * 4 * tt * 256 + halves * 8 * tt * 16 + 128 * 4 + 4);
+  const dim3 grid(p.n_parts + extra, ny);
+  auto kernel = tt == 2 ? (halves == 2 ? matvec_f32_kernel<2, 2> : matvec_f32_kernel<2, 1>)
+                        : (halves == 2 ? matvec_f32_kernel<1, 2> : matvec_f32_kernel<1, 1>);
   CQ_CUDA_TRY(cq_grant_smem((const void*)kernel, smem));
   kernel<<<grid, F32_THREADS, smem, st>>>(p);
   CQ_CUDA_TRY(cudaGetLastError());

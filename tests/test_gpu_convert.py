@@ -195,6 +195,13 @@ def test_fp32_operator(cabi, K, N, G, C, M):
     assert np.array_equal(np.isnan(y), np.isnan(ref))
 
 
+@pytest.mark.parametrize("K,N,G,C,M", [(2176, 20008, 64, 40, 3), (2176, 20008, 128, 8, 16), (1024, 516, 128, 8, 9)])
+def test_fp32_operator_of_wide_layers(cabi, K, N, G, C, M):
+    """Several blocks of 512 columns, the last one short; cherry columns shared by all parts of K, in the last one alone, and
+    in parts of their own.  Bound as in test_fp32_operator."""
+    test_fp32_operator(cabi, K, N, G, C, M)
+
+
 @pytest.mark.parametrize("K,N,C,M,ratio", [(1024, 264, 8, 9, 1e4), (2120, 40, 24, 3, 1e4), (1024, 264, 8, 17, 1e-5)])
 def test_fp32_operator_groups_of_unlike_magnitudes(cabi, K, N, C, M, ratio):
     """Groups of 64 columns whose activations are `ratio` times their neighbours' and whose scales as much smaller: the
