@@ -260,7 +260,11 @@ __device__ __forceinline__ void dequant3(uint32_t w0, uint32_t w1, uint32_t w2, 
 // [token group of 8][k half][token in group][8 fp16]; cherry items (16 cherry columns) first, then the granules
 // (128 compact columns = 8 steps).  A warp stages four octets of eight tokens (128 contiguous bytes per octet) and goes
 // on to the next GROUPS - 1 token groups with the same columns, all their loads in flight together.  An octet without a
-// cherry column inside is two aligned 16-byte loads and a shift by its position in them.
+// cherry column inside is two aligned 16-byte loads and a shift by its position in them; the others are loaded column by
+// column.  Bound by latency: where the columns are is found once, before the kernels before this one have finished (with a
+// search for each token of an octet with a cherry column, after the wait, a call of 16 rows of 4096 x 11008 took 18.6 us
+// instead of 17.1, 45 rows of 5120 x 5120 21.5 and 20.3).  Eight blocks an SM: with nine and ten, spilling registers at
+// ten, 2048 rows of 5120 x 5120 took 2 to 3 us longer.
 // Tokens past M are not written: the padding feeds accumulator columns that are never read back (each output
 // column depends on its own token only).  Also clears the arrival counters of the main kernel.
 // the eight halves that start `off` halves into the two vectors
@@ -275,7 +279,7 @@ __device__ __forceinline__ uint4 shift_halves(uint4 lo, uint4 hi, int off) {
                     __funnelshift_r(w[3], w[4], s));
 }
 template <int GROUPS>
-__global__ void __launch_bounds__(STAGE_THREADS, 10) prefill_stage_x_kernel(
+__global__ void __launch_bounds__(STAGE_THREADS, 8) prefill_stage_x_kernel(
     const __half* __restrict__ x, int ldx, int M, const uint32_t* __restrict__ osh, const uint16_t* __restrict__ cidx,
     int C, int Kc, int n_gran, int n_cher, uint8_t* __restrict__ xb, unsigned long long half_bytes, int NT,
     uint32_t* __restrict__ arrived, int n_arrived, int aligned16) {
@@ -284,67 +288,75 @@ __global__ void __launch_bounds__(STAGE_THREADS, 10) prefill_stage_x_kernel(
   const int lane = threadIdx.x & 31, HT = NT >> 1;
   const int oi = (blockIdx.x * (STAGE_THREADS / 32) + (threadIdx.x >> 5)) * 4 + (lane >> 3);
   const unsigned short* xs = reinterpret_cast<const unsigned short*>(x);
-  asm volatile("griddepcontrol.wait;" ::: "memory");
-  // where the octet's columns are
-  const bool cherry = oi < 2 * n_cher;
-  const int o = oi - 2 * n_cher, k0 = 8 * o;
-  int lo0 = 0, lo7 = 0;
-  bool empty = oi >= n_oct;
-  size_t dst0;
-  if (cherry) {
-    dst0 = (size_t)(oi >> 1) * b_kstep_bytes(NT) + (oi & 1) * 128;
-  } else {
-    dst0 = (size_t)n_cher * b_kstep_bytes(NT) + (size_t)(o >> 4) * b_gran_bytes(NT) + ((o & 15) >> 1) * b_kstep_bytes(NT) + (o & 1) * 128;
-    const uint32_t sh = empty ? 0xFFFFFFFFu : osh[o];
-    empty = sh == 0xFFFFFFFFu;
-    lo0 = (int)(sh & 0xFFFFu);
-    lo7 = (int)(sh >> 16);
+  // Where the octet's columns are (weights: no need to wait for the kernels before): a lane finds one of the eight.  (Shared
+  // memory would keep the block from an SM that has a CTA of the main kernel.)
+  constexpr uint32_t NONE = 0xFFFFu;
+  uint32_t col = NONE;
+  {
+    const int oc = oi - 2 * n_cher, k = 8 * oc + (lane & 7);
+    if (oc < 0) {
+      if (k + 16 * n_cher < C) col = cidx[k + 16 * n_cher];
+    } else if (k < Kc) {
+      const uint32_t sh = osh[oc];
+      if (sh != 0xFFFFFFFFu) {
+        // cherry columns inside the octet: the shift grows from the first column's to the last one's
+        int sft = (int)(sh & 0xFFFFu);
+        while (sft < (int)(sh >> 16) && (int)cidx[sft] - sft <= k) ++sft;
+        col = (uint32_t)(k + sft);
+      }
+    }
   }
-  const bool plain = !cherry && !empty && lo0 == lo7 && aligned16;
-  const int c0 = k0 + lo0, off = c0 & 7;
+  const int c0 = (int)__shfl_sync(0xffffffffu, col, lane & 24), c7 = (int)__shfl_sync(0xffffffffu, col, lane | 7), off = c0 & 7;
+  const bool cherry = oi < 2 * n_cher;
+  const int o = oi - 2 * n_cher;
+  const size_t dst0 = cherry ? (size_t)(oi >> 1) * b_kstep_bytes(NT) + (oi & 1) * 128
+                             : (size_t)n_cher * b_kstep_bytes(NT) + (size_t)(o >> 4) * b_gran_bytes(NT) +
+                                   ((o & 15) >> 1) * b_kstep_bytes(NT) + (o & 1) * 128;
+  const bool plain = !cherry && c7 != (int)NONE && c7 == c0 + 7 && aligned16;      // (the same for an octet's eight lanes)
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   if (blockIdx.x == 0 && blockIdx.y == 0)
     for (int i = threadIdx.x; i < n_arrived; i += STAGE_THREADS) arrived[i] = 0u;
   if (oi >= n_oct) return;
+  auto store = [&](int m, uint4 v) {
+    const int mb = m / NT, ml = m - mb * NT, hf = ml >= HT, mt = ml - hf * HT;
+    *reinterpret_cast<uint4*>(xb + (size_t)(2 * mb + hf) * half_bytes + dst0 + (mt >> 3) * 256 + (mt & 7) * 16) = v;
+  };
   for (int tg0 = blockIdx.y * GROUPS; tg0 < (M + 7) >> 3; tg0 += gridDim.y * GROUPS) {
-    uint4 v[GROUPS], v2[GROUPS];
+    const int m0 = tg0 * 8 + (lane & 7);
+    if (plain) {
+      uint4 v[GROUPS], v2[GROUPS];
 #pragma unroll
-    for (int u = 0; u < GROUPS; ++u) {
-      const int m = (tg0 + u) * 8 + (lane & 7);
-      v[u] = v2[u] = make_uint4(0, 0, 0, 0);
-      if (plain && m < M) {
-        // (K is a multiple of 8 and all eight columns exist: the second vector, where needed, lies inside the row)
-        const uint4* src = reinterpret_cast<const uint4*>(xs + (size_t)m * ldx + (c0 - off));
-        v[u] = __ldg(src);
-        if (off) v2[u] = __ldg(src + 1);
-      }
-    }
-#pragma unroll
-    for (int u = 0; u < GROUPS; ++u) {
-      const int m = (tg0 + u) * 8 + (lane & 7);
-      if (m >= M) break;
-      if (plain) {
-        v[u] = shift_halves(v[u], v2[u], off);
-      } else if (!empty) {
-        const unsigned short* xr = xs + (size_t)m * ldx;
-        unsigned short h[8];
-        int sft = lo0;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-          h[e] = 0;
-          if (cherry) {
-            const int c = 8 * oi + e;
-            if (c < C) h[e] = __ldg(xr + cidx[c]);
-          } else {
-            // cherry columns inside the octet: the shift grows from lo0 to lo7 along it
-            while (sft < lo7 && (int)cidx[sft] - sft <= k0 + e) ++sft;
-            if (k0 + e < Kc) h[e] = __ldg(xr + k0 + e + sft);
-          }
+      for (int u = 0; u < GROUPS; ++u) {
+        const int m = m0 + 8 * u;
+        v[u] = v2[u] = make_uint4(0, 0, 0, 0);
+        if (m < M) {
+          // (K is a multiple of 8 and all eight columns exist: the second vector, where needed, lies inside the row)
+          const uint4* src = reinterpret_cast<const uint4*>(xs + (size_t)m * ldx + (c0 - off));
+          v[u] = __ldg(src);
+          if (off) v2[u] = __ldg(src + 1);
         }
-        v[u] = make_uint4((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16),
-                          (uint32_t)h[4] | ((uint32_t)h[5] << 16), (uint32_t)h[6] | ((uint32_t)h[7] << 16));
       }
-      const int mb = m / NT, ml = m - mb * NT, hf = ml >= HT, mt = ml - hf * HT;
-      *reinterpret_cast<uint4*>(xb + (size_t)(2 * mb + hf) * half_bytes + dst0 + (mt >> 3) * 256 + (mt & 7) * 16) = v[u];
+#pragma unroll
+      for (int u = 0; u < GROUPS; ++u)
+        if (m0 + 8 * u < M) store(m0 + 8 * u, shift_halves(v[u], v2[u], off));
+    } else {
+#pragma unroll 1
+      for (int u = 0; u < GROUPS; u += 2) {
+        uint32_t h[2][8];
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) {
+            const int m = m0 + 8 * (u + i);
+            const uint32_t ce = __shfl_sync(0xFFu << (lane & 24), col, (lane & 24) + e);
+            h[i][e] = u + i < GROUPS && m < M && ce != NONE ? __ldg(xs + (size_t)m * ldx + ce) : 0u;
+          }
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+          if (u + i < GROUPS && m0 + 8 * (u + i) < M)
+            store(m0 + 8 * (u + i), make_uint4(h[i][0] | (h[i][1] << 16), h[i][2] | (h[i][3] << 16), h[i][4] | (h[i][5] << 16),
+                                               h[i][6] | (h[i][7] << 16)));
+      }
     }
   }
 }
