@@ -18,7 +18,7 @@ SYMBOLS = [
     "cq_cache_clear", "cq_cache_stats", "cq_cache_evict", "cq_poll",
     "cq_pack_tmp_bytes", "cq_pack", "cq_unpack_dense", "cq_fake_quant",
     "cq_tlayer_init", "cq_tlayer_prepare", "cq_tlayer_unprepare",
-    "cq_layer_matvec_static", "cq_tlayer_gemm_workspace_bytes", "cq_tlayer_gemm",
+    "cq_layer_matvec_static", "cq_tlayer_gemm_workspace_bytes", "cq_tlayer_gemm", "cq_tlayers_gemm_workspace_bytes", "cq_tlayers_gemm",
     "cq_selftest_bounded_wait", "cq_rmsnorm", "cq_rope_cache", "cq_silu_mul", "cq_silu_mul_full", "cq_attn_decode", "cq_attn_decode_step", "cq_attn_decode_workspace_bytes",
     "cq_peer_region_bytes", "cq_peer_region_create", "cq_peer_region_destroy", "cq_peer_region_export",
     "cq_peer_region_open", "cq_peer_region_close", "cq_peer_allgather",
@@ -86,6 +86,9 @@ def lib():
     L.cq_tlayer_gemm.argtypes = [C.POINTER(cq_tlayer), vp, i32, vp, i32, i32, i32, vp, vp, vp]
     L.cq_tlayer_gemm_workspace_bytes.argtypes = [C.POINTER(cq_tlayer), i32]
     L.cq_tlayer_gemm_workspace_bytes.restype = C.c_size_t
+    L.cq_tlayers_gemm.argtypes = [C.POINTER(C.POINTER(cq_tlayer)), i32, vp, i32, C.POINTER(vp), C.POINTER(i32), i32, i32, vp, vp, vp]
+    L.cq_tlayers_gemm_workspace_bytes.argtypes = [C.POINTER(cq_tlayer), i32, i32]
+    L.cq_tlayers_gemm_workspace_bytes.restype = C.c_size_t
     L.cq_vecquant4matmul_cherryq.argtypes = [vp] * 6 + [i32] * 6 + [u64, vp]
     L.cq_vecquant3matmul_cherryq.argtypes = [vp] * 6 + [i32] * 7 + [u64, vp]
     L.cq_dequantize3_normal.argtypes = [vp, vp, vp] + [i32] * 5 + [vp]

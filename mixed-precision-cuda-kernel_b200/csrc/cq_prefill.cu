@@ -45,6 +45,7 @@
 // 365 that its weights need to arrive from HBM.  (54 us while every decode warp walked over all items, polled without a
 // hint and took every fourth; the hint without the stepping was slower, 61.  With six groups, or with lone CTAs that leave
 // room for seven A slots, it was no faster.)
+#include <algorithm>
 #include <cmath>
 
 #include "cq_tile.cuh"
@@ -69,19 +70,31 @@ constexpr int N_BARS = 2 * SW_MAX + 2 * SB_MAX + 2 * NA + 4;
 __host__ __device__ constexpr int b_kstep_bytes(int nt) { return nt * 16; }
 __host__ __device__ constexpr int b_gran_bytes(int nt) { return nt * 128; }
 
-struct PrefillParams {
+constexpr int MAX_LAYERS = 4;           // layers of one launch, which share an input
+
+struct PrefillLayer {
   const uint8_t* stream;     // tile-layout weight stream
   const uint8_t* xb;         // staged activations: [token block][half][cherry items][granules]
   __half* y;
-  uint32_t* status;
-  int M, N, n_gran, n_tile, n_cher, gran_bytes, tile_bytes, ldy, accumulate, vec_y;
-  int nt;                    // tokens per block
-  uint32_t n_units;          // token blocks x pairs of row tiles
-  uint32_t sk_units, sk_clusters;   // the first sk_units units are cut into runs of items for sk_clusters clusters
-  unsigned long long xb_half_bytes;
-  int wstage_bytes, sw, sb, off_wring, off_bring, off_stage, off_bar;   // sw, sb = ring stages
   float* partial;            // [cluster][first / last run][CTA of the pair][token][128 rows] fp32
   uint32_t* arrived;         // [cut unit][CTA of the pair] runs finished so far
+  int N, n_tile, ldy;
+  uint32_t n_units;          // token blocks x pairs of row tiles
+  uint32_t sk_units, sk_clusters;   // the first sk_units units are cut into runs of items for sk_clusters clusters
+};
+struct PrefillParams {
+  PrefillLayer layer[MAX_LAYERS];
+  uint32_t* status;
+  int n_layers, M, n_gran, n_cher, gran_bytes, tile_bytes, accumulate, vec_y;
+  int nt;                    // tokens per block
+  unsigned long long xb_half_bytes;
+  int wstage_bytes, sw, sb, off_wring, off_bring, off_stage, off_bar;   // sw, sb = ring stages
+};
+// what the pre-pass needs of each layer
+struct StageLayers {
+  const uint32_t* osh[MAX_LAYERS];
+  const uint16_t* cidx[MAX_LAYERS];
+  uint8_t* xb[MAX_LAYERS];
 };
 
 // ------------------------------------------------------------------ PTX helpers
@@ -280,14 +293,16 @@ __device__ __forceinline__ uint4 shift_halves(uint4 lo, uint4 hi, int off) {
 }
 template <int GROUPS>
 __global__ void __launch_bounds__(STAGE_THREADS, 8) prefill_stage_x_kernel(
-    const __half* __restrict__ x, int ldx, int M, const uint32_t* __restrict__ osh, const uint16_t* __restrict__ cidx,
-    int C, int Kc, int n_gran, int n_cher, uint8_t* __restrict__ xb, unsigned long long half_bytes, int NT,
-    uint32_t* __restrict__ arrived, int n_arrived, int aligned16) {
+    const __half* __restrict__ x, int ldx, int M, const __grid_constant__ StageLayers layers, int C, int Kc, int n_gran, int n_cher,
+    unsigned long long half_bytes, int NT, uint32_t* __restrict__ arrived, int n_arrived, int aligned16) {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int n_oct = 2 * n_cher + 16 * n_gran;              // octets per token
   const int lane = threadIdx.x & 31, HT = NT >> 1;
   const int oi = (blockIdx.x * (STAGE_THREADS / 32) + (threadIdx.x >> 5)) * 4 + (lane >> 3);
   const unsigned short* xs = reinterpret_cast<const unsigned short*>(x);
+  const uint32_t* __restrict__ osh = layers.osh[blockIdx.z];
+  const uint16_t* __restrict__ cidx = layers.cidx[blockIdx.z];
+  uint8_t* __restrict__ xb = layers.xb[blockIdx.z];
   // Where the octet's columns are (weights: no need to wait for the kernels before): a lane finds one of the eight.  (Shared
   // memory would keep the block from an SM that has a CTA of the main kernel.)
   constexpr uint32_t NONE = 0xFFFFu;
@@ -314,7 +329,7 @@ __global__ void __launch_bounds__(STAGE_THREADS, 8) prefill_stage_x_kernel(
                                    ((o & 15) >> 1) * b_kstep_bytes(NT) + (o & 1) * 128;
   const bool plain = !cherry && c7 != (int)NONE && c7 == c0 + 7 && aligned16;      // (the same for an octet's eight lanes)
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (blockIdx.x == 0 && blockIdx.y == 0)
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0)
     for (int i = threadIdx.x; i < n_arrived; i += STAGE_THREADS) arrived[i] = 0u;
   if (oi >= n_oct) return;
   auto store = [&](int m, uint4 v) {
@@ -363,39 +378,56 @@ __global__ void __launch_bounds__(STAGE_THREADS, 8) prefill_stage_x_kernel(
 
 // ------------------------------------------------------------------ work list of a cluster
 struct Work {
-  uint32_t unit, j0, j1;     // items [j0, j1) of this unit
+  uint32_t layer, unit, j0, j1;     // items [j0, j1) of this unit of the layer
   int run;                   // -1: a whole unit; 0 / 1: the first / last run of this cluster, a part of its unit
 };
 // first item of cluster c's run over the cut units
-__device__ __forceinline__ uint32_t run_begin(const PrefillParams& p, uint32_t c, uint32_t total) {
-  return c * total / p.sk_clusters;        // (74 clusters x 73 units x a few thousand items at most: fits 32 bits)
+__device__ __forceinline__ uint32_t run_begin(const PrefillLayer& L, uint32_t c, uint32_t total) {
+  return c * total / L.sk_clusters;        // (74 clusters x 73 units x a few thousand items at most: fits 32 bits)
 }
-struct WorkList {
-  uint32_t b, e, b0, u, ipt, n_units, clusters;
-  __device__ __forceinline__ WorkList(const PrefillParams& p, uint32_t cluster, uint32_t n_clusters, uint32_t ipt_)
-      : b(0), e(0), b0(0), u(p.sk_units + cluster), ipt(ipt_), n_units(p.n_units), clusters(n_clusters) {
-    if (cluster < p.sk_clusters) {
-      const uint32_t total = p.sk_units * ipt;
-      b0 = b = run_begin(p, cluster, total);
-      e = run_begin(p, cluster + 1, total);
+// Layer by layer, each divided as in a launch of its own: the sums are the same, and while the last of a layer is stored the
+// next one's weights are on their way.  MANY: more than one layer (with the layer as a variable in launches of one, 45 rows of
+// 5120 x 13824 took 1 us longer).
+template <bool MANY> struct WorkList {
+  const PrefillParams& p;
+  uint32_t layer, b, e, b0, u, ipt, cluster, clusters;
+  __device__ __forceinline__ WorkList(const PrefillParams& p_, uint32_t cluster_, uint32_t n_clusters, uint32_t ipt_)
+      : p(p_), layer(0), ipt(ipt_), cluster(cluster_), clusters(n_clusters) {
+    begin();
+  }
+  __device__ __forceinline__ void begin() {
+    const PrefillLayer& L = p.layer[MANY ? layer : 0];
+    u = L.sk_units + cluster;
+    b = e = b0 = 0;
+    if (cluster < L.sk_clusters) {
+      const uint32_t total = L.sk_units * ipt;
+      b0 = b = run_begin(L, cluster, total);
+      e = run_begin(L, cluster + 1, total);
     }
   }
   __device__ __forceinline__ bool next(Work& w) {
-    if (b < e) {
-      w.unit = b / ipt;
-      w.j0 = b - w.unit * ipt;
-      w.j1 = min(ipt, w.j0 + (e - b));
-      w.run = (w.j0 == 0 && w.j1 == ipt) ? -1 : (b == b0 ? 0 : 1);
-      b += w.j1 - w.j0;
-      return true;
+    for (;;) {
+      w.layer = MANY ? layer : 0;
+      if (b < e) {
+        w.unit = b / ipt;
+        w.j0 = b - w.unit * ipt;
+        w.j1 = min(ipt, w.j0 + (e - b));
+        w.run = (w.j0 == 0 && w.j1 == ipt) ? -1 : (b == b0 ? 0 : 1);
+        b += w.j1 - w.j0;
+        return true;
+      }
+      if (u < p.layer[MANY ? layer : 0].n_units) {
+        w.unit = u;
+        w.j0 = 0;
+        w.j1 = ipt;
+        w.run = -1;
+        u += clusters;
+        return true;
+      }
+      if (!MANY || layer + 1 >= (uint32_t)p.n_layers) return false;
+      ++layer;
+      begin();
     }
-    if (u >= n_units) return false;
-    w.unit = u;
-    w.j0 = 0;
-    w.j1 = ipt;
-    w.run = -1;
-    u += clusters;
-    return true;
   }
 };
 
@@ -427,8 +459,8 @@ struct Ring {
 };
 
 // ------------------------------------------------------------------ main kernel
-template <int BITS, int SETS>
-__global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillParams p) {
+template <int BITS, int SETS, bool MANY>
+__global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const __grid_constant__ PrefillParams p) {
   constexpr int W_MMA = NGRP * 4, W_PROD_W = NGRP * 4 + 1, W_PROD_B = NGRP * 4 + 2;
   extern __shared__ __align__(128) uint8_t smem[];
   __shared__ int s_state;
@@ -442,7 +474,6 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
   const uint32_t NT = (uint32_t)p.nt;
   const uint32_t ND = NT <= 128 ? 2 : 1;                   // accumulator buffers of NT columns
   const uint32_t NCH = (uint32_t)p.n_cher, IPT = NCH + (uint32_t)p.n_gran;
-  const uint32_t NTILE = (uint32_t)p.n_tile, NPAIR = (NTILE + 1) / 2;
   const uint32_t SW = (uint32_t)p.sw, SB = (uint32_t)p.sb;
   const uint32_t B_KSTEP_BYTES = b_kstep_bytes(NT), B_GRAN_BYTES = b_gran_bytes(NT), B_CHER_BYTES = B_KSTEP_BYTES;
 
@@ -487,13 +518,15 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     if (lane == 0) {
       const uint32_t wring = smem_u32(smem + p.off_wring);
       Ring ring;
-      WorkList wl(p, cluster, n_clusters, IPT);
+      WorkList<MANY> wl(p, cluster, n_clusters, IPT);
       Work w;
       while (wl.next(w)) {
         // (an odd number of row tiles: the last pair's second CTA repeats the last tile, its results are dropped)
+        const PrefillLayer& L = p.layer[MANY ? w.layer : 0];
+        const uint32_t NTILE = (uint32_t)L.n_tile, NPAIR = (NTILE + 1) / 2;
         const uint32_t tile = min(2 * (w.unit % NPAIR) + rank, NTILE - 1);
         const uint32_t c0 = min(w.j0, NCH);
-        const uint8_t* src = p.stream + (size_t)tile * p.tile_bytes + (size_t)c0 * CQT_CHER_BYTES + (size_t)(w.j0 - c0) * p.gran_bytes;
+        const uint8_t* src = L.stream + (size_t)tile * p.tile_bytes + (size_t)c0 * CQT_CHER_BYTES + (size_t)(w.j0 - c0) * p.gran_bytes;
         for (uint32_t j = w.j0; j < w.j1; ++j) {
           const uint32_t bytes = j < NCH ? (uint32_t)CQT_CHER_BYTES : (uint32_t)p.gran_bytes;
           if (ring.round) mbar_wait(B_WEMPTY(ring.slot), ring.phase ^ 1, &s_state, p.status, 1u);
@@ -516,13 +549,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
       atomicCAS(&s_state, PENDING, RUNNING);
       const uint32_t bring = smem_u32(smem + p.off_bring);
       Ring ring;
-      WorkList wl(p, cluster, n_clusters, IPT);
+      WorkList<MANY> wl(p, cluster, n_clusters, IPT);
       Work w;
       while (wl.next(w)) {
-        const uint32_t mb = w.unit / NPAIR;
+        const PrefillLayer& L = p.layer[MANY ? w.layer : 0];
+        const uint32_t mb = w.unit / (((uint32_t)L.n_tile + 1) / 2);
         const bool real = (int)(mb * NT + rank * (NT >> 1)) < p.M;       // this half of the block holds tokens
         const uint32_t c0 = min(w.j0, NCH);
-        const uint8_t* src = p.xb + (size_t)(2 * mb + rank) * p.xb_half_bytes + (size_t)c0 * B_CHER_BYTES +
+        const uint8_t* src = L.xb + (size_t)(2 * mb + rank) * p.xb_half_bytes + (size_t)c0 * B_CHER_BYTES +
                              (size_t)(w.j0 - c0) * B_GRAN_BYTES;
         for (uint32_t j = w.j0; j < w.j1; ++j) {
           const uint32_t bytes = j < NCH ? B_CHER_BYTES : B_GRAN_BYTES;
@@ -561,7 +595,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
       __syncwarp();
       uint32_t lu = 0;
       Ring rb, ra;
-      WorkList wl(p, cluster, n_clusters, IPT);
+      WorkList<MANY> wl(p, cluster, n_clusters, IPT);
       Work w;
       for (; wl.next(w); ++lu) {
         const uint32_t dbuf = lu % ND;
@@ -608,7 +642,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     Ring ring, rb;
     ring.slot = rb.slot = grp;
     const uint32_t ready = rank == 0 ? B_READY(a) : cluster_addr(B_READY(a), 0);
-    WorkList wl(p, cluster, n_clusters, IPT);
+    WorkList<MANY> wl(p, cluster, n_clusters, IPT);
     Work w;
     while (wl.next(w)) {
       const uint32_t first = w.j0 + (grp >= (int)n ? grp - n : grp + NGRP - n);
@@ -684,21 +718,23 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
     auto epi_sync = [&]() { asm volatile("bar.sync 2, 128;" ::: "memory"); };
     dependency_wait();
     uint32_t lu = 0;
-    WorkList wl(p, cluster, n_clusters, IPT);
+    WorkList<MANY> wl(p, cluster, n_clusters, IPT);
     Work w;
     for (; wl.next(w); ++lu) {
+      const PrefillLayer& L = p.layer[MANY ? w.layer : 0];
+      const uint32_t NPAIR = ((uint32_t)L.n_tile + 1) / 2;
       const uint32_t mb = w.unit / NPAIR, tile = 2 * (w.unit % NPAIR) + rank;
       const uint32_t dbuf = lu % ND;
       const uint32_t d_lu = tmem + lane_addr + D_BASE + dbuf * NT;
       const int tok0 = (int)(mb * NT), ntok = min((int)NT, p.M - tok0);
-      const int n0 = (int)tile * 128, nrows = min(128, p.N - n0);       // <= 0: the repeated tile of an odd pair
+      const int n0 = (int)tile * 128, nrows = min(128, L.N - n0);       // <= 0: the repeated tile of an odd pair
       if (w.run < 0) {
         if (p.accumulate && nrows > 0) {
           // the old outputs into the staging area while the MMAs run
           for (int i = etid; i < ntok * 16; i += 128) {
             const int t = i >> 4, r8 = (i & 15) * 8;
             if (r8 < nrows) {
-              const __half* yp = p.y + (size_t)(tok0 + t) * p.ldy + n0 + r8;
+              const __half* yp = L.y + (size_t)(tok0 + t) * L.ldy + n0 + r8;
               if (p.vec_y) {
                 *reinterpret_cast<uint4*>(stage + t * 128 + r8) = *reinterpret_cast<const uint4*>(yp);
               } else {
@@ -734,7 +770,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         for (int i = etid; i < ntok * 16; i += 128) {
           const int t = i >> 4, r8 = (i & 15) * 8;
           if (r8 < nrows) {
-            __half* yp = p.y + (size_t)(tok0 + t) * p.ldy + n0 + r8;
+            __half* yp = L.y + (size_t)(tok0 + t) * L.ldy + n0 + r8;
             if (p.vec_y) {
               *reinterpret_cast<uint4*>(yp) = *reinterpret_cast<const uint4*>(stage + t * 128 + r8);
             } else {
@@ -748,7 +784,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         // a part of a unit: park the fp32 tile; the cluster that arrives last adds the parts in item order and
         // stores the outputs
         const size_t part_floats = (size_t)NT * 128;
-        float* mine = p.partial + ((size_t)(cluster * 2 + w.run) * 2 + rank) * part_floats;
+        float* mine = L.partial + ((size_t)(cluster * 2 + w.run) * 2 + rank) * part_floats;
         mbar_wait(B_DFULL(dbuf), (lu / ND) & 1, &s_state, p.status, 128u);
         tc_fence_after();
 #pragma unroll 1
@@ -764,18 +800,18 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
         __syncwarp();
         if (lane == 0) mbar_arrive_cluster(cluster_addr(B_DEMPTY(dbuf), 0));
         // clusters whose runs touch this unit
-        const uint32_t total = p.sk_units * IPT, i0 = w.unit * IPT;
-        const uint32_t c_first = ((i0 + 1) * p.sk_clusters - 1) / total, c_last = ((i0 + IPT) * p.sk_clusters - 1) / total;
+        const uint32_t total = L.sk_units * IPT, i0 = w.unit * IPT;
+        const uint32_t c_first = ((i0 + 1) * L.sk_clusters - 1) / total, c_last = ((i0 + IPT) * L.sk_clusters - 1) / total;
         __threadfence();
         epi_sync();
-        if (etid == 0) s_last = (atomicAdd(p.arrived + 2 * w.unit + rank, 1u) == c_last - c_first) ? 1 : 0;
+        if (etid == 0) s_last = (atomicAdd(L.arrived + 2 * w.unit + rank, 1u) == c_last - c_first) ? 1 : 0;
         epi_sync();
         if (s_last && nrows > 0) {
           __threadfence();
           // a warp takes every fourth token, a lane four rows of it, four tokens' loads in flight; only the first
           // cluster's run can have begun in an earlier unit (its part is then that cluster's last)
-          const uint32_t run0 = run_begin(p, c_first, total) >= i0 ? 0u : 1u;
-          const float4* parts = reinterpret_cast<const float4*>(p.partial + (size_t)(c_first * 4 + rank) * part_floats) + lane;
+          const uint32_t run0 = run_begin(L, c_first, total) >= i0 ? 0u : 1u;
+          const float4* parts = reinterpret_cast<const float4*>(L.partial + (size_t)(c_first * 4 + rank) * part_floats) + lane;
           const size_t part_step = part_floats;               // one cluster's four parts, in float4
           for (int t0 = ewarp; t0 < ntok; t0 += 16) {
             float4 sum[4];
@@ -804,7 +840,7 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const PrefillPa
               const float4 s = sum[u];
               if (t >= ntok) break;
               if (4 * lane < nrows) {
-                __half* yp = p.y + (size_t)(tok0 + t) * p.ldy + n0 + 4 * lane;
+                __half* yp = L.y + (size_t)(tok0 + t) * L.ldy + n0 + 4 * lane;
                 float r[4] = {s.x, s.y, s.z, s.w};
                 if (p.accumulate) {
 #pragma unroll
@@ -856,9 +892,9 @@ PDeviceInfo pdevice_info(int dev) {
 int palign_up(int v, int a) { return (v + a - 1) / a * a; }
 
 typedef void (*PKernelFn)(const PrefillParams);
-PKernelFn ppick(int bits, int sets) {
-  if (bits == 4) return sets == 1 ? cq_prefill_kernel<4, 1> : cq_prefill_kernel<4, 2>;
-  return sets == 1 ? cq_prefill_kernel<3, 1> : cq_prefill_kernel<3, 2>;
+template <bool MANY> PKernelFn ppick(int bits, int sets) {
+  if (bits == 4) return sets == 1 ? cq_prefill_kernel<4, 1, MANY> : cq_prefill_kernel<4, 2, MANY>;
+  return sets == 1 ? cq_prefill_kernel<3, 1, MANY> : cq_prefill_kernel<3, 2, MANY>;
 }
 
 size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
@@ -905,48 +941,75 @@ int pick_runs(uint32_t rem, uint32_t items, int nt, int clusters) {
 
 }  // namespace
 
-extern "C" size_t cq_tlayer_gemm_workspace_bytes(const cq_tlayer* L, int M) {
-  if (!L || M < 1) return 0;
+// Workspace of n layers: staged activations of each | partial tiles of each | arrival counters of each
+extern "C" size_t cq_tlayers_gemm_workspace_bytes(const cq_tlayer* L, int n_layers, int M) {
+  if (!L || M < 1 || n_layers < 1 || n_layers > MAX_LAYERS) return 0;
   int dev = 0;
   PDeviceInfo di;
   if (cudaGetDevice(&dev) == cudaSuccess) di = pdevice_info(dev);
   else (void)cudaGetLastError();
   const int clusters = (di.ok ? di.sms : 148) / 2;
-  return xb_bytes_for(L, M) + partial_bytes_for(M, clusters) + align256((size_t)clusters * 2 * sizeof(uint32_t));
+  return n_layers * (xb_bytes_for(L, M) + partial_bytes_for(M, clusters) + align256((size_t)clusters * 2 * sizeof(uint32_t)));
 }
+extern "C" size_t cq_tlayer_gemm_workspace_bytes(const cq_tlayer* L, int M) { return cq_tlayers_gemm_workspace_bytes(L, 1, M); }
 
 extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* y, int ldy, int M, int accumulate,
                               void* workspace, uint32_t* status_word, cq_stream_t stream) {
-  if (!L || !L->blob || !x || !y || !workspace) return CQ_ERR_BAD_ARG;
-  if (M < 1 || ldx < L->K || ldy < L->N) return CQ_ERR_BAD_ARG;
-  if (((uintptr_t)x & 1) || ((uintptr_t)y & 1) || ((uintptr_t)workspace & 127)) return CQ_ERR_BAD_ARG;
+  return cq_tlayers_gemm(&L, 1, x, ldx, &y, &ldy, M, accumulate, workspace, status_word, stream);
+}
+
+extern "C" int cq_tlayers_gemm(const cq_tlayer* const* layers, int n_layers, const void* x, int ldx, void* const* ys, const int* ldys,
+                               int M, int accumulate, void* workspace, uint32_t* status_word, cq_stream_t stream) {
+  if (!layers || n_layers < 1 || n_layers > MAX_LAYERS || !ys || !ldys || !x || !workspace) return CQ_ERR_BAD_ARG;
+  const cq_tlayer* L = layers[0];
+  if (!L || M < 1 || ldx < L->K || ((uintptr_t)x & 1) || ((uintptr_t)workspace & 127)) return CQ_ERR_BAD_ARG;
+  for (int i = 0; i < n_layers; ++i) {
+    const cq_tlayer* l = layers[i];
+    if (!l || !l->blob || !ys[i] || ldys[i] < l->N || ((uintptr_t)ys[i] & 1)) return CQ_ERR_BAD_ARG;
+    if (l->K != L->K || l->C != L->C || l->G != L->G || l->bits != L->bits) return CQ_ERR_BAD_SHAPE;
+  }
   int dev = 0;
   CQ_CUDA_TRY(cudaGetDevice(&dev));
   const PDeviceInfo di = pdevice_info(dev);
   if (!di.ok) return CQ_ERR_NO_DEVICE;
   cudaStream_t st = (cudaStream_t)stream;
-  const uint8_t* blob = (const uint8_t*)L->blob;
   const int NT = block_tokens(M), n_mblk = (M + NT - 1) / NT;
-  const int clusters = di.sms / 2, n_pair = (L->n_tile + 1) / 2;
+  const int clusters = di.sms / 2;
   const uint32_t items = (uint32_t)(L->n_cher + L->n_gran);
 
-  PrefillParams p;
-  p.stream = blob + L->off_stream;
-  p.xb = (const uint8_t*)workspace;
-  p.y = (__half*)y;
+  PrefillParams p = {};
+  StageLayers stage = {};
   p.status = status_word;
-  p.M = M; p.N = L->N; p.n_gran = L->n_gran; p.n_tile = L->n_tile; p.n_cher = L->n_cher;
-  p.gran_bytes = L->gran_bytes; p.tile_bytes = L->tile_bytes; p.ldy = ldy; p.accumulate = accumulate;
-  p.vec_y = ((uintptr_t)y & 15) == 0 && ldy % 8 == 0;
+  p.n_layers = n_layers;
+  p.M = M; p.n_gran = L->n_gran; p.n_cher = L->n_cher;
+  p.gran_bytes = L->gran_bytes; p.tile_bytes = L->tile_bytes; p.accumulate = accumulate;
+  p.vec_y = 1;
   p.nt = NT;
-  p.n_units = (uint32_t)n_mblk * (uint32_t)n_pair;
-  const uint32_t rem = p.n_units % (uint32_t)clusters;
-  p.sk_clusters = rem ? (uint32_t)pick_runs(rem, items, NT, clusters) : 0;
-  p.sk_units = p.sk_clusters ? rem : 0;
-  p.partial = (float*)((uint8_t*)workspace + xb_bytes_for(L, M));
-  p.arrived = (uint32_t*)((uint8_t*)workspace + xb_bytes_for(L, M) + partial_bytes_for(M, clusters));
   p.xb_half_bytes = xb_half_bytes(L, NT);
-  const uint32_t used = p.n_units >= (uint32_t)clusters ? (uint32_t)clusters : (p.sk_clusters ? p.sk_clusters : p.n_units);
+  uint8_t* xb = (uint8_t*)workspace;
+  uint8_t* partial = xb + n_layers * xb_bytes_for(L, M);
+  uint32_t* arrived = (uint32_t*)(partial + n_layers * partial_bytes_for(M, clusters));
+  uint32_t used = 0, n_arrived = 0;
+  for (int i = 0; i < n_layers; ++i) {
+    const cq_tlayer* l = layers[i];
+    const uint8_t* blob = (const uint8_t*)l->blob;
+    PrefillLayer& d = p.layer[i];
+    d.stream = blob + l->off_stream;
+    d.xb = stage.xb[i] = xb + i * xb_bytes_for(L, M);
+    d.y = (__half*)ys[i];
+    d.N = l->N; d.n_tile = l->n_tile; d.ldy = ldys[i];
+    d.n_units = (uint32_t)n_mblk * (uint32_t)((l->n_tile + 1) / 2);
+    const uint32_t rem = d.n_units % (uint32_t)clusters;
+    d.sk_clusters = rem ? (uint32_t)pick_runs(rem, items, NT, clusters) : 0;
+    d.sk_units = d.sk_clusters ? rem : 0;
+    d.partial = (float*)(partial + i * partial_bytes_for(M, clusters));
+    d.arrived = arrived + n_arrived;
+    n_arrived += 2 * d.sk_units;                     // (fewer than the clusters, for which there is room)
+    used = std::max(used, d.n_units >= (uint32_t)clusters ? (uint32_t)clusters : (d.sk_clusters ? d.sk_clusters : d.n_units));
+    if (((uintptr_t)ys[i] & 15) || ldys[i] % 8) p.vec_y = 0;
+    stage.osh[i] = (const uint32_t*)(blob + l->off_osh);
+    stage.cidx[i] = (const uint16_t*)(blob + l->off_cidx);
+  }
 
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -963,16 +1026,15 @@ extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* 
     // four token groups a thread once that still fills the SMs (2048 rows of 5120: 10 us against 18), one below it
     // (64 rows of 4096: four would add 4 us of latency to a 24 us call)
     const int gx = (quads + STAGE_THREADS / 32 - 1) / (STAGE_THREADS / 32);
-    const bool four = (long long)gx * ((groups + 3) / 4) >= 10ll * di.sms;
+    const bool four = (long long)gx * n_layers * ((groups + 3) / 4) >= 10ll * di.sms;
     const int gy = four ? (groups + 3) / 4 : groups;
-    cfg.gridDim = dim3(gx, gy < 65535 ? gy : 65535);
+    cfg.gridDim = dim3(gx, gy < 65535 ? gy : 65535, n_layers);
     cfg.blockDim = dim3(STAGE_THREADS);
     cfg.numAttrs = 1;
     const int aligned16 = ((uintptr_t)x & 15) == 0 && ldx % 8 == 0;
     CQ_CUDA_TRY(cudaLaunchKernelEx(&cfg, four ? prefill_stage_x_kernel<4> : prefill_stage_x_kernel<1>, (const __half*)x, ldx, M,
-                                   (const uint32_t*)(blob + L->off_osh), (const uint16_t*)(blob + L->off_cidx), (int)L->C,
-                                   (int)L->Kc, (int)L->n_gran, (int)L->n_cher, (uint8_t*)workspace, p.xb_half_bytes, NT,
-                                   p.arrived, (int)(2 * p.sk_units), aligned16));
+                                   stage, (int)L->C, (int)L->Kc, (int)L->n_gran, (int)L->n_cher, p.xb_half_bytes, NT, arrived,
+                                   (int)n_arrived, aligned16));
   }
 
   // shared memory: barriers, output staging tile, activation ring, and weights in what is left
@@ -991,7 +1053,7 @@ extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* 
   if (p.sb < NA || p.sw < NGRP) return CQ_ERR_TOO_LARGE;
   const int smem = off + p.sw * p.wstage_bytes;
 
-  PKernelFn fn = ppick(L->bits, L->sets);
+  PKernelFn fn = n_layers > 1 ? ppick<true>(L->bits, L->sets) : ppick<false>(L->bits, L->sets);
   CQ_CUDA_TRY(cq_grant_smem((const void*)fn, smem));
   cfg.gridDim = dim3(2 * used);
   cfg.blockDim = dim3(NTHREADS);

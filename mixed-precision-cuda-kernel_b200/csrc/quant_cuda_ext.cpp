@@ -695,6 +695,39 @@ torch::Tensor row_layers_matvec_norm(std::vector<RowLayer*> layers, torch::Tenso
   return sum.defined() ? sum : x;
 }
 
+// TileLayer.gemm for layers that take the same activations (q / k / v, gate / up): one pre-pass and one launch per 4096
+// rows.  Returns the outputs, (M, N_i) each.
+std::vector<torch::Tensor> tile_layers_gemm(std::vector<TileLayer*> layers, torch::Tensor x) {
+  TORCH_CHECK(!layers.empty() && layers.size() <= 4, "1 to 4 layers");
+  const at::cuda::OptionalCUDAGuard device_guard(device_of(x));
+  const cq_tlayer& first = layers[0]->layer;
+  check_tensor(x, "x", torch::kFloat16, layers[0]->blob.t);
+  TORCH_CHECK(x.dim() == 2 && x.size(1) == first.K && x.size(0) > 0, "x must be (M, ", first.K, ")");
+  const int M = (int)x.size(0), n = (int)layers.size(), CH = 4096, chunk = M < CH ? M : CH;
+  auto ws = torch::empty({(int64_t)cq_tlayers_gemm_workspace_bytes(&first, n, chunk)}, layers[0]->blob.t.options());
+  auto scratch = scratch_for(x.device());
+  std::vector<torch::Tensor> outs;
+  const cq_tlayer* ls[4];
+  void* ys[4];
+  int ldys[4];
+  for (int i = 0; i < n; ++i) {
+    TORCH_CHECK(layers[i]->blob.t.device() == x.device(), "the layers must be on x's device");
+    layers[i]->blob.use();
+    ls[i] = &layers[i]->layer;
+    ldys[i] = ls[i]->N;
+    outs.push_back(torch::empty({M, ls[i]->N}, x.options()));
+  }
+  uint32_t* status = (uint32_t*)(scratch.data_ptr<uint8_t>() + cq_scratch_bytes());
+  for (int m0 = 0; m0 < M; m0 += CH) {
+    const int rows = M - m0 < CH ? M - m0 : CH;
+    for (int i = 0; i < n; ++i) ys[i] = (uint16_t*)outs[i].data_ptr() + (size_t)m0 * ldys[i];
+    check_status(cq_tlayers_gemm(ls, n, (const uint16_t*)x.data_ptr() + (size_t)m0 * first.K, first.K, ys, ldys, rows, 0, ws.data_ptr(),
+                                 status, current_stream()),
+                 "tile_layers_gemm");
+  }
+  return outs;
+}
+
 // Reads and clears the status word the PreparedLayer launches report into.
 bool device_timed_out(int device_index) {
   torch::Tensor t;
@@ -860,6 +893,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("poll", []() { check_status(cq_poll(current_stream()), "poll"); });
   m.def("device_timed_out", &device_timed_out);
   m.def("row_layers_matvec", &row_layers_matvec, "one launch for row-tile layers sharing an activation row");
+  m.def("tile_layers_gemm", &tile_layers_gemm, "one launch of the GEMM for tile layers sharing their activations");
   m.def("row_layers_matvec_norm", &row_layers_matvec_norm, "row_layers_matvec on the RMS norm of its input");
   m.def("abi_version", &cq_abi_version);
   py::class_<RowLayer>(m, "RowLayer")

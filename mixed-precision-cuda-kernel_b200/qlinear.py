@@ -270,15 +270,50 @@ class QuantLinear(nn.Module):
         return out
 
 
-def _row_copies(layers, rows):
-    """The row-tile copies of layers that one launch of the row kernel can serve for that many rows, or None."""
+def _alike(layers):
+    """Whether one launch can serve these layers, by their sizes."""
     first = layers[0]
     same = all((l.w_bits, l.in_features, l.num_cherries, l.group_size) ==
                (first.w_bits, first.in_features, first.num_cherries, first.group_size) for l in layers)
-    if not (1 < len(layers) <= 4 and same and QuantLinear._layerwise_dequantize and first.w_bits in (3, 4)):
+    return 1 < len(layers) <= 4 and same and QuantLinear._layerwise_dequantize and first.w_bits in (3, 4)
+
+
+def _row_copies(layers, rows):
+    """The row-tile copies of layers that one launch of the row kernel can serve for that many rows, or None."""
+    if not _alike(layers):
         return None
     rls = [l.row_layer(rows) for l in layers]
     return rls if all(r is not None for r in rls) else None
+
+
+# Rows up to which the GEMM serves layers together: one token block of 32.  Microseconds one after another and together, 16
+# and 32 rows: 8192 -> (8192, 1024, 1024) 47 and 34, 53 and 39; 8192 -> 2 x 28672 97 and 90, 97 and 90; 5120 -> 3 x 5120 46 and
+# 36, 54 and 46; 4096 -> 3 x 4096 40 and 34, 47 and 44.  Beyond, storing the layers' parts in one launch costs more than
+# the launches: 64 rows 4096 -> 3 x 4096 61 and 65, 128 rows 5120 -> 3 x 5120 86 and 95, 512 rows 162 and 179.
+GEMM_TOGETHER_ROWS = 32
+
+
+def _tile_copies(layers, x, rows):
+    """The tile-layout copies of layers whose own forward of `x` is the GEMM on them and nothing else, or None."""
+    first = layers[0]
+    if not (rows <= GEMM_TOGETHER_ROWS and _alike(layers) and x.is_cuda and x.dtype == torch.float16 and x.shape[-1] == first.in_features
+            and (first.w_bits == 3 or first.group_size >= 128)):
+        return None
+    for l in layers:
+        hooked = l._forward_hooks or l._forward_pre_hooks or l._backward_hooks or l._backward_pre_hooks
+        if hooked or type(l).forward is not QuantLinear.forward or rows < (l._row_limit() + 1 if l._row_limit() else GEMM_MIN_ROWS):
+            return None
+    return [l.tile_layer() for l in layers]
+
+
+@torch.inference_mode()
+def _gemm_together(layers, tls, x, rows):
+    outs = load_quant_cuda().tile_layers_gemm(tls, x.reshape(rows, x.shape[-1]).contiguous())
+    outs = [o.reshape(x.shape[:-1] + (l.out_features,)) for l, o in zip(layers, outs)]
+    for l, o in zip(layers, outs):
+        if l.bias is not None:
+            o += l.bias
+    return outs
 
 
 def _row_outputs(layers, shape, dtype, rows, device, launch):
@@ -298,15 +333,16 @@ def _row_outputs(layers, shape, dtype, rows, device, launch):
 
 def forward_shared_input(layers, x: torch.Tensor):
     """Outputs of several packed layers applied to the same input (q / k / v, gate / up of the
-    reference's LLaMA, llama/modeling_llama_quant.py): for decode batches (up to the layers' row
-    limit) and layers that agree in bits, in_features, cherry count and group size this is ONE launch
-    of the row-tile kernel per four rows, with the SMs divided among the layers; every other case is
-    the layers' own forward, one by one.  The results are bit-identical to the separate calls."""
+    reference's LLaMA, llama/modeling_llama_quant.py): for layers that agree in bits, in_features, cherry
+    count and group size this is ONE launch of the row-tile kernel per four rows of a decode batch (up to the
+    layers' row limit), with the SMs divided among the layers, and ONE launch of the GEMM for batches beyond, up
+    to 32 rows; every other case is the layers' own forward, one by one.  The results are bit-identical to the separate calls."""
     layers = list(layers)
     rows = x.numel() // x.shape[-1]
     rls = _row_copies(layers, rows)
     if rls is None:
-        return [l(x) for l in layers]
+        tls = _tile_copies(layers, x, rows)
+        return [l(x) for l in layers] if tls is None else _gemm_together(layers, tls, x, rows)
     x2 = x.reshape(rows, x.shape[-1])
     if x2.dtype != torch.float16:
         x2 = x2.half()

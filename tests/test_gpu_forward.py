@@ -119,6 +119,24 @@ def test_norm_in_front_of_a_shared_input(K, bits, G, m, with_delta):
         assert float((out.float() - ref).norm()) <= 3e-4 * float(ref.norm()) and out.shape == (m, lin.out_features)
 
 
+@pytest.mark.parametrize("bits,G", [(4, 128), (3, 64)])
+@pytest.mark.parametrize("shape", [(9,), (2, 16), (33,)])
+def test_shared_input_beyond_the_row_kernel(bits, G, shape):
+    """One launch of the GEMM for the layers equals their own forward, bias included; a hook is still called."""
+    from cherryq_b200.qlinear import forward_shared_input
+    K = 1032
+    lins = [packed(K, N, bits, G, N + i, i == 1, 16) for i, N in enumerate((520, 136, 136))]
+    x = torch.randn(*shape, K, device="cuda").half()
+    want = [l(x) for l in lins]
+    got = forward_shared_input(lins, x)
+    assert all(a.shape == b.shape and torch.equal(a, b) for a, b in zip(got, want))
+    seen = []
+    handle = lins[2].register_forward_hook(lambda m, a, o: seen.append(o))
+    got = forward_shared_input(lins, x)
+    handle.remove()
+    assert len(seen) == 1 and all(torch.equal(a, b) for a, b in zip(got, want))
+
+
 @pytest.mark.parametrize("m,C", [(9, 16), (40, 16), (3, 256)])
 def test_swiglu_beyond_the_row_kernel_is_the_torch_expression(m, C):
     """Rows above the row kernel's limit and layers it does not take: silu in fp32, not the fast exponential.  Every fp16

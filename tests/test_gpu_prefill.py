@@ -219,6 +219,37 @@ def test_gemm_every_fourth_item_of_a_group(cabi, K):
     assert torch.equal(gemm(cabi, p, x), y)
 
 
+@pytest.mark.parametrize("widths", [(264, 8), (1024, 4096, 136), (2440, 128, 128, 9600)])
+@pytest.mark.parametrize("M,offset", [(1, 0), (45, 1), (300, 0), (2049, 0)])
+def test_gemm_of_layers_together_is_the_separate_calls(cabi, widths, M, offset):
+    """Layers with fewer, as many and more units than clusters in one launch: the same bits as one by one, also added to
+    outputs off their alignment."""
+    lib, K, bits, G = cabi.lib(), 1160, 3, 64
+    ps = []
+    for i, N in enumerate(widths):
+        _, _, pk, _ = make_case(K, N, bits, G, seed=N + i)
+        ps.append(TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], bits, K, G))
+    n, g = len(ps), torch.Generator(device="cuda").manual_seed(M)
+    x = torch.randn(M, K, device="cuda", generator=g).half()
+    base = [torch.randn(M * N + offset, device="cuda", generator=g).half() for N in widths]
+    want = []
+    for p, b, N in zip(ps, base, widths):
+        y = b.clone()[offset:].view(M, N)
+        ws = torch.empty(lib.cq_tlayer_gemm_workspace_bytes(C.byref(p.L), M), dtype=torch.uint8, device="cuda")
+        cabi.check(lib.cq_tlayer_gemm(C.byref(p.L), ptr(x), K, y.data_ptr(), N, M, 1, ptr(ws), ptr(p.status), None), "gemm")
+        want.append(y)
+    bufs = [b.clone() for b in base]
+    ws = torch.empty(lib.cq_tlayers_gemm_workspace_bytes(C.byref(ps[0].L), n, M), dtype=torch.uint8, device="cuda")
+    ls = (C.POINTER(type(ps[0].L)) * n)(*[C.pointer(p.L) for p in ps])
+    ys = (C.c_void_p * n)(*[b.data_ptr() + 2 * offset for b in bufs])
+    lds = (C.c_int32 * n)(*widths)
+    cabi.check(lib.cq_tlayers_gemm(ls, n, ptr(x), K, ys, lds, M, 1, ptr(ws), ptr(ps[0].status), None), "gemm")
+    torch.cuda.synchronize()
+    assert all(int(p.status.item()) == 0 for p in ps)
+    for w, b, N in zip(want, bufs, widths):
+        assert torch.equal(b[offset:].view(M, N), w)
+
+
 @pytest.mark.parametrize("bits,G", [(3, 64), (3, 128), (4, 128), (4, 256)])
 def test_gemm_weights_are_unpacked_exactly_at_every_scale(cabi, bits, G):
     """Rows of the identity read the dequantised weights back: bit for bit unpack()'s, with scales from the smallest
