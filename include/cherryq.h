@@ -313,11 +313,12 @@ size_t cq_tlayer_gemm_workspace_bytes(const cq_tlayer* layer, int M);
 int cq_tlayer_gemm(const cq_tlayer* layer, const void* x_f16, int ldx, void* y_f16, int ldy, int M,
                    int accumulate, void* workspace, uint32_t* status_word, cq_stream_t stream);
 /* The same for one to four layers on the same activations (q / k / v, gate / up) in one launch: layers of equal K, C, G
- * and bits, ys[i] with row stride ldys[i].  Bit-identical to separate calls.  `workspace`:
+ * and bits, ys[i] with row stride ldys[i].  Bit-identical to separate calls.  biases (may be null, as each of them): fp16, added
+ * to the rounded outputs and rounded again, as by a kernel after this one; not with `accumulate`.  `workspace`:
  * cq_tlayers_gemm_workspace_bytes(layers[0], n_layers, M) bytes. */
 size_t cq_tlayers_gemm_workspace_bytes(const cq_tlayer* layer, int n_layers, int M);
 int cq_tlayers_gemm(const cq_tlayer* const* layers, int n_layers, const void* x_f16, int ldx, void* const* ys_f16,
-                    const int* ldys, int M, int accumulate, void* workspace, uint32_t* status_word, cq_stream_t stream);
+                    const int* ldys, const void* const* biases_f16, int M, int accumulate, void* workspace, uint32_t* status_word, cq_stream_t stream);
 
 /* ------------------------------------------------------------------------
  * Drop-in operator entry points (reference: csrc/quant_cuda.cpp:41-69, 26-38).

@@ -86,7 +86,7 @@ def lib():
     L.cq_tlayer_gemm.argtypes = [C.POINTER(cq_tlayer), vp, i32, vp, i32, i32, i32, vp, vp, vp]
     L.cq_tlayer_gemm_workspace_bytes.argtypes = [C.POINTER(cq_tlayer), i32]
     L.cq_tlayer_gemm_workspace_bytes.restype = C.c_size_t
-    L.cq_tlayers_gemm.argtypes = [C.POINTER(C.POINTER(cq_tlayer)), i32, vp, i32, C.POINTER(vp), C.POINTER(i32), i32, i32, vp, vp, vp]
+    L.cq_tlayers_gemm.argtypes = [C.POINTER(C.POINTER(cq_tlayer)), i32, vp, i32, C.POINTER(vp), C.POINTER(i32), C.POINTER(vp), i32, i32, vp, vp, vp]
     L.cq_tlayers_gemm_workspace_bytes.argtypes = [C.POINTER(cq_tlayer), i32, i32]
     L.cq_tlayers_gemm_workspace_bytes.restype = C.c_size_t
     L.cq_vecquant4matmul_cherryq.argtypes = [vp] * 6 + [i32] * 6 + [u64, vp]

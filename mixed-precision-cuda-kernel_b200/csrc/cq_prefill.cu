@@ -76,6 +76,7 @@ struct PrefillLayer {
   const uint8_t* stream;     // tile-layout weight stream
   const uint8_t* xb;         // staged activations: [token block][half][cherry items][granules]
   __half* y;
+  const __half* bias;        // null: none
   float* partial;            // [cluster][first / last run][CTA of the pair][token][128 rows] fp32
   uint32_t* arrived;         // [cut unit][CTA of the pair] runs finished so far
   int N, n_tile, ldy;
@@ -755,9 +756,14 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const __grid_co
           tmem_ld16(d_lu + c + 16, v[1]);
           tmem_wait_ld();
           __half* sp = stage + c * 128 + row;
+          // (the bias meets the rounded output, as in a kernel after this one)
           if (p.accumulate) {
 #pragma unroll
             for (int e = 0; e < 32; ++e) sp[e * 128] = __float2half(v[e >> 4][e & 15] + __half2float(sp[e * 128]));
+          } else if (L.bias) {
+            const __half b = row < nrows ? L.bias[n0 + row] : __float2half(0.f);
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sp[e * 128] = __hadd(__float2half(v[e >> 4][e & 15]), b);
           } else {
 #pragma unroll
             for (int e = 0; e < 32; ++e) sp[e * 128] = __float2half(v[e >> 4][e & 15]);
@@ -845,6 +851,9 @@ __global__ void __launch_bounds__(NTHREADS, 1) cq_prefill_kernel(const __grid_co
                 if (p.accumulate) {
 #pragma unroll
                   for (int e = 0; e < 4; ++e) r[e] += __half2float(yp[e]);
+                } else if (L.bias) {
+#pragma unroll
+                  for (int e = 0; e < 4; ++e) r[e] = __half2float(__float2half(r[e])) + __half2float(L.bias[n0 + 4 * lane + e]);
                 }
                 if (p.vec_y) {
                   const __half2 a = __floats2half2_rn(r[0], r[1]), b = __floats2half2_rn(r[2], r[3]);
@@ -955,17 +964,18 @@ extern "C" size_t cq_tlayer_gemm_workspace_bytes(const cq_tlayer* L, int M) { re
 
 extern "C" int cq_tlayer_gemm(const cq_tlayer* L, const void* x, int ldx, void* y, int ldy, int M, int accumulate,
                               void* workspace, uint32_t* status_word, cq_stream_t stream) {
-  return cq_tlayers_gemm(&L, 1, x, ldx, &y, &ldy, M, accumulate, workspace, status_word, stream);
+  return cq_tlayers_gemm(&L, 1, x, ldx, &y, &ldy, nullptr, M, accumulate, workspace, status_word, stream);
 }
 
 extern "C" int cq_tlayers_gemm(const cq_tlayer* const* layers, int n_layers, const void* x, int ldx, void* const* ys, const int* ldys,
-                               int M, int accumulate, void* workspace, uint32_t* status_word, cq_stream_t stream) {
+                               const void* const* biases, int M, int accumulate, void* workspace, uint32_t* status_word, cq_stream_t stream) {
   if (!layers || n_layers < 1 || n_layers > MAX_LAYERS || !ys || !ldys || !x || !workspace) return CQ_ERR_BAD_ARG;
   const cq_tlayer* L = layers[0];
   if (!L || M < 1 || ldx < L->K || ((uintptr_t)x & 1) || ((uintptr_t)workspace & 127)) return CQ_ERR_BAD_ARG;
   for (int i = 0; i < n_layers; ++i) {
     const cq_tlayer* l = layers[i];
     if (!l || !l->blob || !ys[i] || ldys[i] < l->N || ((uintptr_t)ys[i] & 1)) return CQ_ERR_BAD_ARG;
+    if (biases && biases[i] && (accumulate || ((uintptr_t)biases[i] & 1))) return CQ_ERR_BAD_ARG;
     if (l->K != L->K || l->C != L->C || l->G != L->G || l->bits != L->bits) return CQ_ERR_BAD_SHAPE;
   }
   int dev = 0;
@@ -997,6 +1007,7 @@ extern "C" int cq_tlayers_gemm(const cq_tlayer* const* layers, int n_layers, con
     d.stream = blob + l->off_stream;
     d.xb = stage.xb[i] = xb + i * xb_bytes_for(L, M);
     d.y = (__half*)ys[i];
+    d.bias = biases ? (const __half*)biases[i] : nullptr;
     d.N = l->N; d.n_tile = l->n_tile; d.ldy = ldys[i];
     d.n_units = (uint32_t)n_mblk * (uint32_t)((l->n_tile + 1) / 2);
     const uint32_t rem = d.n_units % (uint32_t)clusters;

@@ -243,11 +243,32 @@ def test_gemm_of_layers_together_is_the_separate_calls(cabi, widths, M, offset):
     ls = (C.POINTER(type(ps[0].L)) * n)(*[C.pointer(p.L) for p in ps])
     ys = (C.c_void_p * n)(*[b.data_ptr() + 2 * offset for b in bufs])
     lds = (C.c_int32 * n)(*widths)
-    cabi.check(lib.cq_tlayers_gemm(ls, n, ptr(x), K, ys, lds, M, 1, ptr(ws), ptr(ps[0].status), None), "gemm")
+    cabi.check(lib.cq_tlayers_gemm(ls, n, ptr(x), K, ys, lds, None, M, 1, ptr(ws), ptr(ps[0].status), None), "gemm")
     torch.cuda.synchronize()
     assert all(int(p.status.item()) == 0 for p in ps)
     for w, b, N in zip(want, bufs, widths):
         assert torch.equal(b[offset:].view(M, N), w)
+
+
+@pytest.mark.parametrize("N,M", [(8, 9), (136, 45), (2440, 300), (9600, 2049)])
+def test_gemm_adds_the_bias_to_the_rounded_outputs(cabi, N, M):
+    """Whole units and cut ones, the last rows of a tile; infinite and large biases: the bits of the addition afterwards."""
+    lib, K = cabi.lib(), 1160
+    _, _, pk, _ = make_case(K, N, 3, 64, seed=N)
+    p = TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], 3, K, 64)
+    x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).half()
+    buf = torch.randn(N + 1, device="cuda").half()
+    bias = buf[1:]                                                          # two bytes off
+    bias[2], bias[N - 1] = float("inf"), 60000.0
+    y = torch.empty(M, N, dtype=torch.float16, device="cuda")
+    ws = torch.empty(lib.cq_tlayers_gemm_workspace_bytes(C.byref(p.L), 1, M), dtype=torch.uint8, device="cuda")
+    args = [(C.POINTER(type(p.L)) * 1)(C.pointer(p.L)), 1, ptr(x), K, (C.c_void_p * 1)(y.data_ptr()), (C.c_int32 * 1)(N),
+            (C.c_void_p * 1)(bias.data_ptr())]
+    cabi.check(lib.cq_tlayers_gemm(*args, M, 0, ptr(ws), ptr(p.status), None), "gemm")
+    assert lib.cq_tlayers_gemm(*args, M, 1, ptr(ws), ptr(p.status), None) == 1          # not with accumulate
+    torch.cuda.synchronize()
+    assert int(p.status.item()) == 0
+    assert torch.equal(y, gemm(cabi, p, x) + bias)
 
 
 @pytest.mark.parametrize("bits,G", [(3, 64), (3, 128), (4, 128), (4, 256)])
