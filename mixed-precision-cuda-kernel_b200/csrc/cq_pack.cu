@@ -961,9 +961,10 @@ extern "C" int cq_unpack_dense(const uint8_t* qweight, const void* scales, const
                                                                cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
   };
   // Up to a cherry column in 32, so that most octets have none (4096 x 11008 4-bit, new and old kernel: 16 cherry columns 36.9
-  // and 40.6 us, 64 40.2 and 43.9, 128 44.6 and 46.2, then see the old kernel).  Matrices of few columns have no columns to
-  // spread over the chip but rows: 128 x 65536 13.4 and 12.2.
-  if ((long long)C * 32 <= K && n_cols >= 8) {
+  // and 40.6 us, 64 40.2 and 43.9, 128 44.6 and 46.2, then see the old kernel), and
+  // from 12 million weights on, so that a block has rows to go down (4096 x 8192 19.4 and 21.6, 4096 x 4096 17.5 both, 1536 x
+  // 5000 9.3 and 9.0).  Matrices of few columns have no columns to spread over the chip but rows: 128 x 65536 13.4 and 12.2.
+  if ((long long)C * 32 <= K && n_cols >= 8 && (long long)K * N >= (3ll << 22)) {
     const int n_y = row_blocks(n_cols, n_tiles, UP_BLOCKS);
     bits == 4 ? (C > 0 ? launch(unpack_rows_kernel<4, true>, n_y) : launch(unpack_rows_kernel<4, false>, n_y))
               : (C > 0 ? launch(unpack_rows_kernel<3, true>, n_y) : launch(unpack_rows_kernel<3, false>, n_y));

@@ -100,10 +100,10 @@ def test_pack_of_large_matrices(cabi, K, N, bits, G, C, offset):
 
 
 @pytest.mark.parametrize("offset", [0, 1])
-@pytest.mark.parametrize("K,N,bits,G,C", [(904, 8, 3, 1, 8), (1032, 72, 4, 4, 24), (1160, 136, 3, 12, 32), (2048, 520, 4, 96, 64),
-                                          (1024, 3208, 3, 64, 0)])
+@pytest.mark.parametrize("K,N,bits,G,C", [(904, 13928, 3, 1, 8), (1032, 12232, 4, 4, 24), (1160, 10856, 3, 12, 32),
+                                          (2048, 6152, 4, 96, 64), (1024, 12296, 3, 64, 0)])
 def test_unpack_going_down_the_rows(cabi, K, N, bits, G, C, offset):
-    """Eight and more blocks of columns, few cherry columns: octets with one inside, with group boundaries, of groups narrower
+    """From 12 million weights on, eight and more blocks of columns, few cherry columns: octets with one inside, with group boundaries, of groups narrower
     than an octet; rows that end inside a tile; codes and outputs off their alignment."""
     w, idx = layer(K, N, C, np.float16, K + G)
     ref = O.pack(w, idx, bits, G)
