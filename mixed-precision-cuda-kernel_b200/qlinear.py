@@ -293,6 +293,19 @@ def _row_copies(layers, rows):
 GEMM_TOGETHER_ROWS = 32
 
 
+# what a call runs, as defined here and in torch (a replaced method of the class is not the same object)
+_OWN_METHODS = {name: getattr(QuantLinear, name) for name in ("__call__", "forward", "_forward")}
+
+
+def _calls_only_forward(layer):
+    """Whether layer(x) is QuantLinear.forward and nothing else: no hook on the module or on all modules, no method replaced on
+    the instance (as device-placement wrappers and adapters do) or its class, not compiled."""
+    hooked = layer._forward_hooks or layer._forward_pre_hooks or layer._backward_hooks or layer._backward_pre_hooks
+    if hooked or nn.modules.module._has_any_global_hook() or layer._compiled_call_impl is not None:
+        return False
+    return all(getattr(type(layer), name) is own and name not in layer.__dict__ for name, own in _OWN_METHODS.items())
+
+
 def _tile_copies(layers, x, rows):
     """The tile-layout copies of layers whose own forward of `x` is the GEMM on them and nothing else, or None."""
     first = layers[0]
@@ -300,8 +313,7 @@ def _tile_copies(layers, x, rows):
             and (first.w_bits == 3 or first.group_size >= 128)):
         return None
     for l in layers:
-        hooked = l._forward_hooks or l._forward_pre_hooks or l._backward_hooks or l._backward_pre_hooks
-        if hooked or type(l).forward is not QuantLinear.forward or rows < (l._row_limit() + 1 if l._row_limit() else GEMM_MIN_ROWS):
+        if not _calls_only_forward(l) or rows < (l._row_limit() + 1 if l._row_limit() else GEMM_MIN_ROWS):
             return None
     return [l.tile_layer() for l in layers]
 

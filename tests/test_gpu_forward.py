@@ -137,6 +137,17 @@ def test_shared_input_beyond_the_row_kernel(bits, G, shape):
     assert len(seen) == 1 and all(torch.equal(a, b) for a, b in zip(got, want))
 
 
+@pytest.mark.parametrize("m", [9, 32])
+def test_shared_input_keeps_a_forward_set_on_the_instance(m):
+    from cherryq_b200.qlinear import forward_shared_input
+    lins = [packed(1032, N, 4, 128, N, False, 16) for N in (520, 136)]
+    x = torch.randn(m, 1032, device="cuda").half()
+    want = [lins[0](x), lins[1](x) + 1]
+    own = lins[1].forward
+    lins[1].forward = lambda x: own(x) + 1
+    assert all(torch.equal(a, b) for a, b in zip(forward_shared_input(lins, x), want))
+
+
 @pytest.mark.parametrize("m,C", [(9, 16), (40, 16), (3, 256)])
 def test_swiglu_beyond_the_row_kernel_is_the_torch_expression(m, C):
     """Rows above the row kernel's limit and layers it does not take: silu in fp32, not the fast exponential.  Every fp16

@@ -63,3 +63,46 @@ def test_copy_and_pickle_leave_the_copies_behind():
     lin._prepared_key = "released"
     with pytest.raises(TypeError):
         copy.deepcopy(lin)
+
+
+def _wrapped_call(kind, lin, monkeypatch):
+    """Something that a call of the layer runs besides QuantLinear.forward; returns what takes it away again."""
+    from cherryq_b200 import QuantLinear
+    if kind == "instance forward":                                 # as device-placement wrappers and adapters set it
+        own = lin.forward
+        lin.forward = lambda x: own(x) + 1
+    elif kind == "instance _forward":
+        own = lin._forward
+        lin._forward = lambda x: own(x) + 1
+    elif kind == "class forward":
+        own = QuantLinear.forward
+        monkeypatch.setattr(QuantLinear, "forward", lambda self, x: own(self, x) + 1)
+    elif kind == "subclass call":
+        lin.__class__ = type("Sub", (QuantLinear,), {"__call__": lambda self, x: QuantLinear.__call__(self, x) + 1})
+    elif kind == "hook":
+        return lin.register_forward_hook(lambda m, a, o: o + 1).remove
+    elif kind == "compiled":
+        lin._compiled_call_impl = lambda x: x
+    else:
+        register = getattr(torch.nn.modules.module, kind)
+        return register(lambda *a: None).remove
+    return lambda: None
+
+
+@pytest.mark.parametrize("kind", ["instance forward", "instance _forward", "class forward", "subclass call", "hook", "compiled",
+                                  "register_module_forward_hook", "register_module_forward_pre_hook",
+                                  "register_module_full_backward_hook"])
+def test_layers_that_share_an_input_keep_their_own_calls(kind, monkeypatch):
+    """One launch stands for the calls of several layers only where each call is QuantLinear.forward and nothing else."""
+    from types import SimpleNamespace
+    from cherryq_b200 import QuantLinear, qlinear
+    monkeypatch.setattr(QuantLinear, "_row_limit", lambda self: 8)
+    monkeypatch.setattr(QuantLinear, "tile_layer", lambda self: "copy")
+    x = SimpleNamespace(is_cuda=True, dtype=torch.float16, shape=(16, 1024))
+    lins = [layer(), layer()]
+    assert qlinear._tile_copies(lins, x, 16) == ["copy", "copy"]
+    remove = _wrapped_call(kind, lins[1], monkeypatch)
+    try:
+        assert qlinear._tile_copies(lins, x, 16) is None
+    finally:
+        remove()
