@@ -191,7 +191,9 @@ int cq_rlayer_matvec(const cq_rlayer* layer, const void* x_f16, void* y_f16, int
 /* cq_rlayers_matvec (M = 1..4, one launch) on the RMS norm of x (+ delta): each row's
  * fp16((x + delta) / sqrt(mean((x + delta)^2) + eps)) * norm_weight, the sum x + delta an fp16 tensor, which is stored to
  * sum_out (rows of ldx elements) unless that is null (cq_rmsnorm in front of the layers without its launch).  delta may be
- * null.  x, delta, norm_weight and sum_out 16-byte aligned, ldx a multiple of 8.  CQ_ERR_UNSUPPORTED beyond 4 rows. */
+ * null.  x, delta, norm_weight and sum_out 16-byte aligned, ldx a multiple of 8.  Unlike cq_rmsnorm not in place: every CTA
+ * reads all of x and delta, so CQ_ERR_BAD_ARG where sum_out shares bytes with x, delta or norm_weight (sum_out = x without
+ * a delta is left as it is); the outputs may not share any either.  CQ_ERR_UNSUPPORTED beyond 4 rows. */
 int cq_rlayers_matvec_norm(const cq_rlayer* const* layers, int n_layers, const void* x_f16, const void* delta_f16,
                            const void* norm_weight_f16, float eps, void* sum_out_f16, int ldx, void* const* ys_f16,
                            int ldy, int M, uint32_t* status_word, cq_stream_t stream);

@@ -1200,6 +1200,14 @@ extern "C" int cq_rlayers_matvec(const cq_rlayer* const* layers, int n_layers, c
   return CQ_OK;
 }
 
+// Whether one of `rows` rows at a and one of `other_rows` rows at b, of K elements each, `ld` elements from row to row, share bytes
+static bool rv_rows_overlap(const void* a, const void* b, int K, int ld, int rows, int other_rows) {
+  const long long size = 2ll * K, step = 2ll * ld, off = (long long)((uintptr_t)a - (uintptr_t)b);
+  for (int d = 1 - other_rows; d < rows; ++d)                    // (a's row less b's)
+    if (off + d * step < size && off + d * step > -size) return true;
+  return false;
+}
+
 extern "C" int cq_rlayers_matvec_norm(const cq_rlayer* const* layers, int n_layers, const void* x, const void* delta,
                                       const void* norm_weight, float eps, void* sum_out, int ldx, void* const* ys, int ldy, int M,
                                       uint32_t* status_word, cq_stream_t stream) {
@@ -1215,6 +1223,11 @@ extern "C" int cq_rlayers_matvec_norm(const cq_rlayer* const* layers, int n_laye
   const cq_rlayer* L = layers[0];
   if (ldx < L->K || ldy < nmax || ldx % 8) return CQ_ERR_BAD_ARG;
   if (((uintptr_t)x | (uintptr_t)delta | (uintptr_t)norm_weight | (uintptr_t)sum_out) & 15) return CQ_ERR_BAD_ARG;
+  // The first CTA stores the sum while the others still read x, delta and the weight.  (Without a delta the sum is x.)
+  if (sum_out == x && !delta) sum_out = nullptr;
+  if (sum_out && (rv_rows_overlap(sum_out, x, L->K, ldx, M, M) || (delta && rv_rows_overlap(sum_out, delta, L->K, ldx, M, M)) ||
+                  rv_rows_overlap(sum_out, norm_weight, L->K, ldx, M, 1)))
+    return CQ_ERR_BAD_ARG;
   RvNorm norm;
   norm.w = (const __half*)norm_weight;
   norm.delta = (const __half*)delta;

@@ -56,3 +56,33 @@ def test_package_fails_loudly_without_native_library(monkeypatch, tmp_path):
     monkeypatch.setattr(_cabi, "_lib", None)
     with pytest.raises(cherryq_b200.NativeLibraryMissing):
         _cabi.lib()
+
+
+# offsets of the sum from x or delta, in elements
+@pytest.mark.parametrize("M,with_delta,off,refused", [
+    (1, True, 0, True), (4, True, 0, True), (1, False, 0, False),              # in place; without a delta the sum is x
+    (1, False, 8, True), (1, True, 1016, True), (1, True, -1016, True), (1, True, 1024, False), (1, True, -1024, False),
+    (4, True, 2 * 2080, True), (4, True, -3 * 2080 + 8, True), (4, True, 1024, False), (4, True, 3 * 2080 + 1024, False),
+])
+@pytest.mark.parametrize("about", ["x", "delta"])
+def test_norm_in_front_of_the_layers_is_not_in_place(M, with_delta, off, refused, about):
+    """Every CTA reads all of x and delta while the first one stores the sum: shared bytes are refused before any launch.
+    K = 1024, rows 2080 elements apart (between them there is room for the sum's rows)."""
+    torch = pytest.importorskip("torch")
+    if torch.cuda.is_available():
+        pytest.skip("the addresses are not real: only where nothing can be launched")
+    if about == "delta" and not with_delta:
+        pytest.skip("no delta")
+    from cherryq_b200 import _cabi
+    C = ctypes
+    L = _cabi.rlayer_init(4, 1024, 264, 16, 128)
+    L.blob = 1 << 20
+    fn = _cabi.lib().cq_rlayers_matvec_norm
+    vp, i32 = C.c_void_p, C.c_int
+    fn.argtypes = [vp, i32, vp, vp, vp, C.c_float, vp, i32, vp, i32, i32, vp, vp]
+    x, delta, weight = 1 << 30, 2 << 30, 3 << 30
+    layers, ys = (vp * 1)(C.addressof(L)), (vp * 1)(4 << 30)
+    call = lambda total: fn(layers, 1, x, delta if with_delta else None, weight, 1e-5, total, 2080, ys, 264, M, None, None)
+    rc = call((x if about == "x" else delta) + 2 * off)
+    assert (rc == 1) == refused and rc != 0, rc
+    assert call(weight + 16) == 1 and call(5 << 30) not in (0, 1)
