@@ -135,7 +135,7 @@ __global__ void prepare_index_kernel(LayoutDims d, const int16_t* __restrict__ i
         int low = 0, high = d.C;
         while (low < high) {
           const int mid = (low + high) >> 1;
-          if ((int)idx[mid] - mid <= k) low = mid + 1; else high = mid;
+          if ((int)(uint16_t)idx[mid] - mid <= k) low = mid + 1; else high = mid;
         }
         sh[e] = low;
       }

@@ -9,8 +9,9 @@
 
 namespace {
 
+// The cherry columns are kept as 16-bit words and read as unsigned numbers (a layer may have up to 65534 columns).
 // number of sorted cherry columns with idx[m] - m <= kc (compact -> original shift)
-__device__ __forceinline__ int cherry_shift(const int16_t* __restrict__ idx, int C, int kc) {
+__device__ __forceinline__ int cherry_shift(const uint16_t* __restrict__ idx, int C, int kc) {
   int low = 0, high = C;
   while (low < high) {
     const int mid = (low + high) >> 1;
@@ -36,7 +37,7 @@ __global__ void pack_sort_kernel(const int32_t* __restrict__ in, int C, int16_t*
 }
 
 // llama/qlinear.py:74 — cherry_weight[c, n] = fp16(W[n, idx[c]]).
-__global__ void pack_cherry_kernel(const void* __restrict__ w, int is_f32, const int16_t* __restrict__ idx,
+__global__ void pack_cherry_kernel(const void* __restrict__ w, int is_f32, const uint16_t* __restrict__ idx,
                                    int K, int N, int C, __half* __restrict__ cw) {
   const long long total = (long long)C * N;
   for (long long id = blockIdx.x * (long long)blockDim.x + threadIdx.x; id < total;
@@ -49,7 +50,7 @@ __global__ void pack_cherry_kernel(const void* __restrict__ w, int is_f32, const
 // llama/cherry_linear.py:69-75 + llama/quantizer.py:148-152 + llama/qlinear.py:78:
 // s = fp16((max|w| + 1e-6) / 2^(bits-1)) per (row, group of the compact axis), evaluated in
 // the weight dtype.  One warp per (n, group).
-__global__ void pack_scales_kernel(const void* __restrict__ w, int is_f32, const int16_t* __restrict__ idx,
+__global__ void pack_scales_kernel(const void* __restrict__ w, int is_f32, const uint16_t* __restrict__ idx,
                                    int bits, int K, int N, int C, int G, __half* __restrict__ scales) {
   const int Kc = K - C, ng = (Kc + G - 1) / G;
   const int lane = threadIdx.x & 31;
@@ -78,7 +79,7 @@ __global__ void pack_scales_kernel(const void* __restrict__ w, int is_f32, const
 
 // llama/quantizer.py:154-158 + llama/qlinear.py:81-116: quantize 8 compact columns of one
 // row and write their 3 or 4 bytes.
-__global__ void pack_codes_kernel(const void* __restrict__ w, int is_f32, const int16_t* __restrict__ idx,
+__global__ void pack_codes_kernel(const void* __restrict__ w, int is_f32, const uint16_t* __restrict__ idx,
                                   const __half* __restrict__ scales, int bits, int K, int N, int C,
                                   int G, uint8_t* __restrict__ q) {
   const int Kc = K - C;
@@ -134,7 +135,7 @@ __device__ __forceinline__ float div_fp16(float w, float s_residual, float r) {
 
 template <typename T, int BITS>
 __global__ void __launch_bounds__(PK_THREADS, sizeof(T) == 2 ? 5 : 3) pack_fused_kernel(
-    const T* __restrict__ w, const int16_t* __restrict__ idx, int K, int N, int C, int G, int span, int n_tiles,
+    const T* __restrict__ w, const uint16_t* __restrict__ idx, int K, int N, int C, int G, int span, int n_tiles,
     int n_spans, __half* __restrict__ scales, uint8_t* __restrict__ q, __half* __restrict__ cw) {
   constexpr int ST = PackTile<T>::STRIDE, VEC = 16 / sizeof(T);
   __shared__ __align__(16) T tile[PK_ROWS * ST];
@@ -294,7 +295,7 @@ template <int BITS> __device__ __forceinline__ void codes_of(uint32_t h, uint32_
 
 template <int BITS>
 __global__ void __launch_bounds__(PG_WARPS * 32, PG_BLOCKS) pack_group_kernel(
-    const __half* __restrict__ w, const int16_t* __restrict__ idx, int K, int N, int C, int G,
+    const __half* __restrict__ w, const uint16_t* __restrict__ idx, int K, int N, int C, int G,
     __half* __restrict__ scales, uint8_t* __restrict__ q, __half* __restrict__ cw) {
   __shared__ __align__(16) __half tiles[PG_WARPS][PG_ROWS * PG_STRIDE + 32];      // (+ 32: reads of 32 columns where fewer are left)
   __shared__ int source[PK_COLS], s_at[4], s_gaps[4], s_gap[4], s_end;
@@ -576,7 +577,7 @@ template <int BITS> __device__ __forceinline__ __half2 code_pair(uint32_t word, 
 template <int BITS, bool CHERRY>
 __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
     const uint8_t* __restrict__ q, const __half* __restrict__ scales, const __half* __restrict__ cw,
-    const int16_t* __restrict__ idx, int K, int N, int C, int G, int g_shift, __half* __restrict__ dense, int aligned) {
+    const uint16_t* __restrict__ idx, int K, int N, int C, int G, int g_shift, __half* __restrict__ dense, int aligned) {
   __shared__ __align__(16) uint4 tile[UP_ROWS * (UP_COLS / 8)];
   __shared__ int before[UP_COLS / 8 + 1];           // cherry columns before each octet
   const int tid = threadIdx.x, nq = tid & 15, oct = tid >> 4;
@@ -696,7 +697,7 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
 template <int BITS, bool CHERRY>
 __global__ void __launch_bounds__(256, UP_BLOCKS) unpack_rows_kernel(
     const uint8_t* __restrict__ q, const __half* __restrict__ scales, const __half* __restrict__ cw,
-    const int16_t* __restrict__ idx, int K, int N, int C, int G, int g_shift, __half* __restrict__ dense, int aligned) {
+    const uint16_t* __restrict__ idx, int K, int N, int C, int G, int g_shift, __half* __restrict__ dense, int aligned) {
   __shared__ __align__(16) uint4 tiles[2][UP_ROWS * (UP_COLS / 8)];
   const int tid = threadIdx.x, nq = tid & 15, oct = tid >> 4, lane = tid & 31;
   const int k0 = blockIdx.x * UP_COLS, k = k0 + 8 * oct, k_warp = k0 + 8 * (oct & ~1);       // a warp has two octets
@@ -896,6 +897,7 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
   cudaStream_t st = (cudaStream_t)stream;
   const int T = 256;
   if (C > 0) pack_sort_kernel<<<nblocks(C, T), T, 0, st>>>(cherry_unsorted, C, cherry_indices);
+  const uint16_t* idx = (const uint16_t*)cherry_indices;
   const int ng = (K - C + G - 1) / G;
   // From 12 million weights on a warp of pack_group_kernel has rows enough to go down (4096 x 11008 4-bit: 48.0 and 58.8 us;
   // 16384 x 28672 342 and 542; 4096 x 4096 22.9 and 24.9; 16384 x 1024 25.6 and 27.5; 4096 x 2048 16.5 and 16.5; 2048 x 1024
@@ -904,7 +906,7 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
     const int n_x = (K - C + PK_COLS - 1) / PK_COLS, rows = PG_WARPS * PG_ROWS;
     auto kernel = bits == 4 ? pack_group_kernel<4> : pack_group_kernel<3>;
     kernel<<<dim3(n_x, row_blocks(n_x, (N + rows - 1) / rows, PG_BLOCKS)), PG_WARPS * 32, 0, st>>>(
-        (const __half*)weight, cherry_indices, K, N, C, G, (__half*)scales, qweight, (__half*)cherry_weight);
+        (const __half*)weight, idx, K, N, C, G, (__half*)scales, qweight, (__half*)cherry_weight);
     CQ_CUDA_TRY(cudaGetLastError());
     return CQ_OK;
   }
@@ -922,7 +924,7 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
     const long long blocks = (long long)n_tiles * (n_spans + (C > 0));
     if (blocks <= 0x7fffffffll) {
       auto launch = [&](auto kernel, auto* wp) {
-        kernel<<<(unsigned)blocks, PK_THREADS, 0, st>>>(wp, cherry_indices, K, N, C, G, span, n_tiles, n_spans,
+        kernel<<<(unsigned)blocks, PK_THREADS, 0, st>>>(wp, idx, K, N, C, G, span, n_tiles, n_spans,
                                                        (__half*)scales, qweight, (__half*)cherry_weight);
       };
       if (weight_is_f32)
@@ -934,12 +936,12 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
     }
   }
   if (C > 0)
-    pack_cherry_kernel<<<nblocks((long long)C * N, T), T, 0, st>>>(weight, weight_is_f32, cherry_indices, K, N, C,
+    pack_cherry_kernel<<<nblocks((long long)C * N, T), T, 0, st>>>(weight, weight_is_f32, idx, K, N, C,
                                                                   (__half*)cherry_weight);
-  pack_scales_kernel<<<nblocks((long long)ng * N * 32, T), T, 0, st>>>(weight, weight_is_f32, cherry_indices, bits,
+  pack_scales_kernel<<<nblocks((long long)ng * N * 32, T), T, 0, st>>>(weight, weight_is_f32, idx, bits,
                                                                       K, N, C, G, (__half*)scales);
   pack_codes_kernel<<<nblocks((long long)((K - C) / 8) * N, T), T, 0, st>>>(
-      weight, weight_is_f32, cherry_indices, (const __half*)scales, bits, K, N, C, G, qweight);
+      weight, weight_is_f32, idx, (const __half*)scales, bits, K, N, C, G, qweight);
   CQ_CUDA_TRY(cudaGetLastError());
   return CQ_OK;
 }
@@ -958,7 +960,7 @@ extern "C" int cq_unpack_dense(const uint8_t* qweight, const void* scales, const
   const int n_cols = (K + UP_COLS - 1) / UP_COLS, n_tiles = (N + UP_ROWS - 1) / UP_ROWS;
   auto launch = [&](auto kernel, int n_y) {
     kernel<<<dim3(n_cols, n_y), 256, 0, (cudaStream_t)stream>>>(qweight, (const __half*)scales, (const __half*)cherry_weight,
-                                                               cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
+                                                               (const uint16_t*)cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
   };
   // Up to a cherry column in 32, so that most octets have none (4096 x 11008 4-bit, new and old kernel: 16 cherry columns 36.9
   // and 40.6 us, 64 40.2 and 43.9, 128 44.6 and 46.2, then see the old kernel), and

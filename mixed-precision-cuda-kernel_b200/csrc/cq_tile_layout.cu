@@ -96,7 +96,7 @@ __global__ void tprepare_index_kernel(TileDims d, const int16_t* __restrict__ id
         int low = 0, high = d.C;
         while (low < high) {
           const int mid = (low + high) >> 1;
-          if ((int)idx[mid] - mid <= k) low = mid + 1; else high = mid;
+          if ((int)(uint16_t)idx[mid] - mid <= k) low = mid + 1; else high = mid;
         }
         sh[e] = low;
       }

@@ -99,6 +99,32 @@ def test_pack_of_large_matrices(cabi, K, N, bits, G, C, offset):
         assert np.array_equal(a.cpu().numpy().view(np.uint8), ref[key].view(np.uint8)), key
 
 
+@pytest.mark.parametrize("N,G,dtype", [(64, 128, np.float16), (64, 128, np.float32), (64, 12, np.float16), (400, 128, np.float16)])
+def test_cherry_columns_beyond_32767(cabi, N, G, dtype):
+    """The indices are 16-bit words: as signed numbers the upper half of a layer's columns would be negative.  All pack kernels,
+    both unpack kernels, and the row and GEMM kernels on the layer."""
+    from types import SimpleNamespace
+    from cherryq_b200 import QuantLinear
+    K, C = 33024, 8
+    rng = np.random.default_rng(N + G)
+    idx = rng.permutation([0, 100, 32766, 32767, 32768, 32769, 33000, K - 1])
+    w = (rng.normal(size=(N, K)) * 0.02).astype(dtype)
+    ref = O.pack(w, idx, 4, G)
+    got = gpu_pack(cabi, w, idx, 4, G)
+    for key in ("qweight", "scales", "cherry_weight", "cherry_indices"):
+        assert np.array_equal(got[key].view(np.uint8), ref[key].view(np.uint8)), key
+    columns = ref["cherry_indices"].view(np.uint16).astype(np.int32)
+    dense = O.unpack(ref["qweight"], ref["scales"], ref["cherry_weight"], columns, 4, G, K)
+    assert np.array_equal(gpu_unpack(cabi, ref, 4, K, G).view(np.uint16), dense.view(np.uint16))
+    if dtype == np.float16 and G == 128:
+        lin = QuantLinear(4, G, None, C / K, K, N, bias=False).cuda()
+        lin.pack(SimpleNamespace(weight=dev(w), bias=None, cherry_indices=dev(idx.astype(np.int32)), group_size=G))
+        for m in (1, 40):
+            x = torch.randn(m, K, device="cuda").half()
+            want = x.double() @ dev(dense).double().T
+            assert float((lin(x).double() - want).abs().max() / want.abs().max()) <= 2e-3       # fp16 output, as in the parity tests
+
+
 @pytest.mark.parametrize("offset", [0, 1])
 @pytest.mark.parametrize("K,N,bits,G,C", [(904, 13928, 3, 1, 8), (1032, 12232, 4, 4, 24), (1160, 10856, 3, 12, 32),
                                           (2048, 6152, 4, 96, 64), (1024, 12296, 3, 64, 0)])
