@@ -221,7 +221,7 @@ class CherryDecoder:
         return y, hs
 
     def _norm_lins(self, lay, names, h: torch.Tensor, delta, w: torch.Tensor):
-        """The projections `names` of rmsnorm(h + delta) * w, and h + delta: up to four rows in one launch."""
+        """The projections `names` of rmsnorm(h + delta) * w, and h + delta: one row in one launch."""
         if self.dense:
             xn, h = self._norm(h, delta, w)
             return self._lins(lay, names, xn), h

@@ -365,13 +365,17 @@ def forward_shared_input(layers, x: torch.Tensor):
 
 def forward_normed_input(layers, h: torch.Tensor, delta, weight: torch.Tensor, eps: float):
     """(outputs, h + delta): the layers applied to the RMS norm of h + delta (delta may be None), the residual stream of the
-    reference's decoder layer (llama/modeling_llama_quant.py:724-785).  Up to four fp16 rows: the norm rides in the
-    launch of forward_shared_input; everything else is the norm kernel and that function."""
+    reference's decoder layer (llama/modeling_llama_quant.py:724-785).  One fp16 row: the norm rides in the
+    launch of forward_shared_input; everything else is the norm kernel and that function.
+
+    Every CTA reads the whole rows twice, row after row, so the launch saved pays for one row only.  Microseconds with the norm
+    inside and in front, one and two rows: 4096 -> 3 x 4096 8.0 and 9.3, 21.5 and 19.3; 8192 -> (8192, 1024, 1024) 12.1 and 13.1,
+    27.0 and 25.1; 16384 -> 2 x 4096 18.0 and 18.7, 31.0 and 28.0; four rows 25.6 and 23.0, 34.3 and 29.7, 40.3 and 32.5."""
     layers = list(layers)
     qc = load_quant_cuda()
     rows = h.numel() // h.shape[-1]
     plain = all(t is None or (t.dtype == torch.float16 and t.is_contiguous() and t.data_ptr() % 16 == 0) for t in (h, delta, weight))
-    rls = _row_copies(layers, rows) if rows <= 4 and plain and h.dim() == 2 else None
+    rls = _row_copies(layers, rows) if rows == 1 and plain and h.dim() == 2 else None
     if rls is None:
         if delta is None:
             return forward_shared_input(layers, qc.rmsnorm(h, None, weight, eps, False)[0]), h

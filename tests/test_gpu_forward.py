@@ -119,6 +119,25 @@ def test_norm_in_front_of_a_shared_input(K, bits, G, m, with_delta):
         assert float((out.float() - ref).norm()) <= 3e-4 * float(ref.norm()) and out.shape == (m, lin.out_features)
 
 
+@pytest.mark.parametrize("K,bits,G", [(2048, 4, 128), (1032, 3, 64), (9216, 3, 128)])
+@pytest.mark.parametrize("m", [1, 2, 3, 4])
+def test_row_kernel_with_the_norm_in_front(K, bits, G, m):
+    """The operator itself, for all the rows that it takes."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    lins = [packed(K, n, bits, G, s) for s, n in ((1, 264), (2, 520))]
+    h, delta = torch.randn(m, K, device="cuda").half() * 3, torch.randn(m, K, device="cuda").half()
+    w = (torch.randn(K, device="cuda") * 0.1 + 1).half()
+    buf = torch.empty(m, 784, dtype=torch.float16, device="cuda")
+    outs = list(buf.split([264, 520], dim=1))
+    total = qc.row_layers_matvec_norm([l.row_layer(m) for l in lins], h, delta, w, 1e-5, outs)
+    y, want = qc.rmsnorm(h, delta, w, 1e-5, True)
+    assert torch.equal(total, want)
+    for lin, out in zip(lins, outs):
+        ref = lin(y).float()
+        assert float((out.float() - ref).norm()) <= 3e-4 * float(ref.norm())           # as in test_norm_in_front_of_a_shared_input
+
+
 @pytest.mark.parametrize("bits,G", [(4, 128), (3, 64)])
 @pytest.mark.parametrize("shape", [(9,), (2, 16), (33,)])
 def test_shared_input_beyond_the_row_kernel(bits, G, shape):

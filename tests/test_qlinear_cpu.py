@@ -106,3 +106,31 @@ def test_layers_that_share_an_input_keep_their_own_calls(kind, monkeypatch):
         assert qlinear._tile_copies(lins, x, 16) is None
     finally:
         remove()
+
+
+@pytest.mark.parametrize("rows", [1, 2, 4, 5])
+def test_the_norm_rides_in_the_launch_for_one_row(rows, monkeypatch):
+    """For more rows the norm kernel in front of the layers is the faster way."""
+    from types import SimpleNamespace
+    from cherryq_b200 import qlinear
+    lins = [layer(), layer()]
+    for lin in lins:
+        lin.row_layer = lambda n=1: "copy"
+    calls = []
+
+    def rmsnorm(h, delta, weight, eps, with_sum):
+        calls.append("norm")
+        return h, h
+
+    def matvec(*args):
+        calls.append("layers")
+
+    def matvec_norm(rls, h, *args):
+        calls.append("layers with the norm")
+        return h
+    fake = SimpleNamespace(rmsnorm=rmsnorm, row_layers_matvec=matvec, row_layers_matvec_norm=matvec_norm)
+    monkeypatch.setattr(qlinear, "load_quant_cuda", lambda: fake)
+    h, w = torch.ones(rows, 1024, dtype=torch.float16), torch.ones(1024, dtype=torch.float16)
+    outs, total = qlinear.forward_normed_input(lins, h, h.clone(), w, 1e-5)
+    assert calls == (["layers with the norm"] if rows == 1 else ["norm", "layers"])
+    assert [o.shape for o in outs] == [(rows, 264)] * 2 and total is h
