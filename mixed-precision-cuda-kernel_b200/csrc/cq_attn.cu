@@ -8,12 +8,20 @@
 //     position's key is two or four 16-byte pieces, loaded straight from the cache: the order of the columns inside a
 //     step is free as long as both operands agree;
 //   * the sums land where P . V needs its A operand.  Rows 0-7 take the upper 11 bits of the weights, rows 8-15, which
-//     the heads leave empty, the next 11: weights keep the precision of fp32 sums at no cost;
+//     the heads leave empty, the next 11;
 //   * V is the B operand, two positions' 16-byte pieces interleaved in registers (which columns of the head an MMA
 //     covers is free, too).
 // A warp takes 16 positions a turn with all of their keys and values in flight, and keeps its own running maximum, sum
 // and weighted values; the warps meet once in shared memory, the ranges of positions (blockIdx.z) in the workspace, where
 // the CTA that arrives last merges them.
+//
+// Precision: a weight loses at most 2^-23 of itself in its two halves (a quarter of them their last bit), and what lies below
+// 2^-38 of the largest.  An MMA cuts its sums off instead of rounding them, the more the larger its addend, so each one
+// sums its 16 products alone and fp32 additions do the rest; sums are rescaled by whole powers of two, and added in pairs
+// where warps and ranges meet.  Outputs that differ from the correctly rounded result, against 64 bits over 100 calls of
+// 64- and 128-wide heads, 60 to 4096 positions: 1.1e-4 of them with scores of deviation 1 (the fp32 kernels of cq_model_ops.cu
+// 1.1e-4), 1.1e-3 with deviation 4 (1.25e-3); with the sums left to the MMAs it was 1.8e-4 and 1.7e-3.  The chains of MMAs
+// gone, a call is no slower: 64 query heads on 8 KV heads at 4000 positions, 16 sequences, 50 us and 53.
 //
 // ROPE: the step's rotary embedding and cache write ride along (one launch less a layer): queries are rotated on their way
 // into shared memory, the new position's key and value go into the caches by the CTA whose range ends with it.
@@ -28,17 +36,20 @@ constexpr int AM_HEADS = 8;                  // query heads of a CTA
 constexpr int AM_POS = 16;                   // positions of a turn
 constexpr int AM_MAX_SPLITS = 32;            // (a lane per range in the merge)
 
+// sums of 16 products, without an addend: the unit cuts its sums off, fp32 additions outside round them
 __device__ __forceinline__ void am_mma(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile(
-      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
+      "mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.f));
 }
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// 2^d of a whole number d <= 0; 0 below the normal numbers (and 1 for NaN, whose sums are NaN)
+__device__ __forceinline__ float whole_pow2(float d) { return __int_as_float(max(0, 127 + __float2int_rn(d)) << 23); }
 // 16 bytes of a cache; not as read-only data where the launch itself writes a row of it
 template <bool WRITTEN> __device__ __forceinline__ uint4 ld_cache(const __half* p) {
   if (!WRITTEN) return __ldg(reinterpret_cast<const uint4*>(p));
@@ -85,7 +96,7 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
   extern __shared__ __align__(16) float am_sum[];          // [warp][head][D]
   __shared__ __align__(16) __half s_q[AM_HEADS][D + 32];
   __shared__ float s_m[WARPS][AM_HEADS], s_l[WARPS][AM_HEADS];
-  __shared__ float s_f[AM_HEADS][AM_MAX_SPLITS], s_r[AM_HEADS][AM_MAX_SPLITS], s_tot[AM_HEADS];
+  __shared__ float s_f[AM_HEADS][AM_MAX_SPLITS], s_r[AM_HEADS][AM_MAX_SPLITS], s_top[AM_HEADS], s_tot[AM_HEADS];
   __shared__ int s_last;
   const int kvh = blockIdx.x, seq = blockIdx.y, split = blockIdx.z, nsplit = gridDim.z;
   const int G = H / KV, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g8 = lane >> 2, t4 = lane & 3;
@@ -138,11 +149,9 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
 
   const float scale2 = scale * 1.4426950408889634f;        // scores in powers of two
   float m = -INFINITY, l = 0.f;
-  float o[8 * VS][4];                        // MMA j + 8 s: its column n is column 64 s + 8 n + j of the head
+  float o[8 * VS][2];                        // MMA j + 8 s: its column n is column 64 s + 8 n + j of the head
 #pragma unroll
-  for (int i = 0; i < 8 * VS; ++i)
-#pragma unroll
-    for (int e = 0; e < 4; ++e) o[i][e] = 0.f;
+  for (int i = 0; i < 8 * VS; ++i) o[i][0] = o[i][1] = 0.f;
 
 #pragma unroll 1
   for (int base = warp * AM_POS; base < n_pos; base += WARPS * AM_POS) {
@@ -161,18 +170,17 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
       for (int i = 0; i < VS; ++i)
         vv[u][i] = p < n_pos ? ld_cache<ROPE>(v_cache + first + (size_t)p * row + 8 * g8 + 64 * i) : make_uint4(0, 0, 0, 0);
     }
-    float s[2][4];
-#pragma unroll
-    for (int h = 0; h < 2; ++h)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) s[h][e] = 0.f;
+    float s[2][2] = {};
 #pragma unroll
     for (int i = 0; i < KP; ++i) {
       const uint4 qa = *reinterpret_cast<const uint4*>(mine_q + 32 * i);
 #pragma unroll
       for (int h = 0; h < 2; ++h) {
-        am_mma(s[h], qa.x, 0u, qa.y, 0u, kk[h][i].x, kk[h][i].y);
-        am_mma(s[h], qa.z, 0u, qa.w, 0u, kk[h][i].z, kk[h][i].w);
+        float d0[4], d1[4];
+        am_mma(d0, qa.x, 0u, qa.y, 0u, kk[h][i].x, kk[h][i].y);
+        am_mma(d1, qa.z, 0u, qa.w, 0u, kk[h][i].z, kk[h][i].w);
+        s[h][0] += d0[0] + d1[0];
+        s[h][1] += d0[1] + d1[1];
       }
     }
     // this lane: head g8, positions base + 8 h + 2 t4 + e
@@ -180,29 +188,24 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        s[h][e] = base + 8 * h + 2 * t4 + e < n_pos ? s[h][e] * scale2 : -INFINITY;
-        top = fmaxf(top, s[h][e]);
-      }
+      for (int e = 0; e < 2; ++e) top = fmaxf(top, base + 8 * h + 2 * t4 + e < n_pos ? s[h][e] * scale2 : -INFINITY);
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
     top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
-    // (no finite score so far: weights 0, or NaN where a score is NaN, which no maximum shows)
+    // A whole number at or above the maximum, so that rescaling sums is exact.  (No finite score so far: weights 0, or NaN
+    // where a score is NaN, which no maximum shows.)
+    top = ceilf(top);
     const float ref = top == -INFINITY ? 0.f : top;
-    const float keep = ex2(m - ref);         // (m = -infinity: 0)
+    const float keep = whole_pow2(m - ref);
     m = top;
-    // weights times 2^15: the halves of their split then reach down to 2^-39 of the largest
+    // weights times 2^15: the halves of their split then reach down to 2^-38 of the largest.  (One rounding between the score
+    // and the exponent, of the size of the exponent, not of the score.)
     float w[2][2];
 #pragma unroll
     for (int h = 0; h < 2; ++h)
 #pragma unroll
-      for (int e = 0; e < 2; ++e) w[h][e] = ex2(s[h][e] - ref + 15.f);
+      for (int e = 0; e < 2; ++e)
+        w[h][e] = base + 8 * h + 2 * t4 + e < n_pos ? 32768.f * ex2(__fmaf_rn(s[h][e], scale2, -ref)) : 0.f;
     l = l * keep + ((w[0][0] + w[0][1]) + (w[1][0] + w[1][1]));
-    if (__any_sync(0xffffffffu, keep != 1.f)) {
-#pragma unroll
-      for (int i = 0; i < 8 * VS; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) o[i][e] *= keep;
-    }
     const uint2 w0 = split_weights(w[0][0], w[0][1]), w1 = split_weights(w[1][0], w[1][1]);
 #pragma unroll
     for (int i = 0; i < VS; ++i) {
@@ -213,7 +216,10 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
         const uint32_t sel = (j & 1) ? 0x7632u : 0x5410u;
-        am_mma(o[8 * i + j], w0.x, w0.y, w1.x, w1.y, __byte_perm(v0[j >> 1], v1[j >> 1], sel), __byte_perm(v2[j >> 1], v3[j >> 1], sel));
+        float d[4];
+        am_mma(d, w0.x, w0.y, w1.x, w1.y, __byte_perm(v0[j >> 1], v1[j >> 1], sel), __byte_perm(v2[j >> 1], v3[j >> 1], sel));
+        o[8 * i + j][0] = o[8 * i + j][0] * keep + (d[0] + d[2]);
+        o[8 * i + j][1] = o[8 * i + j][1] * keep + (d[1] + d[3]);
       }
     }
   }
@@ -232,42 +238,66 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
 #pragma unroll
         for (int j = 0; j < 8; j += 4)
           *reinterpret_cast<float4*>(to + 64 * i + 8 * (2 * t4 + c) + j) =
-              make_float4(o[8 * i + j][c] + o[8 * i + j][2 + c], o[8 * i + j + 1][c] + o[8 * i + j + 1][2 + c],
-                          o[8 * i + j + 2][c] + o[8 * i + j + 2][2 + c], o[8 * i + j + 3][c] + o[8 * i + j + 3][2 + c]);
+              make_float4(o[8 * i + j][c], o[8 * i + j + 1][c], o[8 * i + j + 2][c], o[8 * i + j + 3][c]);
   }
   __syncthreads();
-  for (int e = tid; e < G * D; e += THREADS) {
-    const int g = e / D, d = e - g * D;
-    float top = -INFINITY;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) top = fmaxf(top, s_m[w][g]);
-    float sum = 0.f, tot = 0.f;
+  // the warps' shares in each head's sums: a warp without a finite score has none, unless its sum is NaN
+  for (int g = warp; g < G; g += WARPS) {
+    const float mw = lane < WARPS ? s_m[lane][g] : -INFINITY, lw = lane < WARPS ? s_l[lane][g] : 0.f;
+    float top = mw;
+    for (int d = 8; d; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
+    const float f = mw == -INFINITY ? (lw == 0.f ? 0.f : 1.f) : whole_pow2(mw - top);
+    float tot = f == 0.f ? 0.f : f * lw;
+    for (int d = 8; d; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
+    if (lane < WARPS) s_f[g][lane] = f;
+    if (lane == 0) {
+      s_top[g] = top;
+      s_tot[g] = tot;
+    }
+  }
+  __syncthreads();
+  for (int e = tid; e < G * D / 4; e += THREADS) {
+    const int g = e / (D / 4), d = 4 * (e - g * (D / 4));
+    float4 sums[WARPS];
 #pragma unroll
     for (int w = 0; w < WARPS; ++w) {
-      // a warp without a finite score adds nothing, unless its sum is NaN
-      const float lw = s_l[w][g], f = s_m[w][g] == -INFINITY ? (lw == 0.f ? 0.f : 1.f) : ex2(s_m[w][g] - top);
-      if (f != 0.f) {
-        sum += f * am_sum[(w * AM_HEADS + g) * D + d];
-        tot += f * lw;
-      }
+      const float f = s_f[g][w];
+      const float4 x = *reinterpret_cast<const float4*>(am_sum + (w * AM_HEADS + g) * D + d);
+      sums[w] = f != 0.f ? make_float4(f * x.x, f * x.y, f * x.z, f * x.w) : make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    if (!(fabsf(sum) <= 3.0e38f) && tot == tot) {
+#pragma unroll
+    for (int n = WARPS; n > 1; n = (n + 1) / 2)             // (pairs of pairs: fewer roundings in a row)
+#pragma unroll
+      for (int w = 0; w < n / 2; ++w) {
+        sums[w].x += sums[n - 1 - w].x;
+        sums[w].y += sums[n - 1 - w].y;
+        sums[w].z += sums[n - 1 - w].z;
+        sums[w].w += sums[n - 1 - w].w;
+      }
+    float sum[4] = {sums[0].x, sums[0].y, sums[0].z, sums[0].w};
+    const float top = s_top[g], tot = s_tot[g];
+    if (!(fabsf(sum[0]) + fabsf(sum[1]) + fabsf(sum[2]) + fabsf(sum[3]) <= 3.0e38f) && tot == tot) {
       // An infinite or NaN value takes part.  The two halves of a weight turn infinity into NaN where the product does
-      // not: this column is added again, weight by weight.
-      sum = 0.f;
+      // not: these columns are added again, weight by weight.
+      sum[0] = sum[1] = sum[2] = sum[3] = 0.f;
       for (int p = 0; p < n_pos; ++p) {
         const __half* kr = k_cache + first + (size_t)p * row;
         float dot = 0.f;
         for (int c = 0; c < D; ++c) dot += __half2float(s_q[g][c]) * __half2float(kr[c]);
-        sum += ex2(dot * scale2 - (top == -INFINITY ? 0.f : top) + 15.f) * __half2float(v_cache[first + (size_t)p * row + d]);
+        const float w = 32768.f * ex2(__fmaf_rn(dot, scale2, top == -INFINITY ? 0.f : -top));
+#pragma unroll
+        for (int c = 0; c < 4; ++c) sum[c] += w * __half2float(v_cache[first + (size_t)p * row + d + c]);
       }
     }
     if (nsplit == 1) {
-      out[(head0 + g) * D + d] = __float2half(sum / tot);
+      __half2* to = reinterpret_cast<__half2*>(out + (head0 + g) * D + d);
+      to[0] = __floats2half2_rn(sum[0] / tot, sum[1] / tot);
+      to[1] = __floats2half2_rn(sum[2] / tot, sum[3] / tot);
     } else {
       float* mine = part + ((head0 + g) * nsplit + split) * (size_t)(D + 2);
-      mine[2 + d] = sum;
-      if (d == 0) { mine[0] = top; mine[1] = tot; }
+      *reinterpret_cast<float2*>(mine + 2 + d) = make_float2(sum[0], sum[1]);
+      *reinterpret_cast<float2*>(mine + 4 + d) = make_float2(sum[2], sum[3]);
+      if (d == 0) *reinterpret_cast<float2*>(mine) = make_float2(top, tot);
     }
   }
   if (nsplit == 1) return;
@@ -292,7 +322,7 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
     const float mr = lane < nsplit ? s_f[g][lane] : -INFINITY, lr = lane < nsplit ? s_r[g][lane] : 0.f;
     float top = mr;
     for (int d = 16; d; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
-    const float f = mr == -INFINITY ? (lr == 0.f ? 0.f : 1.f) : ex2(mr - top);      // an empty range carries no weight
+    const float f = mr == -INFINITY ? (lr == 0.f ? 0.f : 1.f) : whole_pow2(mr - top);      // an empty range carries no weight
     float tot = f == 0.f ? 0.f : f * lr;
     for (int d = 16; d; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
     if (lane < nsplit) s_f[g][lane] = f;
@@ -302,17 +332,20 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
   for (int e = tid; e < G * D / 2; e += THREADS) {
     const int g = e / (D / 2), d = 2 * (e - g * (D / 2));
     const float* src = all + (size_t)g * nsplit * (D + 2) + 2 + d;
-    float2 v = make_float2(0.f, 0.f);
-#pragma unroll 8
-    for (int r = 0; r < nsplit; ++r) {
-      const float2 x = __ldcg(reinterpret_cast<const float2*>(src + (size_t)r * (D + 2)));
-      const float f = s_f[g][r];
-      if (f != 0.f) {
-        v.x += f * x.x;
-        v.y += f * x.y;
+    float2 v[4] = {};
+    for (int r0 = 0; r0 < nsplit; r0 += 8) {
+      float2 x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u) x[u] = __ldcg(reinterpret_cast<const float2*>(src + (size_t)min(r0 + u, nsplit - 1) * (D + 2)));
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const float f = r0 + u < nsplit ? s_f[g][r0 + u] : 0.f;
+        v[u & 3].x = f != 0.f ? __fmaf_rn(f, x[u].x, v[u & 3].x) : v[u & 3].x;
+        v[u & 3].y = f != 0.f ? __fmaf_rn(f, x[u].y, v[u & 3].y) : v[u & 3].y;
       }
     }
-    *reinterpret_cast<__half2*>(out + (head0 + g) * D + d) = __floats2half2_rn(v.x / s_tot[g], v.y / s_tot[g]);
+    *reinterpret_cast<__half2*>(out + (head0 + g) * D + d) =
+        __floats2half2_rn(((v[0].x + v[1].x) + (v[2].x + v[3].x)) / s_tot[g], ((v[0].y + v[1].y) + (v[2].y + v[3].y)) / s_tot[g]);
   }
   if (tid == 0) counters[cidx] = 0u;                       // ready for the next launch
 }
