@@ -25,6 +25,7 @@
 //
 // ROPE: the step's rotary embedding and cache write ride along (one launch less a layer): queries are rotated on their way
 // into shared memory, the new position's key and value go into the caches by the CTA whose range ends with it.
+#include <algorithm>
 #include <type_traits>
 
 #include "cq_attn.cuh"
@@ -352,15 +353,26 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
 
 }  // namespace
 
-bool cq_attn_mma_takes(int sequences, int n_heads, int n_kv_heads, int head_dim, int max_seq) {
-  const int G = n_heads / n_kv_heads;
+bool cq_attn_mma_takes(int sequences, int n_heads, int n_kv_heads, int head_dim, int max_seq, bool step) {
+  const int G = n_heads / n_kv_heads, sms = cq_sm_count();
   if ((head_dim != 64 && head_dim != 128) || G > AM_HEADS) return false;
   // Without grouped queries the two-sweep kernel has four CTAs of 256 threads on an SM against three of 128 here.  Up to one
-  // wave of those, and for well-filled waves on short caches, this kernel is faster (128-wide heads on cold caches: 32 at
-  // 256 positions 5.8 us against 7.1, at 2100 13.5 and 17.7; 256 at 200 10.5 and 12.9; 320 at 2100 70 and 81; 1280 at 200
-  // 32 and 37), beyond it is not (480 at 700 47 and 37, 1024 at 3900 331 and 322).
-  const long long tasks = (long long)sequences * n_kv_heads, slots = 3ll * cq_sm_count();
+  // wave of those, and for well-filled waves on short caches, this kernel is faster (128-wide heads on cold caches: 40 at
+  // 2200 positions 15.0 us against 19.5; 256 at 192 9.0 and 11.1; 320 at 2200 70 and 81; 1280 at 512 60 and 68), beyond it is
+  // not (512 at 512 37 and 29, 1024 at 4096 325 and 317).
+  const long long tasks = (long long)sequences * n_kv_heads, slots = 3ll * sms;
   const long long waves = (tasks + slots - 1) / slots;
+  if (!step) {
+    // Where the rotation is not part of the call (its launch less, 1.9 us, makes up for it): one CTA for each of up to 148
+    // heads at once, on caches just beyond one turn of twelve warps (256 positions, 32 heads 6.3 us against 4.9, 64 on 8 KV
+    // heads 5.3 and 4.5); one-sweep CTAs of 256 positions that fill the chip once (32 heads at 1024 9.8 and 8.9); about two CTAs
+    // of four warps on an SM on long caches (256 heads, 64-wide, 4096 positions 59 and 53; up to 2048 positions a full cache
+    // takes up to 5 % longer here, one that is filled to a tenth half the time: 1024 21.5 and 19.8, 4.5 and 9.5).
+    const long long one_sweep = tasks * ((max_seq + 255) / 256);
+    if (head_dim == 128 && max_seq > 12 * AM_POS && max_seq <= 256 && (long long)sequences * n_heads <= sms) return false;
+    if (head_dim == 128 && G == 1 && max_seq >= 1024 && one_sweep <= sms && 10 * one_sweep >= 8 * sms) return false;
+    if (G == 1 && 2 * tasks > 3ll * sms && tasks <= 2ll * sms && max_seq > 2048) return false;
+  }
   return G > 1 || waves == 1 || (max_seq <= 512 && 10 * tasks >= 8 * waves * slots);
 }
 
@@ -368,31 +380,35 @@ int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, 
                        int n_heads, int n_kv_heads, int head_dim, int max_seq, float scale, int most, unsigned int* counters,
                        float* part, cudaStream_t stream, const void* k_new, const void* v_new, const float* cos_table,
                        const float* sin_table) {
-  // Twelve warps a CTA, one CTA an SM, and the ranges that cost the fewest turns in a row: a wave's turn brings 192
-  // positions to every SM; a range's start and its warps' meeting count as 1.2 turns, the merge of the ranges as one and
-  // more with the heads it is for.  (64 query heads on 8 KV heads at 4000 positions: 1 sequence 14 us, 4 24, 16 53, 32 101;
-  // the fp32 dot products took 47, 112, 283 and 457, flash_attn 20, 27, 64 and 194.)  Without grouped queries: more heads
-  // than SMs take CTAs of four warps, three on an SM (256 heads at 200 positions 10.5 us against 13.5, 320 at 2100 70 and
-  // 78), and so do few heads on short caches, one turn for each range of 64 positions (32 heads at 500 positions 7.3 us
-  // against 8.3).
+  // CTAs of twelve warps, one on an SM, or of four, three on an SM, and ranges of positions: what takes the least time by a
+  // model.  A turn brings 16 positions to each warp, in at least the latency of its loads (1.75 us with 128-wide heads, 1.0
+  // with 64), or what the warps of an SM need together; a CTA's start and its warps' meeting take 3 us, ranges their merge.
+  // Over 615 calls (1 to 1280 heads, 128 to 4096 positions) the plan is within 1 % of the best one measured, on average.  64
+  // query heads on 8 KV heads at 4096 positions: 1 sequence 12.5 us, 4 20, 16 50, 32 93; the fp32 dot products took 47, 103,
+  // 271 and 429, flash_attn 20, 27, 64 and 194.  32 heads at 512 positions 7.4 us, against 8.1 of the two-sweep kernel; 160 at
+  // 4096 63 and 78.
   const int sms = cq_sm_count(), G = n_heads / n_kv_heads;
   const long long tasks = (long long)sequences * n_kv_heads;
-  const bool few = G == 1 && max_seq > 256 && max_seq <= 512 && tasks * 8 <= 3ll * sms;
-  const int warps = few || (G == 1 && tasks > sms) ? 4 : 12;
+  const double latency = head_dim == 64 ? 1.0 : 1.75, full = head_dim == 64 ? 1.3 : 2.1;      // us a turn: few warps, twelve
   if (most > AM_MAX_SPLITS) most = AM_MAX_SPLITS;
-  int splits = few ? 8 : 1;
-  if (warps == 12) {
-    double best = 0;
+  int warps = 12, splits = 1;
+  double best = 0;
+  for (int w = 12; w >= 4; w -= 8)
     for (int n = 1; n <= most; ++n) {
-      const long long waves = (tasks * n + sms - 1) / sms;
-      const int turns = ((max_seq + n - 1) / n + 12 * AM_POS - 1) / (12 * AM_POS);
-      const double t = (double)waves * (turns + 1.2) + (n > 1 ? 1.0 + 0.15 * G + 0.05 * n : 0.0);
-      if (n == 1 || t < best) {
+      const int per_sm = AM_SM_WARPS / w;
+      const long long waves = (tasks * n + per_sm * sms - 1) / (per_sm * sms), fullest = (tasks * n + sms - 1) / sms;
+      const int turns = ((max_seq + n - 1) / n + w * AM_POS - 1) / (w * AM_POS);
+      const double turn = std::max(latency, full * (double)std::min<long long>(per_sm, fullest) / per_sm);
+      double t = (double)waves * (turns * turn + 3.0) + (n > 1 ? 1.7 + 0.3 * n + 0.3 * G : 0.0);
+      // Ranges in several waves must pay for what they cost while the cache is nearly empty (320 64-wide heads, a tenth of 2048
+      // positions: one range 8.0 us, four 14.2; all of them 43 both).
+      if (n > 1 && waves > 1) t *= 1.2;
+      if ((w == 12 && n == 1) || t < best) {
         best = t;
+        warps = w;
         splits = n;
       }
     }
-  }
   auto pick = [&](auto rope) {
     constexpr bool R = decltype(rope)::value;
     return head_dim == 64 ? (warps == 4 ? attn_decode_mma_kernel<64, 4, R> : attn_decode_mma_kernel<64, 12, R>)

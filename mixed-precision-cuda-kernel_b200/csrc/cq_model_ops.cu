@@ -771,7 +771,7 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
   const int G = n_heads / n_kv_heads;
   const bool wide = (head_dim == 64 || head_dim == 128 || head_dim == 256) &&
                     (((uintptr_t)q | (uintptr_t)k_cache | (uintptr_t)v_cache) & 15) == 0;
-  if (wide && ((uintptr_t)out & 3) == 0 && cq_attn_mma_takes(sequences, n_heads, n_kv_heads, head_dim, max_seq))
+  if (wide && ((uintptr_t)out & 3) == 0 && cq_attn_mma_takes(sequences, n_heads, n_kv_heads, head_dim, max_seq, false))
     return cq_attn_mma_launch(q, k_cache, v_cache, position, out, sequences, n_heads, n_kv_heads, head_dim, max_seq, scale,
                               ATT_MAX_SPLITS, counters, part, (cudaStream_t)stream);
   const int sms = cq_sm_count();
@@ -835,7 +835,7 @@ extern "C" int cq_attn_decode_step(void* q, void* k, const void* v, const float*
     return CQ_ERR_BAD_SHAPE;
   const uintptr_t all = (uintptr_t)q | (uintptr_t)k | (uintptr_t)v | (uintptr_t)cos_table | (uintptr_t)sin_table |
                         (uintptr_t)k_cache | (uintptr_t)v_cache | (uintptr_t)out;
-  if ((all & 15) == 0 && cq_attn_mma_takes(sequences, n_heads, n_kv_heads, head_dim, max_seq)) {
+  if ((all & 15) == 0 && cq_attn_mma_takes(sequences, n_heads, n_kv_heads, head_dim, max_seq, true)) {
     const size_t heads = (size_t)sequences * n_heads;
     float* part = (float*)((uint8_t*)workspace + (heads * sizeof(unsigned int) + 255) / 256 * 256);
     return cq_attn_mma_launch(q, k_cache, v_cache, position, out, sequences, n_heads, n_kv_heads, head_dim, max_seq, scale,
