@@ -122,7 +122,7 @@ template <typename T> __device__ __forceinline__ uint32_t fq_larger(uint32_t u) 
   return max(__float_as_uint(f.x), __float_as_uint(f.y));
 }
 
-constexpr int FQ_LIST = 1024;                // octets on the list; more are looked for again on each turn
+constexpr int FQ_LIST = 1024;                // octets on the list; more are done among the others
 
 // FQ_ROWS rows a turn: one look at the table for all, their loads in flight together.
 template <typename T, int FQ_ROWS>
@@ -138,14 +138,18 @@ __global__ void __launch_bounds__(FQ_THREADS, 4) fake_quant_pairs_kernel(const T
   if (tid == 0) s_n = 0;
   for (int g = tid; g < FQ_ROWS * ng; g += FQ_THREADS) gmax[g] = 0u;
   __syncthreads();
-  for (int o = tid; o < n_oct; o += FQ_THREADS)
-    if (!whole(table[o])) {
-      const int at = atomicAdd(&s_n, 1);
-      if (at < FQ_LIST) list[at] = o;
-    }
-  __syncthreads();
-  const bool listed = s_n <= FQ_LIST;
-  const int n_list = listed ? s_n : n_oct;
+  // (an octet a thread and one row: a list costs more than it saves)
+  bool listed = FQ_ROWS > 1 || n_oct > FQ_THREADS;
+  if (listed) {
+    for (int o = tid; o < n_oct; o += FQ_THREADS)
+      if (!whole(table[o])) {
+        const int at = atomicAdd(&s_n, 1);
+        if (at < FQ_LIST) list[at] = o;
+      }
+    __syncthreads();
+    listed = s_n <= FQ_LIST;
+  }
+  const int n_list = listed ? s_n : 0;
   const float inv = 1.f / (float)(1 << (bits - 1));           // a power of two: the product is the quotient
   const uint32_t lim2 = F::narrow((float)((double)(1 << (bits - 1)) - 1e-2), (float)((double)(1 << (bits - 1)) - 1e-2));
   constexpr uint32_t ABS = 0x7FFF7FFFu;
@@ -155,13 +159,44 @@ __global__ void __launch_bounds__(FQ_THREADS, 4) fake_quant_pairs_kernel(const T
     const uint4* row[FQ_ROWS];                                // (rows past the matrix repeat its last one)
 #pragma unroll
     for (int r = 0; r < FQ_ROWS; ++r) row[r] = reinterpret_cast<const uint4*>(w + (size_t)(n + min(r, rows - 1)) * K);
-    // f(row, octet, table entry) for the octets that are not one whole group's
+    // f(row, octet, table entry) for the listed octets, and of one that is not on a list
     auto others = [&](auto f) {
       for (int i = tid; i < n_list * FQ_ROWS; i += FQ_THREADS) {
-        const int o = listed ? list[i / FQ_ROWS] : i / FQ_ROWS, r = i % FQ_ROWS;
-        const uint32_t t = table[o];
-        if (!whole(t) && r < rows) f(r, o, t);
+        const int o = list[i / FQ_ROWS], r = i % FQ_ROWS;
+        if (r < rows) f(r, o, table[o]);
       }
+    };
+    auto in_place = [&](int o, uint32_t t, auto f) {
+      if (listed) return;
+#pragma unroll 1
+      for (int r = 0; r < rows; ++r) f(r, o, t);
+    };
+    auto take_max = [&](int r, int o, uint32_t t) {
+      const uint4 v = reinterpret_cast<const uint4*>(w + (size_t)(n + r) * K)[o];
+      const uint32_t u[4] = {v.x, v.y, v.z, v.w}, next = (t >> 8) & 0xFFu, own = t & 0xFFu & ~next;
+      uint32_t a = 0, b = 0;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a = F::max(a, u[i] & ABS & fq_halves(own, 2 * i));
+        b = F::max(b, u[i] & ABS & fq_halves(next, 2 * i));
+      }
+      if (own) atomicMax(&gmax[r * ng + (t >> 16)], fq_larger<T>(a));
+      if (next) atomicMax(&gmax[r * ng + (t >> 16) + 1], fq_larger<T>(b));
+    };
+    auto write = [&](int r, int o, uint32_t t) {
+      const uint4 v = reinterpret_cast<const uint4*>(w + (size_t)(n + r) * K)[o];
+      const uint32_t next = (t >> 8) & 0xFFu, own = t & 0xFFu & ~next;
+      const uint2 s0 = scale[r * ng + (t >> 16)], s1 = next ? scale[r * ng + (t >> 16) + 1] : s0;
+      uint32_t u[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint32_t a = fq_halves(own, 2 * i), b = fq_halves(next, 2 * i);
+        uint32_t q = u[i] & ~(a | b);                             // cherry columns keep their value
+        q |= fq_pair<T>(u[i], __uint_as_float(s0.y), s0.x, lim2) & a;
+        q |= fq_pair<T>(u[i], __uint_as_float(s1.y), s1.x, lim2) & b;
+        u[i] = fq_through<T>(q, u[i], ste);
+      }
+      reinterpret_cast<uint4*>(out + (size_t)(n + r) * K)[o] = make_uint4(u[0], u[1], u[2], u[3]);
     };
     // ---- group maxima
     for (int o0 = tid & ~31; o0 < n_oct; o0 += FQ_THREADS) {
@@ -178,6 +213,8 @@ __global__ void __launch_bounds__(FQ_THREADS, 4) fake_quant_pairs_kernel(const T
 #pragma unroll
           for (int r = 0; r < FQ_ROWS; ++r)
             m[r] = fq_larger<T>(F::max(F::max(v[r].x & ABS, v[r].y & ABS), F::max(v[r].z & ABS, v[r].w & ABS)));
+        } else {
+          in_place(o, t, take_max);
         }
       }
       // one maximum per group and warp
@@ -192,18 +229,7 @@ __global__ void __launch_bounds__(FQ_THREADS, 4) fake_quant_pairs_kernel(const T
         if (lane < FQ_ROWS && top) atomicMax(&gmax[lane * ng + q], top);
       }
     }
-    others([&](int r, int o, uint32_t t) {
-      const uint4 v = reinterpret_cast<const uint4*>(w + (size_t)(n + r) * K)[o];
-      const uint32_t u[4] = {v.x, v.y, v.z, v.w}, next = (t >> 8) & 0xFFu, own = t & 0xFFu & ~next;
-      uint32_t a = 0, b = 0;
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        a = F::max(a, u[i] & ABS & fq_halves(own, 2 * i));
-        b = F::max(b, u[i] & ABS & fq_halves(next, 2 * i));
-      }
-      if (own) atomicMax(&gmax[r * ng + (t >> 16)], fq_larger<T>(a));
-      if (next) atomicMax(&gmax[r * ng + (t >> 16) + 1], fq_larger<T>(b));
-    });
+    others(take_max);
     __syncthreads();
     // ---- scales
     for (int g = tid; g < FQ_ROWS * ng; g += FQ_THREADS) {
@@ -216,7 +242,10 @@ __global__ void __launch_bounds__(FQ_THREADS, 4) fake_quant_pairs_kernel(const T
     // ---- weights
     for (int o = tid; o < n_oct; o += FQ_THREADS) {
       const uint32_t t = table[o];
-      if (!whole(t)) continue;
+      if (!whole(t)) {
+        in_place(o, t, write);
+        continue;
+      }
       uint4 v[FQ_ROWS];
 #pragma unroll
       for (int r = 0; r < FQ_ROWS; ++r) v[r] = row[r][o];
@@ -233,21 +262,7 @@ __global__ void __launch_bounds__(FQ_THREADS, 4) fake_quant_pairs_kernel(const T
         dst += n_oct;
       }
     }
-    others([&](int r, int o, uint32_t t) {
-      const uint4 v = reinterpret_cast<const uint4*>(w + (size_t)(n + r) * K)[o];
-      const uint32_t next = (t >> 8) & 0xFFu, own = t & 0xFFu & ~next;
-      const uint2 s0 = scale[r * ng + (t >> 16)], s1 = next ? scale[r * ng + (t >> 16) + 1] : s0;
-      uint32_t u[4] = {v.x, v.y, v.z, v.w};
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const uint32_t a = fq_halves(own, 2 * i), b = fq_halves(next, 2 * i);
-        uint32_t q = u[i] & ~(a | b);                             // cherry columns keep their value
-        q |= fq_pair<T>(u[i], __uint_as_float(s0.y), s0.x, lim2) & a;
-        q |= fq_pair<T>(u[i], __uint_as_float(s1.y), s1.x, lim2) & b;
-        u[i] = fq_through<T>(q, u[i], ste);
-      }
-      reinterpret_cast<uint4*>(out + (size_t)(n + r) * K)[o] = make_uint4(u[0], u[1], u[2], u[3]);
-    });
+    others(write);
   }
 }
 
@@ -338,9 +353,11 @@ extern "C" int cq_fake_quant(const void* weight, int dtype, const uint8_t* quant
   if (dtype == 1) {
     fake_quant_kernel<<<N, FQ_THREADS, (size_t)ng * 4, st>>>((const float*)weight, table, bits, K, ng, ste, (float*)out);
   } else {
-    // Four rows a turn where the matrix has a turn for every block that the chip holds and the groups of four rows fit
-    // shared memory comfortably; two waves of blocks, each of which makes its list once and goes down the rows.
-    const int blocks = 8 * cq_sm_count(), rows = N >= 2 * blocks && ng <= 1000 ? 4 : 1;
+    // Rows a turn: as many as leave the chip blocks enough, and whose groups fit shared memory comfortably.  4096 x 4096 bf16, one,
+    // two and four rows a turn: 33.4, 25.1 and 22.4 us (element by element 45.2); 1024 x 2048 13.0, 9.6 and 7.8 (10.5); 2048 x
+    // 1024 9.9, 7.9 and 8.0 (9.7); 4096 x 256 8.2, 8.3 and 9.2 (8.3).  Two waves of blocks at most, each of which makes its list
+    // once and goes down the rows.
+    const int blocks = 8 * cq_sm_count(), rows = ng > 1000 ? 1 : (N >= blocks ? 4 : (2 * N >= blocks ? 2 : 1));
     const int smem = rows * ng * 12, turns = (N + rows - 1) / rows;
     auto launch = [&](auto kernel, auto* wp, auto* op) -> int {
       CQ_CUDA_TRY(cq_grant_smem((const void*)kernel, smem));
@@ -349,7 +366,9 @@ extern "C" int cq_fake_quant(const void* weight, int dtype, const uint8_t* quant
     };
     auto pick = [&](auto* wp, auto* op) {
       using T = std::remove_pointer_t<decltype(op)>;
-      return rows == 4 ? launch(fake_quant_pairs_kernel<T, 4>, wp, op) : launch(fake_quant_pairs_kernel<T, 1>, wp, op);
+      return rows == 4   ? launch(fake_quant_pairs_kernel<T, 4>, wp, op)
+             : rows == 2 ? launch(fake_quant_pairs_kernel<T, 2>, wp, op)
+                         : launch(fake_quant_pairs_kernel<T, 1>, wp, op);
     };
     const int rc = dtype == 0 ? pick((const __half*)weight, (__half*)out) : pick((const __nv_bfloat16*)weight, (__nv_bfloat16*)out);
     if (rc != CQ_OK) return rc;
