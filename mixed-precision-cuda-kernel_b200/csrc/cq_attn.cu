@@ -366,12 +366,11 @@ bool cq_attn_mma_takes(int sequences, int n_heads, int n_kv_heads, int head_dim,
     // Where the rotation is not part of the call (its launch less, 1.9 us, makes up for it): one CTA for each of up to 148
     // heads at once, on caches just beyond one turn of twelve warps (256 positions, 32 heads 6.3 us against 4.9, 64 on 8 KV
     // heads 5.3 and 4.5); one-sweep CTAs of 256 positions that fill the chip once (32 heads at 1024 9.8 and 8.9); about two CTAs
-    // of four warps on an SM on long caches (256 heads, 64-wide, 4096 positions 59 and 53; up to 2048 positions a full cache
-    // takes up to 5 % longer here, one that is filled to a tenth half the time: 1024 21.5 and 19.8, 4.5 and 9.5).
+    // an SM of 64-wide heads on long caches (256 heads at 1024 positions 20.9 and 19.1, 4096 59 and 53).
     const long long one_sweep = tasks * ((max_seq + 255) / 256);
     if (head_dim == 128 && max_seq > 12 * AM_POS && max_seq <= 256 && (long long)sequences * n_heads <= sms) return false;
     if (head_dim == 128 && G == 1 && max_seq >= 1024 && one_sweep <= sms && 10 * one_sweep >= 8 * sms) return false;
-    if (G == 1 && 2 * tasks > 3ll * sms && tasks <= 2ll * sms && max_seq > 2048) return false;
+    if (head_dim == 64 && G == 1 && 2 * tasks > 3ll * sms && tasks <= 2ll * sms && max_seq > 768) return false;
   }
   return G > 1 || waves == 1 || (max_seq <= 512 && 10 * tasks >= 8 * waves * slots);
 }
@@ -381,15 +380,14 @@ int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, 
                        float* part, cudaStream_t stream, const void* k_new, const void* v_new, const float* cos_table,
                        const float* sin_table) {
   // CTAs of twelve warps, one on an SM, or of four, three on an SM, and ranges of positions: what takes the least time by a
-  // model.  A turn brings 16 positions to each warp, in at least the latency of its loads (1.75 us with 128-wide heads, 1.0
-  // with 64), or what the warps of an SM need together; a CTA's start and its warps' meeting take 3 us, ranges their merge.
-  // Over 615 calls (1 to 1280 heads, 128 to 4096 positions) the plan is within 1 % of the best one measured, on average.  64
-  // query heads on 8 KV heads at 4096 positions: 1 sequence 12.5 us, 4 20, 16 50, 32 93; the fp32 dot products took 47, 103,
-  // 271 and 429, flash_attn 20, 27, 64 and 194.  32 heads at 512 positions 7.4 us, against 8.1 of the two-sweep kernel; 160 at
-  // 4096 63 and 78.
+  // model.  A turn brings 16 positions to each warp, in the latency of its loads where an SM has four warps, else in what its
+  // warps need together; a CTA's start and its warps' meeting take 3 us, ranges their merge.  Over 615 calls (1 to 1280 heads,
+  // 128 to 4096 positions) the plan is within 1 % of the best one measured, on average.  64 query heads on 8 KV heads at 4096
+  // positions: 1 sequence 12.5 us, 4 20, 16 50, 32 93; the fp32 dot products took 47, 103, 271 and 429, flash_attn 20, 27, 64
+  // and 194.  32 heads at 512 positions 7.4 us, against 8.1 of the two-sweep kernel; 160 at 4096 63 and 78.
   const int sms = cq_sm_count(), G = n_heads / n_kv_heads;
   const long long tasks = (long long)sequences * n_kv_heads;
-  const double latency = head_dim == 64 ? 1.0 : 1.75, full = head_dim == 64 ? 1.3 : 2.1;      // us a turn: few warps, twelve
+  const double latency = head_dim == 64 ? 1.0 : 1.75, full = head_dim == 64 ? 1.3 : 2.1;      // us a turn: four warps on an SM, more
   if (most > AM_MAX_SPLITS) most = AM_MAX_SPLITS;
   int warps = 12, splits = 1;
   double best = 0;
@@ -398,7 +396,7 @@ int cq_attn_mma_launch(const void* q, const void* k_cache, const void* v_cache, 
       const int per_sm = AM_SM_WARPS / w;
       const long long waves = (tasks * n + per_sm * sms - 1) / (per_sm * sms), fullest = (tasks * n + sms - 1) / sms;
       const int turns = ((max_seq + n - 1) / n + w * AM_POS - 1) / (w * AM_POS);
-      const double turn = std::max(latency, full * (double)std::min<long long>(per_sm, fullest) / per_sm);
+      const double turn = per_sm > 1 && fullest == 1 ? latency : full;
       double t = (double)waves * (turns * turn + 3.0) + (n > 1 ? 1.7 + 0.3 * n + 0.3 * G : 0.0);
       // Ranges in several waves must pay for what they cost while the cache is nearly empty (320 64-wide heads, a tenth of 2048
       // positions: one range 8.0 us, four 14.2; all of them 43 both).
