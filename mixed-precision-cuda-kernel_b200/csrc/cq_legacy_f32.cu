@@ -17,8 +17,8 @@
 // search for each octet's columns and a digit at a time, and codes were spread to bytes column by column: 1640 instructions
 // a warp and block of 128 columns).  Bound by the issue rate still.  512 columns share the staging, the columns are searched
 // once, the four digits of a value are one addition and one exclusive or, codes are taken out for four columns at once and
-// turned.  Other sizes, before and now: 1 row 33 and 21 us, 64 rows 190 and 103, 16384 x 28672 317 and 208, 1024 x 1024
-// 8.8 and 8.7.
+// turned; four cherry columns' loads are in flight (one after another a column took 0.5 us).  Other sizes, before and now: 1 row 33 and 21 us, 64 rows 190 and 103, 16384 x 28672 317 and 208, 1024 x 1024
+// 8.8 and 8.7; groups of 64 16 rows 58 and 32, 64 rows 221 and 117 (more than 8 rows: 20 bytes of registers spilled).
 #include <algorithm>
 
 #include "cq_common.cuh"
@@ -209,19 +209,42 @@ __global__ void __launch_bounds__(F32_THREADS, 1) matvec_f32_kernel(const __grid
     // ---- this part's share of the cherry columns
     const int share = (int)blockIdx.x - (int)gridDim.x + p.cherry_parts;
     const int c_end = share < 0 ? 0 : (int)((long long)p.C * (share + 1) / p.cherry_parts);
-#pragma unroll 4
-    for (int ci = share < 0 ? 0 : (int)((long long)p.C * share / p.cherry_parts); ci < c_end; ++ci) {
-      const float* xr = p.x + p.idx[ci];
-      float w[4];
-      load4(p.cw + (size_t)ci * p.N, w);
+    constexpr int AHEAD = 4;                                // columns whose loads are in flight together
+    for (int c0 = share < 0 ? 0 : (int)((long long)p.C * share / p.cherry_parts); c0 < c_end; c0 += AHEAD) {
+      int col[AHEAD];
+      float w[AHEAD][4], xv[AHEAD][TT][2];
 #pragma unroll
-      for (int t = 0; t < TT; ++t)
+      for (int u = 0; u < AHEAD; ++u) col[u] = c0 + u < c_end ? __ldg(p.idx + c0 + u) : -1;
+      if (p.aligned_f) {
 #pragma unroll
-        for (int e = 0; e < 2; ++e) {
-          const int m = m0 + 8 * t + 2 * c + e;
-          const float xv = m < p.M ? __ldg(xr + (size_t)m * p.K) : 0.f;
+        for (int u = 0; u < AHEAD; ++u) {
+          const float4 v = n < p.N && col[u] >= 0 ? __ldg(reinterpret_cast<const float4*>(p.cw + (size_t)(c0 + u) * p.N + n)) : make_float4(0.f, 0.f, 0.f, 0.f);
+          w[u][0] = v.x; w[u][1] = v.y; w[u][2] = v.z; w[u][3] = v.w;
+        }
+      } else {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) y[i][t][e] = __fmaf_rn(w[i], xv, y[i][t][e]);
+        for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) w[u][i] = n + i < p.N && col[u] >= 0 ? __ldg(p.cw + (size_t)(c0 + u) * p.N + n + i) : 0.f;
+      }
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u)
+#pragma unroll
+        for (int t = 0; t < TT; ++t)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            const int m = m0 + 8 * t + 2 * c + e;
+            xv[u][t][e] = m < p.M && col[u] >= 0 ? __ldg(p.x + (size_t)m * p.K + col[u]) : 0.f;
+          }
+#pragma unroll
+      for (int u = 0; u < AHEAD; ++u)
+        if (col[u] >= 0) {
+#pragma unroll
+          for (int t = 0; t < TT; ++t)
+#pragma unroll
+            for (int e = 0; e < 2; ++e)
+#pragma unroll
+              for (int i = 0; i < 4; ++i) y[i][t][e] = __fmaf_rn(w[u][i], xv[u][t][e], y[i][t][e]);
         }
     }
     __syncthreads();
@@ -336,11 +359,15 @@ int cq_launch_matvec_f32(const float* x, const uint8_t* q, const float* cw, cons
   }
   p.blk_per_part = per;
   p.n_parts = (p.n_blk + per - 1) / per;
-  // Cherry columns (18 take a warp as long as a block): parts of their own where SMs are left, four columns each; else the
-  // last part, which may be shorter, or more of the last ones where they are many.  (In every part they cost each one more
-  // rounding: 3 % more error at 1024 x 1024.  All in the last part there: 10.9 us and 8.8.)
-  const int spare = C > 0 ? std::min(slots / ny - p.n_parts, (C + 3) / 4) : 0, extra = spare > 0 ? spare : 0;
-  p.cherry_parts = extra > 0 ? extra : (C <= 16 ? 1 : std::min(p.n_parts, C / per + 1));
+  // Cherry columns (18 take a warp as long as a block): parts of their own where SMs are left, four columns each, unless they
+  // are so many that they take longer there than shared by the main parts; else the last part, which may be shorter, or more
+  // of the last ones where they are many.  (In every part they cost each one more rounding: 3 % more error at 1024 x 1024.  All
+  // in the last part there: 10.9 us and 8.8.  11008 x 4096, 16 rows, 344 cherry columns: one part of their own 112 us, all parts
+  // 28; 2048 x 2048, 512: 25 parts of their own 10.9, all parts 19.)
+  const int spare = C > 0 ? std::min(slots / ny - p.n_parts, (C + 3) / 4) : 0;
+  const double own = spare > 0 ? std::max((double)per, C / (18.0 * spare)) : 0.0, shared = per + 0.3 + C / (18.0 * p.n_parts);
+  const int extra = spare > 0 && own <= shared ? spare : 0;
+  p.cherry_parts = extra > 0 ? extra : (spare > 0 ? p.n_parts : (C <= 16 ? 1 : std::min(p.n_parts, C / per + 1)));
   p.aligned_q = N % 4 == 0 && ((uintptr_t)q & 3) == 0;
   p.aligned_f = N % 4 == 0 && ((uintptr_t)sf & 15) == 0 && ((uintptr_t)cw & 15) == 0 && ((uintptr_t)mul & 15) == 0;
   const int tt = M > 8 ? 2 : 1, halves = G == 64 ? 2 : 1;

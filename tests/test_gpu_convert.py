@@ -228,6 +228,13 @@ def test_fp32_operator_of_wide_layers(cabi, K, N, G, C, M):
     test_fp32_operator(cabi, K, N, G, C, M)
 
 
+@pytest.mark.parametrize("K,N,G,C,M", [(2048, 5632, 128, 512, 9), (2048, 5632, 64, 256, 1), (1024, 516, 128, 72, 16)])
+def test_fp32_operator_with_many_cherry_columns(cabi, K, N, G, C, M):
+    """Shared by the main parts although SMs are left, and in parts of their own, four at a time and what remains of them.  Bound
+    as in test_fp32_operator."""
+    test_fp32_operator(cabi, K, N, G, C, M)
+
+
 @pytest.mark.parametrize("K,N,C,M,ratio", [(1024, 264, 8, 9, 1e4), (2120, 40, 24, 3, 1e4), (1024, 264, 8, 17, 1e-5)])
 def test_fp32_operator_groups_of_unlike_magnitudes(cabi, K, N, C, M, ratio):
     """Groups of 64 columns whose activations are `ratio` times their neighbours' and whose scales as much smaller: the
