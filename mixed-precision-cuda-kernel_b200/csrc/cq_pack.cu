@@ -314,7 +314,7 @@ __global__ void __launch_bounds__(PG_WARPS * 32, PG_BLOCKS) pack_group_kernel(
   const int first = c_begin < c_end ? min(idx[c_begin], source[0]) : source[0];
   const int last = c_begin < c_end ? max(idx[c_end - 1], source[cols - 1]) : source[cols - 1];
   const int base = first & ~7, pieces = (last - base) / 8 + 1;
-  const bool wide = (reinterpret_cast<uintptr_t>(w) & 15) == 0 && pieces * 8 <= PG_SPAN;      // (K is a multiple of 8)
+  const bool wide = pieces * 8 <= PG_SPAN;                        // (K is a multiple of 8, w aligned to 16 bytes)
   // of each 32 columns: where the first is in the tile, how many cherry columns lie among them, the first of these
   const int parts = (cols + 31) / 32;
   if (tid < parts) {
@@ -344,7 +344,7 @@ __global__ void __launch_bounds__(PG_WARPS * 32, PG_BLOCKS) pack_group_kernel(
         dst += (dr * PG_STRIDE + 8 * dc) * 2;
       }
     } else {
-      // unaligned weights, or so many cherry columns inside the chunk that it does not fit: compact columns one by one
+      // so many cherry columns inside the chunk that it does not fit: compact columns one by one
       for (int j = lane; j < cols; j += 32) {
         const __half* src = w + (size_t)n0 * K + source[j];
 #pragma unroll 16
@@ -902,7 +902,15 @@ extern "C" int cq_pack(const void* weight, int weight_is_f32, const int32_t* che
   // From 12 million weights on a warp of pack_group_kernel has rows enough to go down (4096 x 11008 4-bit: 48.0 and 58.8 us;
   // 16384 x 28672 342 and 542; 4096 x 4096 22.9 and 24.9; 16384 x 1024 25.6 and 27.5; 4096 x 2048 16.5 and 16.5; 2048 x 1024
   // 12.3 and 10.3; 1032 x 1000 12.3 and 9.6).
-  if (!weight_is_f32 && (G == 64 || G == PK_COLS) && (long long)K * N >= (3ll << 22)) {
+  // Its weights come in 16 bytes at a time (off that alignment 4096 x 11008 would take 61 us, 55 with the other kernel), and each
+  // cherry column among them moves the others: with more than a cherry column in 128 the other kernel is faster on matrices
+  // below 25 million weights (2048 x 6144, one in 256 18.9 and 19.1, in 64 20.5 and 19.9, in 16 28 and 25, in 8 37 and 31) and on
+  // narrow ones (1024 x 24576, one in 32 34 and 36, in 8 54 and 46; 4096 x 8192, in 8 78 and 86), but its last blocks copy the
+  // cherry columns one after another (8192 x 1536, in 64 22 and 24, in 8 60 and 86; 1024 x 12288, in 4 26 and 38).
+  const long long weights_all = (long long)K * N;
+  const bool fits = (long long)C * 128 <= K || K >= 8192 || (long long)C * 5 >= K ||
+                    (weights_all >= (3ll << 23) && ((long long)C * 32 <= K || K >= 4096));
+  if (!weight_is_f32 && (G == 64 || G == PK_COLS) && weights_all >= (3ll << 22) && fits && ((uintptr_t)weight & 15) == 0) {
     const int n_x = (K - C + PK_COLS - 1) / PK_COLS, rows = PG_WARPS * PG_ROWS;
     auto kernel = bits == 4 ? pack_group_kernel<4> : pack_group_kernel<3>;
     kernel<<<dim3(n_x, row_blocks(n_x, (N + rows - 1) / rows, PG_BLOCKS)), PG_WARPS * 32, 0, st>>>(

@@ -99,6 +99,22 @@ def test_pack_of_large_matrices(cabi, K, N, bits, G, C, offset):
         assert np.array_equal(a.cpu().numpy().view(np.uint8), ref[key].view(np.uint8)), key
 
 
+@pytest.mark.parametrize("K,N,bits,G,C", [(1032, 12296, 4, 128, 8), (8192, 1544, 4, 64, 128), (2064, 12296, 3, 128, 64)])
+def test_pack_of_large_matrices_into_unaligned_codes(cabi, K, N, bits, G, C):
+    """On the kernel whose warps go down the rows, up to a cherry column in 128, in 64 of wide layers, in 32 of larger ones."""
+    w, idx = layer(K, N, C, np.float16, K + N)
+    ref = O.pack(w, idx, bits, G)
+    q = torch.zeros(ref["qweight"].size + 1, dtype=torch.uint8, device="cuda")
+    t = [dev(np.zeros_like(ref[k])) for k in ("scales", "cherry_weight", "cherry_indices")]
+    wd, idd = dev(w), dev(idx.astype(np.int32))
+    cabi.check(cabi.lib().cq_pack(ptr(wd), 0, ptr(idd), bits, K, N, C, G, q.data_ptr() + 1,
+                                  *[ptr(a) for a in t], None, None), "pack")
+    torch.cuda.synchronize()
+    assert np.array_equal(q[1:].cpu().numpy(), ref["qweight"].ravel())
+    for a, key in zip(t, ("scales", "cherry_weight", "cherry_indices")):
+        assert np.array_equal(a.cpu().numpy().view(np.uint8), ref[key].view(np.uint8)), key
+
+
 @pytest.mark.parametrize("N,G,dtype", [(64, 128, np.float16), (64, 128, np.float32), (64, 12, np.float16), (400, 128, np.float16)])
 def test_cherry_columns_beyond_32767(cabi, N, G, dtype):
     """The indices are 16-bit words: as signed numbers the upper half of a layer's columns would be negative.  All pack kernels,
