@@ -805,20 +805,6 @@ __global__ void __launch_bounds__(256, UP_BLOCKS) unpack_rows_kernel(
 #pragma unroll
           for (int j = 0; j < 4; ++j) reinterpret_cast<__half*>(slot + 16 * j)[e] = cw[(size_t)(low + t) * N + n + j];
         }
-        if (!whole && G < 8) {
-          // groups narrower than 8 columns can put more than two into an octet: column by column
-#pragma unroll 1
-          for (int e = 0, m = low; e < 8; ++e) {
-            if ((own >> e) & 1u) { ++m; continue; }
-            const int c = k + e - m;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float a = (float)((int)cq_ref_code(q, BITS, c, n + j, N) - (1 << (BITS - 1))) + 0.5f;
-              reinterpret_cast<__half*>(slot + 16 * j)[e] =
-                  __float2half_rn(__fmul_rn(a, __half2float(scales[(size_t)group_of(c) * N + n + j])));
-            }
-          }
-        }
       }
     }
     __syncthreads();                                            // (the other tile was read before this barrier)
@@ -970,11 +956,12 @@ extern "C" int cq_unpack_dense(const uint8_t* qweight, const void* scales, const
     kernel<<<dim3(n_cols, n_y), 256, 0, (cudaStream_t)stream>>>(qweight, (const __half*)scales, (const __half*)cherry_weight,
                                                                (const uint16_t*)cherry_indices, K, N, C, G, g_shift, (__half*)dense, aligned);
   };
-  // Up to a cherry column in 32, so that most octets have none (4096 x 11008 4-bit, new and old kernel: 16 cherry columns 36.9
-  // and 40.6 us, 64 40.2 and 43.9, 128 44.6 and 46.2, then see the old kernel), and
-  // from 12 million weights on, so that a block has rows to go down (4096 x 8192 19.4 and 21.6, 4096 x 4096 17.5 both, 1536 x
-  // 5000 9.3 and 9.0).  Matrices of few columns have no columns to spread over the chip but rows: 128 x 65536 13.4 and 12.2.
-  if ((long long)C * 32 <= K && n_cols >= 8 && (long long)K * N >= (3ll << 22)) {
+  // From 25 million weights on, so that a block has rows to go down, up to a cherry column in 48, so that most octets have none,
+  // and groups that put at most two into an octet.  New and old kernel: 4096 x 11008 4-bit, 16 cherry columns 36.9 us and 40.6, 64
+  // 40.2 and 43.9, 128 44.6 and 46.2, groups of 4 66 and 62; 16384 x 1024, 64 cherry columns 18.4 and 18.6, 512 25.3 and 20.0; 2048
+  // x 8192, groups of 96 17.3 and 17.0.  Matrices of few columns have no columns to spread over the chip but rows: 128 x 65536
+  // 13.4 and 12.2.
+  if ((long long)C * 48 <= K && G >= 8 && n_cols >= 8 && (long long)K * N >= (3ll << 23)) {
     const int n_y = row_blocks(n_cols, n_tiles, UP_BLOCKS);
     bits == 4 ? (C > 0 ? launch(unpack_rows_kernel<4, true>, n_y) : launch(unpack_rows_kernel<4, false>, n_y))
               : (C > 0 ? launch(unpack_rows_kernel<3, true>, n_y) : launch(unpack_rows_kernel<3, false>, n_y));

@@ -159,6 +159,14 @@ def test_unpack_going_down_the_rows(cabi, K, N, bits, G, C, offset):
     assert np.array_equal(out[offset:].cpu().numpy().view(np.uint16), dense.view(np.uint16).ravel())
 
 
+@pytest.mark.parametrize("offset", [0, 1])
+@pytest.mark.parametrize("K,N,bits,G,C", [(1032, 24416, 4, 12, 16), (1160, 21704, 3, 96, 24), (2056, 12256, 4, 64, 40), (1032, 24416, 3, 8, 8),
+                                          (1024, 24584, 3, 64, 0)])
+def test_unpack_of_the_largest_matrices(cabi, K, N, bits, G, C, offset):
+    """From 25 million weights on the blocks go down the rows: the edges of test_unpack_going_down_the_rows."""
+    test_unpack_going_down_the_rows(cabi, K, N, bits, G, C, offset)
+
+
 def test_unpack_into_unaligned_buffers(cabi):
     K, N, bits, G, C = 264, 72, 3, 128, 8
     w, idx = layer(K, N, C, np.float16, 5)
