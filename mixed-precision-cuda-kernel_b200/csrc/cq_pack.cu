@@ -104,8 +104,8 @@ __global__ void pack_codes_kernel(const void* __restrict__ w, int is_f32, const 
   }
 }
 
-// One pass over the weights for groups of several chunks of 128 compact columns (multiples of 128, one group per row) and
-// for fp32 weights: a block owns PK_ROWS output rows of one group (two 64-wide ones), reads them once in chunks, reduces
+// One pass over the weights for groups of several chunks of 128 compact columns (multiples of 128, one group per row), for
+// fp32 weights and for what the rule at cq_pack leaves of fp16 weights in groups of one chunk: a block owns PK_ROWS output rows of one group (two 64-wide ones), reads them once in chunks, reduces
 // the maxima and writes scales and codes.  The general pair of kernels above reads the matrix twice, lanes a row
 // apart, and divides per weight.  The loads are 2 bytes a lane, 64 contiguous bytes a warp, because the removed
 // cherry columns leave the compact columns at any alignment; the tile turns them so that a thread quantises 32
@@ -506,16 +506,11 @@ __global__ void __launch_bounds__(PG_WARPS * 32, PG_BLOCKS) pack_group_kernel(
 
 // ------------------------------------------------------------------ dense unpack
 // llama/qlinear.py:120-162: dense[n, k] = cherry ? cherry_weight : fp16((q + 0.5) * s).
-// A block keeps 128 original columns and goes down the rows, 64 at a time: what depends on the columns alone (the search for
-// the cherry columns among it) is done once, the next rows' codes are on their way while these are written.  A thread makes
-// one octet of 8 columns of four consecutive rows.  The octet's codes are consecutive compact columns: the bytes of two
-// compact octets (one 32-bit load per byte row covers the four rows), shifted by the position inside the first.  Pairs of
-// codes become mantissa bits of 1024; one exact multiply-add and the product with the scale, rounded once as in the
-// reference, make the values.  Warps whose octets have a cherry column or a group's end inside take a general path: a gap
-// in the word for each cherry column, whose values go over the finished octet, and a scale for each column.  The tile in
-// shared memory (16-byte slots, slot number XOR row quad against bank conflicts) turns the octets into rows of 256
-// contiguous bytes.  Bound by the issue rate: 11008 x 4096 3-bit 35.6 us (108 MB), 38.9 with the kernel above; 4096 x 11008
-// 4-bit 36.9 and 40.6; 16384 x 28672 335 and 360.
+// Two kernels, both with blocks of 64 rows x 128 columns.  A thread makes one octet of 8 original columns of four consecutive
+// rows.  The octet's codes are consecutive compact columns: the bytes of two compact octets (one 32-bit load per byte row
+// covers the four rows), shifted by the position inside the first; a cherry column inside leaves a gap in the word, and its
+// values go over the finished octet.  The tile in shared memory (16-byte slots, slot number XOR row quad against bank
+// conflicts) turns the octets into rows of 256 contiguous bytes.
 constexpr int UP_ROWS = 64, UP_COLS = 128, UP_BLOCKS = 4;       // blocks of an SM
 
 __device__ __forceinline__ uint32_t load_quad(const uint8_t* p, bool aligned) {
@@ -561,8 +556,10 @@ template <int BITS> __device__ __forceinline__ uint4 scaled_octet(uint32_t word,
   return v;
 }
 
-// For layers with many cherry columns: a block makes one tile of 64 rows x 128 columns, each value by itself, gaps and groups
-// included.  (4096 x 11008 4-bit, 512 cherry columns: 54.5 us, the kernel below 62.4; 256: 48.4 and 50.5.)
+// A block makes one tile, with gaps and group boundaries in every octet: for layers with many cherry columns, narrow groups, and
+// matrices that are small or narrow (the rule and both sides' times stand at cq_unpack_dense).  Pairs of codes become the low
+// mantissa bits of 1024 + u, minus (1024 + off), times the scale: each step but the last exact, so the product is rounded once
+// as in the reference.
 // codes 2 i, 2 i + 1 of a word as fp16 (u - off)
 template <int BITS> __device__ __forceinline__ __half2 code_pair(uint32_t word, int i) {
   const uint32_t x = word >> (2 * BITS * i);
@@ -692,7 +689,12 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
   }
 }
 
-
+// A block keeps its 128 columns and goes down the rows: what depends on the columns alone (the search for the cherry columns
+// among it) is done once, the next rows' codes are on their way while these are written.  Pairs of codes become mantissa bits
+// of 1024; one exact multiply-add and the product with the scale, rounded once, make the values.  Warps whose octets have
+// neither a cherry column nor a group's end inside take a short path, the others a general one with a scale for each column.
+// Bound by the issue rate: 11008 x 4096 3-bit 35.6 us (108 MB), 38.9 with the kernel above; 4096 x 11008 4-bit 36.9 and 40.6;
+// 16384 x 28672 335 and 360.
 // CHERRY = the layer has cherry columns
 template <int BITS, bool CHERRY>
 __global__ void __launch_bounds__(256, UP_BLOCKS) unpack_rows_kernel(
