@@ -271,6 +271,33 @@ def test_gemm_adds_the_bias_to_the_rounded_outputs(cabi, N, M):
     assert torch.equal(y, gemm(cabi, p, x) + bias)
 
 
+@pytest.mark.parametrize("M,offset", [(9, 1), (45, 0), (300, 0), (2049, 1)])
+def test_gemm_of_layers_together_adds_each_bias(cabi, M, offset):
+    """Layers with whole and with cut units in one launch, every second one with a bias (two bytes off): the bits of the
+    separate calls and the addition afterwards, into outputs on and off their alignment."""
+    lib, K, bits, G = cabi.lib(), 1160, 3, 64
+    widths = (2440, 8, 9600, 136)
+    ps = []
+    for N in widths:
+        _, _, pk, _ = make_case(K, N, bits, G, seed=N)
+        ps.append(TilePrepared(cabi, pk["qweight"], pk["scales"], pk["cherry_weight"], pk["cherry_indices"], bits, K, G))
+    n = len(ps)
+    x = torch.randn(M, K, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M)).half()
+    biases = [torch.randn(N + 1, device="cuda").half()[1:] if i % 2 == 0 else None for i, N in enumerate(widths)]
+    biases[0][3], biases[2][9599] = float("-inf"), 60000.0
+    bufs = [torch.empty(M * N + offset, dtype=torch.float16, device="cuda") for N in widths]
+    ws = torch.empty(lib.cq_tlayers_gemm_workspace_bytes(C.byref(ps[0].L), n, M), dtype=torch.uint8, device="cuda")
+    ls = (C.POINTER(type(ps[0].L)) * n)(*[C.pointer(p.L) for p in ps])
+    ys = (C.c_void_p * n)(*[b.data_ptr() + 2 * offset for b in bufs])
+    bs = (C.c_void_p * n)(*[None if b is None else b.data_ptr() for b in biases])
+    cabi.check(lib.cq_tlayers_gemm(ls, n, ptr(x), K, ys, (C.c_int32 * n)(*widths), bs, M, 0, ptr(ws), ptr(ps[0].status), None), "gemm")
+    torch.cuda.synchronize()
+    assert all(int(p.status.item()) == 0 for p in ps)
+    for p, buf, b, N in zip(ps, bufs, biases, widths):
+        want = gemm(cabi, p, x)
+        assert torch.equal(buf[offset:].view(M, N), want if b is None else want + b)
+
+
 @pytest.mark.parametrize("bits,G", [(3, 64), (3, 128), (4, 128), (4, 256)])
 def test_gemm_weights_are_unpacked_exactly_at_every_scale(cabi, bits, G):
     """Rows of the identity read the dequantised weights back: bit for bit unpack()'s, with scales from the smallest
