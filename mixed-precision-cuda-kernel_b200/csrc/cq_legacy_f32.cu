@@ -15,7 +15,7 @@
 // multiply-adds needs 25 us of the FMA pipe for 16 rows of 4096 x 13824, before the decode of each code by the one
 // thread that uses it.  That case: 32 us a call (93 with the loop; 52 while every 256 columns staged x for themselves, with a
 // search for each octet's columns and a digit at a time, and codes were spread to bytes column by column: 1640 instructions
-// a warp and block of 128 columns).  Bound by the issue rate still.  512 columns share the staging, the columns are searched
+// a warp and block of 128 columns).  Bound by its instructions still (54 % of the issue slots busy with 16 warps).  512 columns share the staging, the columns are searched
 // once, the four digits of a value are one addition and one exclusive or, codes are taken out for four columns at once and
 // turned; four cherry columns' loads are in flight (one after another a column took 0.5 us).  Other sizes, before and now: 1 row 33 and 21 us, 64 rows 190 and 103, 16384 x 28672 317 and 208, 1024 x 1024
 // 8.8 and 8.7; groups of 64 16 rows 58 and 32, 64 rows 221 and 117 (more than 8 rows: 20 bytes of registers spilled).

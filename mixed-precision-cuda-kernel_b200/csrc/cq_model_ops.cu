@@ -776,7 +776,8 @@ extern "C" int cq_attn_decode(const void* q, const void* k_cache, const void* v_
                               ATT_MAX_SPLITS, counters, part, (cudaStream_t)stream);
   const int sms = cq_sm_count();
   const int splits = attn_splits(sms, sequences, n_heads, max_seq);
-  // What is left: 256-wide heads, more than 8 query heads per KV head, and many heads without grouped queries.
+  // What is left: 256-wide heads, more than 8 query heads per KV head, many heads without grouped queries, and the calls that
+  // cq_attn_mma_takes names.
   // One CTA per KV head reads every cache row once for the query heads that share it; with several query heads
   // per KV head its per-position arithmetic is G times larger, which only pays on long caches (measured on 128-wide heads,
   // 8 per KV head: 103 us against 174 at 4000 positions, but 21 against 15 at 200): short grouped-query caches take

@@ -257,10 +257,10 @@ __global__ void __launch_bounds__(PK_THREADS, sizeof(T) == 2 ? 5 : 3) pack_fused
 
 // fp16 weights of large matrices in groups of one chunk: a block keeps 128 compact columns, one group (two 64-wide ones); each
 // of its warps goes down the rows, 32 at a time, a lane a row, without a barrier.
-//   * Bound by the issue rate: the kernel above executes 31 instructions a weight, much of it set-up per 32 weights.  Here
-//     the rows come in with 16-byte copies, in their original order; the removed cherry columns only show when a lane takes
-//     32 compact columns of its row from shared memory, at some position (the same for the whole warp: each position has
-//     its own straight code): those after a cherry column move up.  (Picked one by one where a cherry column lay among
+//   * Bound by its instructions (62 % of the issue slots busy): the kernel above executes 31 a weight, much of it set-up per 32
+//     weights, this one 19.  Here the rows come in with 16-byte copies, in their original order; the removed cherry columns
+//     only show when a lane takes 32 compact columns of its row from shared memory, at some position (the same for the whole
+//     warp: each position has its own straight code): those after a cherry column move up.  (Picked one by one where a cherry column lay among
 //     them, such blocks were the last to end: 57 us for 11008 x 4096 3-bit with 40, 36 without.)  Maxima, clamps and
 //     roundings run on packed pairs.  Four rows' bytes are turned into words for the stores.
 //   * The 128 columns go in four turns of one loop, twice, instead of 64 registers a lane: unrolled, a fourth of the issue
@@ -693,8 +693,8 @@ __global__ void __launch_bounds__(256, 5) unpack_dense_kernel(
 // among it) is done once, the next rows' codes are on their way while these are written.  Pairs of codes become mantissa bits
 // of 1024; one exact multiply-add and the product with the scale, rounded once, make the values.  Warps whose octets have
 // neither a cherry column nor a group's end inside take a short path, the others a general one with a scale for each column.
-// Bound by the issue rate: 11008 x 4096 3-bit 35.6 us (108 MB), 38.9 with the kernel above; 4096 x 11008 4-bit 36.9 and 40.6;
-// 16384 x 28672 335 and 360.
+// Bound by its instructions (15 a weight, 65 % of the issue slots busy): 11008 x 4096 3-bit 35.6 us (108 MB), 38.9 with the
+// kernel above; 4096 x 11008 4-bit 36.9 and 40.6; 16384 x 28672 335 and 360.
 // CHERRY = the layer has cherry columns
 template <int BITS, bool CHERRY>
 __global__ void __launch_bounds__(256, UP_BLOCKS) unpack_rows_kernel(

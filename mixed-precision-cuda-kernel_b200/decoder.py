@@ -88,8 +88,8 @@ class CherryDecoder:
         # flash_attn package's flash_attn_with_kvcache (a library call, like the lm_head's cuBLAS matmul);
         # "auto" = own, except for grouped-query models with caches of more than 1024 positions whose heads the tensor-core
         # kernel does not take, where that package imports.  Measured on B200 with cold caches, own against flash_attn:
-        # 7B at 256 positions 5.8 us and 9.5; 13B shapes at 2100 positions, batch 8, 70 and 159; 8 query heads per KV head
-        # at 4000 positions 14 and 20 at batch 1, 24 and 27 at 4, 53 and 64 at 16, 101 and 194 at 32.
+        # 7B at 256 positions 4.9 us and 9.5; 13B shapes at 2100 positions, batch 8, 70 and 159; 8 query heads per KV head
+        # at 4000 positions 12.5 and 20 at batch 1, 20 and 27 at 4, 50 and 64 at 16, 93 and 194 at 32.
         if attention not in ("auto", "own", "flash"):
             raise ValueError("attention is 'auto', 'own' or 'flash'")
         self._flash = None
