@@ -134,3 +134,21 @@ def test_the_norm_rides_in_the_launch_for_one_row(rows, monkeypatch):
     outs, total = qlinear.forward_normed_input(lins, h, h.clone(), w, 1e-5)
     assert calls == (["layers with the norm"] if rows == 1 else ["norm", "layers"])
     assert [o.shape for o in outs] == [(rows, 264)] * 2 and total is h
+
+
+def test_layers_that_share_an_input_are_looked_at_once(monkeypatch):
+    """The host's part of a call beyond the row kernel's limit: each layer's buffers are compared once, the first one's once
+    more for the row kernel."""
+    from types import SimpleNamespace
+    from cherryq_b200 import QuantLinear, qlinear
+    looks = []
+    own = QuantLinear._sync_key
+    monkeypatch.setattr(QuantLinear, "_sync_key", lambda self: (looks.append(self), own(self)))
+    monkeypatch.setattr(qlinear, "_gemm_together", lambda layers, tls, x, rows: tls)
+    lins = [layer(), layer(), layer()]
+    for lin in lins:
+        lin._row_rows = 8
+    looks.clear()
+    x = SimpleNamespace(is_cuda=True, dtype=torch.float16, shape=(16, 1024), numel=lambda: 16 * 1024)
+    assert qlinear.forward_shared_input(lins, x) == ["copy"] * 3
+    assert [sum(l is lin for l in looks) for lin in lins] == [2, 1, 1]
