@@ -310,8 +310,15 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  // the ranges' weights, then two columns a thread
+  // the ranges' weights, then two columns a thread, whose first sums are on their way meanwhile
   const float* all = part + head0 * nsplit * (size_t)(D + 2);
+  float2 x[8];
+  auto fetch = [&](int e, int r0) {
+    const float* src = all + (size_t)(e / (D / 2)) * nsplit * (D + 2) + 2 + 2 * (e % (D / 2));
+#pragma unroll
+    for (int u = 0; u < 8; ++u) x[u] = __ldcg(reinterpret_cast<const float2*>(src + (size_t)min(r0 + u, nsplit - 1) * (D + 2)));
+  };
+  if (tid < G * D / 2) fetch(tid, 0);
   for (int e = tid; e < G * nsplit; e += THREADS) {
     const int g = e / nsplit, r = e - g * nsplit;
     const float2 ml = __ldcg(reinterpret_cast<const float2*>(all + (size_t)e * (D + 2)));
@@ -332,12 +339,9 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
   __syncthreads();
   for (int e = tid; e < G * D / 2; e += THREADS) {
     const int g = e / (D / 2), d = 2 * (e - g * (D / 2));
-    const float* src = all + (size_t)g * nsplit * (D + 2) + 2 + d;
     float2 v[4] = {};
     for (int r0 = 0; r0 < nsplit; r0 += 8) {
-      float2 x[8];
-#pragma unroll
-      for (int u = 0; u < 8; ++u) x[u] = __ldcg(reinterpret_cast<const float2*>(src + (size_t)min(r0 + u, nsplit - 1) * (D + 2)));
+      if (e != tid || r0) fetch(e, r0);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
         const float f = r0 + u < nsplit ? s_f[g][r0 + u] : 0.f;
