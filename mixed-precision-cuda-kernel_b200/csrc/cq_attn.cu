@@ -49,8 +49,21 @@ __device__ __forceinline__ float ex2(float x) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
 }
+// with results below the normal numbers
+__device__ __forceinline__ float ex2_full(float x) {
+  float y;
+  asm("ex2.approx.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
 // 2^d of a whole number d <= 0; 0 below the normal numbers (and 1 for NaN, whose sums are NaN)
 __device__ __forceinline__ float whole_pow2(float d) { return __int_as_float(max(0, 127 + __float2int_rn(d)) << 23); }
+// the share of a warp's or range's sums (maximum m, sum of weights l) in those that reach up to `top`: 0 where it has no
+// position, but 1 where its only scores are NaN
+__device__ __forceinline__ float share_of(float m, float l, float top) {
+  if (m == -INFINITY) return l == 0.f ? 0.f : 1.f;
+  const int d = __float2int_rn(m - top);
+  return d < -126 ? (d < -149 ? 0.f : __int_as_float(1 << (149 + d))) : whole_pow2(m - top);
+}
 // 16 bytes of a cache; not as read-only data where the launch itself writes a row of it
 template <bool WRITTEN> __device__ __forceinline__ uint4 ld_cache(const __half* p) {
   if (!WRITTEN) return __ldg(reinterpret_cast<const uint4*>(p));
@@ -242,13 +255,14 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
               make_float4(o[8 * i + j][c], o[8 * i + j + 1][c], o[8 * i + j + 2][c], o[8 * i + j + 3][c]);
   }
   __syncthreads();
-  // the warps' shares in each head's sums: a warp without a finite score has none, unless its sum is NaN
+  // The warps' shares in each head's sums.  (A share of 0 is multiplied all the same: what is NaN or infinite stays so or
+  // becomes NaN, as a weight of 0 does.)
   for (int g = warp; g < G; g += WARPS) {
     const float mw = lane < WARPS ? s_m[lane][g] : -INFINITY, lw = lane < WARPS ? s_l[lane][g] : 0.f;
     float top = mw;
     for (int d = 8; d; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
-    const float f = mw == -INFINITY ? (lw == 0.f ? 0.f : 1.f) : whole_pow2(mw - top);
-    float tot = f == 0.f ? 0.f : f * lw;
+    const float f = share_of(mw, lw, top);
+    float tot = f * lw;
     for (int d = 8; d; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
     if (lane < WARPS) s_f[g][lane] = f;
     if (lane == 0) {
@@ -264,7 +278,7 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
     for (int w = 0; w < WARPS; ++w) {
       const float f = s_f[g][w];
       const float4 x = *reinterpret_cast<const float4*>(am_sum + (w * AM_HEADS + g) * D + d);
-      sums[w] = f != 0.f ? make_float4(f * x.x, f * x.y, f * x.z, f * x.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+      sums[w] = make_float4(f * x.x, f * x.y, f * x.z, f * x.w);
     }
 #pragma unroll
     for (int n = WARPS; n > 1; n = (n + 1) / 2)             // (pairs of pairs: fewer roundings in a row)
@@ -285,7 +299,7 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
         const __half* kr = k_cache + first + (size_t)p * row;
         float dot = 0.f;
         for (int c = 0; c < D; ++c) dot += __half2float(s_q[g][c]) * __half2float(kr[c]);
-        const float w = 32768.f * ex2(__fmaf_rn(dot, scale2, top == -INFINITY ? 0.f : -top));
+        const float w = 32768.f * ex2_full(__fmaf_rn(dot, scale2, top == -INFINITY ? 0.f : -top));
 #pragma unroll
         for (int c = 0; c < 4; ++c) sum[c] += w * __half2float(v_cache[first + (size_t)p * row + d + c]);
       }
@@ -330,8 +344,8 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
     const float mr = lane < nsplit ? s_f[g][lane] : -INFINITY, lr = lane < nsplit ? s_r[g][lane] : 0.f;
     float top = mr;
     for (int d = 16; d; d >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, d));
-    const float f = mr == -INFINITY ? (lr == 0.f ? 0.f : 1.f) : whole_pow2(mr - top);      // an empty range carries no weight
-    float tot = f == 0.f ? 0.f : f * lr;
+    const float f = share_of(mr, lr, top);
+    float tot = f * lr;
     for (int d = 16; d; d >>= 1) tot += __shfl_xor_sync(0xffffffffu, tot, d);
     if (lane < nsplit) s_f[g][lane] = f;
     if (lane == 0) s_tot[g] = tot;
@@ -344,9 +358,10 @@ __global__ void __launch_bounds__(WARPS * 32, AM_SM_WARPS / WARPS) attn_decode_m
       if (e != tid || r0) fetch(e, r0);
 #pragma unroll
       for (int u = 0; u < 8; ++u) {
-        const float f = r0 + u < nsplit ? s_f[g][r0 + u] : 0.f;
-        v[u & 3].x = f != 0.f ? __fmaf_rn(f, x[u].x, v[u & 3].x) : v[u & 3].x;
-        v[u & 3].y = f != 0.f ? __fmaf_rn(f, x[u].y, v[u & 3].y) : v[u & 3].y;
+        const bool in = r0 + u < nsplit;
+        const float f = in ? s_f[g][r0 + u] : 0.f;
+        v[u & 3].x = in ? __fmaf_rn(f, x[u].x, v[u & 3].x) : v[u & 3].x;
+        v[u & 3].y = in ? __fmaf_rn(f, x[u].y, v[u & 3].y) : v[u & 3].y;
       }
     }
     *reinterpret_cast<__half2*>(out + (head0 + g) * D + d) =

@@ -319,6 +319,33 @@ def test_attention_on_tensor_cores(D, B, H, KV, max_seq):
     assert bool(out[:, :G, 3:].isfinite().all() and out[:, :G, 0].isfinite().all() and out[:, G:].isfinite().all())
 
 
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("B,H,KV,n", [(1, 32, 32, 40), (1, 32, 32, 300), (2, 8, 1, 193), (1, 8, 8, 1100), (20, 64, 8, 400)])
+def test_attention_keeps_nan_where_the_weights_are_zero(D, B, H, KV, n):
+    """One position takes all the weight (2^-400 is left for each other one).  Zero times a NaN or infinite value is NaN, a NaN score
+    makes its head NaN: of positions in the same turn, in other warps and in other ranges."""
+    import cherryq_b200
+    qc = cherryq_b200.load_quant_cuda()
+    g = torch.Generator(device="cuda").manual_seed(n)
+    q = torch.randn(B, H, D, device="cuda", generator=g).half() * 0.1
+    k, v = (torch.randn(B, n, KV, D, device="cuda", generator=g).half() * 0.1 for _ in range(2))
+    q[:, :, 0] = 60
+    k[:, :, :, 0] = 0
+    at = torch.full((B,), n - 1, device="cuda")
+    for top in (0, n - 1):
+        keys = k.clone()
+        keys[:, top, :, 0] = 60                                     # score 3600 / sqrt(D)
+        for other in (1, 9, n // 2, n - 2):
+            values = v.clone()
+            values[:, other, 0, 1], values[:, other, 0, 2] = float("nan"), float("inf")
+            out = qc.attn_decode(q, keys, values, at).view(B, KV, H // KV, D)
+            assert bool(out[:, 0, :, 1:3].isnan().all() and out[:, 0, :, 3:].isfinite().all() and out[:, 1:].isfinite().all())
+            bad = keys.clone()
+            bad[:, other, 0, 5] = float("nan")
+            out = qc.attn_decode(q, bad, v, at).view(B, KV, H // KV, D)
+            assert bool(out[:, 0].isnan().all() and out[:, 1:].isfinite().all())
+
+
 @pytest.mark.parametrize("H,KV", [(32, 32), (64, 8)])
 @pytest.mark.parametrize("B,n", [(4, 1100), (2, 4096)])
 def test_attention_is_as_exact_as_fp32_sums(H, KV, B, n):
